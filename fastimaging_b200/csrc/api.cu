@@ -32,6 +32,7 @@
 
 #include "common.cuh"
 #include "imager_kernels.cuh"
+#include "gridder_kernels.cuh"
 #include "sourcefind_kernels.cuh"
 #include "visibility_kernels.cuh"
 #include "aproj_kernels.cuh"
@@ -539,6 +540,125 @@ inline int form_of(int lay)
     return (lay & kLayoutRecs) ? 3 : ((lay & kLayoutCols) ? 1 : ((lay & kLayoutTaps) ? 2 : 0));
 }
 
+// Exclusive scan of n counts into off[0 .. n] (off[n] = the total).
+void scan_counts(stpgpu_context* c, uint32_t* cnt, uint32_t* off, int n)
+{
+    cudaStream_t st = c->stream;
+    if (n <= 4096) {
+        k_scan_single<<<1, 1024, 0, st>>>(cnt, off, n);
+        STPGPU_CHECK_LAUNCH();
+        return;
+    }
+    // many counts: the multi-block scan (cnt[n] is 0, so off[n] receives the total)
+    size_t tb = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, off, n + 1, st);
+    void* tmp = c->buf<unsigned char>("cubtmp_tiles", tb);
+    if (cub::DeviceScan::ExclusiveSum(tmp, tb, cnt, off, n + 1, st) != cudaSuccess)
+        fail(STPGPU_ERR_CUDA, "tile offset scan failed");
+    g_launches += 2;
+}
+
+// Binning by first cell and the block gridder (gridder_kernels.cuh) for the
+// separable and the exact kernels.
+template <typename R>
+void grid_separable(stpgpu_context* c, const ImagerSetup& s, GridOut& g, const Item<R>* items, int64_t n, bool exact,
+    int os, int cs, const double* k1d64, const double* frac, bool wide)
+{
+    cudaStream_t st = c->stream;
+    const int K = 2 * s.support + 1;
+    const int64_t nn = std::max<int64_t>(n, 1);
+    BlockBins b {};
+    b.N = s.N;
+    b.rows = g.image_rows;
+    b.pad = int(ceil_div(K - 1, kBlk));
+    b.brn = int(ceil_div(b.rows, kBlk)) + b.pad;
+    b.bcn = int(ceil_div(b.N, kBlk)) + b.pad;
+    b.wrap_neg = exact;
+    b.support = s.support;
+    b.ntimesteps = 1;
+    b.n = n;
+    const int nbins = b.brn * b.bcn;
+    uint32_t* off = c->buf<uint32_t>("toff", nbins + 1);
+    b.count = c->buf<uint32_t>("tcount", nbins + 1);
+    b.cursor = c->buf<uint32_t>("tcur", nbins + 1);
+    b.ranks = c->buf<uint32_t>("tranks", size_t(nn) * kEntrySlots);
+    b.rank_overflow = c->buf<uint32_t>("trankovf", 1);
+    b.off = off;
+    zero_words(st, { { b.count, nbins + 1 }, { b.cursor, nbins + 1 }, { b.rank_overflow, 1 } });
+    // entries per visibility: two copies (original, mirrored) of up to two
+    // columns; more wraps only on grids smaller than two footprints
+    const uint64_t cap = uint64_t(nn) * (s.N >= 2 * K + 2 ? 4 : 18);
+    if (cap > 0xffffffffull)
+        fail(STPGPU_ERR_INVALID_ARG, "too many visibilities for one snapshot");
+    BinFill<R> q {};
+    q.rec = c->buf<GridRec<R>>("trecs", cap);
+    q.wts = s.beam ? c->buf<R>("trecw", cap) : nullptr;
+    q.cap = cap;
+    q.cs = cs;
+    q.os = os;
+    q.exact = exact;
+    q.err = g.d_err;
+    if (n > 0) {
+        k_bin_count<R><<<grid1d(n, 256), 256, 0, st>>>(b, items);
+        STPGPU_CHECK_LAUNCH();
+    }
+    scan_counts(c, b.count, off, nbins);
+    if (n > 0) {
+        k_bin_fill<R><<<grid1d(n, 256), 256, 0, st>>>(b, items, q);
+        STPGPU_CHECK_LAUNCH();
+    }
+    g.d_nitems = off + nbins;
+    SepParams<R> p {};
+    p.N = b.N;
+    p.rows = b.rows;
+    p.pad = b.pad;
+    p.brn = b.brn;
+    p.off = off;
+    p.recs = q.rec;
+    p.wts = q.wts;
+    p.K = K;
+    if (exact) {
+        double* tab = c->buf<double>("exact_tab", size_t(nn) * 2 * K);
+        if (n > 0) {
+            k_exact_tables<<<grid1d(2 * n, 256), 256, 0, st>>>(s.kf, s.trunc, s.support, frac, n, tab);
+            STPGPU_CHECK_LAUNCH();
+        }
+        p.tab = tab;
+    } else {
+        p.tw = kBlk * b.pad + 15;
+        p.zrow = cs * p.tw;
+        double* tab = c->buf<double>("k1dpad", size_t(cs + 1) * p.tw);
+        if (!c->memo("k1dpad", std::to_string(s.kf) + "/" + fkey(s.trunc) + "/" + std::to_string(s.support) + "/"
+                    + std::to_string(os))) {
+            k_pad_table<<<grid1d(int64_t(cs + 1) * p.tw, 256), 256, 0, st>>>(k1d64, cs, K, p.tw, tab);
+            STPGPU_CHECK_LAUNCH();
+        }
+        p.tab = tab;
+    }
+    const size_t cells = size_t(b.rows) * b.N;
+    const bool f64 = sizeof(R) == 8 || wide;
+    p.grid = g.grid = c->buf<unsigned char>("grid", cells * (f64 ? 16 : 8));
+    p.beam = g.beam = s.beam ? c->buf<unsigned char>("beamgrid", cells * (f64 ? 16 : 8)) : nullptr;
+    const dim3 blocks(unsigned(ceil_div(ceil_div(b.rows, kBlk), kGridWarps)), unsigned(ceil_div(b.N, kBlk)));
+    auto launch = [&](auto kern) {
+        c->mark(1);
+        kern<<<blocks, 32 * kGridWarps, 0, st>>>(p);
+        STPGPU_CHECK_LAUNCH();
+        c->mark(2);
+    };
+    auto pick = [&](auto cell) {
+        using G = decltype(cell);
+        if (exact)
+            s.beam ? launch(k_grid_blocks<SepCore<R, G, true, true>>) : launch(k_grid_blocks<SepCore<R, G, true, false>>);
+        else
+            s.beam ? launch(k_grid_blocks<SepCore<R, G, false, true>>) : launch(k_grid_blocks<SepCore<R, G, false, false>>);
+    };
+    if constexpr (sizeof(R) == 8)
+        pick(double());
+    else
+        f64 ? pick(double()) : pick(float());
+}
+
 template <typename R, int COMP>
 GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, int vis_c64, const double* d_wts,
     const double* d_uv, int uv_is_pixels, int64_t n, int tile_c = TILE_C_DEFAULT, GridLaunch<R>* defer = nullptr,
@@ -611,7 +731,7 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
     Item<R>* items_sorted = nullptr; // W-projection: the items in |w| order
     const int64_t* plane_first = nullptr;
     int nplanes = 0;
-    const R* k1d = nullptr;
+    const double* k1d64 = nullptr;
     const C2* wconv = nullptr;
     const R* winv = nullptr;
     int lh = 0;
@@ -629,16 +749,7 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
             k_kernel_table<<<grid1d(cs, 64), 64, 0, st>>>(s.kf, s.trunc, s.support, os, t64);
             STPGPU_CHECK_LAUNCH();
         }
-        if (sizeof(R) == 8) {
-            k1d = reinterpret_cast<const R*>(t64);
-        } else {
-            float* t32 = c->buf<float>("k1d32", size_t(cs) * K);
-            if (!c->memo("k1d32", key)) {
-                k_d2f<<<grid1d(int64_t(cs) * K, 256), 256, 0, st>>>(t64, t32, int64_t(cs) * K);
-                STPGPU_CHECK_LAUNCH();
-            }
-            k1d = reinterpret_cast<const R*>(t32);
-        }
+        k1d64 = t64;
     }
     const uint16_t* plane16 = nullptr;
     if (wproj && n > 0 && s.wsel) {
@@ -915,6 +1026,14 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
     }
 
     const int kind = (wproj && n > 0) ? GK_WPROJ : (kernel_exact ? GK_EXACT : (!wproj ? GK_SEP : GK_NONE));
+    if (kind == GK_SEP || kind == GK_EXACT) {
+        grid_separable<R>(c, s, g, items, n, kind == GK_EXACT, os, cs, k1d64, pp.frac, COMP == 1 && s.wide_fft);
+        if (defer) {
+            defer->kind = GK_NONE; // gridded: nothing is left to launch
+            defer->ntiles = 0;
+        }
+        return g;
+    }
     // the clipped forms need one footprint segment per axis and tile
     const bool clip_ok = kind != GK_EXACT && N >= 2 * (2 * conv_support + 1 + 32) + 2;
     // staged records: tabulated kernels, no beam (else the lane-per-tap form)
@@ -1047,7 +1166,6 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
     gp.items = bin_items;
     gp.tile_off = toff;
     gp.list = list;
-    gp.k1d = k1d;
     gp.kf = s.kf;
     gp.trunc = s.trunc;
     gp.frac = pp.frac;
@@ -1387,8 +1505,8 @@ void run_imager(stpgpu_context* c, const ImagerSetup& s_in, int image_size, int 
                 w | (std::strchr(pin, 'c') ? kLayoutCols : 0) | (std::strchr(pin, 't') ? kLayoutTaps : 0)
                     | (std::strchr(pin, 'r') ? kLayoutRecs : 0));
     }
-    int tuned_lay = 0;
-    const bool have_tune = c->tune_get(cls, tuned_lay);
+    int tuned_lay = TILE_C_DEFAULT;
+    const bool have_tune = c->tune_get(cls, tuned_lay) || s.nplanes == 0;
     // Device-pointer calls that repeat the previous call exactly (parameters,
     // sizes, buffers) replay a CUDA graph of the gridding, FFT and
     // normalisation kernels, captured on the first repeat; any other call
@@ -1993,7 +2111,7 @@ void run_batch(stpgpu_context* c, const stpgpu_snapshot* sn, int nb, int precisi
         // tile autotuner: time both tile widths for classes not seen before
         std::vector<std::string> fresh;
         for (auto& b : B)
-            if (int v; !c->tune_get(b.cls, v) && std::find(fresh.begin(), fresh.end(), b.cls) == fresh.end())
+            if (int v; b.s.nplanes > 0 && !c->tune_get(b.cls, v) && std::find(fresh.begin(), fresh.end(), b.cls) == fresh.end())
                 fresh.push_back(b.cls);
         if (!fresh.empty()) {
             constexpr int NC = 12;

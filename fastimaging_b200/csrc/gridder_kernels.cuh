@@ -1,0 +1,583 @@
+// Block gridder: binning of the footprints by their first cell and the
+// output-stationary gridding kernels over 8 x 8 blocks of grid cells
+// (gridder.h:596-994 for the gridding semantics).
+#pragma once
+
+#include "imager_kernels.cuh"
+
+namespace stpgpu {
+
+// ---------------------------------------------------------------- binning
+
+// A footprint (item, mirror) becomes one entry per place where its K x K
+// cells land in the grid after wrapping: the first cell (row0, col0) may lie
+// up to K - 1 before the grid, and cells outside [0, rows) x [0, N) are not
+// gridded.  Almost every item has one entry; footprints across a grid edge
+// and the mirrored copies near v = 0 have more.  Entries are binned by
+// (row0, col0) into 8 x 8 bins, `pad` bins before the first block on either
+// axis, so the entries that reach a block are those of the block's own bin
+// and of the `pad` bins before it on each axis; bins are numbered down the
+// rows first, which makes them pad + 1 contiguous ranges of records.  An
+// entry is stored once, whatever number of blocks it reaches (the tile lists
+// of a binning by overlap hold about 2.1 records per item at K = 7).
+constexpr int kBlk = 8;        // block edge in cells
+constexpr int kEntrySlots = 4; // entries per item whose places the count pass keeps
+
+struct BlockBins {
+    int N, rows;  // grid columns and rows
+    int pad;      // ceil((largest K - 1) / 8)
+    int brn, bcn; // bins along the rows and along the columns
+    int wrap_neg; // exact gridder: rows below 0 wrap to the top
+    int support;  // without W-projection
+    const int* plane_support;
+    const uint16_t* plane16; // W-projection without the |w| sort: plane of each item (input order), else null
+    const uint32_t* order;   // W-projection with the sort: input index of each item (items in |w| order), else null
+    const int64_t* first;    // then the first item of each plane
+    int P;
+    const uint8_t* ts_of; // A-projection: time step per visibility (nullable)
+    int ntimesteps;
+    int64_t n;
+    uint32_t* count;  // entries per bin
+    uint32_t* cursor; // fill cursors, used when some item has more than kEntrySlots entries
+    uint32_t* ranks;  // [kEntrySlots][n] place of an item's entries in their bins
+    uint32_t* rank_overflow;
+    const uint32_t* off; // first entry of each bin
+};
+
+// One entry.  geom: row0 and col0 modulo 1024 (10 bits each), the support
+// (7 bits), conjugated W-kernel (bit 27), mirrored copy (bit 28).
+// koff: W-projection, the entry's kernel in the expanded tables; separable
+// kernels, cpy | cpx << 16 (offset indices); exact kernels, the visibility.
+template <typename R>
+struct alignas(16) GridRec {
+    R vr, vi;
+    uint32_t koff, geom;
+};
+static_assert(sizeof(GridRec<float>) == 16 && sizeof(GridRec<double>) == 32, "record sizes");
+
+__device__ __forceinline__ int item_plane(const BlockBins& b, int64_t k)
+{
+    if (b.plane16)
+        return b.plane16[k];
+    if (!b.order)
+        return 0;
+    int plane = plane_of(b.first, b.P, k);
+    if (b.ts_of)
+        plane = plane * b.ntimesteps + b.ts_of[b.order[k]];
+    return plane;
+}
+
+// f(row0, col0, bin) for every entry of one footprint.
+template <typename F>
+__device__ __forceinline__ void for_entries(const BlockBins& b, int cx, int cy, int S, F f)
+{
+    const int K = 2 * S + 1;
+    const int rb = cy - S, cb = cx - S;
+#pragma unroll 1
+    for (int ri = 0; ri < 3; ri++) {
+        // in place; rows at or beyond N wrap once; rows below 0 wrap for the exact gridder
+        if (ri == 1 && rb + K <= b.N)
+            continue;
+        if (ri == 2 && !(b.wrap_neg && rb < 0))
+            continue;
+        const int row0 = ri == 0 ? rb : (ri == 1 ? rb - b.N : rb + b.N);
+        if (row0 >= b.rows || row0 + K <= 0)
+            continue;
+#pragma unroll 1
+        for (int ci = 0; ci < 3; ci++) {
+            if (ci == 1 && cb + K <= b.N)
+                continue;
+            if (ci == 2 && cb >= 0)
+                continue;
+            const int col0 = ci == 0 ? cb : (ci == 1 ? cb - b.N : cb + b.N);
+            if (col0 >= b.N || col0 + K <= 0)
+                continue;
+            f(row0, col0,
+                uint32_t((col0 + kBlk * b.pad) / kBlk) * uint32_t(b.brn) + uint32_t((row0 + kBlk * b.pad) / kBlk));
+        }
+    }
+}
+
+template <typename R>
+__global__ void __launch_bounds__(256) k_bin_count(BlockBins b, const Item<R>* __restrict__ items)
+{
+    const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k >= b.n)
+        return;
+    const Item<R> it = items[k];
+    if (!it.good)
+        return;
+    const int S = b.plane_support ? b.plane_support[item_plane(b, k)] : b.support;
+    int q = 0;
+    for (int mir = 0; mir < int(it.good); mir++) {
+        int cx, cy;
+        item_centre(it, mir, b.N, cx, cy);
+        for_entries(b, cx, cy, S, [&](int, int, uint32_t bin) {
+            const uint32_t r = atomicAdd(&b.count[bin], 1u);
+            if (q < kEntrySlots)
+                b.ranks[size_t(q) * size_t(b.n) + size_t(k)] = r; // slot-major: coalesced
+            else
+                *b.rank_overflow = 1u;
+            q++;
+        });
+    }
+}
+
+// Records at their places.  The capacity holds every entry there can be
+// (bit 1 of *err otherwise, never expected).
+template <typename R>
+struct BinFill {
+    GridRec<R>* rec;
+    R* wts; // weight per record (beam), nullable
+    uint64_t cap;
+    const uint32_t* wk_off; // W-projection: table offset per plane (x time step)
+    int cs, os, exact;
+    unsigned int* err;
+};
+
+template <typename R>
+__global__ void __launch_bounds__(256) k_bin_fill(BlockBins b, const Item<R>* __restrict__ items, BinFill<R> q)
+{
+    const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k >= b.n)
+        return;
+    const Item<R> it = items[k];
+    if (!it.good)
+        return;
+    int S = b.support, plane = 0;
+    if (b.plane_support) {
+        plane = item_plane(b, k);
+        S = b.plane_support[plane];
+    }
+    const int K = 2 * S + 1;
+    const bool ranked = *b.rank_overflow == 0u;
+    int e = 0;
+    for (int mir = 0; mir < int(it.good); mir++) {
+        int cx, cy;
+        item_centre(it, mir, b.N, cx, cy);
+        int cpx = it.cpx, cpy = it.cpy;
+        if (mir && q.os > 1) {
+            cpx = q.os - cpx;
+            cpy = q.os - cpy;
+        }
+        GridRec<R> r;
+        r.vr = it.vr * it.w;
+        r.vi = (mir ? -it.vi : it.vi) * it.w;
+        const uint32_t conj = (it.flags >> (mir ? 1 : 0)) & 1u;
+        if (b.plane_support)
+            r.koff = q.wk_off[plane] + uint32_t((cpy * q.cs + cpx) * K * K);
+        else
+            r.koff = q.exact ? uint32_t(k) : uint32_t(cpy) | (uint32_t(cpx) << 16);
+        for_entries(b, cx, cy, S, [&](int row0, int col0, uint32_t bin) {
+            const uint32_t place = ranked ? b.ranks[size_t(e) * size_t(b.n) + size_t(k)] : atomicAdd(&b.cursor[bin], 1u);
+            e++;
+            r.geom = uint32_t(row0 & 1023) | (uint32_t(col0 & 1023) << 10) | (uint32_t(S) << 20) | (conj << 27)
+                | (uint32_t(mir) << 28);
+            const uint64_t pos = uint64_t(b.off[bin]) + place;
+            if (pos < q.cap) {
+                q.rec[pos] = r;
+                if (q.wts)
+                    q.wts[pos] = it.w;
+            } else {
+                atomicOr(q.err, 1u);
+            }
+        });
+    }
+}
+
+// ---------------------------------------------------------------- kernel tables
+
+// The 1-D kernel table in rows of `tw` values with zeros around the K taps
+// (tap d of offset c at [c * tw + d + 7]), so a block kernel indexes it
+// without a range check, and a last row of zeros.
+__global__ void k_pad_table(const double* k1d, int cs, int K, int tw, double* out)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (cs + 1) * tw)
+        return;
+    const int c = t / tw, d = t % tw - 7;
+    out[t] = c < cs && d >= 0 && d < K ? k1d[c * K + d] : 0.0;
+}
+
+// Exact gridder: the two 1-D kernels of every visibility, tab[k][axis][K]
+// (axis 0: v, 1: u).  make_kernel_array divides the outer product by its
+// sum (conv_func.h:279-303), which is the product of the two sums; the
+// functors are even, so the mirrored copy reads them backwards.
+__global__ void __launch_bounds__(256) k_exact_tables(int kf, double trunc, int S, const double* __restrict__ frac,
+    int64_t n, double* __restrict__ tab)
+{
+    const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (t >= 2 * n)
+        return;
+    const int64_t k = t >> 1;
+    const int axis = int(t & 1), K = 2 * S + 1;
+    const double f = frac[(axis ? 0 : n) + k];
+    double* o = tab + size_t(t) * K;
+    double sum = 0.0;
+    for (int i = 0; i < K; i++) {
+        const double v = kernel_value(kf, trunc, (double(i) - S) - f);
+        o[i] = v;
+        sum += v;
+    }
+    for (int i = 0; i < K; i++)
+        o[i] = o[i] / sum;
+}
+
+// ---------------------------------------------------------------- block gridder
+
+// One warp per 8 x 8 block of cells, eight warps (64 rows x 8 columns) per
+// CTA.  The cells stay in registers: nothing is read back, zeroed or
+// updated in memory, and every cell of the grid is written exactly once.
+// The warp walks its pad + 1 ranges of records as one stream, 32 at a time:
+// each lane fetches and decodes one record, those that reach the block are
+// packed into shared memory, and the core C accumulates them.  Blocks with
+// more than kHeavy entries (the centre of a concentrated uv coverage) are
+// taken by all eight warps of the CTA together, their partial cells summed
+// in a fixed order through shared memory.
+constexpr int kGridWarps = 8;
+constexpr uint32_t kHeavy = 512;
+
+struct BlockRanges {
+    uint32_t pre, delta; // lane j: entries before range j, and range j's first record minus that
+    uint32_t total;
+    int nb;
+};
+
+// Ranges j0 .. j0 + nb - 1 (nb <= 32) of block (br, bc): the bins' columns.
+__device__ __forceinline__ BlockRanges block_ranges(const uint32_t* __restrict__ off, int brn, int br, int bc, int rows_nb,
+    int nb)
+{
+    const int lane = threadIdx.x & 31;
+    uint32_t beg = 0, len = 0;
+    if (lane < nb) {
+        const uint32_t* o = off + size_t(bc + lane) * size_t(brn) + size_t(br);
+        beg = o[0];
+        len = o[rows_nb] - beg;
+    }
+    uint32_t incl = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o)
+            incl += y;
+    }
+    BlockRanges r;
+    r.pre = incl - len;
+    r.delta = beg - r.pre;
+    r.total = __shfl_sync(0xffffffffu, incl, 31);
+    r.nb = nb;
+    return r;
+}
+
+// Record of stream position t.
+__device__ __forceinline__ uint32_t stream_record(const BlockRanges& r, uint32_t t)
+{
+    uint32_t d = __shfl_sync(0xffffffffu, r.delta, 0);
+    for (int j = 1; j < r.nb; j++) {
+        const uint32_t pj = __shfl_sync(0xffffffffu, r.pre, j), dj = __shfl_sync(0xffffffffu, r.delta, j);
+        if (t >= pj)
+            d = dj;
+    }
+    return t + d;
+}
+
+template <class C>
+__device__ __forceinline__ void block_walk(const typename C::Params& p, const BlockRanges& r, int r0, int c0, int first,
+    int stride, typename C::Staged* st, typename C::A (&acc)[C::NACC])
+{
+    const int lane = threadIdx.x & 31;
+    uint32_t t = uint32_t(first) * 32u;
+    typename C::Raw raw {};
+    if (t < r.total) {
+        const uint32_t i = stream_record(r, t + lane);
+        if (t + lane < r.total)
+            raw = C::fetch(p, i);
+    }
+    while (t < r.total) {
+        typename C::Staged s;
+        const bool reach = C::decode(p, raw, r0, c0, s) && t + lane < r.total;
+        const unsigned mask = __ballot_sync(0xffffffffu, reach);
+        if (reach)
+            st[__popc(mask & ((1u << lane) - 1u))] = s;
+        const int m = __popc(mask);
+        C::fill_up(p, st, m);
+        __syncwarp();
+        // the next 32 records are in flight while these are gridded
+        const uint32_t tn = t + uint32_t(stride) * 32u;
+        if (tn < r.total) {
+            const uint32_t i = stream_record(r, tn + lane);
+            if (tn + lane < r.total)
+                raw = C::fetch(p, i);
+        }
+        C::accumulate(p, st, m, acc);
+        __syncwarp();
+        t = tn;
+    }
+}
+
+template <class C>
+__global__ void __launch_bounds__(32 * kGridWarps) k_grid_blocks(const __grid_constant__ typename C::Params p)
+{
+    using A = typename C::A;
+    constexpr size_t kStage = sizeof(typename C::Staged) * 36 * kGridWarps;
+    constexpr size_t kRed = sizeof(A) * C::NACC * 32 * kGridWarps;
+    __shared__ __align__(16) unsigned char smem[kStage > kRed ? kStage : kRed];
+    __shared__ uint32_t s_heavy;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    typename C::Staged* st = reinterpret_cast<typename C::Staged*>(smem) + warp * 36;
+    const int nbr = (p.rows + kBlk - 1) / kBlk;
+    const int br = int(blockIdx.x) * kGridWarps + warp, bc = int(blockIdx.y);
+    const int nb = C::bins(p);      // bins that reach a block on either axis
+    const int skip = p.pad + 1 - nb; // (those further away cannot)
+    if (threadIdx.x == 0)
+        s_heavy = 0;
+    __syncthreads();
+    if (br < nbr) {
+        A acc[C::NACC] = {};
+        uint32_t total = 0;
+        bool heavy = false;
+        // at most 32 ranges at a time (33 for the largest supports)
+        for (int j = 0; j < nb; j += 32) {
+            const BlockRanges r = block_ranges(p.off, p.brn, br + skip, bc + skip + j, nb, min(nb - j, 32));
+            total += r.total;
+            heavy = total > kHeavy;
+            if (heavy)
+                break;
+            block_walk<C>(p, r, br * kBlk, bc * kBlk, 0, 1, st, acc);
+        }
+        if (heavy) {
+            if (lane == 0)
+                atomicOr(&s_heavy, 1u << warp);
+        } else {
+            C::store(p, br * kBlk, bc * kBlk, acc);
+        }
+    }
+    __syncthreads();
+    for (uint32_t h = s_heavy; h; h &= h - 1) {
+        const int hw = __ffs(int(h)) - 1;
+        const int hbr = int(blockIdx.x) * kGridWarps + hw;
+        A acc[C::NACC] = {};
+        for (int j = 0; j < nb; j += 32) {
+            const BlockRanges r = block_ranges(p.off, p.brn, hbr + skip, bc + skip + j, nb, min(nb - j, 32));
+            block_walk<C>(p, r, hbr * kBlk, bc * kBlk, warp, kGridWarps, st, acc);
+        }
+        __syncthreads(); // the staged records are read; the same memory takes the partial cells
+        A* red = reinterpret_cast<A*>(smem);
+        for (int q = 0; q < C::NACC; q++)
+            red[(q * kGridWarps + warp) * 32 + lane] = acc[q];
+        __syncthreads();
+        if (warp == hw) {
+            for (int q = 0; q < C::NACC; q++) {
+                A v = A(0);
+                for (int w = 0; w < kGridWarps; w++)
+                    v += red[(q * kGridWarps + w) * 32 + lane];
+                acc[q] = v;
+            }
+            C::store(p, hbr * kBlk, bc * kBlk, acc);
+        }
+        __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------- separable kernels
+
+template <typename R>
+struct SepParams {
+    int N, rows, pad, brn;
+    const uint32_t* off;
+    const GridRec<R>* recs;
+    const R* wts;      // per record (beam)
+    const double* tab; // padded table (k_pad_table), or per-visibility kernels (k_exact_tables)
+    int tw, zrow, K; // padded row length, position of the row of zeros
+    void* grid;
+    void* beam;
+};
+
+// Separable kernels on the FP64 tensor cores.  An entry adds the rank-one
+// block kv (V ku)^T, so four entries are one 8 x 8 x 4 product: A holds the
+// four v kernels at the block's rows, B the four u kernels at its columns
+// times the visibility (one product for the real and one for the imaginary
+// part), zeros where a footprint does not reach.  Two DMMA add four entries
+// to all 64 cells; a lane looks up one tap of either axis per product.  The
+// bound is instruction issue (about 5 warp instructions per entry and block)
+// and the FP64 pipe (8 cycles); the shared-memory tile gridder it replaces
+// spent about 85 warp instructions per entry and tile on decode and
+// read-modify-write.  Calls, before and after: 4M visibilities on 8192^2
+// (PSWF S = 4, compensated single precision) 2604 -> 1630 us; 100k on 2048^2
+// in double 182 -> 159 us; 78k exact kernels with beam on 2160^2 (where the
+// functor was evaluated per tap) 2016 -> 316 us.
+// Products and sums are in double whatever the record's precision.  Entries
+// with a weight, visibility or kernel that is not finite are added tap by
+// tap instead, so that they reach their own footprint only.
+template <typename R, typename G, bool EXACT, bool BEAM>
+struct SepCore {
+    using Params = SepParams<R>;
+    using A = double;
+    static constexpr int NACC = BEAM ? 6 : 4;
+    struct Raw {
+        GridRec<R> r;
+        R w;
+    };
+    struct alignas(16) StagedB {
+        double vr, vi;
+        int ty, tx;  // table position of the entry's tap at the block's first row / column
+        uint32_t vis; // exact: the visibility
+        int back;     // bit 0: exact, the mirrored copy; bit 1: not finite
+        double w, unused;
+    };
+    struct alignas(16) StagedP {
+        double vr, vi;
+        int ty, tx;
+        uint32_t vis;
+        int back;
+    };
+    using Staged = std::conditional_t<BEAM, StagedB, StagedP>;
+
+    static __device__ __forceinline__ int bins(const Params& p) { return p.pad + 1; }
+    static __device__ __forceinline__ Raw fetch(const Params& p, uint32_t i)
+    {
+        Raw w {};
+        w.r = p.recs[i];
+        if (BEAM)
+            w.w = p.wts[i];
+        return w;
+    }
+    static __device__ __forceinline__ bool decode(const Params& p, const Raw& w, int r0, int c0, Staged& s)
+    {
+        const uint32_t g = w.r.geom;
+        const int row0 = int((g - uint32_t(r0)) << 22) >> 22, col0 = int((g - (uint32_t(c0) << 10)) << 12) >> 22;
+        s.vr = double(w.r.vr);
+        s.vi = double(w.r.vi);
+        double chk = s.vr + s.vi;
+        if constexpr (BEAM) {
+            s.w = double(w.w);
+            chk += s.w;
+        }
+        if (EXACT) {
+            s.ty = -row0;
+            s.tx = -col0;
+            s.vis = w.r.koff;
+            s.back = int((g >> 28) & 1u);
+        } else {
+            s.ty = int(w.r.koff & 0xffffu) * p.tw + 7 - row0;
+            s.tx = int(w.r.koff >> 16) * p.tw + 7 - col0;
+            s.vis = 0;
+            s.back = 0;
+        }
+        if (!(row0 + p.K > 0 && col0 + p.K > 0))
+            return false;
+        // a kernel whose samples sum to zero is not finite in all its taps
+        if (EXACT) {
+            const double* t = p.tab + size_t(s.vis) * size_t(2 * p.K);
+            chk += __ldg(t) + __ldg(t + p.K);
+        } else {
+            chk += __ldg(p.tab + s.ty + row0) + __ldg(p.tab + s.tx + col0);
+        }
+        if (!(fabs(chk) <= 1.7976931348623157e308))
+            s.back |= 2;
+        return true;
+    }
+    // entries of zero weight up to a multiple of four
+    static __device__ __forceinline__ void fill_up(const Params& p, Staged* st, int m)
+    {
+        const int lane = threadIdx.x & 31;
+        if (lane < ((4 - m) & 3))
+            st[m + lane] = none(p);
+    }
+    static __device__ __forceinline__ Staged none(const Params& p)
+    {
+        Staged z {};
+        z.ty = z.tx = EXACT ? -kBlk : p.zrow;
+        return z;
+    }
+    // the tap of either axis at the block's row / column q
+    static __device__ __forceinline__ void taps(const Params& p, const Staged& s, int row, int col, double& a, double& b)
+    {
+        if (EXACT) {
+            const int K = p.K;
+            const int dr = s.ty + row, dc = s.tx + col;
+            const double* t = p.tab + size_t(s.vis) * size_t(2 * K);
+            a = unsigned(dr) < unsigned(K) ? __ldg(t + (s.back & 1 ? K - 1 - dr : dr)) : 0.0;
+            b = unsigned(dc) < unsigned(K) ? __ldg(t + K + (s.back & 1 ? K - 1 - dc : dc)) : 0.0;
+        } else {
+            a = __ldg(p.tab + s.ty + row);
+            b = __ldg(p.tab + s.tx + col);
+        }
+    }
+    static __device__ __noinline__ void odd_entries(const Params& p, Staged* st, int m, unsigned odd, A (&acc)[NACC])
+    {
+        const int lane = threadIdx.x & 31;
+        for (; odd; odd &= odd - 1) {
+            const int e = __ffs(int(odd)) - 1;
+            const Staged s = st[e];
+            const int tr = EXACT ? 0 : (s.ty / p.tw) * p.tw + 7, tc = EXACT ? 0 : (s.tx / p.tw) * p.tw + 7;
+            for (int k = 0; k < 2; k++) {
+                const int row = lane >> 2, col = 2 * (lane & 3) + k;
+                const int dr = s.ty + row - tr, dc = s.tx + col - tc;
+                if (unsigned(dr) < unsigned(p.K) && unsigned(dc) < unsigned(p.K)) {
+                    double a, b;
+                    taps(p, s, row, col, a, b);
+                    acc[k] += a * b * s.vr;
+                    acc[2 + k] += a * b * s.vi;
+                    if constexpr (BEAM)
+                        acc[4 + k] += a * b * s.w;
+                }
+            }
+            __syncwarp();
+            if (lane == 0)
+                st[e] = none(p);
+            __syncwarp();
+        }
+    }
+    static __device__ __forceinline__ void mma(double& c0, double& c1, double a, double b)
+    {
+        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+            : "+d"(c0), "+d"(c1)
+            : "d"(a), "d"(b));
+    }
+    static __device__ __forceinline__ void accumulate(const Params& p, Staged* st, int m, A (&acc)[NACC])
+    {
+        const int lane = threadIdx.x & 31;
+        const unsigned odd = __ballot_sync(0xffffffffu, lane < m && (st[lane].back & 2));
+        if (odd)
+            odd_entries(p, st, m, odd, acc);
+#pragma unroll 2
+        for (int g = 0; g < m; g += 4) {
+            const Staged s = st[g + (lane & 3)];
+            double a, b;
+            taps(p, s, lane >> 2, lane >> 2, a, b);
+            mma(acc[0], acc[1], a, b * s.vr);
+            mma(acc[2], acc[3], a, b * s.vi);
+            if constexpr (BEAM)
+                mma(acc[4], acc[5], a, b * s.w);
+        }
+    }
+    // lane: row lane / 4, columns 2 (lane % 4) and the next
+    static __device__ __forceinline__ void store(const Params& p, int r0, int c0, const A (&acc)[NACC])
+    {
+        using G2 = typename Cplx<G>::T;
+        const int lane = threadIdx.x & 31;
+        const int r = r0 + (lane >> 2);
+        if (r >= p.rows)
+            return;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int c = c0 + 2 * (lane & 3) + k;
+            if (c >= p.N)
+                continue;
+            const size_t i = size_t(c) * size_t(p.rows) + size_t(r);
+            G2 v;
+            v.x = G(acc[k]);
+            v.y = G(acc[2 + k]);
+            static_cast<G2*>(p.grid)[i] = v;
+            if constexpr (BEAM) {
+                G2 w;
+                w.x = G(acc[4 + k]);
+                w.y = G(0);
+                static_cast<G2*>(p.beam)[i] = w;
+            }
+        }
+    }
+};
+
+} // namespace stpgpu
