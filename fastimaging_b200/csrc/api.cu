@@ -168,8 +168,7 @@ struct stpgpu_context {
     std::string ns;
 
     // batch path: worker streams, fork/join events, the captured graph of
-    // the last batch signature, the tile-width choice per size class and a
-    // pinned staging area (gridder parameter tables, scalar read-back)
+    // the last batch signature and a pinned staging area (scalar read-back)
     std::vector<cudaStream_t> wstreams;
     std::vector<cudaEvent_t> wevents;
     cudaEvent_t fork_ev = nullptr;
@@ -177,28 +176,6 @@ struct stpgpu_context {
     int batch_calls = 0;
     cudaGraph_t batch_graph = nullptr;
     cudaGraphExec_t batch_exec = nullptr;
-    // gridder layouts chosen by the autotuner, per size class; shared by the
-    // slot contexts of a server so that a class is tuned once
-    struct TuneTable {
-        std::mutex mu;
-        std::map<std::string, int> m;
-    };
-    std::shared_ptr<TuneTable> tunes = std::make_shared<TuneTable>();
-    bool tune_get(const std::string& k, int& v)
-    {
-        std::lock_guard<std::mutex> lk(tunes->mu);
-        auto it = tunes->m.find(k);
-        if (it == tunes->m.end())
-            return false;
-        v = it->second;
-        return true;
-    }
-    void tune_set(const std::string& k, int v)
-    {
-        std::lock_guard<std::mutex> lk(tunes->mu);
-        tunes->m[k] = v;
-    }
-    cudaEvent_t tev[2] = { nullptr, nullptr };
     void* batch_host = nullptr;
     size_t batch_host_cap = 0;
 
@@ -261,9 +238,6 @@ struct stpgpu_context {
     void* pinned_dev = nullptr; // the device's address of the staging area (mapped)
     size_t pinned_cap = 0;
     std::map<std::string, std::string> memo_keys; // buffer name -> key of its current contents
-    // staged gridder: records per visibility last counted, per namespace,
-    // tile width, support and truncation (absent: count at the next call)
-    std::map<std::string, double> rec_ratio;
 
     // True when buffer `name` already holds the data described by `key`
     // (static tables: gcf, kernel tables, cos tables); records `key`.
@@ -500,7 +474,8 @@ void check_pars(const ImagerSetup& s)
         fail(STPGPU_ERR_INVALID_ARG, "oversampling too large");
 }
 
-// Key of the tile autotuner: calls of one class share the tile width.
+// Size class of a call: those whose data could not take the W-planes without
+// the |w| sort are remembered by it.
 std::string size_class(const ImagerSetup& s, int precision)
 {
     const int conv = s.nplanes > 0 ? s.max_support : s.support;
@@ -510,34 +485,11 @@ std::string size_class(const ImagerSetup& s, int precision)
         + (s.nplanes > 0 ? "/t" + fkey(s.trunc_perc) : std::string());
 }
 
-// Gridder launch prepared by run_gridder when the caller launches it itself
-// (the batch path merges the tiles of many snapshots into one launch).
-enum GridKind { GK_NONE = 0, GK_SEP, GK_EXACT, GK_WPROJ };
-template <typename R>
-struct GridLaunch {
-    int kind = GK_NONE;
-    int beam = 0;
-    int form = 0; // gridder form the binning was built for (0 lanes-per-item, 2 lane-per-tap, 3 staged)
-    int tile_c = TILE_C_DEFAULT;
-    int ntiles = 0;
-    size_t smem = 0;
-    GridParams<R> gp {};
-};
-
-// convolve_to_grid (gridder.h:240-997): grids into context buffers "grid"
-// and "beamgrid" of precision R (complex), image_rows x N column-major.
-// tile_c: grid columns per tile (32 or 16).  With `defer` the gridder kernel
-// is not launched: its parameters are returned there instead.
-// Autotuned gridder layout bits beside the tile width (low 8 bits).
-constexpr int kLayoutPersist = 1 << 8; // batch: persistent work queue
-constexpr int kLayoutCols = 1 << 9;    // column-packed tile gridder (grid_tile_cols)
-constexpr int kLayoutTaps = 1 << 10;   // lane-per-tap tile gridder (grid_tile_taps)
-constexpr int kLayoutRecs = 1 << 11;   // staged tile gridder over decoded records (grid_tile_recs)
-// gridder form of a layout: 0 lanes-per-item, 1 column-packed, 2 lane-per-tap
-// (3: staged records)
-inline int form_of(int lay)
+// Entries that n visibilities can have: two copies (original, mirrored) of up
+// to two columns; more wraps only on grids smaller than two footprints.
+uint64_t entry_capacity(int N, int K, int64_t n)
 {
-    return (lay & kLayoutRecs) ? 3 : ((lay & kLayoutCols) ? 1 : ((lay & kLayoutTaps) ? 2 : 0));
+    return uint64_t(std::max<int64_t>(n, 1)) * (N >= 2 * K + 2 ? 4 : 18);
 }
 
 // Exclusive scan of n counts into off[0 .. n] (off[n] = the total).
@@ -558,14 +510,34 @@ void scan_counts(stpgpu_context* c, uint32_t* cnt, uint32_t* off, int n)
     g_launches += 2;
 }
 
-// Binning by first cell and the block gridder (gridder_kernels.cuh) for the
-// separable and the exact kernels.
+// Where a call's items and kernel tables are, for grid_blocks.
 template <typename R>
-void grid_separable(stpgpu_context* c, const ImagerSetup& s, GridOut& g, const Item<R>* items, int64_t n, bool exact,
-    int os, int cs, const double* k1d64, const double* frac, bool wide)
+struct GridInputs {
+    bool wproj = false, exact = false;
+    int os = 1, cs = 1;
+    const Item<R>* items = nullptr;
+    // W-projection: planes (k_wsel_* or the sorting path) and kernels
+    const int* plane_support = nullptr;
+    const uint16_t* plane16 = nullptr;
+    const uint32_t* order = nullptr;
+    const int64_t* first = nullptr;
+    int P = 0;
+    const uint8_t* ts_of = nullptr;
+    const uint32_t* wk_off = nullptr;
+    const void* wk = nullptr;
+    const unsigned int* max_support = nullptr;
+    // separable kernels: 1-D table; exact: fractional positions
+    const double* k1d = nullptr;
+    const double* frac = nullptr;
+};
+
+// Binning by first cell and the block gridder (gridder_kernels.cuh).  wide:
+// a single-precision call's grid holds double cells.
+template <typename R, typename T, typename ACC>
+void grid_blocks(stpgpu_context* c, const ImagerSetup& s, GridOut& g, int64_t n, const GridInputs<R>& in, bool wide)
 {
     cudaStream_t st = c->stream;
-    const int K = 2 * s.support + 1;
+    const int K = 2 * (in.wproj ? s.max_support : s.support) + 1;
     const int64_t nn = std::max<int64_t>(n, 1);
     BlockBins b {};
     b.N = s.N;
@@ -573,9 +545,15 @@ void grid_separable(stpgpu_context* c, const ImagerSetup& s, GridOut& g, const I
     b.pad = int(ceil_div(K - 1, kBlk));
     b.brn = int(ceil_div(b.rows, kBlk)) + b.pad;
     b.bcn = int(ceil_div(b.N, kBlk)) + b.pad;
-    b.wrap_neg = exact;
+    b.wrap_neg = in.exact;
     b.support = s.support;
-    b.ntimesteps = 1;
+    b.plane_support = in.plane_support;
+    b.plane16 = in.plane16;
+    b.order = in.order;
+    b.first = in.first;
+    b.P = in.P;
+    b.ts_of = in.ts_of;
+    b.ntimesteps = std::max(s.ntimesteps, 1);
     b.n = n;
     const int nbins = b.brn * b.bcn;
     uint32_t* off = c->buf<uint32_t>("toff", nbins + 1);
@@ -585,88 +563,110 @@ void grid_separable(stpgpu_context* c, const ImagerSetup& s, GridOut& g, const I
     b.rank_overflow = c->buf<uint32_t>("trankovf", 1);
     b.off = off;
     zero_words(st, { { b.count, nbins + 1 }, { b.cursor, nbins + 1 }, { b.rank_overflow, 1 } });
-    // entries per visibility: two copies (original, mirrored) of up to two
-    // columns; more wraps only on grids smaller than two footprints
-    const uint64_t cap = uint64_t(nn) * (s.N >= 2 * K + 2 ? 4 : 18);
+    const uint64_t cap = entry_capacity(s.N, K, nn);
     if (cap > 0xffffffffull)
         fail(STPGPU_ERR_INVALID_ARG, "too many visibilities for one snapshot");
     BinFill<R> q {};
     q.rec = c->buf<GridRec<R>>("trecs", cap);
     q.wts = s.beam ? c->buf<R>("trecw", cap) : nullptr;
     q.cap = cap;
-    q.cs = cs;
-    q.os = os;
-    q.exact = exact;
+    q.wk_off = in.wk_off;
+    q.cs = in.cs;
+    q.os = in.os;
+    q.exact = in.exact;
     q.err = g.d_err;
     if (n > 0) {
-        k_bin_count<R><<<grid1d(n, 256), 256, 0, st>>>(b, items);
+        k_bin_count<R><<<grid1d(n, 256), 256, 0, st>>>(b, in.items);
         STPGPU_CHECK_LAUNCH();
     }
     scan_counts(c, b.count, off, nbins);
     if (n > 0) {
-        k_bin_fill<R><<<grid1d(n, 256), 256, 0, st>>>(b, items, q);
+        k_bin_fill<R><<<grid1d(n, 256), 256, 0, st>>>(b, in.items, q);
         STPGPU_CHECK_LAUNCH();
     }
     g.d_nitems = off + nbins;
-    SepParams<R> p {};
-    p.N = b.N;
-    p.rows = b.rows;
-    p.pad = b.pad;
-    p.brn = b.brn;
-    p.off = off;
-    p.recs = q.rec;
-    p.wts = q.wts;
-    p.K = K;
-    if (exact) {
-        double* tab = c->buf<double>("exact_tab", size_t(nn) * 2 * K);
-        if (n > 0) {
-            k_exact_tables<<<grid1d(2 * n, 256), 256, 0, st>>>(s.kf, s.trunc, s.support, frac, n, tab);
-            STPGPU_CHECK_LAUNCH();
-        }
-        p.tab = tab;
-    } else {
-        p.tw = kBlk * b.pad + 15;
-        p.zrow = cs * p.tw;
-        double* tab = c->buf<double>("k1dpad", size_t(cs + 1) * p.tw);
-        if (!c->memo("k1dpad", std::to_string(s.kf) + "/" + fkey(s.trunc) + "/" + std::to_string(s.support) + "/"
-                    + std::to_string(os))) {
-            k_pad_table<<<grid1d(int64_t(cs + 1) * p.tw, 256), 256, 0, st>>>(k1d64, cs, K, p.tw, tab);
-            STPGPU_CHECK_LAUNCH();
-        }
-        p.tab = tab;
-    }
     const size_t cells = size_t(b.rows) * b.N;
     const bool f64 = sizeof(R) == 8 || wide;
-    p.grid = g.grid = c->buf<unsigned char>("grid", cells * (f64 ? 16 : 8));
-    p.beam = g.beam = s.beam ? c->buf<unsigned char>("beamgrid", cells * (f64 ? 16 : 8)) : nullptr;
+    g.grid = c->buf<unsigned char>("grid", cells * (f64 ? 16 : 8));
+    g.beam = s.beam ? c->buf<unsigned char>("beamgrid", cells * (f64 ? 16 : 8)) : nullptr;
+    auto geometry = [&](auto& p) {
+        p.N = b.N;
+        p.rows = b.rows;
+        p.pad = b.pad;
+        p.brn = b.brn;
+        p.off = off;
+        p.recs = q.rec;
+        p.wts = q.wts;
+        p.grid = g.grid;
+        p.beam = g.beam;
+    };
     const dim3 blocks(unsigned(ceil_div(ceil_div(b.rows, kBlk), kGridWarps)), unsigned(ceil_div(b.N, kBlk)));
-    auto launch = [&](auto kern) {
+    auto launch = [&](auto kern, const auto& p) {
         c->mark(1);
         kern<<<blocks, 32 * kGridWarps, 0, st>>>(p);
         STPGPU_CHECK_LAUNCH();
         c->mark(2);
     };
-    auto pick = [&](auto cell) {
-        using G = decltype(cell);
-        if (exact)
-            s.beam ? launch(k_grid_blocks<SepCore<R, G, true, true>>) : launch(k_grid_blocks<SepCore<R, G, true, false>>);
+    auto by_cell = [&](auto f) { // f(the grid's scalar type)
+        if constexpr (sizeof(R) == 8)
+            f(double());
         else
-            s.beam ? launch(k_grid_blocks<SepCore<R, G, false, true>>) : launch(k_grid_blocks<SepCore<R, G, false, false>>);
+            f64 ? f(double()) : f(float());
     };
-    if constexpr (sizeof(R) == 8)
-        pick(double());
-    else
-        f64 ? pick(double()) : pick(float());
+    if (in.wproj) {
+        WprojParams<R, T> p {};
+        geometry(p);
+        p.wk = static_cast<const typename Cplx<T>::T*>(in.wk);
+        p.max_support = in.max_support;
+        by_cell([&](auto cell) {
+            using G = decltype(cell);
+            s.beam ? launch(k_grid_blocks<WprojCore<R, G, T, ACC, true>>, p)
+                   : launch(k_grid_blocks<WprojCore<R, G, T, ACC, false>>, p);
+        });
+        return;
+    }
+    SepParams<R> p {};
+    geometry(p);
+    p.K = K;
+    if (in.exact) {
+        double* tab = c->buf<double>("exact_tab", size_t(nn) * 2 * K);
+        if (n > 0) {
+            k_exact_tables<<<grid1d(2 * n, 256), 256, 0, st>>>(s.kf, s.trunc, s.support, in.frac, n, tab);
+            STPGPU_CHECK_LAUNCH();
+        }
+        p.tab = tab;
+    } else {
+        p.tw = kBlk * b.pad + 15;
+        p.zrow = in.cs * p.tw;
+        double* tab = c->buf<double>("k1dpad", size_t(in.cs + 1) * p.tw);
+        if (!c->memo("k1dpad", std::to_string(s.kf) + "/" + fkey(s.trunc) + "/" + std::to_string(s.support) + "/"
+                    + std::to_string(in.os))) {
+            k_pad_table<<<grid1d(int64_t(in.cs + 1) * p.tw, 256), 256, 0, st>>>(in.k1d, in.cs, K, p.tw, tab);
+            STPGPU_CHECK_LAUNCH();
+        }
+        p.tab = tab;
+    }
+    by_cell([&](auto cell) {
+        using G = decltype(cell);
+        if (in.exact)
+            s.beam ? launch(k_grid_blocks<SepCore<R, G, true, true>>, p)
+                   : launch(k_grid_blocks<SepCore<R, G, true, false>>, p);
+        else
+            s.beam ? launch(k_grid_blocks<SepCore<R, G, false, true>>, p)
+                   : launch(k_grid_blocks<SepCore<R, G, false, false>>, p);
+    });
 }
 
+// convolve_to_grid (gridder.h:240-997): grids into context buffers "grid"
+// and "beamgrid" of precision R (complex), image_rows x N column-major.
 template <typename R, int COMP>
 GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, int vis_c64, const double* d_wts,
-    const double* d_uv, int uv_is_pixels, int64_t n, int tile_c = TILE_C_DEFAULT, GridLaunch<R>* defer = nullptr,
-    int form = 0)
+    const double* d_uv, int uv_is_pixels, int64_t n)
 {
-    if (tile_c != 32 && tile_c != 16 && !(tile_c == 8 && (form == 2 || form == 3)))
-        fail(STPGPU_ERR_INVALID_ARG, "tile width must be 16 or 32 (8 with the lane-per-tap or staged gridder)");
-    using C2 = typename Cplx<R>::T;
+    // W-projection: kernel tables in the call's precision, sums in double except for plain FP32
+    using KT = R;
+    using ACC = std::conditional_t<sizeof(R) == 8 || COMP == 1, double, float>;
+    using C2 = typename Cplx<KT>::T;
     check_pars(s);
     cudaStream_t st = c->stream;
     GridOut g;
@@ -696,7 +696,7 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
     g.d_total = c->buf<double>("total", 4);
     g.d_ngood = c->buf<unsigned long long>("ngood", 2);
     g.d_err = c->buf<unsigned int>("err", 2);
-    zero_words(st, { { g.d_err, 1 } });
+    zero_words(st, { { g.d_err, 2 } }); // error flags, largest plane support
     PrepassParams pp {};
     pp.n = n;
     pp.vis = d_vis;
@@ -732,9 +732,6 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
     const int64_t* plane_first = nullptr;
     int nplanes = 0;
     const double* k1d64 = nullptr;
-    const C2* wconv = nullptr;
-    const R* winv = nullptr;
-    int lh = 0;
     C2* wk = nullptr;
     uint32_t* wk_off = nullptr;
     uint8_t* ts_of = nullptr; // A-projection time step per visibility
@@ -1015,276 +1012,36 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
         wk = c->buf<C2>("wkexp", cap_wk);
         wk_off = c->buf<uint32_t>("wkoff", PT);
         if (aconv)
-            k_aproj_expand<R><<<dim3(PT, cs * cs), 256, 0, st>>>(aconv, arr, plane_support, cs, os, wk, wk_off);
+            k_aproj_expand<KT><<<dim3(PT, cs * cs), 256, 0, st>>>(aconv, arr, plane_support, cs, os, wk, wk_off,
+                g.d_err + 1);
         else
-            k_wk_expand<R><<<dim3(P, cs * cs), 64, 0, st>>>(wq.convd, wq.invd, plane_support, P, cs, os, Lh, wk,
-                wk_off);
+            k_wk_expand<KT><<<dim3(P, cs * cs), 64, 0, st>>>(wq.convd, wq.invd, plane_support, P, cs, os, Lh, wk,
+                wk_off, g.d_err + 1);
         STPGPU_CHECK_LAUNCH();
-        lh = Lh;
         g.d_plane_support = plane_support;
         g.nplanes = PT;
     }
 
-    const int kind = (wproj && n > 0) ? GK_WPROJ : (kernel_exact ? GK_EXACT : (!wproj ? GK_SEP : GK_NONE));
-    if (kind == GK_SEP || kind == GK_EXACT) {
-        grid_separable<R>(c, s, g, items, n, kind == GK_EXACT, os, cs, k1d64, pp.frac, COMP == 1 && s.wide_fft);
-        if (defer) {
-            defer->kind = GK_NONE; // gridded: nothing is left to launch
-            defer->ntiles = 0;
-        }
-        return g;
-    }
-    // the clipped forms need one footprint segment per axis and tile
-    const bool clip_ok = kind != GK_EXACT && N >= 2 * (2 * conv_support + 1 + 32) + 2;
-    // staged records: tabulated kernels, no beam (else the lane-per-tap form)
-    // and four warps' shared memory within the 227 KB of a block
-    const size_t rec_wb = sizeof(Acc<R, COMP>) * TILE_R * size_t(tile_c) + 2 * kRecChunk * sizeof(TapRec<R>) + 16
-        + (kind == GK_SEP ? sizeof(R) * size_t(cs) * size_t(2 * s.support + 1) : 0);
-    const bool use_recs = form == 3 && clip_ok && !s.beam && (kind == GK_WPROJ || kind == GK_SEP)
-        && 4 * (rec_wb + 15) <= 227 * 1024;
-    if (form == 3 && !use_recs)
-        form = 2;
-    // 8-column tiles exist for the clipped lane-per-tap and staged forms only
-    if (tile_c == 8 && !(clip_ok && (form == 2 || form == 3)))
-        tile_c = 16;
-
-    // ---- binning into 32x32 uv tiles
-    const int tiles_r = int(ceil_div(image_rows, TILE_R));
-    const int tiles_c = int(ceil_div(N, tile_c));
-    const int ntiles = tiles_r * tiles_c;
-    uint32_t* tcount = c->buf<uint32_t>("tcount", ntiles + 1);
-    uint32_t* toff = c->buf<uint32_t>("toff", ntiles + 1);
-    uint32_t* tcur = c->buf<uint32_t>("tcur", ntiles + 1);
-    const int Kx = 2 * conv_support + 1;
-    const uint64_t per_dim = uint64_t(ceil_div(Kx - 1, std::min(TILE_R, tile_c))) + 2;
-    uint64_t cap = std::max<uint64_t>(1, uint64_t(nn) * 2 * per_dim * per_dim);
-    if (!large_support(s) && cap > 0xffffffffull)
-        fail(STPGPU_ERR_INVALID_ARG, "too many visibilities for one snapshot");
-    uint32_t* list = (large_support(s) || use_recs) ? nullptr : c->buf<uint32_t>("tlist", cap);
-    Item<R>* bin_items = items_sorted ? items_sorted : items;
-    BinParams bp {};
-    bp.plane16 = plane16;
-    bp.N = N;
-    bp.image_rows = image_rows;
-    bp.tiles_r = tiles_r;
-    bp.tiles_c = tiles_c;
-    bp.tile_c = tile_c;
-    bp.support = s.support;
-    bp.plane_support = plane_support;
-    bp.ts_of = ts_of;
-    bp.ntimesteps = std::max(s.ntimesteps, 1);
-    bp.exact = kernel_exact;
-    bp.n = n;
-    bp.tile_count = tcount;
-    bp.tile_off = toff;
-    bp.tile_cursor = tcur;
-    // list slots kept by the count pass (the fill then needs no atomics)
-    bp.ranks = c->buf<uint32_t>("tranks", size_t(std::max<int64_t>(n, 1)) * 2 * kRankSlots);
-    bp.rank_overflow = c->buf<uint32_t>("trankovf", 1);
-    bp.list = list;
-    bp.list_capacity = cap;
-    bp.err = g.d_err;
-    zero_words(st, { { tcount, ntiles + 1 }, { tcur, ntiles + 1 }, { bp.rank_overflow, 1 } });
-    if (n > 0) {
-        k_count_tiles<R><<<grid1d(n, 256), 256, 0, st>>>(bp, bin_items, sorted_perm, plane_first, nplanes);
-        STPGPU_CHECK_LAUNCH();
-    }
-    if (ntiles <= 4096) {
-        k_scan_single<<<1, 1024, 0, st>>>(tcount, toff, ntiles);
-        STPGPU_CHECK_LAUNCH();
-    } else {
-        // many tiles: the multi-block scan (tcount[ntiles] is 0, so
-        // toff[ntiles] receives the total)
-        size_t tb = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, tb, tcount, toff, ntiles + 1, st);
-        void* tmp = c->buf<unsigned char>("cubtmp_tiles", tb);
-        if (cub::DeviceScan::ExclusiveSum(tmp, tb, tcount, toff, ntiles + 1, st) != cudaSuccess)
-            fail(STPGPU_ERR_CUDA, "tile offset scan failed");
-        g_launches += 2;
-    }
-    TapRec<R>* recs = nullptr;
-    uint64_t rec_cap = 0;
-    if (use_recs) {
-        // records sized from the records per visibility counted on the first
-        // call of this namespace and class (one host round trip), scaled by
-        // the call's visibilities with a quarter spare; a call that exceeds
-        // the capacity sets bit 8 and the caller grids again after a fresh
-        // count
-        const std::string rkey = c->ns + "/" + std::to_string(tile_c) + "/S" + std::to_string(conv_support) + "/t"
-            + fkey(s.trunc_perc) + "/os" + std::to_string(os);
-        auto it = c->rec_ratio.find(rkey);
-        if (it == c->rec_ratio.end() || large_support(s)) {
-            uint32_t total = 0;
-            STPGPU_CUDA_TRY(cudaMemcpyAsync(&total, toff + ntiles, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-            STPGPU_CUDA_TRY(cudaStreamSynchronize(st));
-            const double r = double(total) / double(nn);
-            it = c->rec_ratio.insert_or_assign(rkey, it == c->rec_ratio.end() ? r : std::max(r, it->second)).first;
-        }
-        rec_cap = uint64_t(std::ceil(double(nn) * it->second * 1.25)) + 1024;
-        recs = c->buf<TapRec<R>>("trecs", rec_cap);
-        if (n > 0) {
-            RecFill<R> rf { recs, rec_cap, wk_off, cs, os };
-            if (kind == GK_WPROJ)
-                k_fill_recs<R, KM_WPROJ><<<grid1d(n, 256), 256, 0, st>>>(bp, bin_items, sorted_perm, plane_first,
-                    nplanes, rf);
-            else
-                k_fill_recs<R, KM_SEP><<<grid1d(n, 256), 256, 0, st>>>(bp, bin_items, sorted_perm, plane_first,
-                    nplanes, rf);
-            STPGPU_CHECK_LAUNCH();
-        }
-    } else {
-        if (large_support(s)) { // size the list from the counted entries
-            uint32_t total = 0;
-            STPGPU_CUDA_TRY(cudaMemcpyAsync(&total, toff + ntiles, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-            STPGPU_CUDA_TRY(cudaStreamSynchronize(st));
-            cap = std::max<uint64_t>(total, 1);
-            list = c->buf<uint32_t>("tlist", cap);
-            bp.list = list;
-            bp.list_capacity = cap;
-        }
-        if (n > 0) {
-            k_fill_tiles<R><<<grid1d(n, 256), 256, 0, st>>>(bp, bin_items, sorted_perm, plane_first, nplanes);
-            STPGPU_CHECK_LAUNCH();
-        }
-    }
-    g.d_nitems = toff + ntiles;
-
-    // ---- tile gridding
-    // a wide grid (compensated FP32 for a double-precision c2r) holds double2 cells
-    const int wide = (COMP == 1 && s.wide_fft) ? 1 : 0;
-    const size_t cells = size_t(image_rows) * N * (wide ? 2 : 1);
-    C2* grid = c->buf<C2>("grid", cells);
-    C2* beam = s.beam ? c->buf<C2>("beamgrid", cells) : nullptr;
-    GridParams<R> gp {};
-    gp.N = N;
-    gp.image_rows = image_rows;
-    gp.tiles_r = tiles_r;
-    gp.support = s.support;
-    gp.os = os;
-    gp.cs = cs;
-    gp.exact_wrap = kernel_exact;
-    gp.items = bin_items;
-    gp.tile_off = toff;
-    gp.list = list;
-    gp.kf = s.kf;
-    gp.trunc = s.trunc;
-    gp.frac = pp.frac;
-    gp.n = n;
-    gp.wconv = wconv;
-    gp.winv = winv;
-    gp.lh = lh;
-    gp.plane_support = plane_support;
-    gp.wk = wk;
-    gp.wk_off = wk_off;
-    gp.recs = recs;
-    gp.rec_cap = rec_cap;
-    gp.err = g.d_err;
-    gp.grid = grid;
-    gp.beam = beam;
-    gp.wide = wide;
-    using A = Acc<R, COMP>;
-    size_t smem = size_t(TILE_R) * tile_c * sizeof(A) * (s.beam ? 2 : 1);
-    if (!wproj && !kernel_exact)
-        smem += sizeof(R) * size_t(cs) * (2 * s.support + 1);
     if (2 * conv_support + 1 > 255)
         fail(STPGPU_ERR_UNSUPPORTED, "kernel support > 127 is outside the GPU path");
-    if (kind == GK_NONE) {
-        STPGPU_CUDA_TRY(cudaMemsetAsync(grid, 0, sizeof(C2) * cells, st));
-        if (beam)
-            STPGPU_CUDA_TRY(cudaMemsetAsync(beam, 0, sizeof(C2) * cells, st));
-    }
-    if (defer) {
-        defer->kind = kind;
-        defer->beam = s.beam ? 1 : 0;
-        defer->form = use_recs ? 3 : (form == 2 && clip_ok && kind != GK_EXACT ? 2 : 0);
-        defer->tile_c = tile_c;
-        defer->ntiles = kind == GK_NONE ? 0 : ntiles;
-        defer->smem = use_recs ? (rec_wb + 15) / 16 * 16 : smem;
-        defer->gp = gp;
-    } else if (kind != GK_NONE) {
-        auto launch = [&](auto kern) {
-            if (smem > 48 * 1024)
-                STPGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-            c->mark(1);
-            kern<<<ntiles, 32, smem, st>>>(gp);
-            STPGPU_CHECK_LAUNCH();
-            c->mark(2);
-        };
-        const bool b = s.beam != 0;
-        const bool t32 = tile_c == 32;
-        const bool use_cols = form == 1 && clip_ok, use_taps = form == 2 && clip_ok;
-        if (use_recs) {
-            // four warps per block, each on its own tile
-            const int sep_len = kind == GK_SEP ? cs * (2 * s.support + 1) : 0;
-            auto launch_recs = [&](auto kern, size_t wb) {
-                const size_t bs = 4 * wb;
-                if (bs > 48 * 1024)
-                    STPGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bs)));
-                c->mark(1);
-                kern<<<unsigned((ntiles + 3) / 4), 128, bs, st>>>(gp, ntiles, int(wb));
-                STPGPU_CHECK_LAUNCH();
-                c->mark(2);
-            };
-            if (kind == GK_WPROJ) {
-                if (tile_c == 8)
-                    launch_recs(k_grid_tiles_recs<R, COMP, KM_WPROJ, 8, 4>, rec_warp_bytes<R, COMP, 8>(0));
-                else if (tile_c == 16)
-                    launch_recs(k_grid_tiles_recs<R, COMP, KM_WPROJ, 16, 4>, rec_warp_bytes<R, COMP, 16>(0));
-                else
-                    launch_recs(k_grid_tiles_recs<R, COMP, KM_WPROJ, 32, 4>, rec_warp_bytes<R, COMP, 32>(0));
-            } else {
-                if (tile_c == 8)
-                    launch_recs(k_grid_tiles_recs<R, COMP, KM_SEP, 8, 4>, rec_warp_bytes<R, COMP, 8>(sep_len));
-                else if (tile_c == 16)
-                    launch_recs(k_grid_tiles_recs<R, COMP, KM_SEP, 16, 4>, rec_warp_bytes<R, COMP, 16>(sep_len));
-                else
-                    launch_recs(k_grid_tiles_recs<R, COMP, KM_SEP, 32, 4>, rec_warp_bytes<R, COMP, 32>(sep_len));
-            }
-        } else if (use_cols && kind == GK_WPROJ)
-            b ? (t32 ? launch(k_grid_tiles<R, COMP, KM_WPROJ, true, 32, 1>) : launch(k_grid_tiles<R, COMP, KM_WPROJ, true, 16, 1>))
-              : (t32 ? launch(k_grid_tiles<R, COMP, KM_WPROJ, false, 32, 1>) : launch(k_grid_tiles<R, COMP, KM_WPROJ, false, 16, 1>));
-        else if (use_cols)
-            b ? (t32 ? launch(k_grid_tiles<R, COMP, KM_SEP, true, 32, 1>) : launch(k_grid_tiles<R, COMP, KM_SEP, true, 16, 1>))
-              : (t32 ? launch(k_grid_tiles<R, COMP, KM_SEP, false, 32, 1>) : launch(k_grid_tiles<R, COMP, KM_SEP, false, 16, 1>));
-        else if (use_taps && tile_c == 8) {
-            // four 8-column tiles per block (k_grid_tiles_mw)
-            const int tb = int((smem + 15) / 16 * 16);
-            auto launch_mw = [&](auto kern) {
-                const size_t bs = size_t(4) * size_t(tb);
-                if (bs > 48 * 1024)
-                    STPGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bs)));
-                c->mark(1);
-                kern<<<unsigned((ntiles + 3) / 4), 128, bs, st>>>(gp, ntiles, tb);
-                STPGPU_CHECK_LAUNCH();
-                c->mark(2);
-            };
-            if (kind == GK_WPROJ)
-                b ? launch_mw(k_grid_tiles_mw<R, COMP, KM_WPROJ, true, 8, 4>)
-                  : launch_mw(k_grid_tiles_mw<R, COMP, KM_WPROJ, false, 8, 4>);
-            else
-                b ? launch_mw(k_grid_tiles_mw<R, COMP, KM_SEP, true, 8, 4>)
-                  : launch_mw(k_grid_tiles_mw<R, COMP, KM_SEP, false, 8, 4>);
-        } else if (use_taps && kind == GK_WPROJ)
-            b ? (t32 ? launch(k_grid_tiles<R, COMP, KM_WPROJ, true, 32, 2>) : launch(k_grid_tiles<R, COMP, KM_WPROJ, true, 16, 2>))
-              : (t32 ? launch(k_grid_tiles<R, COMP, KM_WPROJ, false, 32, 2>) : launch(k_grid_tiles<R, COMP, KM_WPROJ, false, 16, 2>));
-        else if (use_taps)
-            b ? (t32 ? launch(k_grid_tiles<R, COMP, KM_SEP, true, 32, 2>) : launch(k_grid_tiles<R, COMP, KM_SEP, true, 16, 2>))
-              : (t32 ? launch(k_grid_tiles<R, COMP, KM_SEP, false, 32, 2>) : launch(k_grid_tiles<R, COMP, KM_SEP, false, 16, 2>));
-        else if (kind == GK_WPROJ)
-            b ? (t32 ? launch(k_grid_tiles<R, COMP, KM_WPROJ, true, 32>) : launch(k_grid_tiles<R, COMP, KM_WPROJ, true, 16>))
-              : (t32 ? launch(k_grid_tiles<R, COMP, KM_WPROJ, false, 32>) : launch(k_grid_tiles<R, COMP, KM_WPROJ, false, 16>));
-        else if (kind == GK_EXACT)
-            b ? (t32 ? launch(k_grid_tiles<R, COMP, KM_EXACT, true, 32>) : launch(k_grid_tiles<R, COMP, KM_EXACT, true, 16>))
-              : (t32 ? launch(k_grid_tiles<R, COMP, KM_EXACT, false, 32>) : launch(k_grid_tiles<R, COMP, KM_EXACT, false, 16>));
-        else
-            b ? (t32 ? launch(k_grid_tiles<R, COMP, KM_SEP, true, 32>) : launch(k_grid_tiles<R, COMP, KM_SEP, true, 16>))
-              : (t32 ? launch(k_grid_tiles<R, COMP, KM_SEP, false, 32>) : launch(k_grid_tiles<R, COMP, KM_SEP, false, 16>));
-    } else {
-        c->mark(1);
-        c->mark(2);
-    }
-    g.grid = grid;
-    g.beam = beam;
+    GridInputs<R> in;
+    in.wproj = wproj;
+    in.exact = kernel_exact != 0;
+    in.os = os;
+    in.cs = cs;
+    in.items = items_sorted ? items_sorted : items;
+    in.plane_support = plane_support;
+    in.plane16 = plane16;
+    in.order = sorted_perm;
+    in.first = plane_first;
+    in.P = nplanes;
+    in.ts_of = ts_of;
+    in.wk_off = wk_off;
+    in.wk = wk;
+    in.max_support = g.d_err + 1;
+    in.k1d = k1d64;
+    in.frac = pp.frac;
+    grid_blocks<R, KT, ACC>(c, s, g, n, in, COMP == 1 && s.wide_fft);
     return g;
 }
 
@@ -1306,12 +1063,10 @@ ScalarsBack read_back(stpgpu_context* c, const GridOut& g)
     STPGPU_CUDA_TRY(cudaStreamSynchronize(c->stream));
     ScalarsBack r { h->total, h->ngood, h->nitems, h->err, h->max_support };
     // bit 4: the 32-bit |w| sort met a long run of distinct |w| (the caller
-    // repeats the gridding with the 64-bit sort); bit 8: the staged
-    // gridder's records exceeded their capacity (the caller grids again with
-    // the buffer sized from the count); bit 16: the W-planes without the
-    // sort did not apply (the caller grids again on the sorting path); other
-    // bits are errors
-    if (r.err & ~(4u | 8u | 16u))
+    // repeats the gridding with the 64-bit sort); bit 16: the W-planes
+    // without the sort did not apply (the caller grids again on the sorting
+    // path); other bits are errors
+    if (r.err & ~(4u | 16u))
         fail(STPGPU_ERR_DEVICE, "gridder reported internal error flags " + std::to_string(r.err));
     return r;
 }
@@ -1487,26 +1242,11 @@ void run_imager(stpgpu_context* c, const ImagerSetup& s_in, int image_size, int 
     // its last call (visibilities outside the grid, non-finite w) sorts
     s.wsel = s.nplanes > 0 && s.nplanes <= WSEL_MAXP && !s.wmedian && s.ntimesteps == 0 && !s.full_wsort
         && n < (int64_t(1) << 31);
-    // tile width: the autotuned choice of this size class; the first call of
-    // a class grids with both widths, times them, keeps the faster for later
-    // calls (every pass produces the complete grid; the last one is used)
     const int precision = sizeof(R) == 8 ? STPGPU_FP64 : (COMP ? STPGPU_FP32C : STPGPU_FP32);
     const std::string cls = size_class(s, precision);
     if (s.wsel && c->wsel_off.count(cls))
         s.wsel = 0;
     GridOut g;
-    // STPGPU_GRIDDER_LAYOUT=32|16|32c|16c|32t|16t|8t|32r|16r|8r pins the tile
-    // width and gridder form (c: column-packed, t: lane-per-tap, r: staged
-    // records) instead of the autotuner's choice
-    if (const char* pin = std::getenv("STPGPU_GRIDDER_LAYOUT")) {
-        const int w = std::atoi(pin);
-        if (w == 16 || w == 32 || (w == 8 && (std::strchr(pin, 't') || std::strchr(pin, 'r'))))
-            c->tune_set(cls,
-                w | (std::strchr(pin, 'c') ? kLayoutCols : 0) | (std::strchr(pin, 't') ? kLayoutTaps : 0)
-                    | (std::strchr(pin, 'r') ? kLayoutRecs : 0));
-    }
-    int tuned_lay = TILE_C_DEFAULT;
-    const bool have_tune = c->tune_get(cls, tuned_lay) || s.nplanes == 0;
     // Device-pointer calls that repeat the previous call exactly (parameters,
     // sizes, buffers) replay a CUDA graph of the gridding, FFT and
     // normalisation kernels, captured on the first repeat; any other call
@@ -1531,12 +1271,11 @@ void run_imager(stpgpu_context* c, const ImagerSetup& s_in, int image_size, int 
         STPGPU_CUDA_TRY(cudaGraphLaunch(c->single_exec, c->stream));
         g_launches += c->single_launches; // the replay runs the captured kernels
         g = c->single_g;
-    } else if (repeat && have_tune) {
+    } else if (repeat) {
         const int before = g_launches;
         STPGPU_CUDA_TRY(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
         try {
-            g = run_gridder<R, COMP>(c, s, d_vis, vis_c64, d_wts, d_uvw, 0, n, tuned_lay & 0xff, nullptr,
-                form_of(tuned_lay));
+            g = run_gridder<R, COMP>(c, s, d_vis, vis_c64, d_wts, d_uvw, 0, n);
             finish_imager<R>(c, s, image_size, correction, g, d_image, d_beam, out_f32);
         } catch (...) {
             cudaGraph_t dead = nullptr;
@@ -1554,65 +1293,8 @@ void run_imager(stpgpu_context* c, const ImagerSetup& s_in, int image_size, int 
         STPGPU_CUDA_TRY(cudaGraphLaunch(c->single_exec, c->stream));
         c->single_g = g;
         c->single_launches = g_launches - before;
-    } else if (have_tune || c->timing) {
-        const int lay = have_tune ? tuned_lay : TILE_C_DEFAULT;
-        g = run_gridder<R, COMP>(c, s, d_vis, vis_c64, d_wts, d_uvw, 0, n, lay & 0xff, nullptr,
-            form_of(lay));
     } else {
-        for (auto& e : c->tev)
-            if (!e)
-                STPGPU_CUDA_TRY(cudaEventCreate(&e));
-        // an untimed pass first grows every buffer (16 columns: the most
-        // tiles) and fills the cached tables, so no timed pass pays that
-        // the column-packed form is a candidate for large kernels only (with
-        // K <= 17 the lane-per-item form is faster on every measured workload)
-        g = run_gridder<R, COMP>(c, s, d_vis, vis_c64, d_wts, d_uvw, 0, n, 16);
-        // the widest kernel the data actually uses (W-planes are truncated
-        // below the maximum support), read back from the untimed pass
-        const int used_support = s.nplanes > 0 ? std::max(read_back(c, g).max_support, 0) : s.support;
-        // the clipped forms need one footprint segment per axis and tile
-        const bool clip_ok = !s.kernel_exact && s.N >= 2 * (2 * (s.nplanes > 0 ? s.max_support : s.support) + 33) + 2;
-        std::vector<int> lays = { 32, 16 };
-        if (clip_ok) {
-            for (int w : { 32 | kLayoutTaps, 16 | kLayoutTaps, 8 | kLayoutTaps })
-                lays.push_back(w);
-            if (2 * used_support + 1 > 17)
-                for (int w : { 32 | kLayoutCols, 16 | kLayoutCols })
-                    lays.push_back(w);
-            if (!s.beam)
-                for (int w : { 32 | kLayoutRecs, 16 | kLayoutRecs, 8 | kLayoutRecs })
-                    lays.push_back(w);
-        }
-        const int ncand = int(lays.size());
-        std::vector<float> ms(size_t(ncand), 1e30f);
-        // each candidate timed twice, the faster pass kept (single passes
-        // of close candidates swap order from run to run)
-        for (int rep = 0; rep < 2; rep++)
-            for (int k = 0; k < ncand; k++) {
-                STPGPU_CUDA_TRY(cudaEventRecord(c->tev[0], c->stream));
-                g = run_gridder<R, COMP>(c, s, d_vis, vis_c64, d_wts, d_uvw, 0, n, lays[k] & 0xff, nullptr,
-                    form_of(lays[k]));
-                STPGPU_CUDA_TRY(cudaEventRecord(c->tev[1], c->stream));
-                STPGPU_CUDA_TRY(cudaEventSynchronize(c->tev[1]));
-                float t = 0.f;
-                STPGPU_CUDA_TRY(cudaEventElapsedTime(&t, c->tev[0], c->tev[1]));
-                ms[k] = std::min(ms[k], t);
-            }
-        int best = 0;
-        for (int k = 1; k < ncand; k++)
-            if (ms[k] < ms[best])
-                best = k;
-        c->tune_set(cls, lays[best]);
-        if (std::getenv("STPGPU_LOG_TUNING")) {
-            std::string line;
-            for (int k = 0; k < ncand; k++) {
-                const int f = form_of(lays[k]);
-                line += " " + std::to_string(lays[k] & 0xff)
-                    + (f == 1 ? "c" : (f == 2 ? "t" : (f == 3 ? "r" : ""))) + " " + std::to_string(ms[k]);
-            }
-            std::fprintf(stderr, "stpgpu gridder tuner: %s (layout ms):%s -> candidate %d (single call)\n", cls.c_str(),
-                line.c_str(), best);
-        }
+        g = run_gridder<R, COMP>(c, s, d_vis, vis_c64, d_wts, d_uvw, 0, n);
     }
     if (!(repeat && c->single_exec))
         finish_imager<R>(c, s, image_size, correction, g, d_image, d_beam, out_f32);
@@ -1620,27 +1302,13 @@ void run_imager(stpgpu_context* c, const ImagerSetup& s_in, int image_size, int 
         c->single_sig = sig;
     const int N = s.N;
     ScalarsBack sb = read_back(c, g);
-    if (sb.err & 8u) {
-        // records outgrew the remembered capacity: size them from a fresh
-        // count (the next run_gridder reads the total) and grid again
-        for (auto it = c->rec_ratio.begin(); it != c->rec_ratio.end();)
-            it = it->first.compare(0, c->ns.size() + 1, c->ns + "/") == 0 ? c->rec_ratio.erase(it) : std::next(it);
-        c->drop_single();
-        int lay = TILE_C_DEFAULT;
-        c->tune_get(cls, lay);
-        g = run_gridder<R, COMP>(c, s, d_vis, vis_c64, d_wts, d_uvw, 0, n, lay & 0xff, nullptr, form_of(lay));
-        finish_imager<R>(c, s, image_size, correction, g, d_image, d_beam, out_f32);
-        sb = read_back(c, g);
-    }
     if (sb.err & 16u) {
         // the W-planes without the sort did not apply: the sorting path, for
         // this call and the size class's next ones
         c->wsel_off.insert(cls);
         c->drop_single();
         s.wsel = 0;
-        int lay = TILE_C_DEFAULT;
-        c->tune_get(cls, lay);
-        g = run_gridder<R, COMP>(c, s, d_vis, vis_c64, d_wts, d_uvw, 0, n, lay & 0xff, nullptr, form_of(lay));
+        g = run_gridder<R, COMP>(c, s, d_vis, vis_c64, d_wts, d_uvw, 0, n);
         finish_imager<R>(c, s, image_size, correction, g, d_image, d_beam, out_f32);
         sb = read_back(c, g);
     }
@@ -1648,10 +1316,7 @@ void run_imager(stpgpu_context* c, const ImagerSetup& s_in, int image_size, int 
         // rare data (many distinct |w| within one single-precision step): redo with the 64-bit |w| sort
         ImagerSetup s64 = s;
         s64.full_wsort = 1;
-        int lay = TILE_C_DEFAULT;
-        c->tune_get(cls, lay);
-        g = run_gridder<R, COMP>(c, s64, d_vis, vis_c64, d_wts, d_uvw, 0, n, lay & 0xff, nullptr,
-            form_of(lay));
+        g = run_gridder<R, COMP>(c, s64, d_vis, vis_c64, d_wts, d_uvw, 0, n);
         finish_imager<R>(c, s64, image_size, correction, g, d_image, d_beam, out_f32);
         sb = read_back(c, g);
     }
@@ -1762,24 +1427,8 @@ struct BatchSnap {
     const double* uvw = nullptr;
     int64_t n = 0;
     void* image = nullptr;
-    std::string cls; // size class of the tile autotuner
-    int tile_c = TILE_C_DEFAULT;
-    int persist = 0;
-    int form = 0; // gridder form: 0 lanes-per-item, 2 lane-per-tap
+    std::string cls; // size class
 };
-
-// Tuned layout of a batch snapshot.  The lane-per-tap form clips footprints
-// to tiles and needs one segment per axis and tile (as in run_gridder).
-void apply_layout(BatchSnap& b, int lay)
-{
-    b.tile_c = lay & 0xff;
-    b.persist = (lay & kLayoutPersist) ? 1 : 0;
-    const int conv = b.s.nplanes > 0 ? b.s.max_support : b.s.support;
-    const bool clip_ok = !b.s.kernel_exact && b.s.N >= 2 * (2 * conv + 1 + 32) + 2;
-    // the staged form: run_gridder falls back to the lane-per-tap form where
-    // it does not apply and reports the form it built in GridLaunch::form
-    b.form = ((lay & kLayoutRecs) && clip_ok) ? 3 : (((lay & kLayoutTaps) && clip_ok) ? 2 : 0);
-}
 
 void batch_streams(stpgpu_context* c)
 {
@@ -1813,109 +1462,15 @@ void batch_join(stpgpu_context* c, cudaStream_t main)
     }
 }
 
-template <typename R, int COMP, int KMODE, int TC, bool PERSIST, int FORM>
-void launch_grid_batch(cudaStream_t st, size_t smem, const BatchGridParams<R>& P, uint32_t total_tiles, bool capturing)
-{
-    auto kern = k_grid_batch<R, COMP, KMODE, false, TC, PERSIST, FORM>;
-    if (!capturing && smem > 48 * 1024)
-        STPGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    uint32_t blocks = std::max<uint32_t>(1, total_tiles);
-    if (PERSIST) {
-        static int sms = 0;
-        if (sms == 0) {
-            int dev = 0;
-            STPGPU_CUDA_TRY(cudaGetDevice(&dev));
-            STPGPU_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        }
-        int per_sm = 0;
-        STPGPU_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32, smem));
-        blocks = std::min<uint32_t>(blocks, uint32_t(std::max(per_sm, 1) * sms));
-    }
-    kern<<<blocks, 32, smem, st>>>(P);
-    STPGPU_CHECK_LAUNCH();
-}
-
-
-template <typename R, int COMP, int KMODE, int FORM>
-void launch_mode_form(cudaStream_t st, int layout, size_t smem, const BatchGridParams<R>& P, uint32_t total, bool cap)
-{
-    const bool t32 = (layout & 0xff) == 32;
-    if (layout & kLayoutPersist)
-        t32 ? launch_grid_batch<R, COMP, KMODE, 32, true, FORM>(st, smem, P, total, cap)
-            : launch_grid_batch<R, COMP, KMODE, 16, true, FORM>(st, smem, P, total, cap);
-    else
-        t32 ? launch_grid_batch<R, COMP, KMODE, 32, false, FORM>(st, smem, P, total, cap)
-            : launch_grid_batch<R, COMP, KMODE, 16, false, FORM>(st, smem, P, total, cap);
-}
-
-template <typename R, int COMP, int KMODE>
-void launch_mode(cudaStream_t st, int layout, size_t smem, const BatchGridParams<R>& P, uint32_t total, bool cap)
-{
-    if (KMODE != KM_EXACT && (layout & kLayoutRecs))
-        launch_mode_form<R, COMP, KMODE, 3>(st, layout, smem, P, total, cap);
-    else if (KMODE != KM_EXACT && (layout & kLayoutTaps))
-        launch_mode_form<R, COMP, KMODE, 2>(st, layout, smem, P, total, cap);
-    else
-        launch_mode_form<R, COMP, KMODE, 0>(st, layout, smem, P, total, cap);
-}
-
+// Enqueue one batch: every snapshot's whole pipeline (with host buffers, its
+// transfers too) on its worker stream, so that the snapshots overlap, and the
+// scalars of each read back into `scal` (pinned host memory).
 template <typename R, int COMP>
-void launch_group(cudaStream_t st, int kind, int layout, size_t smem, const BatchGridParams<R>& P, uint32_t total,
-    bool capturing)
-{
-    if (kind == GK_WPROJ)
-        launch_mode<R, COMP, KM_WPROJ>(st, layout, smem, P, total, capturing);
-    else if (kind == GK_EXACT)
-        launch_mode<R, COMP, KM_EXACT>(st, layout, smem, P, total, capturing);
-    else
-        launch_mode<R, COMP, KM_SEP>(st, layout, smem, P, total, capturing);
-}
-
-// Enqueue one batch: preparation of every snapshot on the worker streams,
-// persistent gridder launches on the main stream (one per kernel variant,
-// or one per size class when class_ms is given, each timed), then c2r +
-// normalisation per snapshot on the worker streams, and the scalars of every
-// snapshot gathered into `scal` (pinned host memory) by the main stream.
-template <typename R, int COMP>
-int batch_enqueue(stpgpu_context* c, std::vector<BatchSnap>& B, int out_f32, int device_ptrs, bool capturing,
-    BatchScalars* scal, unsigned char* host_params, std::map<std::string, float>* class_ms)
+void batch_enqueue(stpgpu_context* c, std::vector<BatchSnap>& B, int out_f32, int device_ptrs, BatchScalars* scal)
 {
     const cudaStream_t main = c->stream;
     const int nb = int(B.size());
     const int K = int(c->wstreams.size());
-    const size_t vb = 16;
-    std::vector<GridLaunch<R>> L(nb);
-    std::vector<GridOut> G(nb);
-    std::vector<void*> dimg(nb);
-    if (!device_ptrs && !class_ms) {
-        // host buffers: each snapshot runs its whole pipeline on its worker
-        // stream (H2D, preparation, gridder, c2r, normalisation, D2H), so the
-        // transfers of one snapshot overlap the compute of the others
-        batch_fork(c, main);
-        for (int i = 0; i < nb; i++) {
-            c->stream = c->wstreams[i % K];
-            c->ns = "b" + std::to_string(i) + "/";
-            BatchSnap& b = B[i];
-            const void* dv = to_device<unsigned char>(c, "in_vis", b.vis, (b.c64 ? 8 : vb) * size_t(b.n));
-            const double* dw = to_device<double>(c, "in_w", b.wts, size_t(b.n));
-            const double* duvw = to_device<double>(c, "in_uvw", b.uvw, 3 * size_t(b.n));
-            const size_t ob = (out_f32 ? 4 : 8) * size_t(b.image_size) * b.image_size;
-            void* di = c->buf<unsigned char>("out_img", ob);
-            GridOut g = run_gridder<R, COMP>(c, b.s, dv, b.c64, dw, duvw, 0, b.n, b.tile_c, nullptr, b.form);
-            finish_imager<R>(c, b.s, b.image_size, b.correction, g, di, nullptr, out_f32);
-            BatchScalars* ds = c->buf<BatchScalars>("scal", 1);
-            k_collect_scalars<<<1, 1, 0, c->stream>>>(g.d_total, g.d_ngood, g.d_nitems, g.d_err,
-                g.d_plane_support ? g.d_plane_support : reinterpret_cast<const int*>(g.d_err),
-                g.d_plane_support ? g.nplanes : 0, ds);
-            STPGPU_CHECK_LAUNCH();
-            STPGPU_CUDA_TRY(cudaMemcpyAsync(&scal[i], ds, sizeof(BatchScalars), cudaMemcpyDeviceToHost, c->stream));
-            STPGPU_CUDA_TRY(cudaMemcpyAsync(b.image, di, ob, cudaMemcpyDeviceToHost, c->stream));
-        }
-        c->stream = main;
-        c->ns = "";
-        batch_join(c, main);
-        return nb;
-    }
     batch_fork(c, main);
     for (int i = 0; i < nb; i++) {
         c->stream = c->wstreams[i % K];
@@ -1924,91 +1479,29 @@ int batch_enqueue(stpgpu_context* c, std::vector<BatchSnap>& B, int out_f32, int
         const void* dv = b.vis;
         const double* dw = b.wts;
         const double* duvw = b.uvw;
-        dimg[i] = b.image;
+        void* di = b.image;
+        const size_t ob = (out_f32 ? 4 : 8) * size_t(b.image_size) * b.image_size;
         if (!device_ptrs) {
-            const size_t vbytes = b.c64 ? 8 : vb;
-            dv = to_device<unsigned char>(c, "in_vis", b.vis, vbytes * size_t(b.n));
+            dv = to_device<unsigned char>(c, "in_vis", b.vis, (b.c64 ? 8 : 16) * size_t(b.n));
             dw = to_device<double>(c, "in_w", b.wts, size_t(b.n));
             duvw = to_device<double>(c, "in_uvw", b.uvw, 3 * size_t(b.n));
-            dimg[i] = c->buf<unsigned char>("out_img", (out_f32 ? 4 : 8) * size_t(b.image_size) * b.image_size);
+            di = c->buf<unsigned char>("out_img", ob);
         }
-        G[i] = run_gridder<R, COMP>(c, b.s, dv, b.c64, dw, duvw, 0, b.n, b.tile_c, &L[i], b.form);
-    }
-    c->stream = main;
-    c->ns = "batch/";
-    batch_join(c, main);
-
-    // ---- persistent gridder launches over (snapshot, tile) work queues
-    std::map<std::string, std::vector<int>> groups;
-    for (int i = 0; i < nb; i++) {
-        if (L[i].kind == GK_NONE || L[i].ntiles == 0)
-            continue;
-        std::string key = std::to_string(L[i].kind) + "/" + std::to_string(L[i].tile_c) + "/"
-            + std::to_string(B[i].persist) + "/" + std::to_string(L[i].form);
-        if (class_ms)
-            key += "|" + B[i].cls;
-        groups[key].push_back(i);
-    }
-    int gi = 0, nlaunch = 0;
-    for (auto& kv : groups) {
-        const std::vector<int>& all = kv.second;
-        for (size_t c0 = 0; c0 < all.size(); c0 += kBatchGrid) {
-            const int m = int(std::min<size_t>(kBatchGrid, all.size() - c0));
-            auto* P = reinterpret_cast<BatchGridParams<R>*>(host_params); // host-side scratch, copied by value
-            size_t smem = 0;
-            uint32_t tot = 0;
-            for (int k = 0; k < m; k++) {
-                const GridLaunch<R>& l = L[all[c0 + k]];
-                P->ps[k] = l.gp;
-                P->tile_base[k] = tot;
-                tot += uint32_t(l.ntiles);
-                smem = std::max(smem, l.smem);
-            }
-            P->tile_base[m] = tot;
-            P->nsnap = m;
-            P->counter = c->buf<uint32_t>("g" + std::to_string(gi++) + "ctr", 1);
-            STPGPU_CUDA_TRY(cudaMemsetAsync(P->counter, 0, sizeof(uint32_t), main));
-            if (class_ms)
-                STPGPU_CUDA_TRY(cudaEventRecord(c->pev[0], main));
-            const GridLaunch<R>& l0 = L[all[c0]];
-            launch_group<R, COMP>(main, l0.kind,
-                l0.tile_c | (B[all[c0]].persist ? kLayoutPersist : 0) | (l0.form == 2 ? kLayoutTaps : 0)
-                    | (l0.form == 3 ? kLayoutRecs : 0),
-                smem, *P, tot, capturing);
-            nlaunch++;
-            if (class_ms) {
-                STPGPU_CUDA_TRY(cudaEventRecord(c->pev[1], main));
-                STPGPU_CUDA_TRY(cudaEventSynchronize(c->pev[1]));
-                float ms = 0.f;
-                STPGPU_CUDA_TRY(cudaEventElapsedTime(&ms, c->pev[0], c->pev[1]));
-                (*class_ms)[B[all[c0]].cls] += ms;
-            }
-        }
-    }
-
-    // ---- c2r + normalise per snapshot, scalars
-    batch_fork(c, main);
-    for (int i = 0; i < nb; i++) {
-        c->stream = c->wstreams[i % K];
-        c->ns = "b" + std::to_string(i) + "/";
-        BatchSnap& b = B[i];
-        finish_imager<R>(c, b.s, b.image_size, b.correction, G[i], dimg[i], nullptr, out_f32);
+        const GridOut g = run_gridder<R, COMP>(c, b.s, dv, b.c64, dw, duvw, 0, b.n);
+        finish_imager<R>(c, b.s, b.image_size, b.correction, g, di, nullptr, out_f32);
         BatchScalars* ds = c->buf<BatchScalars>("scal", 1);
-        k_collect_scalars<<<1, 1, 0, c->stream>>>(G[i].d_total, G[i].d_ngood, G[i].d_nitems, G[i].d_err,
-            G[i].d_plane_support ? G[i].d_plane_support : reinterpret_cast<const int*>(G[i].d_err),
-            G[i].d_plane_support ? G[i].nplanes : 0, ds);
+        k_collect_scalars<<<1, 1, 0, c->stream>>>(g.d_total, g.d_ngood, g.d_nitems, g.d_err,
+            g.d_plane_support ? g.d_plane_support : reinterpret_cast<const int*>(g.d_err),
+            g.d_plane_support ? g.nplanes : 0, ds);
         STPGPU_CHECK_LAUNCH();
         STPGPU_CUDA_TRY(cudaMemcpyAsync(&scal[i], ds, sizeof(BatchScalars), cudaMemcpyDeviceToHost, c->stream));
         if (!device_ptrs)
-            STPGPU_CUDA_TRY(cudaMemcpyAsync(b.image, dimg[i], (out_f32 ? 4 : 8) * size_t(b.image_size) * b.image_size,
-                cudaMemcpyDeviceToHost, c->stream));
+            STPGPU_CUDA_TRY(cudaMemcpyAsync(b.image, di, ob, cudaMemcpyDeviceToHost, c->stream));
     }
     c->stream = main;
     c->ns = "";
     batch_join(c, main);
-    return nlaunch;
 }
-
 
 template <typename R, int COMP>
 void run_batch(stpgpu_context* c, const stpgpu_snapshot* sn, int nb, int precision, int out_f32, int device_ptrs,
@@ -2066,9 +1559,8 @@ void run_batch(stpgpu_context* c, const stpgpu_snapshot* sn, int nb, int precisi
         c->batch_calls = 0;
     }
     c->batch_calls++;
-    // pinned staging: scalars read back by the device + host scratch for the
-    // by-value gridder parameter block
-    const size_t need = pad256(sizeof(BatchScalars) * nb) + pad256(sizeof(BatchGridParams<R>)) + 4096;
+    // pinned staging: the scalars read back
+    const size_t need = pad256(sizeof(BatchScalars) * nb) + 4096;
     if (c->batch_host_cap < need) {
         if (c->batch_host) {
             for (auto w : c->wstreams)
@@ -2083,7 +1575,6 @@ void run_batch(stpgpu_context* c, const stpgpu_snapshot* sn, int nb, int precisi
         c->batch_host_cap = need;
     }
     BatchScalars* scal = reinterpret_cast<BatchScalars*>(c->batch_host);
-    unsigned char* hparams = reinterpret_cast<unsigned char*>(c->batch_host) + pad256(sizeof(BatchScalars) * nb);
     const bool saved_timing = c->timing;
     c->timing = false;
     struct Restore {
@@ -2098,7 +1589,7 @@ void run_batch(stpgpu_context* c, const stpgpu_snapshot* sn, int nb, int precisi
         }
     } restore { c, c->stream, saved_timing };
     const cudaStream_t main = c->stream;
-    int tuned = 0, glaunch = 0, graph = 0;
+    int graph = 0;
     g_launches = 0;
     if (device_ptrs && c->batch_exec) {
         // replay
@@ -2108,62 +1599,14 @@ void run_batch(stpgpu_context* c, const stpgpu_snapshot* sn, int nb, int precisi
         g_launches = c->batch_launches; // the replay runs the captured kernels
         graph = 1;
     } else {
-        // tile autotuner: time both tile widths for classes not seen before
-        std::vector<std::string> fresh;
-        for (auto& b : B)
-            if (int v; b.s.nplanes > 0 && !c->tune_get(b.cls, v) && std::find(fresh.begin(), fresh.end(), b.cls) == fresh.end())
-                fresh.push_back(b.cls);
-        if (!fresh.empty()) {
-            constexpr int NC = 12;
-            const int layouts[NC] = { 32, 16, 32 | kLayoutPersist, 16 | kLayoutPersist, 32 | kLayoutTaps,
-                16 | kLayoutTaps, 32 | kLayoutPersist | kLayoutTaps, 16 | kLayoutPersist | kLayoutTaps, 32 | kLayoutRecs,
-                16 | kLayoutRecs, 32 | kLayoutPersist | kLayoutRecs, 16 | kLayoutPersist | kLayoutRecs };
-            std::map<std::string, float> t[NC];
-            for (int k = 0; k < 5; k++)
-                if (!c->pev[k])
-                    STPGPU_CUDA_TRY(cudaEventCreate(&c->pev[k]));
-            for (int cand = 0; cand < NC; cand++) {
-                for (auto& b : B) {
-                    int lay = layouts[cand];
-                    c->tune_get(b.cls, lay);
-                    apply_layout(b, lay);
-                }
-                batch_enqueue<R, COMP>(c, B, out_f32, device_ptrs, false, scal, hparams, &t[cand]);
-                STPGPU_CUDA_TRY(cudaStreamSynchronize(main));
-            }
-            static const bool log_tuning = std::getenv("STPGPU_LOG_TUNING") != nullptr;
-            for (auto& cls : fresh) {
-                int best = 0;
-                for (int cand = 1; cand < NC; cand++)
-                    if (t[cand][cls] < t[best][cls])
-                        best = cand;
-                c->tune_set(cls, layouts[best]);
-                if (log_tuning)
-                    std::fprintf(stderr,
-                        "stpgpu gridder tuner: %s  32/16 cols %.3f/%.3f ms, persistent %.3f/%.3f ms, lane-per-tap"
-                        " %.3f/%.3f ms, lane-per-tap persistent %.3f/%.3f ms, staged %.3f/%.3f ms, staged"
-                        " persistent %.3f/%.3f ms -> %d%s%s\n",
-                        cls.c_str(), double(t[0][cls]), double(t[1][cls]), double(t[2][cls]), double(t[3][cls]),
-                        double(t[4][cls]), double(t[5][cls]), double(t[6][cls]), double(t[7][cls]),
-                        double(t[8][cls]), double(t[9][cls]), double(t[10][cls]), double(t[11][cls]),
-                        layouts[best] & 0xff, (layouts[best] & kLayoutPersist) ? " persistent" : "",
-                        (layouts[best] & kLayoutRecs) ? " staged" : ((layouts[best] & kLayoutTaps) ? " lane-per-tap" : ""));
-            }
-            tuned = int(fresh.size());
-        }
-        for (auto& b : B) {
-            int lay = TILE_C_DEFAULT;
-            c->tune_get(b.cls, lay);
-            apply_layout(b, lay);
-        }
         bool capturable = true;
         for (auto& b : B)
             capturable = capturable && !large_support(b.s);
-        if (device_ptrs && capturable && c->batch_calls >= 2 && tuned == 0) {
+        if (device_ptrs && capturable && c->batch_calls >= 2) {
             // capture the batch (buffers, plans and tables exist from the previous call)
             STPGPU_CUDA_TRY(cudaStreamBeginCapture(main, cudaStreamCaptureModeThreadLocal));
             try {
-                glaunch = batch_enqueue<R, COMP>(c, B, out_f32, device_ptrs, true, scal, hparams, nullptr);
+                batch_enqueue<R, COMP>(c, B, out_f32, device_ptrs, scal);
             } catch (...) {
                 cudaGraph_t g = nullptr;
                 cudaStreamEndCapture(main, &g);
@@ -2183,7 +1626,7 @@ void run_batch(stpgpu_context* c, const stpgpu_snapshot* sn, int nb, int precisi
             graph = 1;
         } else {
             STPGPU_CUDA_TRY(cudaEventRecord(c->ev0, main));
-            glaunch = batch_enqueue<R, COMP>(c, B, out_f32, device_ptrs, false, scal, hparams, nullptr);
+            batch_enqueue<R, COMP>(c, B, out_f32, device_ptrs, scal);
             STPGPU_CUDA_TRY(cudaEventRecord(c->ev1, main));
         }
     }
@@ -2206,7 +1649,7 @@ void run_batch(stpgpu_context* c, const stpgpu_snapshot* sn, int nb, int precisi
         c->batch_calls = 0;
         c->batch_sig.clear();
         STPGPU_CUDA_TRY(cudaEventRecord(c->ev0, main));
-        glaunch = batch_enqueue<R, COMP>(c, B, out_f32, device_ptrs, false, scal, hparams, nullptr);
+        batch_enqueue<R, COMP>(c, B, out_f32, device_ptrs, scal);
         STPGPU_CUDA_TRY(cudaEventRecord(c->ev1, main));
         STPGPU_CUDA_TRY(cudaStreamSynchronize(main));
         graph = 0;
@@ -2234,8 +1677,8 @@ void run_batch(stpgpu_context* c, const stpgpu_snapshot* sn, int nb, int precisi
         std::memset(bi, 0, sizeof(*bi));
         bi->device_ms = ms;
         bi->graph = graph;
-        bi->gridder_launches = glaunch;
-        bi->tuned_classes = tuned;
+        bi->gridder_launches = nb;
+        bi->tuned_classes = 0;
         bi->n_launches = g_launches;
     }
 }
@@ -2951,9 +2394,6 @@ stpgpu_status stpgpu_destroy(stpgpu_context* c)
         cudaEventDestroy(e);
     if (c->fork_ev)
         cudaEventDestroy(c->fork_ev);
-    for (auto e : c->tev)
-        if (e)
-            cudaEventDestroy(e);
     if (c->ev0)
         cudaEventDestroy(c->ev0);
     if (c->ev1)
@@ -3276,9 +2716,11 @@ int64_t request_bytes(const ImagerSetup& s, int image_size, int64_t n, int vis_c
     const int64_t N = s.N, rows = N / 2 + 1;
     const int conv = s.nplanes > 0 ? s.max_support : s.support;
     int64_t b = n * ((vis_c64 ? 8 : 16) + 8 + 24) + n * (rb == 8 ? 48 : 32); // items: 48 / 32 B records
-    const int64_t per_dim = ceil_div(2 * conv, 16) + 2;
-    b += std::max<int64_t>(n, 1) * 2 * per_dim * per_dim * 4; // tile-list capacity
-    b += std::max<int64_t>(n, 1) * 2 * kRankSlots * 4;         // list slots kept by the count pass
+    b += int64_t(entry_capacity(s.N, 2 * conv + 1, n)) * (rb == 8 ? 32 : 16); // entry records
+    b += std::max<int64_t>(n, 1) * kEntrySlots * 4;                           // their places in the bins
+    b += 12 * (rows / kBlk + 40) * (N / kBlk + 40);                           // bins
+    if (s.kernel_exact)
+        b += n * (2 * 8 + 2 * 8 * (2 * conv + 1)); // fractional positions, 1-D kernels
     if (s.nplanes > 0) {
         b += n * (rb == 8 ? 48 : 32); // items in |w| order
         const int64_t os = std::max(1, (s.os >> 1) << 1), cs = (os / 2) * 2 + 1, K = 2 * conv + 1;
@@ -3456,8 +2898,6 @@ stpgpu_status stpgpu_server_create(const stpgpu_server_pars* pars, stpgpu_server
             delete sv;
             return s;
         }
-        if (!sv->slots.empty())
-            c->tunes = sv->slots[0]->tunes; // a size class is tuned once for all slots
         sv->slots.push_back(c);
     }
     for (int k = 0; k < pars->slots; k++)

@@ -310,7 +310,7 @@ __global__ void k_aproj_rotate(const double2* src, int64_t src_stride, double2* 
 // cs^2 K_q^2.
 template <typename R>
 __global__ void __launch_bounds__(256) k_aproj_expand(const double2* conv_base, int arr, const int* support, int cs,
-    int os, typename Cplx<R>::T* out, uint32_t* off)
+    int os, typename Cplx<R>::T* out, uint32_t* off, unsigned int* max_support)
 {
     const int pt = blockIdx.x;
     const int pair = blockIdx.y;
@@ -320,9 +320,11 @@ __global__ void __launch_bounds__(256) k_aproj_expand(const double2* conv_base, 
         const uint32_t Kq = uint32_t(2 * support[q] + 1);
         base += uint32_t(cs) * uint32_t(cs) * Kq * Kq;
     }
-    if (pair == 0 && threadIdx.x == 0)
-        off[pt] = base;
     const int S = support[pt];
+    if (pair == 0 && threadIdx.x == 0) {
+        off[pt] = base;
+        atomicMax(max_support, unsigned(S));
+    }
     const int K = 2 * S + 1;
     const double2* conv = conv_base + int64_t(pt) * arr * arr;
     auto at = [&](int i, int j) {
@@ -347,7 +349,7 @@ __global__ void __launch_bounds__(256) k_aproj_expand(const double2* conv_base, 
     const double inv = 1 / red[0];
     typename Cplx<R>::T* dst = out + base + uint32_t(pair) * uint32_t(K * K);
     for (int t = threadIdx.x; t < K * K; t += blockDim.x) {
-        const int i = t / K, j = t % K;
+        const int i = t % K, j = t / K; // column j, row i
         const double2 v = at(i, j);
         typename Cplx<R>::T o;
         o.x = R(v.x * inv);

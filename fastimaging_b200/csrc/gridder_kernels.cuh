@@ -580,4 +580,144 @@ struct SepCore {
     }
 };
 
+// ---------------------------------------------------------------- W-projection
+
+template <typename R, typename T>
+struct WprojParams {
+    int N, rows, pad, brn;
+    const uint32_t* off;
+    const GridRec<R>* recs;
+    const R* wts;                     // per record (beam)
+    const typename Cplx<T>::T* wk;    // expanded kernels: column j, row i at [koff + j K + i]
+    const unsigned int* max_support; // largest support of the call's planes
+    void* grid;
+    void* beam;
+};
+
+// W-kernels: each lane keeps two cells of the block (row lane % 8, columns
+// lane / 8 and that + 4) in registers and adds the entries one after the
+// other: eight lanes read eight consecutive kernel values (rows of one
+// column), so a warp's load touches the footprint's columns once each.  The
+// kernel values of the next entries are in flight while one is added.  Sums
+// (type A) are in double for FP64 and compensated FP32.
+template <typename R, typename G, typename T, typename ACC, bool BEAM>
+struct WprojCore {
+    using Params = WprojParams<R, T>;
+    using A = ACC;
+    static constexpr int NACC = BEAM ? 8 : 4;
+    struct Raw {
+        GridRec<R> r;
+        R w;
+    };
+    struct alignas(16) StagedB {
+        A vr, vi;
+        int row0, col0;
+        uint32_t koff;
+        uint32_t kc; // K, and the sign bit when the kernel is conjugated
+        A w, unused;
+    };
+    struct alignas(16) StagedP {
+        A vr, vi;
+        int row0, col0;
+        uint32_t koff;
+        uint32_t kc;
+    };
+    using Staged = std::conditional_t<BEAM, StagedB, StagedP>;
+
+    static __device__ __forceinline__ int bins(const Params& p) { return int((2u * p.max_support[0] + 7u) / 8u) + 1; }
+    static __device__ __forceinline__ Raw fetch(const Params& p, uint32_t i)
+    {
+        Raw w {};
+        w.r = p.recs[i];
+        if (BEAM)
+            w.w = p.wts[i];
+        return w;
+    }
+    static __device__ __forceinline__ bool decode(const Params&, const Raw& w, int r0, int c0, Staged& s)
+    {
+        const uint32_t g = w.r.geom;
+        s.row0 = int((g - uint32_t(r0)) << 22) >> 22;
+        s.col0 = int((g - (uint32_t(c0) << 10)) << 12) >> 22;
+        s.vr = A(w.r.vr);
+        s.vi = A(w.r.vi);
+        const int K = int(2u * ((g >> 20) & 127u) + 1u);
+        s.koff = w.r.koff;
+        s.kc = uint32_t(K) | ((g << 4) & 0x80000000u);
+        if constexpr (BEAM)
+            s.w = A(w.w);
+        return s.row0 + K > 0 && s.col0 + K > 0 && s.row0 < kBlk && s.col0 < kBlk;
+    }
+    static __device__ __forceinline__ void fill_up(const Params&, Staged*, int) {}
+    static __device__ __forceinline__ float flip(float x, uint32_t sign)
+    {
+        return __uint_as_float(__float_as_uint(x) ^ sign);
+    }
+    static __device__ __forceinline__ double flip(double x, uint32_t sign)
+    {
+        return __hiloint2double(int(uint32_t(__double2hiint(x)) ^ sign), __double2loint(x));
+    }
+    static __device__ __forceinline__ void accumulate(const Params& p, const Staged* st, int m, A (&acc)[NACC])
+    {
+        using C2 = typename Cplx<T>::T;
+        const int lane = threadIdx.x & 31;
+        const int r = lane & 7, c = lane >> 3;
+        const C2* __restrict__ wk = p.wk;
+#pragma unroll 4
+        for (int e = 0; e < m; e++) {
+            const Staged s = st[e];
+            const int K = int(s.kc & 0xffffu);
+            const uint32_t sign = s.kc & 0x80000000u;
+            const int dr = r - s.row0, dc = c - s.col0;
+            const bool in = unsigned(dr) < unsigned(K);
+            const bool in0 = in && unsigned(dc) < unsigned(K), in1 = in && unsigned(dc + 4) < unsigned(K);
+            const uint32_t i = s.koff + uint32_t(dc * K + dr);
+            C2 v[2];
+            v[0].x = v[0].y = v[1].x = v[1].y = T(0);
+            if (in0)
+                v[0] = __ldg(wk + i);
+            if (in1)
+                v[1] = __ldg(wk + (i + uint32_t(4 * K)));
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                if (k ? in1 : in0) {
+                    const A kr = A(v[k].x), ki = A(flip(v[k].y, sign));
+                    acc[2 * k] = fma(s.vr, kr, acc[2 * k]);
+                    acc[2 * k] = fma(-s.vi, ki, acc[2 * k]);
+                    acc[2 * k + 1] = fma(s.vr, ki, acc[2 * k + 1]);
+                    acc[2 * k + 1] = fma(s.vi, kr, acc[2 * k + 1]);
+                    if constexpr (BEAM) {
+                        acc[4 + 2 * k] = fma(s.w, kr, acc[4 + 2 * k]);
+                        acc[5 + 2 * k] = fma(s.w, ki, acc[5 + 2 * k]);
+                    }
+                }
+            }
+        }
+    }
+    static __device__ __forceinline__ void store(const Params& p, int r0, int c0, const A (&acc)[NACC])
+    {
+        using G2 = typename Cplx<G>::T;
+        const int lane = threadIdx.x & 31;
+        const int r = r0 + (lane & 7);
+        if (r >= p.rows)
+            return;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int c = c0 + (lane >> 3) + 4 * k;
+            if (c >= p.N)
+                continue;
+            const size_t i = size_t(c) * size_t(p.rows) + size_t(r);
+            G2 v;
+            v.x = G(acc[2 * k]);
+            v.y = G(acc[2 * k + 1]);
+            static_cast<G2*>(p.grid)[i] = v;
+            if constexpr (BEAM) {
+                G2 w;
+                w.x = G(acc[4 + 2 * k]);
+                w.y = G(acc[5 + 2 * k]);
+                static_cast<G2*>(p.beam)[i] = w;
+            }
+        }
+    }
+};
+
 } // namespace stpgpu

@@ -4,13 +4,7 @@
 //   k_prepass      uvw -> pixel scaling, half-plane conversion, rint split,
 //                  bounds check, uv shift, oversampled index  (gridder.h:369-504)
 //   [W-proj]       |w| sort (CUB), plane boundaries/averages, FP64 W-kernels
-//   k_count_tiles  footprint -> uv tiles it overlaps (counting pass)
-//   k_scan_*       tile offsets
-//   k_fill_tiles   tile -> item lists
-//   k_grid_tiles   one CTA per 32x32 tile of the half-plane grid: all items
-//                  whose footprint touches the tile accumulate in shared
-//                  memory, then the tile is written once with coalesced
-//                  stores (no memset, no global atomics)          (gridder.h:596-994)
+//   k_bin_*, k_grid_blocks  binning and gridding (gridder_kernels.cuh)
 //   cuFFT Z2D/C2R  (fft.cpp:45-135)
 //   k_normalise    crop + 1/sum + gcf division                    (imager.h:97-150)
 #pragma once
@@ -19,18 +13,13 @@
 
 namespace stpgpu {
 
-constexpr int TILE_R = 32; // tile rows (v, the fast grid axis)
-constexpr int TILE_C_DEFAULT = 32; // tile columns (u); 16-column tiles are the other tuned shape
 constexpr int GRID_THREADS = 256;
-
-enum KMode { KM_SEP = 0, KM_EXACT = 1, KM_WPROJ = 2 };
 
 // Per-visibility record written by the prepass.  flags: bit0 conj(kernel)
 // for the original item (w < 0), bit1 conj(kernel) for the mirrored item
 // (-w < 0).  The visibility is stored conjugated when the half-plane
 // conversion flipped it.  16-byte aligned (32 B single, 48 B double
-// precision): a record never straddles a 32-byte sector more than it must,
-// and the gridder's random fetch of a record is two or three 16-byte loads.
+// precision): two or three 16-byte loads.
 template <typename R>
 struct alignas(16) Item {
     R vr, vi, w;
@@ -298,187 +287,11 @@ __global__ void k_zero_ranges(ZeroRanges z)
                 z.p[r][i] = 0;
 }
 
-// ---------------------------------------------------------------- footprint segments
-
-// Footprint index mapping (gridder.h:645-667 columns/rows, :970-983 exact).
-// Column tap j of a kernel whose left edge is cb lands in grid column
-// cb + j wrapped once into [0, N).  Row tap i lands in cb-style wrapped row
-// rb + i, except that negative rows are skipped by the oversampled gridder
-// and wrapped by the exact one; rows >= `rows` (half plane) are dropped.
-// Returns -1 when the tap is not gridded.
-__device__ __forceinline__ int map_col(int raw, int N)
-{
-    return raw < 0 ? raw + N : (raw >= N ? raw - N : raw);
-}
-__device__ __forceinline__ int map_row(int raw, int N, int rows, bool wrap_neg)
-{
-    if (raw < 0) {
-        if (!wrap_neg)
-            return -1;
-        raw += N;
-    } else if (raw >= N) {
-        raw -= N;
-    }
-    return raw < rows ? raw : -1;
-}
-
-constexpr int kRankSlots = 4; // tiles per (item, mirror) whose list slots the count pass keeps
-
-// One (entry, tile) pair of the binning, decoded for the staged gridder
-// (grid_tile_recs): the entry's footprint clipped to the tile, the weighted
-// visibility and the kernel-table offset of the window's first tap.  The
-// fill pass writes these records contiguously in tile order, so a tile's
-// entries are one contiguous byte range that the gridder copies into shared
-// memory with bulk (TMA) copies.  16 B in single precision, 32 B in double.
-//   geom: row0 (5 bits, local row of the window's first tap), col0 (5 bits),
-//         nrows (6 bits, 1..32), ncols (6 bits), conj (1 bit, W-kernel
-//         conjugated), K (8 bits, kernel width; the row stride of W-kernels)
-//   koff: W-projection: index of tap (ilo, jlo) in the expanded kernel
-//         tables; separable: (cpy*K + ilo) << 16 | (cpx*K + jlo)
-template <typename R>
-struct alignas(16) TapRec {
-    R vr, vi;
-    uint32_t koff;
-    uint32_t geom;
-};
-static_assert(sizeof(TapRec<float>) == 16 && sizeof(TapRec<double>) == 32, "tile record sizes");
-
-__host__ __device__ __forceinline__ uint32_t rec_geom(int row0, int col0, int nrows, int ncols, int conj, int K)
-{
-    return uint32_t(row0) | (uint32_t(col0) << 5) | (uint32_t(nrows) << 10) | (uint32_t(ncols) << 16)
-        | (uint32_t(conj & 1) << 22) | (uint32_t(K) << 23);
-}
-
-struct BinParams {
-    int N, image_rows, tiles_r, tiles_c;
-    int tile_c;              // tile width in grid columns (TILE_R rows per tile)
-    int support;             // non-W-proj support
-    const int* plane_support; // W-proj truncated support per plane (nullable)
-    const uint16_t* plane16;  // W-proj without the |w| sort: plane of each item (input order), else null
-    const uint8_t* ts_of;     // A-projection: time step per visibility (nullable)
-    int ntimesteps;           // planes are indexed plane * ntimesteps + step
-    int exact;               // rows wrap negative (exact gridder)
-    int64_t n;
-    uint32_t* tile_count;
-    const uint32_t* tile_off;
-    uint32_t* tile_cursor;
-    uint32_t* ranks;          // nullable: [kRankSlots][2][n] list slots taken by the count pass
-    uint32_t* rank_overflow;  // set when some (item, mirror) touched more than kRankSlots tiles
-    uint32_t* list;
-    uint64_t list_capacity;
-    unsigned int* err;
-};
-
 template <typename R>
 __device__ __forceinline__ void item_centre(const Item<R>& it, int mir, int N, int& cx, int& cy)
 {
     cx = mir ? N - it.gcx : it.gcx;
     cy = mir ? N - it.gcy : it.gcy;
-}
-
-// Tiles overlapped by one item: calls f(tile) once per distinct tile.  The
-// footprint's raw rows [rb, rb+K) and columns [cb, cb+K) are split into the
-// segments that map_row / map_col send to distinct grid ranges (in place,
-// wrapped from >= N, and for the exact gridder wrapped from < 0; rows at or
-// beyond the half plane dropped); each segment becomes a range of tile
-// indices, overlapping ranges are merged, and the tiles of the row ranges x
-// column ranges are visited once each.
-struct TileRanges {
-    int lo[3], hi[3];
-    int n;
-    __device__ __forceinline__ void add(int l, int h)
-    {
-        if (l > h)
-            return;
-        for (int k = 0; k < n; k++) {
-            if (l <= hi[k] + 1 && h >= lo[k] - 1) { // overlapping or adjacent: merge
-                lo[k] = min(lo[k], l);
-                hi[k] = max(hi[k], h);
-                return;
-            }
-        }
-        lo[n] = l;
-        hi[n] = h;
-        n++;
-    }
-    // merge ranges that a later add made overlap
-    __device__ __forceinline__ void merge()
-    {
-        for (int a = 0; a < n; a++)
-            for (int b = a + 1; b < n; b++)
-                if (lo[b] <= hi[a] + 1 && hi[b] >= lo[a] - 1) {
-                    lo[a] = min(lo[a], lo[b]);
-                    hi[a] = max(hi[a], hi[b]);
-                    lo[b] = lo[n - 1];
-                    hi[b] = hi[n - 1];
-                    n--;
-                    b = a; // restart the scan of a
-                }
-    }
-};
-
-template <typename R, typename F>
-__device__ __forceinline__ void for_item_tiles(const Item<R>& it, int mir, int S, const BinParams& p, F f)
-{
-    const int K = 2 * S + 1;
-    int cx, cy;
-    item_centre(it, mir, p.N, cx, cy);
-    const int N = p.N, rows_max = p.image_rows - 1;
-    const int a = cy - S, b = cy - S + K - 1; // raw rows
-    {
-        // common case: the footprint wraps on neither axis, so it covers one
-        // range of tile rows and one of tile columns (tile sizes are powers
-        // of two; every index here is non-negative)
-        const int c = cx - S, d = cx - S + K - 1;
-        if (a >= 0 && b < N && c >= 0 && d < N) {
-            const int h = min(b, rows_max);
-            if (a > h)
-                return;
-            const int cshift = p.tile_c == 32 ? 5 : (p.tile_c == 16 ? 4 : 3);
-            for (int t_r = a / TILE_R; t_r <= h / TILE_R; t_r++)
-                for (int t_c = c >> cshift; t_c <= (d >> cshift); t_c++)
-                    f(uint32_t(t_c) * uint32_t(p.tiles_r) + uint32_t(t_r));
-            return;
-        }
-    }
-    TileRanges tr;
-    tr.n = 0;
-    {
-        const int l = max(a, 0), h = min(min(b, N - 1), rows_max);
-        if (l <= h)
-            tr.add(l / TILE_R, h / TILE_R);
-    }
-    if (b >= N) {
-        const int l = max(a, N) - N, h = min(b - N, rows_max);
-        if (l <= h)
-            tr.add(l / TILE_R, h / TILE_R);
-    }
-    if (p.exact && a < 0) {
-        const int l = a + N, h = min(min(b, -1) + N, rows_max);
-        if (l <= h)
-            tr.add(l / TILE_R, h / TILE_R);
-    }
-    if (tr.n == 0)
-        return;
-    const int c = cx - S, d = cx - S + K - 1; // raw columns
-    TileRanges tc;
-    tc.n = 0;
-    {
-        const int l = max(c, 0), h = min(d, N - 1);
-        if (l <= h)
-            tc.add(l / p.tile_c, h / p.tile_c);
-    }
-    if (c < 0)
-        tc.add((c + N) / p.tile_c, (min(d, -1) + N) / p.tile_c);
-    if (d >= N)
-        tc.add((max(c, N) - N) / p.tile_c, (d - N) / p.tile_c);
-    tr.merge();
-    tc.merge();
-    for (int r = 0; r < tr.n; r++)
-        for (int t_r = tr.lo[r]; t_r <= tr.hi[r]; t_r++)
-            for (int q = 0; q < tc.n; q++)
-                for (int t_c = tc.lo[q]; t_c <= tc.hi[q]; t_c++)
-                    f(uint32_t(t_c) * uint32_t(p.tiles_r) + uint32_t(t_r));
 }
 
 // W-plane of sorted position k: the last plane whose first position <= k.
@@ -493,88 +306,6 @@ __device__ __forceinline__ int plane_of(const int64_t* first, int P, int64_t k)
             hi = mid - 1;
     }
     return lo;
-}
-
-// With W-projection (`order` = the |w| permutation, `first` = plane starts)
-// `items` is already permuted into |w| order (item k is sorted position k);
-// each item takes the plane of its position, which the fill pass records in
-// the item for the gridder (order[k] is the item's input index, used for
-// per-visibility inputs such as the A-projection time step).
-template <typename R>
-__global__ void k_count_tiles(BinParams p, const Item<R>* items, const uint32_t* order, const int64_t* first, int P)
-{
-    const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k >= p.n)
-        return;
-    const Item<R> it = items[k];
-    if (!it.good)
-        return;
-    int S = p.support;
-    if (p.plane16) {
-        S = p.plane_support[p.plane16[k]];
-    } else if (order) {
-        int plane = plane_of(first, P, k);
-        if (p.ts_of)
-            plane = plane * p.ntimesteps + p.ts_of[order[k]];
-        S = p.plane_support[plane];
-    }
-    for (int mir = 0; mir < int(it.good); mir++) {
-        // the count's atomic returns the entry's slot in the tile list; up to
-        // kRankSlots of them per (item, mirror) are kept for the fill pass
-        int q = 0;
-        for_item_tiles(it, mir, S, p, [&](uint32_t t) {
-            const uint32_t r = atomicAdd(&p.tile_count[t], 1u);
-            if (p.ranks) {
-                if (q < kRankSlots)
-                    p.ranks[size_t(q * 2 + mir) * size_t(p.n) + size_t(k)] = r; // slot-major: coalesced
-                else
-                    *p.rank_overflow = 1u;
-            }
-            q++;
-        });
-    }
-}
-
-// Lists are filled in |w| order for W-projection, so that a warp's items
-// mostly share one plane.
-template <typename R>
-__global__ void k_fill_tiles(BinParams p, Item<R>* items, const uint32_t* order, const int64_t* first, int P)
-{
-    const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k >= p.n)
-        return;
-    const int64_t i = k;
-    const Item<R> it = items[k];
-    if (!it.good)
-        return;
-    int S = p.support;
-    if (p.plane16) {
-        const int plane = p.plane16[k];
-        S = p.plane_support[plane];
-        items[k].plane = uint16_t(plane);
-    } else if (order) {
-        int plane = plane_of(first, P, k);
-        if (p.ts_of)
-            plane = plane * p.ntimesteps + p.ts_of[order[k]];
-        S = p.plane_support[plane];
-        items[k].plane = uint16_t(plane);
-    }
-    // slots from the count pass when every (item, mirror) kept its slots
-    // (no footprint with more than kRankSlots tiles), else from cursors
-    const bool ranked = p.ranks && *p.rank_overflow == 0u;
-    for (int mir = 0; mir < int(it.good); mir++) {
-        int q = 0;
-        for_item_tiles(it, mir, S, p, [&](uint32_t t) {
-            const uint32_t slot = ranked ? p.ranks[size_t(q * 2 + mir) * size_t(p.n) + size_t(k)]
-                                         : atomicAdd(&p.tile_cursor[t], 1u);
-            q++;
-            const uint64_t pos = uint64_t(p.tile_off[t]) + slot;
-            if (pos < p.list_capacity)
-                p.list[pos] = uint32_t(i) * 2u + uint32_t(mir);
-            else
-                atomicOr(p.err, 1u);
-        });
-    }
 }
 
 // Exclusive scan of n counts into off[0..n] (single block of 1024 threads,
@@ -644,98 +375,6 @@ __global__ void __launch_bounds__(1024) k_scan_rows(const uint32_t* cnt, uint32_
         tot[blockIdx.x] = t;
 }
 
-// ---------------------------------------------------------------- accumulators
-
-// Shared-memory cell accumulators.  Each cell is owned by one warp and
-// updated with plain read-modify-write (no atomics), so the two-sum
-// compensation of FP32C is exact: s + c carries the full sum.
-template <typename R, int COMP>
-struct Acc;
-template <>
-struct __align__(16) Acc<double, 0> {
-    double2 s;
-};
-template <>
-struct __align__(8) Acc<float, 0> {
-    float2 s;
-};
-template <>
-struct __align__(16) Acc<float, 1> {
-    float2 s, c;
-};
-
-__device__ __forceinline__ void acc_rmw(Acc<double, 0>* a, double re, double im)
-{
-    double2 v = a->s;
-    v.x += re;
-    v.y += im;
-    a->s = v;
-}
-__device__ __forceinline__ void acc_rmw(Acc<float, 0>* a, float re, float im)
-{
-    float2 v = a->s;
-    v.x += re;
-    v.y += im;
-    a->s = v;
-}
-// Packed single-precision pairs (sm_100 f32x2: one instruction rounds both
-// halves, each as its scalar form would).
-__device__ __forceinline__ unsigned long long f2_pack(float x, float y)
-{
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ float2 f2_unpack(unsigned long long r)
-{
-    float2 v;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(r));
-    return v;
-}
-__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b)
-{
-    unsigned long long r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ unsigned long long f2_sub(unsigned long long a, unsigned long long b)
-{
-    unsigned long long r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-// FP32C update: t = s + x and Knuth's TwoSum error term
-// e = (s - (t - bb)) + (x - bb), bb = t - s, added to c, with explicit
-// rounding (no contraction), the real and imaginary parts side by side in
-// seven packed adds.  TwoSum is exact whatever the magnitudes: Dekker's
-// cheaper Fast2Sum needs |s| >= |x|, which fails throughout a cell whose
-// running sum cancels, and there it loses about one rounding of each term
-// (enough to move a 256^2 PSWF image by 3e-5 of its peak with the order of
-// the updates).
-__device__ __forceinline__ void acc_rmw(Acc<float, 1>* a, float re, float im)
-{
-    const Acc<float, 1> v = *a;
-    const unsigned long long s = f2_pack(v.s.x, v.s.y), x = f2_pack(re, im);
-    const unsigned long long t = f2_add(s, x);
-    const unsigned long long bb = f2_sub(t, s);
-    const unsigned long long e = f2_add(f2_sub(s, f2_sub(t, bb)), f2_sub(x, bb));
-    Acc<float, 1> w;
-    w.s = f2_unpack(t);
-    w.c = f2_unpack(f2_add(f2_pack(v.c.x, v.c.y), e));
-    *a = w;
-}
-template <typename R, int COMP>
-__device__ __forceinline__ void acc_zero(Acc<R, COMP>* a)
-{
-    *a = Acc<R, COMP> {};
-}
-__device__ __forceinline__ double2 acc_value(const Acc<double, 0>& a) { return a.s; }
-__device__ __forceinline__ float2 acc_value(const Acc<float, 0>& a) { return a.s; }
-__device__ __forceinline__ float2 acc_value(const Acc<float, 1>& a)
-{
-    return make_float2(__fadd_rn(a.s.x, a.c.x), __fadd_rn(a.s.y, a.c.y));
-}
-
 template <typename R>
 struct Cplx;
 template <>
@@ -746,1097 +385,6 @@ template <>
 struct Cplx<float> {
     using T = float2;
 };
-
-// Store of one finished cell: the accumulator's value in the grid's
-// precision, or (compensated FP32 into a wide grid) sum + error in double.
-template <typename R, int COMP>
-__device__ __forceinline__ void cell_store(typename Cplx<R>::T* g, size_t i, const Acc<R, COMP>& a, int wide)
-{
-    if constexpr (COMP == 1) {
-        if (wide) {
-            reinterpret_cast<double2*>(g)[i]
-                = make_double2(double(a.s.x) + double(a.c.x), double(a.s.y) + double(a.c.y));
-            return;
-        }
-    }
-    g[i] = acc_value(a);
-}
-
-// ---------------------------------------------------------------- gridder
-
-template <typename R>
-struct GridParams {
-    int N, image_rows, tiles_r;
-    int support, os, cs; // cs = cache size per dimension = (os/2)*2+1
-    int exact_wrap;      // exact gridder row wrap
-    const Item<R>* items;
-    const uint32_t* tile_off;
-    const uint32_t* list;
-    // KM_SEP: 1-D kernel table [cs][K] (R)
-    const R* k1d;
-    // KM_EXACT: functor + per-visibility fractions
-    int kf;
-    double trunc;
-    const double* frac;
-    int64_t n;
-    // KM_WPROJ: per plane the W-kernel quadrant conv[p][l][k] (stride lh,
-    // |offsets| index it) and 1/sum(Re) per oversampled offset inv[p][y][x]:
-    // the cached kernel of aw_projection.cpp:415-448 is conv * inv.
-    const typename Cplx<R>::T* wconv;
-    const R* winv;
-    int lh;
-    const int* plane_support;
-    // KM_WPROJ: per plane and oversampled offset pair (cpy, cpx) the K x K
-    // cached kernel (conv * inv, tap i*K + j) at wk + wk_off[plane] + (cpy*cs + cpx)*K*K
-    const typename Cplx<R>::T* wk;
-    const uint32_t* wk_off;
-    // staged form (grid_tile_recs): the decoded entries in tile order, and
-    // how many the buffer holds
-    const TapRec<R>* recs;
-    uint64_t rec_cap;
-    unsigned int* err; // error flags of the call (staged form: bits 8 and 16)
-    typename Cplx<R>::T* grid; // image_rows x N column-major
-    typename Cplx<R>::T* beam; // nullable
-    // compensated FP32 only: grid and beam hold double2 cells (sum + error
-    // term carried into double) for a double-precision c2r transform
-    int wide;
-};
-
-// One warp per 32x32 tile of the (half-plane) grid.  Lanes take 32 items of
-// the tile's list at a time and walk their K x K footprints in lockstep, so
-// at every step distinct lanes touch distinct cells unless two items share a
-// kernel corner; such items are deferred to a later round (match_any).  The
-// tile is zeroed in shared memory, accumulated with plain read-modify-write,
-// and stored once with coalesced 512-byte column writes: no memset of the
-// grid, no global or shared atomics, and every cell of the grid is written
-// exactly once.  (Gridding semantics: gridder.h:596-994.)
-// Kernel value of tap (i, j) of the lane's item, times the visibility weight.
-template <typename R, int KMODE>
-struct TapCtx {
-    int K, S, cpx, cpy, os, lh;
-    R wt, winv;
-    bool conj_k;
-    const typename Cplx<R>::T* wconv;
-    double fx, fy, ksum;
-};
-
-template <typename R, int KMODE>
-__device__ __forceinline__ void tap_value(const GridParams<R>& p, const R* tab, const TapCtx<R, KMODE>& t, int i, int j,
-    R& kr, R& ki)
-{
-    if (KMODE == KM_SEP) {
-        kr = tab[t.cpy * t.K + i] * tab[t.cpx * t.K + j];
-        ki = R(0);
-    } else if (KMODE == KM_EXACT) {
-        // make_kernel_array (conv_func.h:279-303): outer product / accu
-        const double y = kernel_value(p.kf, p.trunc, (double(i) - t.S) - t.fy);
-        const double x = kernel_value(p.kf, p.trunc, (double(j) - t.S) - t.fx);
-        kr = R((y * x) / t.ksum);
-        ki = R(0);
-    } else {
-        const typename Cplx<R>::T cv = t.wconv[i * t.K + j];
-        kr = cv.x;
-        ki = t.conj_k ? -cv.y : cv.y;
-    }
-}
-
-template <typename R, int COMP, int KMODE, bool BEAM, int TILE_C>
-__device__ __forceinline__ void grid_tile(const GridParams<R>& p, int tile, unsigned char* smem_raw)
-{
-    using A = Acc<R, COMP>;
-    A* acc = reinterpret_cast<A*>(smem_raw);
-    A* bacc = acc + (BEAM ? TILE_R * TILE_C : 0);
-    R* tab = reinterpret_cast<R*>(acc + (BEAM ? 2 : 1) * TILE_R * TILE_C);
-    const int lane = threadIdx.x;
-    // hot scalars in registers (the batch kernel reads p from parameter
-    // space with a run-time index, which costs a load per use)
-    const int gN = p.N, grows = p.image_rows, gos = p.os, glh = p.lh;
-    const int tr = tile % p.tiles_r, tc = tile / p.tiles_r;
-    const int r0 = tr * TILE_R, c0 = tc * TILE_C;
-    const bool wrap_neg = p.exact_wrap != 0;
-
-    for (int t = lane; t < TILE_R * TILE_C; t += 32) {
-        acc_zero(&acc[t]);
-        if (BEAM)
-            acc_zero(&bacc[t]);
-    }
-    if (KMODE == KM_SEP) {
-        const int K = 2 * p.support + 1;
-        for (int t = lane; t < p.cs * K; t += 32)
-            tab[t] = p.k1d[t];
-    }
-    __syncwarp();
-
-    const uint32_t beg = p.tile_off[tile], end = p.tile_off[tile + 1];
-    for (uint32_t base = beg; base < end; base += 32) {
-        const uint32_t e = base + lane;
-        const bool active = e < end;
-        TapCtx<R, KMODE> t;
-        t.K = 0;
-        t.S = 0;
-        t.cpx = t.cpy = 0;
-        t.os = gos;
-        t.lh = glh;
-        t.wt = R(0);
-        t.winv = R(1);
-        t.conj_k = false;
-        t.wconv = nullptr;
-        t.fx = t.fy = 0.0;
-        t.ksum = 1.0;
-        R vr = R(0), vim = R(0);
-        int rb = 0, cb = 0;
-        int cbase = 0, jlo = 0, jhi = 0;
-        bool cwrap = false;
-        unsigned long long key = ~0ull;
-        if (active) {
-            const uint32_t code = p.list[e];
-            const uint32_t vi = code >> 1;
-            const int mir = int(code & 1u);
-            const Item<R> it = p.items[vi];
-            int cx, cy;
-            item_centre(it, mir, gN, cx, cy);
-            t.S = (KMODE == KM_WPROJ) ? p.plane_support[it.plane] : p.support;
-            t.K = 2 * t.S + 1;
-            t.cpx = it.cpx;
-            t.cpy = it.cpy;
-            if (mir && gos > 1) {
-                t.cpx = gos - t.cpx;
-                t.cpy = gos - t.cpy;
-            }
-            vr = it.vr;
-            vim = mir ? -it.vi : it.vi;
-            t.wt = it.w;
-            rb = cy - t.S;
-            cb = cx - t.S;
-            // column window of the footprint inside this tile; only footprints
-            // crossing the grid edge need the per-tap wrap
-            cwrap = cb < 0 || cb + t.K > gN;
-            cbase = cb - c0;
-            jlo = cwrap ? 0 : max(0, -cbase);
-            jhi = cwrap ? t.K : min(t.K, TILE_C - cbase);
-            const int krow = ((rb % gN) + gN) % gN, kcol = ((cb % gN) + gN) % gN;
-            key = (unsigned long long)krow * (unsigned long long)gN + (unsigned long long)kcol;
-            if (KMODE == KM_WPROJ) {
-                t.conj_k = (it.flags >> (mir ? 1 : 0)) & 1u;
-                t.wconv = p.wk + p.wk_off[it.plane] + uint32_t((t.cpy * p.cs + t.cpx) * t.K * t.K);
-            }
-            if (KMODE == KM_EXACT) {
-                t.fx = p.frac[vi];
-                t.fy = p.frac[p.n + vi];
-                if (mir) {
-                    t.fx *= -1;
-                    t.fy *= -1;
-                }
-                // arma::accu of the column-major outer product (two accumulators)
-                double a1 = 0.0, a2 = 0.0;
-                int lin = 0;
-                for (int c = 0; c < t.K; c++) {
-                    const double xc = kernel_value(p.kf, p.trunc, (double(c) - t.S) - t.fx);
-                    for (int r = 0; r < t.K; r++, lin++) {
-                        const double v = kernel_value(p.kf, p.trunc, (double(r) - t.S) - t.fy) * xc;
-                        if (lin & 1)
-                            a2 += v;
-                        else
-                            a1 += v;
-                    }
-                }
-                t.ksum = a1 + a2;
-            }
-        }
-        // rounds: one item per kernel corner per round, so that at every
-        // step of the lockstep walk distinct lanes touch distinct cells
-        unsigned pending = __ballot_sync(0xffffffffu, active);
-        while (pending) {
-            const unsigned peers
-                = __match_any_sync(0xffffffffu, (active && ((pending >> lane) & 1u)) ? key : ~0ull);
-            const bool mine = active && ((pending >> lane) & 1u) && (__ffs(peers & pending) - 1 == lane);
-            const unsigned sel = __ballot_sync(0xffffffffu, mine);
-            pending &= ~sel;
-            int kmax = mine ? t.K : 0;
-            for (int o = 16; o > 0; o >>= 1)
-                kmax = max(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
-            const bool anywrap = __any_sync(0xffffffffu, mine && cwrap);
-            if (KMODE != KM_EXACT && !anywrap && !BEAM) {
-                // common case: no footprint of the round crosses the grid's
-                // column edge, so each lane's in-tile columns are the window
-                // [jl, jh) and tap (i, j) sits at a fixed slot stride; the
-                // weight is folded into the visibility once per item
-                const int jl = mine ? jlo : 0;
-                const int jh = mine ? min(jhi, t.K) : 0;
-                const R vrw = vr * t.wt, viw = vim * t.wt;
-                for (int i = 0; i < kmax; i++) {
-                    const int rm = (mine && i < t.K) ? map_row(rb + i, gN, grows, wrap_neg) : -1;
-                    const int rl = rm - r0;
-                    const bool rok = rm >= 0 && rl >= 0 && rl < TILE_R;
-                    const int jhi_r = rok ? jh : 0;
-                    const int slot0 = cbase * TILE_R + rl;
-                    for (int j0 = 0; j0 < kmax; j0 += 8) {
-                        R kr[8], ki[8];
-#pragma unroll
-                        for (int jj = 0; jj < 8; jj++) {
-                            const int j = j0 + jj;
-                            kr[jj] = R(0);
-                            ki[jj] = R(0);
-                            if (j >= jl && j < jhi_r)
-                                tap_value<R, KMODE>(p, tab, t, i, j, kr[jj], ki[jj]);
-                        }
-#pragma unroll
-                        for (int jj = 0; jj < 8; jj++) {
-                            const int j = j0 + jj;
-                            if (j < kmax) {
-                                if (j >= jl && j < jhi_r) {
-                                    const R re = vrw * kr[jj] - viw * ki[jj];
-                                    const R im = vrw * ki[jj] + viw * kr[jj];
-                                    acc_rmw(&acc[slot0 + j * TILE_R], re, im);
-                                }
-                                __syncwarp();
-                            }
-                        }
-                    }
-                }
-            } else if (KMODE != KM_EXACT) {
-                // tabulated kernels: the lane's kernel row is fetched into
-                // registers eight taps at a time, so the loads are in flight
-                // together, then accumulated tap by tap in lockstep
-                for (int i = 0; i < kmax; i++) {
-                    const int rm = (mine && i < t.K) ? map_row(rb + i, gN, grows, wrap_neg) : -1;
-                    const int rl = rm - r0;
-                    const bool rok = rm >= 0 && rl >= 0 && rl < TILE_R;
-                    for (int j0 = 0; j0 < kmax; j0 += 8) {
-                        R kr[8], ki[8];
-#pragma unroll
-                        for (int jj = 0; jj < 8; jj++) {
-                            const int j = j0 + jj;
-                            kr[jj] = R(0);
-                            ki[jj] = R(0);
-                            if (rok && j < t.K && j >= jlo && j < jhi) {
-                                tap_value<R, KMODE>(p, tab, t, i, j, kr[jj], ki[jj]);
-                                kr[jj] = kr[jj] * t.wt;
-                                ki[jj] = ki[jj] * t.wt;
-                            }
-                        }
-#pragma unroll
-                        for (int jj = 0; jj < 8; jj++) {
-                            const int j = j0 + jj;
-                            if (j < kmax) {
-                                if (rok && j < t.K && j >= jlo && j < jhi) {
-                                    const int cl = cwrap ? map_col(cb + j, gN) - c0 : cbase + j;
-                                    if (cl >= 0 && cl < TILE_C) {
-                                        const R re = vr * kr[jj] - vim * ki[jj];
-                                        const R im = vr * ki[jj] + vim * kr[jj];
-                                        acc_rmw(&acc[cl * TILE_R + rl], re, im);
-                                        if (BEAM)
-                                            acc_rmw(&bacc[cl * TILE_R + rl], kr[jj], ki[jj]);
-                                    }
-                                }
-                                __syncwarp();
-                            }
-                        }
-                    }
-                }
-            } else {
-                for (int i = 0; i < kmax; i++) {
-                    const int rm = (mine && i < t.K) ? map_row(rb + i, gN, grows, wrap_neg) : -1;
-                    const int rl = rm - r0;
-                    const bool rok = rm >= 0 && rl >= 0 && rl < TILE_R;
-                    for (int j = 0; j < kmax; j++) {
-                        if (rok && j < t.K && j >= jlo && j < jhi) {
-                            const int cl = cwrap ? map_col(cb + j, gN) - c0 : cbase + j;
-                            if (cl >= 0 && cl < TILE_C) {
-                                R kr, ki;
-                                tap_value<R, KMODE>(p, tab, t, i, j, kr, ki);
-                                kr = kr * t.wt;
-                                ki = ki * t.wt;
-                                const R re = vr * kr - vim * ki;
-                                const R im = vr * ki + vim * kr;
-                                acc_rmw(&acc[cl * TILE_R + rl], re, im);
-                                if (BEAM)
-                                    acc_rmw(&bacc[cl * TILE_R + rl], kr, ki);
-                            }
-                        }
-                        __syncwarp();
-                    }
-                }
-            }
-        }
-    }
-    __syncwarp();
-    const int nr = min(TILE_R, grows - r0);
-    const int nc = min(TILE_C, gN - c0);
-    for (int q = lane; q < TILE_R * TILE_C; q += 32) {
-        const int rl = q % TILE_R, cl = q / TILE_R;
-        if (rl < nr && cl < nc) {
-            const size_t g = size_t(c0 + cl) * grows + (r0 + rl);
-            cell_store<R, COMP>(p.grid, g, acc[q], p.wide);
-            if (BEAM)
-                cell_store<R, COMP>(p.beam, g, bacc[q], p.wide);
-        }
-    }
-}
-
-// In-tile part of one footprint axis: taps t in [lo, hi) of raw index
-// base + t land on tile positions base + t + shift - origin.  `wrap_pos`:
-// raw indices >= N map to raw - N; `wrap_neg`: raw < 0 map to raw + N (else
-// they are dropped); only positions < limit exist.  Assumes N is large
-// against K + the tile size, so that at most one of the three candidate
-// segments meets the tile.
-__device__ __forceinline__ void tile_span(int base, int K, int N, int origin, int width, int limit, bool wrap_neg,
-    int& lo, int& hi, int& shift)
-{
-    const int top = min(origin + width, limit); // tile positions [origin, top)
-    // non-wrapped raw in [0, N)
-    lo = max(max(origin - base, -base), 0);
-    hi = min(min(top - base, N - base), K);
-    shift = 0;
-    if (lo < hi)
-        return;
-    // raw >= N -> raw - N
-    lo = max(max(origin + N - base, N - base), 0);
-    hi = min(top + N - base, K);
-    shift = -N;
-    if (lo < hi)
-        return;
-    if (wrap_neg) { // raw < 0 -> raw + N
-        lo = max(origin - N - base, 0);
-        hi = min(min(top - N - base, -base), K);
-        shift = N;
-        if (lo < hi)
-            return;
-    }
-    lo = hi = 0;
-}
-
-// Column-packed tile gridder (tabulated kernels).  One warp per tile.  Each
-// list entry (item, mirrored bit) is clipped to the tile: in-tile taps rows
-// [ilo, ihi) x columns [jlo, jhi).  A round packs the in-tile columns of
-// several entries side by side into the 32 lanes (lane = one column of one
-// entry) and walks their rows in lock-step, so lanes are spent on in-tile taps
-// only.  Lanes whose cells coincide in one step (two entries of a round
-// overlapping) are serialised by __match_any_sync; consecutive steps are
-// ordered by __syncwarp.  Requires N >= 2 (Kmax + tile) + 2 (one segment per
-// axis and tile); smaller grids use grid_tile.
-template <typename R, int COMP, int KMODE, bool BEAM, int TILE_C>
-__device__ __forceinline__ void grid_tile_cols(const GridParams<R>& p, int tile, unsigned char* smem_raw)
-{
-    using A = Acc<R, COMP>;
-    using C2 = typename Cplx<R>::T;
-    A* acc = reinterpret_cast<A*>(smem_raw);
-    A* bacc = acc + (BEAM ? TILE_R * TILE_C : 0);
-    R* tab = reinterpret_cast<R*>(acc + (BEAM ? 2 : 1) * TILE_R * TILE_C);
-    __shared__ int owner[32];
-    const int lane = threadIdx.x;
-    const int gN = p.N, grows = p.image_rows, gos = p.os;
-    const int tr = tile % p.tiles_r, tc = tile / p.tiles_r;
-    const int r0 = tr * TILE_R, c0 = tc * TILE_C;
-
-    for (int t = lane; t < TILE_R * TILE_C; t += 32) {
-        acc_zero(&acc[t]);
-        if (BEAM)
-            acc_zero(&bacc[t]);
-    }
-    if (KMODE == KM_SEP) {
-        const int K = 2 * p.support + 1;
-        for (int t = lane; t < p.cs * K; t += 32)
-            tab[t] = p.k1d[t];
-    }
-    __syncwarp();
-
-    const uint32_t beg = p.tile_off[tile], end = p.tile_off[tile + 1];
-    for (uint32_t base = beg; base < end; base += 32) {
-        // this lane's entry, clipped to the tile
-        const uint32_t e = base + lane;
-        int K = 1, ilo = 0, nrows = 0, jlo = 0, ncols = 0, rowb = 0, colb = 0;
-        uint32_t koff = 0; // W-proj: table offset of the item's K x K kernel; separable: cpy*K << 16 | cpx*K
-        R vr = R(0), vi = R(0), wt = R(0);
-        int conj = 0;
-        if (e < end) {
-            const uint32_t code = p.list[e];
-            const uint32_t idx = code >> 1;
-            const int mir = int(code & 1u);
-            const Item<R> it = p.items[idx];
-            int cx, cy;
-            item_centre(it, mir, gN, cx, cy);
-            const int S = (KMODE == KM_WPROJ) ? p.plane_support[it.plane] : p.support;
-            K = 2 * S + 1;
-            int cpx = it.cpx, cpy = it.cpy;
-            if (mir && gos > 1) {
-                cpx = gos - cpx;
-                cpy = gos - cpy;
-            }
-            const int rb = cy - S, cb = cx - S;
-            int ihi, jhi, rsh, csh;
-            tile_span(rb, K, gN, r0, TILE_R, grows, false, ilo, ihi, rsh);
-            tile_span(cb, K, gN, c0, TILE_C, gN, true, jlo, jhi, csh);
-            nrows = max(ihi - ilo, 0);
-            ncols = nrows > 0 ? max(jhi - jlo, 0) : 0;
-            rowb = rb + rsh - r0; // local row of tap i: rowb + i
-            colb = cb + csh - c0; // local column of tap j: colb + j
-            vr = it.vr;
-            vi = mir ? -it.vi : it.vi;
-            wt = it.w;
-            if (KMODE == KM_WPROJ) {
-                conj = (it.flags >> (mir ? 1 : 0)) & 1u;
-                koff = p.wk_off[it.plane] + uint32_t((cpy * p.cs + cpx) * K * K);
-            } else {
-                koff = (uint32_t(cpy * K) << 16) | uint32_t(cpx * K);
-            }
-        }
-        const R vrw = vr * wt, viw = vi * wt;
-        bool pending = ncols > 0;
-        while (__any_sync(0xffffffffu, pending)) {
-            // pack a prefix of the pending entries into the lanes
-            const int x = pending ? ncols : 0;
-            int incl = x;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o)
-                    incl += y;
-            }
-            const bool take = pending && incl <= 32;
-            const int off = incl - x;
-            if (take)
-                for (int t = 0; t < ncols; t++)
-                    owner[off + t] = lane;
-            int total = take ? incl : 0, steps = take ? nrows : 0;
-            for (int o = 16; o > 0; o >>= 1) {
-                total = max(total, __shfl_xor_sync(0xffffffffu, total, o));
-                steps = max(steps, __shfl_xor_sync(0xffffffffu, steps, o));
-            }
-            __syncwarp();
-            const int own = lane < total ? owner[lane] : lane;
-            __syncwarp();
-            const bool mine = lane < total;
-            // the owner entry's parameters
-            const int o_ilo = __shfl_sync(0xffffffffu, ilo, own);
-            const int o_nrows = __shfl_sync(0xffffffffu, nrows, own);
-            const int o_jlo = __shfl_sync(0xffffffffu, jlo, own);
-            const int o_off = __shfl_sync(0xffffffffu, off, own);
-            const int o_rowb = __shfl_sync(0xffffffffu, rowb, own);
-            const int o_colb = __shfl_sync(0xffffffffu, colb, own);
-            const int o_K = __shfl_sync(0xffffffffu, K, own);
-            const uint32_t o_koff = __shfl_sync(0xffffffffu, koff, own);
-            const R o_vr = __shfl_sync(0xffffffffu, vrw, own);
-            const R o_vi = __shfl_sync(0xffffffffu, viw, own);
-            const R o_wt = BEAM ? __shfl_sync(0xffffffffu, wt, own) : R(0);
-            const int o_conj = __shfl_sync(0xffffffffu, conj, own);
-            const int j = o_jlo + (lane - o_off);
-            const int col = o_colb + j;
-            for (int st = 0; st < steps; st++) {
-                const bool act = mine && st < o_nrows;
-                const int i = o_ilo + st;
-                R kr = R(0), ki = R(0);
-                if (act) {
-                    if (KMODE == KM_WPROJ) {
-                        const C2 v = p.wk[o_koff + uint32_t(i * o_K + j)];
-                        kr = v.x;
-                        ki = o_conj ? -v.y : v.y;
-                    } else {
-                        kr = tab[(o_koff >> 16) + uint32_t(i)] * tab[(o_koff & 0xffffu) + uint32_t(j)];
-                    }
-                }
-                const int slot = col * TILE_R + (o_rowb + i);
-                bool todo = act;
-                while (__any_sync(0xffffffffu, todo)) {
-                    const unsigned peers = __match_any_sync(0xffffffffu, todo ? slot : -1 - lane);
-                    const bool lead = todo && (__ffs(peers) - 1 == lane);
-                    if (lead) {
-                        const R re = o_vr * kr - o_vi * ki;
-                        const R im = o_vr * ki + o_vi * kr;
-                        acc_rmw(&acc[slot], re, im);
-                        if (BEAM)
-                            acc_rmw(&bacc[slot], kr * o_wt, ki * o_wt);
-                    }
-                    todo = todo && !lead;
-                    __syncwarp();
-                }
-            }
-            pending = pending && !take;
-        }
-    }
-    __syncwarp();
-    const int nr = min(TILE_R, grows - r0);
-    const int nc = min(TILE_C, gN - c0);
-    for (int q = lane; q < TILE_R * TILE_C; q += 32) {
-        const int rl = q % TILE_R, cl = q / TILE_R;
-        if (rl < nr && cl < nc) {
-            const size_t g = size_t(c0 + cl) * grows + (r0 + rl);
-            cell_store<R, COMP>(p.grid, g, acc[q], p.wide);
-            if (BEAM)
-                cell_store<R, COMP>(p.beam, g, bacc[q], p.wide);
-        }
-    }
-}
-
-// One CTA (one warp) per tile of one snapshot.
-// Residency target: the shared-memory tile allows ~28 CTAs per SM at 16
-// columns (8 KB FP32/FP32C cell tile) and ~14 at 32; registers are capped to match.
-// Lane-per-tap tile gridder (tabulated kernels).  One warp per tile; the
-// 32 list entries of a batch are clipped to the tile by their own lanes
-// (window rows [ilo, ihi) x columns [jlo, jhi)), then taken one at a time:
-// the entry's parameters are broadcast and its in-tile taps are spread over
-// the lanes, 32 per pass (lane = tap, column-major in the window, so that
-// consecutive lanes touch consecutive accumulator cells).  All taps of one
-// pass hit distinct cells, so there are no conflicts; consecutive passes are
-// ordered by __syncwarp.  Every lane does useful work on windows of 32 taps
-// or more; small kernels (K = 5 or 7 at one tile per footprint) fill most of
-// a pass.  Requires N >= 2 (Kmax + tile) + 2, as grid_tile_cols.
-template <typename R, int COMP, int KMODE, bool BEAM, int TILE_C>
-__device__ __forceinline__ void grid_tile_taps(const GridParams<R>& p, int tile, unsigned char* smem_raw)
-{
-    using A = Acc<R, COMP>;
-    using C2 = typename Cplx<R>::T;
-    A* acc = reinterpret_cast<A*>(smem_raw);
-    A* bacc = acc + (BEAM ? TILE_R * TILE_C : 0);
-    R* tab = reinterpret_cast<R*>(acc + (BEAM ? 2 : 1) * TILE_R * TILE_C);
-    const int lane = threadIdx.x & 31;
-    const int gN = p.N, grows = p.image_rows, gos = p.os;
-    const int tr = tile % p.tiles_r, tc = tile / p.tiles_r;
-    const int r0 = tr * TILE_R, c0 = tc * TILE_C;
-
-    for (int t = lane; t < TILE_R * TILE_C; t += 32) {
-        acc_zero(&acc[t]);
-        if (BEAM)
-            acc_zero(&bacc[t]);
-    }
-    if (KMODE == KM_SEP) {
-        const int K = 2 * p.support + 1;
-        for (int t = lane; t < p.cs * K; t += 32)
-            tab[t] = p.k1d[t];
-    }
-    __syncwarp();
-
-    const uint32_t beg = p.tile_off[tile], end = p.tile_off[tile + 1];
-    for (uint32_t base = beg; base < end; base += 32) {
-        // this lane's entry, clipped to the tile
-        const uint32_t e = base + lane;
-        int K = 1, ilo = 0, nrows = 0, jlo = 0, ncols = 0, rowb = 0, colb = 0;
-        uint32_t koff = 0; // W-proj: table offset of the item's K x K kernel; separable: cpy*K << 16 | cpx*K
-        R vr = R(0), vi = R(0), wt = R(0);
-        int conj = 0;
-        if (e < end) {
-            const uint32_t code = p.list[e];
-            const uint32_t idx = code >> 1;
-            const int mir = int(code & 1u);
-            const Item<R> it = p.items[idx];
-            int cx, cy;
-            item_centre(it, mir, gN, cx, cy);
-            const int S = (KMODE == KM_WPROJ) ? p.plane_support[it.plane] : p.support;
-            K = 2 * S + 1;
-            int cpx = it.cpx, cpy = it.cpy;
-            if (mir && gos > 1) {
-                cpx = gos - cpx;
-                cpy = gos - cpy;
-            }
-            const int rb = cy - S, cb = cx - S;
-            int ihi, jhi, rsh, csh;
-            tile_span(rb, K, gN, r0, TILE_R, grows, false, ilo, ihi, rsh);
-            tile_span(cb, K, gN, c0, TILE_C, gN, true, jlo, jhi, csh);
-            nrows = max(ihi - ilo, 0);
-            ncols = nrows > 0 ? max(jhi - jlo, 0) : 0;
-            if (ncols == 0)
-                nrows = 0;
-            rowb = rb + rsh - r0; // local row of tap i: rowb + i
-            colb = cb + csh - c0; // local column of tap j: colb + j
-            vr = it.vr;
-            vi = mir ? -it.vi : it.vi;
-            wt = it.w;
-            if (KMODE == KM_WPROJ) {
-                conj = (it.flags >> (mir ? 1 : 0)) & 1u;
-                koff = p.wk_off[it.plane] + uint32_t((cpy * p.cs + cpx) * K * K);
-            } else {
-                koff = (uint32_t(cpy * K) << 16) | uint32_t(cpx * K);
-            }
-        }
-        const R vrw = vr * wt, viw = vi * wt;
-        const int nt = nrows * ncols;
-        const int np = (nt + 31) >> 5;
-        // passes of the batch: unit u belongs to the last lane whose start <= u
-        int incl = np;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o)
-                incl += y;
-        }
-        const int start = incl - np;
-        const int units = __shfl_sync(0xffffffffu, incl, 31);
-        // packed per-entry words for the broadcasts
-        const int geo = (ilo & 0xff) | ((jlo & 0xff) << 8) | ((nrows & 0xff) << 16) | ((conj & 1) << 24);
-        const int loc = (rowb & 0xffff) | int(unsigned(colb) << 16);
-        const int kn = (K & 0xffff) | (nt << 16);
-        const float rcp = nrows > 0 ? 1.0f / float(nrows) : 0.0f;
-        for (int u = 0; u < units; u++) {
-            const unsigned le = __ballot_sync(0xffffffffu, np > 0 && start <= u);
-            const int own = 31 - __clz(le);
-            const int pass = u - __shfl_sync(0xffffffffu, start, own);
-            const int o_geo = __shfl_sync(0xffffffffu, geo, own);
-            const int o_loc = __shfl_sync(0xffffffffu, loc, own);
-            const int o_kn = __shfl_sync(0xffffffffu, kn, own);
-            const uint32_t o_koff = __shfl_sync(0xffffffffu, koff, own);
-            const float o_rcp = __shfl_sync(0xffffffffu, rcp, own);
-            const R o_vr = __shfl_sync(0xffffffffu, vrw, own);
-            const R o_vi = __shfl_sync(0xffffffffu, viw, own);
-            const R o_wt = BEAM ? __shfl_sync(0xffffffffu, wt, own) : R(0);
-            const int o_nt = o_kn >> 16, o_K = o_kn & 0xffff;
-            const int t = pass * 32 + lane;
-            if (t < o_nt) {
-                // window column-major: consecutive lanes take consecutive rows,
-                // i.e. consecutive accumulator cells
-                const int o_nrows = (o_geo >> 16) & 0xff;
-                const int dj = int((float(t) + 0.5f) * o_rcp);
-                const int di = t - dj * o_nrows;
-                const int i = (o_geo & 0xff) + di, j = ((o_geo >> 8) & 0xff) + dj;
-                R kr, ki;
-                if (KMODE == KM_WPROJ) {
-                    const C2 v = p.wk[o_koff + uint32_t(i * o_K + j)];
-                    kr = v.x;
-                    ki = ((o_geo >> 24) & 1) ? -v.y : v.y;
-                } else {
-                    kr = tab[(o_koff >> 16) + uint32_t(i)] * tab[(o_koff & 0xffffu) + uint32_t(j)];
-                    ki = R(0);
-                }
-                const int row = int(short(o_loc & 0xffff)) + i, col = (o_loc >> 16) + j;
-                const int slot = col * TILE_R + row;
-                const R re = o_vr * kr - o_vi * ki;
-                const R im = o_vr * ki + o_vi * kr;
-                acc_rmw(&acc[slot], re, im);
-                if (BEAM)
-                    acc_rmw(&bacc[slot], kr * o_wt, ki * o_wt);
-            }
-            __syncwarp();
-        }
-    }
-    __syncwarp();
-    const int nr = min(TILE_R, grows - r0);
-    const int nc = min(TILE_C, gN - c0);
-    for (int q = lane; q < TILE_R * TILE_C; q += 32) {
-        const int rl = q % TILE_R, cl = q / TILE_R;
-        if (rl < nr && cl < nc) {
-            const size_t g = size_t(c0 + cl) * grows + (r0 + rl);
-            cell_store<R, COMP>(p.grid, g, acc[q], p.wide);
-            if (BEAM)
-                cell_store<R, COMP>(p.beam, g, bacc[q], p.wide);
-        }
-    }
-}
-
-// ---------------------------------------------------------------- staged gridder
-
-// Record fill: like k_fill_tiles, but each (entry, tile) pair is written as a
-// decoded TapRec at its slot of the tile's range (tile order), the footprint
-// already clipped to the tile (tile_span, as grid_tile_taps clips it).  Slots
-// beyond `cap` are not written and set bit 8 of *err (the caller grows the
-// buffer to the counted total and grids again).
-template <typename R>
-struct RecFill {
-    TapRec<R>* rec;
-    uint64_t cap;
-    const uint32_t* wk_off; // W-projection: table offset per plane (x time step)
-    int cs, os;
-};
-
-template <typename R, int KMODE>
-__global__ void k_fill_recs(BinParams p, Item<R>* items, const uint32_t* order, const int64_t* first, int P,
-    RecFill<R> q)
-{
-    const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k >= p.n)
-        return;
-    const Item<R> it = items[k];
-    if (!it.good)
-        return;
-    int S = p.support, plane = 0;
-    if (p.plane16) {
-        plane = p.plane16[k];
-        S = p.plane_support[plane];
-        items[k].plane = uint16_t(plane);
-    } else if (order) {
-        plane = plane_of(first, P, k);
-        if (p.ts_of)
-            plane = plane * p.ntimesteps + p.ts_of[order[k]];
-        S = p.plane_support[plane];
-        items[k].plane = uint16_t(plane);
-    }
-    const int K = 2 * S + 1;
-    const bool ranked = p.ranks && *p.rank_overflow == 0u;
-    for (int mir = 0; mir < int(it.good); mir++) {
-        int cx, cy;
-        item_centre(it, mir, p.N, cx, cy);
-        int cpx = it.cpx, cpy = it.cpy;
-        if (mir && q.os > 1) {
-            cpx = q.os - cpx;
-            cpy = q.os - cpy;
-        }
-        TapRec<R> r;
-        r.vr = it.vr * it.w;
-        r.vi = (mir ? -it.vi : it.vi) * it.w;
-        const int conj = KMODE == KM_WPROJ ? int((it.flags >> (mir ? 1 : 0)) & 1u) : 0;
-        const uint32_t kbase = KMODE == KM_WPROJ ? q.wk_off[plane] + uint32_t((cpy * q.cs + cpx) * K * K) : 0u;
-        const int rb = cy - S, cb = cx - S;
-        int qn = 0;
-        for_item_tiles(it, mir, S, p, [&](uint32_t t) {
-            const uint32_t slot = ranked ? p.ranks[size_t(qn * 2 + mir) * size_t(p.n) + size_t(k)]
-                                         : atomicAdd(&p.tile_cursor[t], 1u);
-            qn++;
-            const int r0 = int(t % uint32_t(p.tiles_r)) * TILE_R, c0 = int(t / uint32_t(p.tiles_r)) * p.tile_c;
-            int ilo, ihi, rsh, jlo, jhi, csh;
-            tile_span(rb, K, p.N, r0, TILE_R, p.image_rows, false, ilo, ihi, rsh);
-            tile_span(cb, K, p.N, c0, p.tile_c, p.N, true, jlo, jhi, csh);
-            int nrows = max(ihi - ilo, 0), ncols = max(jhi - jlo, 0);
-            if (nrows == 0 || ncols == 0)
-                nrows = ncols = 0;
-            const int row0 = nrows ? rb + rsh - r0 + ilo : 0;
-            const int col0 = ncols ? cb + csh - c0 + jlo : 0;
-            r.koff = KMODE == KM_WPROJ ? kbase + uint32_t(ilo * K + jlo)
-                                       : (uint32_t(cpy * K + ilo) << 16) | uint32_t(cpx * K + jlo);
-            r.geom = rec_geom(row0, col0, nrows, ncols, conj, K);
-            const uint64_t pos = uint64_t(p.tile_off[t]) + slot;
-            if (pos < q.cap)
-                q.rec[pos] = r;
-            else
-                atomicOr(p.err, 8u);
-        });
-    }
-}
-
-// Bulk (TMA) copies into shared memory completing on an mbarrier, and a
-// bounded wait for a barrier phase.
-constexpr int kRecChunk = 64;              // records per staged chunk (two chunks in flight per warp)
-constexpr uint32_t kWaitLimit = 1u << 22; // try_wait rounds before a wait gives up
-
-__device__ __forceinline__ uint32_t smem_addr(const void* p)
-{
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(1u) : "memory");
-}
-
-__device__ __forceinline__ void mbar_init_fence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-
-// one arrival that expects `bytes`, then the copy that delivers them
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
-                 : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_addr(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_addr(bar))
-                 : "memory");
-}
-
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity)
-{
-    const uint32_t a = smem_addr(bar);
-    for (uint32_t it = 0; it < kWaitLimit; it++) {
-        uint32_t done;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                     "selp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(done)
-                     : "r"(a), "r"(parity)
-                     : "memory");
-        if (done)
-            return true;
-    }
-    return false;
-}
-
-// ceil(65536 / n), n = 1..32: (t * m) >> 16 == t / n for t < 1024
-__constant__ uint32_t c_div_magic[33] = { 0, 65536, 32768, 21846, 16384, 13108, 10923, 9363, 8192, 7282, 6554, 5958,
-    5462, 5042, 4682, 4370, 4096, 3856, 3641, 3450, 3277, 3121, 2979, 2850, 2731, 2622, 2521, 2428, 2341, 2260, 2185,
-    2115, 2048 };
-
-// Shared memory of one warp of the staged gridder: accumulators, two record
-// buffers, two barriers and the separable kernel table.
-template <typename R, int COMP, int TILE_C>
-__host__ __device__ constexpr size_t rec_warp_bytes(int sep_table_len)
-{
-    return ((sizeof(Acc<R, COMP>) * TILE_R * TILE_C + 2 * kRecChunk * sizeof(TapRec<R>) + 16
-                + sizeof(R) * size_t(sep_table_len))
-               + 15)
-        / 16 * 16;
-}
-
-// Staged tile gridder: one warp per tile.  The tile's records (k_fill_recs)
-// arrive in chunks of kRecChunk by bulk copies into two shared-memory
-// buffers (the next chunk is in flight while one is processed); the warp
-// takes the entries one at a time, each lane one tap of the entry's clipped
-// window (column-major, so consecutive lanes update consecutive cells: the
-// taps of one entry are distinct cells, entries are ordered by __syncwarp),
-// the record read from shared memory by all lanes at once.  Accumulation,
-// zeroing and the single coalesced store are those of grid_tile_taps.  A
-// barrier wait that gives up (never expected) sets bit 16 of *err, waits for
-// the copies still in flight and leaves the tile unwritten.
-template <typename R, int COMP, int KMODE, int TILE_C>
-__device__ __forceinline__ bool grid_tile_recs(const GridParams<R>& p, int tile, unsigned char* smem_raw)
-{
-    unsigned int* err = p.err;
-    using A = Acc<R, COMP>;
-    using C2 = typename Cplx<R>::T;
-    A* acc = reinterpret_cast<A*>(smem_raw);
-    TapRec<R>* rbuf = reinterpret_cast<TapRec<R>*>(acc + TILE_R * TILE_C);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(rbuf + 2 * kRecChunk);
-    R* tab = reinterpret_cast<R*>(bar + 2);
-    const int lane = threadIdx.x & 31;
-    const int gN = p.N, grows = p.image_rows;
-    const int tr = tile % p.tiles_r, tc = tile / p.tiles_r;
-    const int r0 = tr * TILE_R, c0 = tc * TILE_C;
-    const uint32_t beg = p.tile_off[tile];
-    uint32_t cnt = p.tile_off[tile + 1] - beg;
-    if (uint64_t(beg) + cnt > p.rec_cap) { // the fill overflowed (bit 8 is set): copy nothing
-        cnt = 0;
-        if (lane == 0)
-            atomicOr(err, 8u);
-    }
-    const int nch = int((cnt + kRecChunk - 1) / kRecChunk);
-    auto issue = [&](int c) {
-        const uint32_t n = min(uint32_t(kRecChunk), cnt - uint32_t(c) * kRecChunk);
-        bulk_copy_g2s(rbuf + (c & 1) * kRecChunk, p.recs + beg + uint32_t(c) * kRecChunk,
-            n * uint32_t(sizeof(TapRec<R>)), &bar[c & 1]);
-    };
-    if (lane == 0) {
-        mbar_init(&bar[0]);
-        mbar_init(&bar[1]);
-        mbar_init_fence();
-        if (nch > 0)
-            issue(0);
-        if (nch > 1)
-            issue(1);
-    }
-    for (int t = lane; t < TILE_R * TILE_C; t += 32)
-        acc_zero(&acc[t]);
-    if (KMODE == KM_SEP) {
-        const int K = 2 * p.support + 1;
-        for (int t = lane; t < p.cs * K; t += 32)
-            tab[t] = p.k1d[t];
-    }
-    __syncwarp();
-    for (int c = 0; c < nch; c++) {
-        const bool ok = __all_sync(0xffffffffu, mbar_wait(&bar[c & 1], uint32_t(c >> 1) & 1u));
-        if (!ok) {
-            if (lane == 0) {
-                // record the failure, then wait (bounded again) for this
-                // chunk's copy and the other buffer's before leaving
-                atomicOr(err, 16u);
-                mbar_wait(&bar[c & 1], uint32_t(c >> 1) & 1u);
-                if (c + 1 < nch)
-                    mbar_wait(&bar[(c + 1) & 1], uint32_t((c + 1) >> 1) & 1u);
-            }
-            __syncwarp();
-            return false;
-        }
-        const TapRec<R>* rb = rbuf + (c & 1) * kRecChunk;
-        const int ne = min(kRecChunk, int(cnt) - c * kRecChunk);
-        // an entry decoded once: window shape, divisor magic, first cell,
-        // kernel offsets and the weighted visibility (pvr, pvi: its parts
-        // negated when the W-kernel is conjugated, so that the product
-        // needs no per-tap sign)
-        struct Ent {
-            int nrows, nt, sbase, K;
-            uint32_t m, koff, ky, kx;
-            R vr, vi, pvr, pvi;
-        };
-        auto decode = [&](const TapRec<R>& r) {
-            Ent x;
-            const uint32_t g = r.geom;
-            x.nrows = int((g >> 10) & 63u);
-            x.nt = x.nrows * int((g >> 16) & 63u);
-            x.m = c_div_magic[x.nrows];
-            x.sbase = int((g >> 5) & 31u) * TILE_R + int(g & 31u);
-            x.K = int(g >> 23);
-            const bool conj = (g >> 22) & 1u;
-            x.koff = r.koff;
-            x.ky = r.koff >> 16;
-            x.kx = r.koff & 0xffffu;
-            x.vr = r.vr;
-            x.vi = r.vi;
-            x.pvr = conj ? -r.vr : r.vr;
-            x.pvi = conj ? -r.vi : r.vi;
-            return x;
-        };
-        // tap t of an entry: its accumulator cell and weighted value
-        auto tap = [&](const Ent& x, int t, int& cell, R& re, R& im) {
-            const int dj = int((uint32_t(t) * x.m) >> 16);
-            const int di = t - dj * x.nrows;
-            if (KMODE == KM_WPROJ) {
-                // (vr + i vi)(kr + i ki), ki = -v.y for a conjugated kernel
-                const C2 v = __ldg(&p.wk[x.koff + uint32_t(di * x.K + dj)]);
-                re = x.vr * R(v.x) - x.pvi * R(v.y);
-                im = x.pvr * R(v.y) + x.vi * R(v.x);
-            } else {
-                const R kr = tab[x.ky + uint32_t(di)] * tab[x.kx + uint32_t(dj)];
-                re = x.vr * kr;
-                im = x.vi * kr;
-            }
-            cell = x.sbase + dj * TILE_R + di;
-        };
-        // two single-pass entries at a time where possible: both kernel
-        // loads in flight before either entry's cells are updated
-        for (int e = 0; e < ne;) {
-            const Ent ea = decode(rb[e]);
-            if (ea.nt <= 32 && e + 1 < ne) {
-                const Ent eb = decode(rb[e + 1]);
-                if (eb.nt <= 32) {
-                    int ca = 0, cb = 0;
-                    R xa = R(0), ya = R(0), xb = R(0), yb = R(0);
-                    const bool ia = lane < ea.nt, ib = lane < eb.nt;
-                    if (ia)
-                        tap(ea, lane, ca, xa, ya);
-                    if (ib)
-                        tap(eb, lane, cb, xb, yb);
-                    if (ia)
-                        acc_rmw(&acc[ca], xa, ya);
-                    __syncwarp();
-                    if (ib)
-                        acc_rmw(&acc[cb], xb, yb);
-                    __syncwarp();
-                    e += 2;
-                    continue;
-                }
-            }
-            // an entry's taps are distinct cells: up to four passes' kernel
-            // loads are issued before their updates, with no ordering
-            // between the passes
-            for (int t0 = lane; t0 < ea.nt; t0 += 128) {
-                int cell[4];
-                R xr[4], yi[4];
-                bool in[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    in[q] = t0 + q * 32 < ea.nt;
-                    if (in[q])
-                        tap(ea, t0 + q * 32, cell[q], xr[q], yi[q]);
-                }
-#pragma unroll
-                for (int q = 0; q < 4; q++)
-                    if (in[q])
-                        acc_rmw(&acc[cell[q]], xr[q], yi[q]);
-            }
-            __syncwarp();
-            e++;
-        }
-        if (lane == 0 && c + 2 < nch) {
-            // the buffer's records were read by every lane (ordered by the
-            // __syncwarp above) before the async proxy overwrites it
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            issue(c + 2);
-        }
-        __syncwarp();
-    }
-    const int nr = min(TILE_R, grows - r0);
-    const int nc = min(TILE_C, gN - c0);
-    for (int q = lane; q < TILE_R * TILE_C; q += 32) {
-        const int rl = q % TILE_R, cl = q / TILE_R;
-        if (rl < nr && cl < nc) {
-            cell_store<R, COMP>(p.grid, size_t(c0 + cl) * grows + (r0 + rl), acc[q], p.wide);
-        }
-    }
-    // every copy has completed: the barriers can be initialised again for
-    // the warp's next tile (persistent batch gridder)
-    if (lane == 0) {
-        asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_addr(&bar[0])) : "memory");
-        asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_addr(&bar[1])) : "memory");
-    }
-    __syncwarp();
-    return true;
-}
-
-// Staged gridder with WPB warps per block, each on its own tile (tile
-// blockIdx.x * WPB + warp; its shared memory at warp * warp_bytes).
-template <typename R, int COMP, int KMODE, int TILE_C, int WPB>
-__global__ void __launch_bounds__(32 * WPB) k_grid_tiles_recs(GridParams<R> p, int ntiles, int warp_bytes)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int warp = threadIdx.x >> 5;
-    const int tile = int(blockIdx.x) * WPB + warp;
-    if (tile < ntiles)
-        grid_tile_recs<R, COMP, KMODE, TILE_C>(p, tile, smem_raw + size_t(warp) * size_t(warp_bytes));
-}
-
-// Lane-per-tap gridder with WPB warps per block, each on its own tile (tile
-// blockIdx.x * WPB + warp, its accumulators at warp * tile_bytes): narrow
-// tiles keep the shared memory per warp small, and several warps per block
-// raise the resident warps past the per-SM block limit.
-template <typename R, int COMP, int KMODE, bool BEAM, int TILE_C, int WPB>
-__global__ void __launch_bounds__(32 * WPB, 44 / WPB) k_grid_tiles_mw(GridParams<R> p, int ntiles, int tile_bytes)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int warp = threadIdx.x >> 5;
-    const int tile = int(blockIdx.x) * WPB + warp;
-    if (tile < ntiles)
-        grid_tile_taps<R, COMP, KMODE, BEAM, TILE_C>(p, tile, smem_raw + size_t(warp) * size_t(tile_bytes));
-}
-
-// FORM: 0 lanes-per-item (grid_tile), 1 column-packed (grid_tile_cols),
-// 2 lane-per-tap (grid_tile_taps); the exact gridder always uses grid_tile.
-template <typename R, int COMP, int KMODE, bool BEAM, int TILE_C, int FORM = 0>
-__global__ void __launch_bounds__(32, TILE_C == 16 ? (sizeof(R) == 8 ? 24 : 28) : 14) k_grid_tiles(GridParams<R> p)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    if constexpr (FORM == 1 && KMODE != KM_EXACT)
-        grid_tile_cols<R, COMP, KMODE, BEAM, TILE_C>(p, int(blockIdx.x), smem_raw);
-    else if constexpr (FORM == 2 && KMODE != KM_EXACT)
-        grid_tile_taps<R, COMP, KMODE, BEAM, TILE_C>(p, int(blockIdx.x), smem_raw);
-    else
-        grid_tile<R, COMP, KMODE, BEAM, TILE_C>(p, int(blockIdx.x), smem_raw);
-}
-
-// Parameters of one persistent gridder launch: up to kBatchGrid snapshots,
-// passed by value (kernel parameter space, read through the constant cache
-// with a warp-uniform index).
-constexpr int kBatchGrid = 64;
-template <typename R>
-struct BatchGridParams {
-    GridParams<R> ps[kBatchGrid];
-    uint32_t tile_base[kBatchGrid + 1];
-    int nsnap;
-    uint32_t* counter;
-};
-
-// Persistent gridder over the tiles of many snapshots: a (snapshot, tile)
-// work queue.  Work item w is tile w - tile_base[s] of the snapshot s with
-// tile_base[s] <= w < tile_base[s + 1]; warps take items from one atomic
-// counter (zeroed before the launch) until the queue is empty.
-// PERSIST = false: one CTA per work item (w = blockIdx.x), the hardware
-// block scheduler being the queue; the autotuner picks the faster form.
-template <typename R, int COMP, int KMODE, bool BEAM, int TILE_C, bool PERSIST, int FORM = 0>
-__global__ void __launch_bounds__(32, TILE_C == 16 ? (sizeof(R) == 8 ? 24 : 28) : 14) k_grid_batch(const __grid_constant__ BatchGridParams<R> P)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const uint32_t total = P.tile_base[P.nsnap];
-    for (int once = 0;; once++) {
-        uint32_t w = 0;
-        if (PERSIST) {
-            if (threadIdx.x == 0)
-                w = atomicAdd(P.counter, 1u);
-            w = __shfl_sync(0xffffffffu, w, 0);
-        } else {
-            if (once)
-                break;
-            w = blockIdx.x;
-        }
-        if (w >= total)
-            break;
-        int lo = 0, hi = P.nsnap - 1;
-        while (lo < hi) { // last snapshot whose first tile <= w
-            const int mid = (lo + hi + 1) / 2;
-            if (P.tile_base[mid] <= w)
-                lo = mid;
-            else
-                hi = mid - 1;
-        }
-        __syncwarp();
-        if constexpr (FORM == 3 && KMODE != KM_EXACT && !BEAM) {
-            if (!grid_tile_recs<R, COMP, KMODE, TILE_C>(P.ps[lo], int(w - P.tile_base[lo]), smem_raw))
-                break; // a staged copy's wait gave up (flagged): this warp stops
-        } else if constexpr (FORM == 2 && KMODE != KM_EXACT)
-            grid_tile_taps<R, COMP, KMODE, BEAM, TILE_C>(P.ps[lo], int(w - P.tile_base[lo]), smem_raw);
-        else
-            grid_tile<R, COMP, KMODE, BEAM, TILE_C>(P.ps[lo], int(w - P.tile_base[lo]), smem_raw);
-        __syncwarp();
-    }
-}
 
 // ---------------------------------------------------------------- kernel tables
 
@@ -3009,13 +1557,13 @@ __global__ void k_collect_scalars(const double* total, const unsigned long long*
 }
 
 // Expanded W-kernel tables for the gridder: one block per (plane, oversampled
-// offset pair); entry t = i*K + j holds the reference's cached kernel value
-// conv(|oy|, |ox|) * inv (aw_projection.cpp:415-448), formed in FP64 and
-// rounded once to R.  Plane p's tables start at off[p] = sum over q < p of
-// cs^2 * K_q^2.
+// offset pair); entry j*K + i (column j, row i) holds the reference's cached
+// kernel value conv(|oy|, |ox|) * inv (aw_projection.cpp:415-448), formed in
+// FP64 and rounded once to R.  Plane p's tables start at off[p] = sum over q <
+// p of cs^2 * K_q^2; *max_support (zeroed before) = the largest support.
 template <typename R>
 __global__ void k_wk_expand(const double2* convd, const double* invd, const int* support, int P, int cs, int os,
-    int lh, typename Cplx<R>::T* out, uint32_t* off)
+    int lh, typename Cplx<R>::T* out, uint32_t* off, unsigned int* max_support)
 {
     const int p = blockIdx.x;
     const int pair = blockIdx.y;
@@ -3025,15 +1573,17 @@ __global__ void k_wk_expand(const double2* convd, const double* invd, const int*
         const uint32_t Kq = uint32_t(2 * support[q] + 1);
         base += uint32_t(cs) * uint32_t(cs) * Kq * Kq;
     }
-    if (pair == 0 && threadIdx.x == 0)
-        off[p] = base;
     const int S = support[p];
+    if (pair == 0 && threadIdx.x == 0) {
+        off[p] = base;
+        atomicMax(max_support, unsigned(S));
+    }
     const int K = 2 * S + 1;
     const double inv = invd[(size_t(p) * cs + cy) * cs + cx];
     const double2* conv = convd + size_t(p) * lh * lh;
     typename Cplx<R>::T* dst = out + base + uint32_t(pair) * uint32_t(K * K);
     for (int t = threadIdx.x; t < K * K; t += blockDim.x) {
-        const int i = t / K, j = t % K;
+        const int i = t % K, j = t / K;
         int oy = (i - S) * os + os / 2 - cy;
         int ox = (j - S) * os + os / 2 - cx;
         oy = oy < 0 ? -oy : oy;

@@ -69,3 +69,48 @@ def test_entries_that_are_not_finite_stay_in_their_footprint(ctx, exact):
         assert 0 < (~fine).sum() <= 2 * (2 * S + 1) ** 2
         assert np.array_equal(fine, np.isfinite(a.real) & np.isfinite(a.imag))
         assert np.abs(a[fine] - b[fine]).max() <= 1e-12 * np.abs(b[fine]).max()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32c"])
+@pytest.mark.parametrize("N,P,smax,trunc", [(28, 2, 3, 0.0), (66, 4, 8, 0.0), (102, 8, 12, 2.0), (130, 5, 16, 0.0),
+                                            (256, 3, 40, 0.0)])
+def test_w_kernels_match_oracle(ctx, N, P, smax, trunc, precision):
+    """Supports below, at and beyond a block's width, planes of different supports, both signs of w, dense blocks."""
+    uv, vis, wts = _points(N + smax, 900, N, 1.05)
+    uv[::3] *= 0.1  # several hundred entries in the blocks around the origin
+    w = np.random.default_rng(N).uniform(-3000.0, 3000.0, len(vis))
+    cell = 20.0
+    kw = dict(num_wplanes=P, max_wpconv_support=smax, kernel_trunc_perc=trunc, w=w, cell_size=cell, analytic_gcf=False)
+    r = orc.convolve_to_grid(capi.GaussianSinc, 3, N, uv, vis, wts, False, 4, True, True, True,
+                             wproj=orc.WProj(P, smax, 1, trunc), w=w, cell_size=cell, analytic_gcf=False)
+    if precision == "fp64":
+        g = ctx.convolve_to_grid(capi.GaussianSinc, 3.0, 3, N, uv, vis, wts, kernel_exact=False, oversampling=4, **kw)
+        assert np.abs(g[0] - r.vis_grid).max() <= 1e-11 * np.abs(r.vis_grid).max()
+        assert np.abs(g[1] - r.sampling_grid).max() <= 1e-11 * np.abs(r.sampling_grid).max()
+        return
+    # single-precision kernel values and weighted visibilities (relative error 2^-23 in all, or 1.2e-7 per tap):
+    # the image before correction is within that of the peak of the sum of all taps' magnitudes
+    inv = N * np.deg2rad(cell / 3600.0)
+    uvw = np.column_stack([uv / inv, w])
+    kwi = dict(kernel_func=capi.GaussianSinc, kernel_support=3, kernel_exact=False, oversampling=4,
+               gridding_correction=False, num_wplanes=P, max_wpconv_support=smax, kernel_trunc_perc=trunc)
+    img = ctx.image_visibilities(vis, wts, uvw, N, cell, precision=capi.FP32C, **kwi)[0]
+    ref = ctx.image_visibilities(vis, wts, uvw, N, cell, precision=capi.FP64, **kwi)[0]
+    assert np.abs(img - ref).max() <= 5e-6 * np.abs(ref).max()
+
+
+def test_w_kernel_entries_that_are_not_finite_stay_in_their_footprint(ctx):
+    N, smax = 64, 4
+    uv, vis, wts = _points(5, 200, N, 0.8)
+    vis[17] = np.nan
+    uv[17] = (10.3, 12.2)
+    w = np.linspace(-500.0, 500.0, 200)
+    with np.errstate(all="ignore"):
+        r = orc.convolve_to_grid(capi.GaussianSinc, 3, N, uv, vis, wts, False, 4, True, True, True,
+                                 wproj=orc.WProj(2, smax, 1, 0.0), w=w, cell_size=5.0, analytic_gcf=False)
+    g = ctx.convolve_to_grid(capi.GaussianSinc, 3.0, 3, N, uv, vis, wts, kernel_exact=False, oversampling=4,
+                             num_wplanes=2, max_wpconv_support=smax, w=w, cell_size=5.0, analytic_gcf=False)
+    fine = np.isfinite(r.vis_grid.real) & np.isfinite(r.vis_grid.imag)
+    assert (~fine).sum() == (2 * smax + 1) ** 2
+    assert np.array_equal(fine, np.isfinite(g[0].real) & np.isfinite(g[0].imag))
+    assert np.abs(g[0][fine] - r.vis_grid[fine]).max() <= 1e-11 * np.abs(r.vis_grid[fine]).max()
