@@ -132,6 +132,9 @@ struct DevBuf {
     size_t cap = 0;
 };
 
+// Words zeroed at the start of a call (GridOut::d_err points at them).
+enum CallFlags { CF_ERR = 0, CF_MAX_SUPPORT, CF_RANK_OVERFLOW, CF_ENTRIES, CF_TICKET, CF_WORDS };
+
 // Device outputs of one gridding pass (context buffers).
 struct GridOut {
     void* grid = nullptr;
@@ -139,8 +142,8 @@ struct GridOut {
     int image_rows = 0;
     double* d_total = nullptr;             // [0] sample_grid_total
     unsigned long long* d_ngood = nullptr; // [0] good visibilities
-    uint32_t* d_nitems = nullptr;          // tile-list entries
-    unsigned int* d_err = nullptr;
+    uint32_t* d_nitems = nullptr;          // binned entries
+    unsigned int* d_err = nullptr;         // error flags, then the other words of CallFlags
     int* d_plane_support = nullptr;
     int nplanes = 0;
 };
@@ -492,22 +495,28 @@ uint64_t entry_capacity(int N, int K, int64_t n)
     return uint64_t(std::max<int64_t>(n, 1)) * (N >= 2 * K + 2 ? 4 : 18);
 }
 
-// Exclusive scan of n counts into off[0 .. n] (off[n] = the total).
-void scan_counts(stpgpu_context* c, uint32_t* cnt, uint32_t* off, int n)
+// The bins of a call's entries; the count, off, cursor and rank buffers are
+// sized here and the flags attached.
+BlockBins make_bins(stpgpu_context* c, const ImagerSetup& s, const GridOut& g, int64_t n, bool exact)
 {
-    cudaStream_t st = c->stream;
-    if (n <= 4096) {
-        k_scan_single<<<1, 1024, 0, st>>>(cnt, off, n);
-        STPGPU_CHECK_LAUNCH();
-        return;
-    }
-    // many counts: the multi-block scan (cnt[n] is 0, so off[n] receives the total)
-    size_t tb = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, off, n + 1, st);
-    void* tmp = c->buf<unsigned char>("cubtmp_tiles", tb);
-    if (cub::DeviceScan::ExclusiveSum(tmp, tb, cnt, off, n + 1, st) != cudaSuccess)
-        fail(STPGPU_ERR_CUDA, "tile offset scan failed");
-    g_launches += 2;
+    BlockBins b {};
+    const int K = 2 * (s.nplanes > 0 ? s.max_support : s.support) + 1;
+    b.N = s.N;
+    b.rows = g.image_rows;
+    b.pad = int(ceil_div(K - 1, kBlk));
+    b.brn = int(ceil_div(b.rows, kBlk)) + b.pad;
+    b.bcn = int(ceil_div(b.N, kBlk)) + b.pad;
+    b.wrap_neg = exact;
+    b.support = s.support;
+    b.ntimesteps = std::max(s.ntimesteps, 1);
+    b.n = n;
+    const size_t nbins = size_t(b.brn) * size_t(b.bcn);
+    b.off = c->buf<uint32_t>("toff", nbins + size_t(b.bcn));
+    b.count = c->buf<uint32_t>("tcount", nbins);
+    b.cursor = c->buf<uint32_t>("tcur", nbins);
+    b.ranks = c->buf<uint32_t>("tranks", size_t(std::max<int64_t>(n, 1)) * kEntrySlots);
+    b.rank_overflow = g.d_err + CF_RANK_OVERFLOW;
+    return b;
 }
 
 // Where a call's items and kernel tables are, for grid_blocks.
@@ -534,35 +543,18 @@ struct GridInputs {
 // Binning by first cell and the block gridder (gridder_kernels.cuh).  wide:
 // a single-precision call's grid holds double cells.
 template <typename R, typename T, typename ACC>
-void grid_blocks(stpgpu_context* c, const ImagerSetup& s, GridOut& g, int64_t n, const GridInputs<R>& in, bool wide)
+void grid_blocks(stpgpu_context* c, const ImagerSetup& s, GridOut& g, int64_t n, BlockBins b, const GridInputs<R>& in,
+    bool wide)
 {
     cudaStream_t st = c->stream;
     const int K = 2 * (in.wproj ? s.max_support : s.support) + 1;
     const int64_t nn = std::max<int64_t>(n, 1);
-    BlockBins b {};
-    b.N = s.N;
-    b.rows = g.image_rows;
-    b.pad = int(ceil_div(K - 1, kBlk));
-    b.brn = int(ceil_div(b.rows, kBlk)) + b.pad;
-    b.bcn = int(ceil_div(b.N, kBlk)) + b.pad;
-    b.wrap_neg = in.exact;
-    b.support = s.support;
     b.plane_support = in.plane_support;
     b.plane16 = in.plane16;
     b.order = in.order;
     b.first = in.first;
     b.P = in.P;
     b.ts_of = in.ts_of;
-    b.ntimesteps = std::max(s.ntimesteps, 1);
-    b.n = n;
-    const int nbins = b.brn * b.bcn;
-    uint32_t* off = c->buf<uint32_t>("toff", nbins + 1);
-    b.count = c->buf<uint32_t>("tcount", nbins + 1);
-    b.cursor = c->buf<uint32_t>("tcur", nbins + 1);
-    b.ranks = c->buf<uint32_t>("tranks", size_t(nn) * kEntrySlots);
-    b.rank_overflow = c->buf<uint32_t>("trankovf", 1);
-    b.off = off;
-    zero_words(st, { { b.count, nbins + 1 }, { b.cursor, nbins + 1 }, { b.rank_overflow, 1 } });
     const uint64_t cap = entry_capacity(s.N, K, nn);
     if (cap > 0xffffffffull)
         fail(STPGPU_ERR_INVALID_ARG, "too many visibilities for one snapshot");
@@ -575,16 +567,18 @@ void grid_blocks(stpgpu_context* c, const ImagerSetup& s, GridOut& g, int64_t n,
     q.os = in.os;
     q.exact = in.exact;
     q.err = g.d_err;
-    if (n > 0) {
+    if (n > 0 && in.wproj) {
         k_bin_count<R><<<grid1d(n, 256), 256, 0, st>>>(b, in.items);
         STPGPU_CHECK_LAUNCH();
     }
-    scan_counts(c, b.count, off, nbins);
+    g.d_nitems = g.d_err + CF_ENTRIES;
+    k_bin_scan<<<unsigned(b.bcn), 256, 0, st>>>(b.count, const_cast<uint32_t*>(b.off), b.cursor, b.brn, b.rank_overflow,
+        g.d_nitems);
+    STPGPU_CHECK_LAUNCH();
     if (n > 0) {
         k_bin_fill<R><<<grid1d(n, 256), 256, 0, st>>>(b, in.items, q);
         STPGPU_CHECK_LAUNCH();
     }
-    g.d_nitems = off + nbins;
     const size_t cells = size_t(b.rows) * b.N;
     const bool f64 = sizeof(R) == 8 || wide;
     g.grid = c->buf<unsigned char>("grid", cells * (f64 ? 16 : 8));
@@ -594,7 +588,7 @@ void grid_blocks(stpgpu_context* c, const ImagerSetup& s, GridOut& g, int64_t n,
         p.rows = b.rows;
         p.pad = b.pad;
         p.brn = b.brn;
-        p.off = off;
+        p.off = b.off;
         p.recs = q.rec;
         p.wts = q.wts;
         p.grid = g.grid;
@@ -695,8 +689,12 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
     unsigned long long* npart = c->buf<unsigned long long>("npart", nb_pre);
     g.d_total = c->buf<double>("total", 4);
     g.d_ngood = c->buf<unsigned long long>("ngood", 2);
-    g.d_err = c->buf<unsigned int>("err", 2);
-    zero_words(st, { { g.d_err, 2 } }); // error flags, largest plane support
+    g.d_err = c->buf<unsigned int>("err", CF_WORDS);
+    BlockBins bins = make_bins(c, s, g, n, kernel_exact != 0);
+    const bool use_wsel = wproj && n > 0 && s.wsel;
+    WselState* ws = use_wsel ? c->buf<WselState>("wsel", 1) : nullptr;
+    zero_words(st, { { g.d_err, CF_WORDS }, { bins.count, int64_t(bins.brn) * bins.bcn },
+                       { ws, use_wsel ? int64_t(kWselZeroWords) : 0 } });
     PrepassParams pp {};
     pp.n = n;
     pp.vis = d_vis;
@@ -719,12 +717,15 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
     pp.wmax_part = (wproj && !s.full_wsort) ? c->buf<double>("wmaxpart", 2 * size_t(nb_pre)) : nullptr;
     pp.iota = (wproj && !s.wsel) ? c->buf<uint32_t>("perm_in", nn) : nullptr;
     pp.w_out = nullptr;
-    if (n > 0) {
-        k_prepass<R><<<nb_pre, GRID_THREADS, 0, st>>>(pp, items);
-        STPGPU_CHECK_LAUNCH();
-    }
-    k_finish_wsum<<<1, 1024, 0, st>>>(wpart, npart, pp.wmax_part, n > 0 ? int(nb_pre) : 0, g.d_total, g.d_ngood);
+    pp.ticket = g.d_err + CF_TICKET;
+    pp.total = g.d_total;
+    pp.ngood = g.d_ngood;
+    if (wproj)
+        bins.count = nullptr; // (counted once the supports are known)
+    k_prepass<R><<<nb_pre, GRID_THREADS, 0, st>>>(pp, items, bins); // n = 0 too: one block, totals of zero
     STPGPU_CHECK_LAUNCH();
+    if (wproj)
+        bins.count = c->buf<uint32_t>("tcount", 1);
 
     // ---- kernels
     const uint32_t* sorted_perm = nullptr;
@@ -749,20 +750,15 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
         k1d64 = t64;
     }
     const uint16_t* plane16 = nullptr;
-    if (wproj && n > 0 && s.wsel) {
+    if (use_wsel) {
         // the planes without sorting (k_wsel_*, see imager_kernels.cuh); a
         // condition it cannot meet sets error bit 16 and the caller grids
         // again on the sorting path
         const int P = s.nplanes;
         const unsigned g2 = std::min<unsigned>(grid1d(n, 256), 148 * 8);
-        WselState* ws = c->buf<WselState>("wsel", 1);
-        zero_words(st, { { ws, int64_t(kWselZeroWords) } });
-        k_wsel_hist<<<std::min<unsigned>(grid1d(n, 256), 148 * 4), 256, 0, st>>>(pp.absw_key, n, g.d_total, ws);
-        STPGPU_CHECK_LAUNCH();
-        static_assert(WSEL_BINS == 1024 * 64, "chunks of 64 bins, 32 a block");
-        k_wsel_chunks<<<32, 1024, 0, st>>>(ws);
-        STPGPU_CHECK_LAUNCH();
-        k_wsel_plan<<<1, 1024, 0, st>>>(ws, n, P, g.d_ngood, g.d_err);
+        static_assert(WSEL_BINS == 1024 * 64, "chunks of 64 bins, one per thread of the planning block");
+        k_wsel_hist<<<std::min<unsigned>(grid1d(n, 1024), 148), 1024, 0, st>>>(pp.absw_key, n, g.d_total, ws, P, g.d_ngood,
+            g.d_err);
         STPGPU_CHECK_LAUNCH();
         // members of the start bins: at most P - 1 bins of WSEL_CAP
         unsigned long long* mbits = c->buf<unsigned long long>("wsel_mb", size_t(std::max(P - 1, 1)) * WSEL_CAP);
@@ -774,11 +770,9 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
             STPGPU_CHECK_LAUNCH();
         }
         uint16_t* pl = c->buf<uint16_t>("wsel_plane", nn);
-        k_wsel_classify<<<g2, 256, 0, st>>>(pp.absw_key, n, P, g.d_total, ws, pl, g.d_err);
-        STPGPU_CHECK_LAUNCH();
         int64_t* first = c->buf<int64_t>("pfirst", P);
         double* w_avg = c->buf<double>("wavg", P);
-        k_wsel_finish<<<1, 256, 0, st>>>(ws, n, P, g.d_total, w_avg, first);
+        k_wsel_classify<<<g2, 256, 0, st>>>(pp.absw_key, n, P, g.d_total, ws, pl, g.d_err, w_avg, first);
         STPGPU_CHECK_LAUNCH();
         plane16 = pl;
         plane_first = first;
@@ -1013,10 +1007,10 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
         wk_off = c->buf<uint32_t>("wkoff", PT);
         if (aconv)
             k_aproj_expand<KT><<<dim3(PT, cs * cs), 256, 0, st>>>(aconv, arr, plane_support, cs, os, wk, wk_off,
-                g.d_err + 1);
+                g.d_err + CF_MAX_SUPPORT);
         else
             k_wk_expand<KT><<<dim3(P, cs * cs), 64, 0, st>>>(wq.convd, wq.invd, plane_support, P, cs, os, Lh, wk,
-                wk_off, g.d_err + 1);
+                wk_off, g.d_err + CF_MAX_SUPPORT);
         STPGPU_CHECK_LAUNCH();
         g.d_plane_support = plane_support;
         g.nplanes = PT;
@@ -1038,30 +1032,29 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
     in.ts_of = ts_of;
     in.wk_off = wk_off;
     in.wk = wk;
-    in.max_support = g.d_err + 1;
+    in.max_support = g.d_err + CF_MAX_SUPPORT;
     in.k1d = k1d64;
     in.frac = pp.frac;
-    grid_blocks<R, KT, ACC>(c, s, g, n, in, COMP == 1 && s.wide_fft);
+    grid_blocks<R, KT, ACC>(c, s, g, n, bins, in, COMP == 1 && s.wide_fft);
     return g;
 }
 
-struct ScalarsBack {
-    double total;
-    unsigned long long ngood;
-    uint32_t nitems;
-    unsigned int err;
-    int max_support;
-};
-
-ScalarsBack read_back(stpgpu_context* c, const GridOut& g)
+PackArgs pack_args(const GridOut& g, ScalarPack* out)
 {
-    // the scalars packed by one kernel straight into the page-locked stage
+    return PackArgs { g.d_total, g.d_ngood, g.d_nitems, g.d_err, g.d_plane_support, g.nplanes, out };
+}
+
+// The call's scalars, once its kernels are done.  packed: the normalisation
+// wrote them to the page-locked stage.
+ScalarPack read_back(stpgpu_context* c, const GridOut& g, bool packed)
+{
     ScalarPack* h = c->host_stage<ScalarPack>(1);
-    k_pack_scalars<<<1, 32, 0, c->stream>>>(g.d_total, g.d_ngood, g.d_nitems, g.d_err, g.d_plane_support,
-        g.nplanes > 0 ? g.nplanes : 0, c->host_stage_dev(h));
-    STPGPU_CHECK_LAUNCH();
+    if (!packed) {
+        k_pack_scalars<<<1, 32, 0, c->stream>>>(pack_args(g, c->host_stage_dev(h)));
+        STPGPU_CHECK_LAUNCH();
+    }
     STPGPU_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    ScalarsBack r { h->total, h->ngood, h->nitems, h->err, h->max_support };
+    const ScalarPack r = *h;
     // bit 4: the 32-bit |w| sort met a long run of distinct |w| (the caller
     // repeats the gridding with the 64-bit sort); bit 16: the W-planes
     // without the sort did not apply (the caller grids again on the sorting
@@ -1101,14 +1094,15 @@ const double* device_gcf(stpgpu_context* c, const ImagerSetup& s)
 }
 
 // c2r FFT + crop/normalise of a gridded snapshot (fft.cpp:45-135,
-// imager.h:97-213) on the context's current stream.
+// imager.h:97-213) on the context's current stream; the call's scalars go
+// to `pack`.
 template <typename R>
 void finish_imager(stpgpu_context* c, const ImagerSetup& s, int image_size, int correction, const GridOut& g,
-    void* d_image, void* d_beam, int out_f32)
+    void* d_image, void* d_beam, int out_f32, ScalarPack* pack)
 {
     if constexpr (sizeof(R) == 4) {
         if (s.wide_fft) { // the gridder wrote double2 cells: Z2D + double normalisation
-            finish_imager<double>(c, s, image_size, correction, g, d_image, d_beam, out_f32);
+            finish_imager<double>(c, s, image_size, correction, g, d_image, d_beam, out_f32, pack);
             return;
         }
     }
@@ -1134,32 +1128,33 @@ void finish_imager(stpgpu_context* c, const ImagerSetup& s, int image_size, int 
     const bool vec4 = (image_size % 8) == 0 && (N % 4) == 0
         && (reinterpret_cast<uintptr_t>(d_image) % 16) == 0 && (!d_beam || (reinterpret_cast<uintptr_t>(d_beam) % 16) == 0);
     const dim3 ngrid4(grid1d(image_size / 4, 256), (image_size + kNormCols - 1) / kNormCols);
-    auto normalise = [&](void* out) {
+    auto normalise = [&](void* out, ScalarPack* pk) {
+        const PackArgs pa = pack_args(g, pk);
         if (vec4) {
             if (out_f32)
                 k_normalise4<R, float><<<ngrid4, 256, 0, st>>>(img, N, image_size, g.d_total, ginv, correction,
-                    reinterpret_cast<float*>(out));
+                    reinterpret_cast<float*>(out), pa);
             else
                 k_normalise4<R, double><<<ngrid4, 256, 0, st>>>(img, N, image_size, g.d_total, ginv, correction,
-                    reinterpret_cast<double*>(out));
+                    reinterpret_cast<double*>(out), pa);
             STPGPU_CHECK_LAUNCH();
             return;
         }
         if (out_f32)
             k_normalise<R, float><<<ngrid, 256, 0, st>>>(img, N, image_size, g.d_total, ginv, correction,
-                reinterpret_cast<float*>(out));
+                reinterpret_cast<float*>(out), pa);
         else
             k_normalise<R, double><<<ngrid, 256, 0, st>>>(img, N, image_size, g.d_total, ginv, correction,
-                reinterpret_cast<double*>(out));
+                reinterpret_cast<double*>(out), pa);
         STPGPU_CHECK_LAUNCH();
     };
     exec(g.grid, img);
     c->mark(3);
-    normalise(d_image);
+    normalise(d_image, pack);
     c->mark(4);
     if (s.beam && d_beam) {
         exec(g.beam, img);
-        normalise(d_beam);
+        normalise(d_beam, nullptr);
     }
 }
 
@@ -1247,6 +1242,7 @@ void run_imager(stpgpu_context* c, const ImagerSetup& s_in, int image_size, int 
     if (s.wsel && c->wsel_off.count(cls))
         s.wsel = 0;
     GridOut g;
+    ScalarPack* pack = c->host_stage_dev(c->host_stage<ScalarPack>(1));
     // Device-pointer calls that repeat the previous call exactly (parameters,
     // sizes, buffers) replay a CUDA graph of the gridding, FFT and
     // normalisation kernels, captured on the first repeat; any other call
@@ -1261,7 +1257,7 @@ void run_imager(stpgpu_context* c, const ImagerSetup& s_in, int image_size, int 
         put(&vis_c64, sizeof(vis_c64));
         put(&n, sizeof(n));
         put(&out_f32, sizeof(out_f32));
-        const void* ptrs[6] = { d_vis, d_wts, d_uvw, d_image, d_beam, reinterpret_cast<const void*>(c->stream) };
+        const void* ptrs[7] = { d_vis, d_wts, d_uvw, d_image, d_beam, pack, reinterpret_cast<const void*>(c->stream) };
         put(ptrs, sizeof(ptrs));
     }
     const bool repeat = !sig.empty() && sig == c->single_sig;
@@ -1276,7 +1272,7 @@ void run_imager(stpgpu_context* c, const ImagerSetup& s_in, int image_size, int 
         STPGPU_CUDA_TRY(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
         try {
             g = run_gridder<R, COMP>(c, s, d_vis, vis_c64, d_wts, d_uvw, 0, n);
-            finish_imager<R>(c, s, image_size, correction, g, d_image, d_beam, out_f32);
+            finish_imager<R>(c, s, image_size, correction, g, d_image, d_beam, out_f32, pack);
         } catch (...) {
             cudaGraph_t dead = nullptr;
             cudaStreamEndCapture(c->stream, &dead);
@@ -1297,11 +1293,11 @@ void run_imager(stpgpu_context* c, const ImagerSetup& s_in, int image_size, int 
         g = run_gridder<R, COMP>(c, s, d_vis, vis_c64, d_wts, d_uvw, 0, n);
     }
     if (!(repeat && c->single_exec))
-        finish_imager<R>(c, s, image_size, correction, g, d_image, d_beam, out_f32);
+        finish_imager<R>(c, s, image_size, correction, g, d_image, d_beam, out_f32, pack);
     if (!sig.empty())
         c->single_sig = sig;
     const int N = s.N;
-    ScalarsBack sb = read_back(c, g);
+    ScalarPack sb = read_back(c, g, true);
     if (sb.err & 16u) {
         // the W-planes without the sort did not apply: the sorting path, for
         // this call and the size class's next ones
@@ -1309,16 +1305,16 @@ void run_imager(stpgpu_context* c, const ImagerSetup& s_in, int image_size, int 
         c->drop_single();
         s.wsel = 0;
         g = run_gridder<R, COMP>(c, s, d_vis, vis_c64, d_wts, d_uvw, 0, n);
-        finish_imager<R>(c, s, image_size, correction, g, d_image, d_beam, out_f32);
-        sb = read_back(c, g);
+        finish_imager<R>(c, s, image_size, correction, g, d_image, d_beam, out_f32, pack);
+        sb = read_back(c, g, true);
     }
     if ((sb.err & 4u) && !s.full_wsort) {
         // rare data (many distinct |w| within one single-precision step): redo with the 64-bit |w| sort
         ImagerSetup s64 = s;
         s64.full_wsort = 1;
         g = run_gridder<R, COMP>(c, s64, d_vis, vis_c64, d_wts, d_uvw, 0, n);
-        finish_imager<R>(c, s64, image_size, correction, g, d_image, d_beam, out_f32);
-        sb = read_back(c, g);
+        finish_imager<R>(c, s64, image_size, correction, g, d_image, d_beam, out_f32, pack);
+        sb = read_back(c, g, true);
     }
     if (info) {
         info->sample_grid_total = sb.total;
@@ -1464,9 +1460,10 @@ void batch_join(stpgpu_context* c, cudaStream_t main)
 
 // Enqueue one batch: every snapshot's whole pipeline (with host buffers, its
 // transfers too) on its worker stream, so that the snapshots overlap, and the
-// scalars of each read back into `scal` (pinned host memory).
+// scalars of each written to `scal` (the device's address of pinned host
+// memory).
 template <typename R, int COMP>
-void batch_enqueue(stpgpu_context* c, std::vector<BatchSnap>& B, int out_f32, int device_ptrs, BatchScalars* scal)
+void batch_enqueue(stpgpu_context* c, std::vector<BatchSnap>& B, int out_f32, int device_ptrs, ScalarPack* scal)
 {
     const cudaStream_t main = c->stream;
     const int nb = int(B.size());
@@ -1488,13 +1485,7 @@ void batch_enqueue(stpgpu_context* c, std::vector<BatchSnap>& B, int out_f32, in
             di = c->buf<unsigned char>("out_img", ob);
         }
         const GridOut g = run_gridder<R, COMP>(c, b.s, dv, b.c64, dw, duvw, 0, b.n);
-        finish_imager<R>(c, b.s, b.image_size, b.correction, g, di, nullptr, out_f32);
-        BatchScalars* ds = c->buf<BatchScalars>("scal", 1);
-        k_collect_scalars<<<1, 1, 0, c->stream>>>(g.d_total, g.d_ngood, g.d_nitems, g.d_err,
-            g.d_plane_support ? g.d_plane_support : reinterpret_cast<const int*>(g.d_err),
-            g.d_plane_support ? g.nplanes : 0, ds);
-        STPGPU_CHECK_LAUNCH();
-        STPGPU_CUDA_TRY(cudaMemcpyAsync(&scal[i], ds, sizeof(BatchScalars), cudaMemcpyDeviceToHost, c->stream));
+        finish_imager<R>(c, b.s, b.image_size, b.correction, g, di, nullptr, out_f32, scal + i);
         if (!device_ptrs)
             STPGPU_CUDA_TRY(cudaMemcpyAsync(b.image, di, ob, cudaMemcpyDeviceToHost, c->stream));
     }
@@ -1560,7 +1551,7 @@ void run_batch(stpgpu_context* c, const stpgpu_snapshot* sn, int nb, int precisi
     }
     c->batch_calls++;
     // pinned staging: the scalars read back
-    const size_t need = pad256(sizeof(BatchScalars) * nb) + 4096;
+    const size_t need = pad256(sizeof(ScalarPack) * nb) + 4096;
     if (c->batch_host_cap < need) {
         if (c->batch_host) {
             for (auto w : c->wstreams)
@@ -1574,7 +1565,9 @@ void run_batch(stpgpu_context* c, const stpgpu_snapshot* sn, int nb, int precisi
         STPGPU_CUDA_TRY(cudaMallocHost(&c->batch_host, need));
         c->batch_host_cap = need;
     }
-    BatchScalars* scal = reinterpret_cast<BatchScalars*>(c->batch_host);
+    ScalarPack* scal = reinterpret_cast<ScalarPack*>(c->batch_host);
+    ScalarPack* scal_dev = nullptr;
+    STPGPU_CUDA_TRY(cudaHostGetDevicePointer(reinterpret_cast<void**>(&scal_dev), scal, 0));
     const bool saved_timing = c->timing;
     c->timing = false;
     struct Restore {
@@ -1606,7 +1599,7 @@ void run_batch(stpgpu_context* c, const stpgpu_snapshot* sn, int nb, int precisi
             // capture the batch (buffers, plans and tables exist from the previous call)
             STPGPU_CUDA_TRY(cudaStreamBeginCapture(main, cudaStreamCaptureModeThreadLocal));
             try {
-                batch_enqueue<R, COMP>(c, B, out_f32, device_ptrs, scal);
+                batch_enqueue<R, COMP>(c, B, out_f32, device_ptrs, scal_dev);
             } catch (...) {
                 cudaGraph_t g = nullptr;
                 cudaStreamEndCapture(main, &g);
@@ -1626,7 +1619,7 @@ void run_batch(stpgpu_context* c, const stpgpu_snapshot* sn, int nb, int precisi
             graph = 1;
         } else {
             STPGPU_CUDA_TRY(cudaEventRecord(c->ev0, main));
-            batch_enqueue<R, COMP>(c, B, out_f32, device_ptrs, scal);
+            batch_enqueue<R, COMP>(c, B, out_f32, device_ptrs, scal_dev);
             STPGPU_CUDA_TRY(cudaEventRecord(c->ev1, main));
         }
     }
@@ -1649,7 +1642,7 @@ void run_batch(stpgpu_context* c, const stpgpu_snapshot* sn, int nb, int precisi
         c->batch_calls = 0;
         c->batch_sig.clear();
         STPGPU_CUDA_TRY(cudaEventRecord(c->ev0, main));
-        batch_enqueue<R, COMP>(c, B, out_f32, device_ptrs, scal);
+        batch_enqueue<R, COMP>(c, B, out_f32, device_ptrs, scal_dev);
         STPGPU_CUDA_TRY(cudaEventRecord(c->ev1, main));
         STPGPU_CUDA_TRY(cudaStreamSynchronize(main));
         graph = 0;
@@ -2623,11 +2616,11 @@ stpgpu_status stpgpu_convolve_to_grid(stpgpu_context* c, int kernel_function, do
         const double* dw = to_device<double>(c, "in_w", weights, size_t(n_vis));
         c->drop_single(); // this call reuses the imager's buffers
         GridOut g = run_gridder<double, 0>(c, s, dvis, 0, dw, duv, 1, n_vis);
-        ScalarsBack sb = read_back(c, g);
+        ScalarPack sb = read_back(c, g, false);
         if (sb.err & 4u) { // redo with the 64-bit |w| sort
             s.full_wsort = 1;
             g = run_gridder<double, 0>(c, s, dvis, 0, dw, duv, 1, n_vis);
-            sb = read_back(c, g);
+            sb = read_back(c, g, false);
         }
         const size_t cells = size_t(g.image_rows) * size_t(image_size);
         STPGPU_CUDA_TRY(cudaMemcpyAsync(vis_grid, g.grid, sizeof(double2) * cells, cudaMemcpyDeviceToHost, c->stream));

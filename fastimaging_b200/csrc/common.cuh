@@ -172,4 +172,25 @@ __host__ __device__ inline double kernel_zero_beyond(int kf, double trunc) { ret
 
 __host__ __device__ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
+// True in exactly one block, the last to finish the pass; every other
+// block's writes before the call are visible to it (the barrier, then one
+// fenced ticket per block, as in a grid-wide barrier).  Resets the ticket
+// for the next pass.
+__device__ __forceinline__ bool last_block(unsigned int* ticket)
+{
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const unsigned int t = atomicAdd(ticket, 1u);
+        last = t == gridDim.x - 1;
+        if (last) {
+            *ticket = 0;
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    return last;
+}
+
 } // namespace stpgpu

@@ -10,25 +10,11 @@
 #pragma once
 
 #include "common.cuh"
+#include "binning_kernels.cuh"
 
 namespace stpgpu {
 
 constexpr int GRID_THREADS = 256;
-
-// Per-visibility record written by the prepass.  flags: bit0 conj(kernel)
-// for the original item (w < 0), bit1 conj(kernel) for the mirrored item
-// (-w < 0).  The visibility is stored conjugated when the half-plane
-// conversion flipped it.  16-byte aligned (32 B single, 48 B double
-// precision): two or three 16-byte loads.
-template <typename R>
-struct alignas(16) Item {
-    R vr, vi, w;
-    int32_t gcx, gcy;
-    int16_t cpx, cpy;
-    uint16_t plane;
-    uint8_t good, flags;
-};
-static_assert(sizeof(Item<float>) == 32 && sizeof(Item<double>) == 48, "item record sizes");
 
 struct PrepassParams {
     int64_t n;
@@ -47,10 +33,58 @@ struct PrepassParams {
     double* w_out;    // n half-plane-converted w (W-proj), may be null
     double* wmax_part; // per block: the maximum and the sum of the finite |w| (W-proj), may be null
     uint32_t* iota;    // n identity permutation (W-proj), may be null
+    unsigned int* ticket; // blocks done (zeroed before)
+    double* total;        // results of the last block (finish_wsum)
+    unsigned long long* ngood;
 };
 
+// Sum of block partials in a fixed order (one block of GRID_THREADS).  out[0]
+// = 2 * sum (the half-plane doubling of gridder.h:423), out_n[0] = count;
+// with mpart, out[1] = the largest finite |w| and out[2] = the sum of the
+// finite |w|.
+__device__ __forceinline__ void finish_wsum(const double* part, const unsigned long long* npart, const double* mpart, int nb,
+    double* out, unsigned long long* out_n)
+{
+    __shared__ double s[GRID_THREADS], sm[GRID_THREADS], sa[GRID_THREADS];
+    __shared__ unsigned long long sn[GRID_THREADS];
+    double t = 0.0, m = 0.0, a = 0.0;
+    unsigned long long c = 0;
+    for (int k = threadIdx.x; k < nb; k += GRID_THREADS) {
+        t += __ldcg(part + k);
+        c += __ldcg(npart + k);
+        if (mpart) {
+            m = fmax(m, __ldcg(mpart + 2 * k));
+            a += __ldcg(mpart + 2 * k + 1);
+        }
+    }
+    s[threadIdx.x] = t;
+    sn[threadIdx.x] = c;
+    sm[threadIdx.x] = m;
+    sa[threadIdx.x] = a;
+    __syncthreads();
+    for (int o = GRID_THREADS / 2; o > 0; o >>= 1) {
+        if (int(threadIdx.x) < o) {
+            s[threadIdx.x] += s[threadIdx.x + o];
+            sn[threadIdx.x] += sn[threadIdx.x + o];
+            sm[threadIdx.x] = fmax(sm[threadIdx.x], sm[threadIdx.x + o]);
+            sa[threadIdx.x] += sa[threadIdx.x + o];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        out[0] = s[0] * 2.0;
+        out_n[0] = sn[0];
+        if (mpart) {
+            out[1] = sm[0];
+            out[2] = sa[0];
+        }
+    }
+}
+
+// b.count: null with W-projection (the footprints are not known yet), else
+// the entries are counted here.  The last block sums the blocks' partials.
 template <typename R>
-__global__ void k_prepass(PrepassParams p, Item<R>* items)
+__global__ void __launch_bounds__(GRID_THREADS) k_prepass(PrepassParams p, Item<R>* items, BlockBins b)
 {
     __shared__ double s_w[GRID_THREADS / 32];
     __shared__ unsigned long long s_n[GRID_THREADS / 32];
@@ -148,6 +182,8 @@ __global__ void k_prepass(PrepassParams p, Item<R>* items)
         if (good) {
             wgood = wt;
             ngood = 1;
+            if (b.count)
+                count_entries(b, it, i, b.support);
         }
     }
     // deterministic block partial sums
@@ -180,49 +216,8 @@ __global__ void k_prepass(PrepassParams p, Item<R>* items)
             p.wmax_part[2 * blockIdx.x + 1] = a;
         }
     }
-}
-
-// Sum of block partials in a fixed order (one block).  out[0] = 2 * sum
-// (the half-plane doubling of gridder.h:423), out_n[0] = count; with mpart,
-// out[1] = the largest finite |w| and out[2] = the sum of the finite |w|.
-__global__ void k_finish_wsum(const double* part, const unsigned long long* npart, const double* mpart, int nb,
-    double* out, unsigned long long* out_n)
-{
-    __shared__ double s[1024];
-    __shared__ unsigned long long sn[1024];
-    __shared__ double sm[1024], sa[1024];
-    double t = 0.0, m = 0.0, a = 0.0;
-    unsigned long long c = 0;
-    for (int k = threadIdx.x; k < nb; k += blockDim.x) {
-        t += part[k];
-        c += npart[k];
-        if (mpart) {
-            m = fmax(m, mpart[2 * k]);
-            a += mpart[2 * k + 1];
-        }
-    }
-    s[threadIdx.x] = t;
-    sn[threadIdx.x] = c;
-    sm[threadIdx.x] = m;
-    sa[threadIdx.x] = a;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) {
-            s[threadIdx.x] += s[threadIdx.x + o];
-            sn[threadIdx.x] += sn[threadIdx.x + o];
-            sm[threadIdx.x] = fmax(sm[threadIdx.x], sm[threadIdx.x + o]);
-            sa[threadIdx.x] += sa[threadIdx.x + o];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        out[0] = s[0] * 2.0;
-        out_n[0] = sn[0];
-        if (mpart) {
-            out[1] = sm[0];
-            out[2] = sa[0];
-        }
-    }
+    if (last_block(p.ticket))
+        finish_wsum(p.wsum_part, p.ngood_part, p.wmax_part, int(gridDim.x), p.total, p.ngood);
 }
 
 // Sort keys of |w| for the W-plane order, 24 bits, monotone in |w| (|a| <=
@@ -287,27 +282,6 @@ __global__ void k_zero_ranges(ZeroRanges z)
                 z.p[r][i] = 0;
 }
 
-template <typename R>
-__device__ __forceinline__ void item_centre(const Item<R>& it, int mir, int N, int& cx, int& cy)
-{
-    cx = mir ? N - it.gcx : it.gcx;
-    cy = mir ? N - it.gcy : it.gcy;
-}
-
-// W-plane of sorted position k: the last plane whose first position <= k.
-__device__ __forceinline__ int plane_of(const int64_t* first, int P, int64_t k)
-{
-    int lo = 0, hi = P - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) / 2;
-        if (first[mid] <= k)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    return lo;
-}
-
 // Exclusive scan of n counts into off[0..n] (single block of 1024 threads,
 // n up to a few hundred thousand).  off[n] = total.  Each thread first
 // loads 16 elements (16 coalesced rows of 1024), then the rows are scanned
@@ -359,11 +333,6 @@ __device__ __forceinline__ uint32_t scan_block_1024(const uint32_t* cnt, uint32_
     if (tid == 0)
         off[n] = carry;
     return carry;
-}
-
-__global__ void __launch_bounds__(1024) k_scan_single(const uint32_t* cnt, uint32_t* off, int n)
-{
-    scan_block_1024(cnt, off, n);
 }
 
 // One such scan per block: row blockIdx.x of cnt and off (row stride
@@ -452,6 +421,47 @@ __global__ void k_imgdom_kernel(int kf, double trunc, int n, int analytic, doubl
     out[i] = r;
 }
 
+// The scalars a call reads back: sampling-grid total, good visibilities,
+// binned entries, error flags and the largest plane support.  One warp
+// writes them straight into page-locked host memory through its device
+// address; the normalisation, a call's last kernel, does it in its first
+// block (out non-null), so that they cost no launch of their own.
+struct ScalarPack {
+    double total;
+    unsigned long long ngood;
+    uint32_t nitems;
+    unsigned int err;
+    int max_support;
+    int pad;
+};
+
+struct PackArgs {
+    const double* total;
+    const unsigned long long* ngood;
+    const uint32_t* nitems;
+    const unsigned int* err;
+    const int* sup;
+    int nsup;
+    ScalarPack* out;
+};
+
+__device__ __forceinline__ void pack_scalars(const PackArgs& k)
+{
+    int m = 0;
+    for (int i = threadIdx.x; i < k.nsup; i += 32)
+        m = max(m, k.sup[i]);
+    for (int o = 16; o > 0; o >>= 1)
+        m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (threadIdx.x == 0) {
+        k.out->total = *k.total;
+        k.out->ngood = *k.ngood;
+        k.out->nitems = *k.nitems;
+        k.out->err = *k.err;
+        k.out->max_support = m;
+        k.out->pad = 0;
+    }
+}
+
 // ---------------------------------------------------------------- normalise
 
 // normalise_image_beam_result_1D, non-FFTSHIFT branch (imager.h:97-150):
@@ -460,8 +470,10 @@ __global__ void k_imgdom_kernel(int kf, double trunc, int n, int analytic, doubl
 // factor 1/sum is read from the device (0 when the sampling total is 0).
 template <typename RI, typename RO>
 __global__ void __launch_bounds__(256) k_normalise(const RI* __restrict__ img, int padded, int image_size,
-    const double* total, const double* __restrict__ ginv, int corr, RO* __restrict__ out)
+    const double* total, const double* __restrict__ ginv, int corr, RO* __restrict__ out, PackArgs pk)
 {
+    if (pk.out && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 32)
+        pack_scalars(pk);
     const int j = blockIdx.y;
     const double tot = total[0];
     const double nf = tot > 0.0 ? 1.0 / tot : 0.0;
@@ -489,8 +501,10 @@ __global__ void __launch_bounds__(256) k_normalise(const RI* __restrict__ img, i
 constexpr int kNormCols = 8;
 template <typename RI, typename RO>
 __global__ void __launch_bounds__(256) k_normalise4(const RI* __restrict__ img, int padded, int image_size,
-    const double* total, const double* __restrict__ ginv, int corr, RO* __restrict__ out)
+    const double* total, const double* __restrict__ ginv, int corr, RO* __restrict__ out, PackArgs pk)
 {
+    if (pk.out && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 32)
+        pack_scalars(pk);
     const double tot = total[0];
     const double nf = tot > 0.0 ? 1.0 / tot : 0.0;
     const int hp = padded / 2, hs = image_size / 2;
@@ -755,14 +769,14 @@ __global__ void k_gather_good(const uint32_t* perm, const Item<R>* items, const 
 // p)), so an item's plane follows from how many plane-start items precede
 // it in the sort order ((|w| bits, input index), the stable order).  Those
 // P - 1 items are found without sorting: a histogram of the 24-bit keys'
-// top 12 bits (k_wsel_hist) places each start rank in a bin and at a rank
-// within it (k_wsel_plan); the members of those bins are collected
+// top 16 bits places each start rank in a bin and at a rank within it
+// (k_wsel_hist and, in its last block, wsel_plan); the members of those bins are collected
 // (k_wsel_collect) and each start item is the member of its bin with the
 // wanted rank under the exact order (k_wsel_resolve: every member counts the
 // members before it).  k_wsel_classify then gives every item its plane (a
 // binary search over the start items) and sums |w| per plane exactly, in
 // 64-bit fixed point relative to the plane's smallest |w| (so the sums do
-// not depend on the order of the additions); k_wsel_finish forms the means
+// not depend on the order of the additions); its last block forms the means
 // and plane starts.  Items not all good, non-finite |w|, more than WSEL_MAXP
 // planes or a start bin of more than WSEL_CAP members set bit 16 of the
 // error word: the host then runs the sorting path.
@@ -775,33 +789,21 @@ struct WselState {
     // zeroed before the pass
     uint32_t hist[WSEL_BINS];
     uint32_t cursor[WSEL_MAXP];
+    uint32_t tickets[2];
     unsigned long long sum[WSEL_MAXP];
-    // written by k_wsel_plan / k_wsel_resolve
+    // written by wsel_plan / k_wsel_resolve
     int32_t binmap[WSEL_BINS];      // list of a start bin, -1 otherwise
     uint32_t list_off[WSEL_MAXP + 1];
     uint32_t list_cnt[WSEL_MAXP];
     int32_t start_list[WSEL_MAXP];  // per plane p >= 1: its start item's list
     uint32_t start_rank[WSEL_MAXP]; // and rank within the list's bin
     uint32_t start_bin[WSEL_MAXP];
-    uint32_t chunk_tot[1024];       // bins per 64-bin chunk (k_wsel_chunks)
     unsigned long long start_bits[WSEL_MAXP]; // the start item: |w| bits, input index
     uint32_t start_idx[WSEL_MAXP];
     int64_t G[WSEL_MAXP + 1];
     int valid;
 };
-constexpr size_t kWselZeroWords = (sizeof(uint32_t) * (WSEL_BINS + WSEL_MAXP) + sizeof(unsigned long long) * WSEL_MAXP) / 4;
-
-// (the keys of k_wkey24, formed here and again in k_wsel_collect from |w|)
-__global__ void __launch_bounds__(256) k_wsel_hist(const double* __restrict__ absw, int64_t n, const double* total,
-    WselState* ws)
-{
-    const WKey kf(total, n);
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-        atomicAdd(&ws->hist[kf(absw[i]) >> (24 - WSEL_BINS_LOG)], 1u);
-    // no start bins yet (k_wsel_plan marks them)
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < WSEL_BINS; b += gridDim.x * blockDim.x)
-        ws->binmap[b] = -1;
-}
+constexpr size_t kWselZeroWords = (sizeof(uint32_t) * (WSEL_BINS + WSEL_MAXP + 2) + sizeof(unsigned long long) * WSEL_MAXP) / 4;
 
 // Exclusive scan over the 1024 threads of a block of the values v; *total =
 // their sum.
@@ -834,31 +836,26 @@ __device__ __forceinline__ uint32_t wsel_block_scan(uint32_t v, uint32_t* total)
     return r;
 }
 
-// Totals of the 1024 chunks of 64 bins, one warp a chunk (coalesced).
-__global__ void __launch_bounds__(1024) k_wsel_chunks(WselState* ws)
-{
-    const int c = blockIdx.x * 32 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const uint2 v = reinterpret_cast<const uint2*>(ws->hist + 64 * c)[lane];
-    uint32_t t = v.x + v.y;
-    for (int o = 16; o > 0; o >>= 1)
-        t += __shfl_down_sync(0xffffffffu, t, o);
-    if (lane == 0)
-        ws->chunk_tot[c] = t;
-}
-
 // One block of 1024 threads.  The plane starts have a closed form: with q =
 // n / P and r = n % P, ceil((n - G_p) / (P - p)) = q + [p < r], so G_p = p q +
-// min(p, r).  A block scan of the chunk totals (k_wsel_chunks) locates each
-// start rank's chunk, and the plane's thread walks the chunk's 64 bins to the
-// bin and the rank within it.  The start bins become lists in plane order.
-__global__ void __launch_bounds__(1024) k_wsel_plan(WselState* ws, int64_t n, int P, const unsigned long long* ngood,
-    unsigned int* err)
+// min(p, r).  A block scan of the totals of 1024 chunks of 64 bins locates
+// each start rank's chunk, and the plane's thread walks the chunk's bins to
+// the bin and the rank within it.  The start bins become lists in plane order.
+__device__ __forceinline__ void wsel_plan(WselState* ws, int64_t n, int P, const unsigned long long* ngood, unsigned int* err)
 {
     constexpr int PER = WSEL_BINS / 1024;
     __shared__ uint32_t chunk[1025]; // prefix at each thread's first bin
     const int tid = threadIdx.x;
     const bool ok0 = ngood[0] == (unsigned long long)n && P >= 1 && P <= WSEL_MAXP;
-    const uint32_t t = ws->chunk_tot[tid];
+    uint32_t t = 0;
+    {
+        const uint4* c4 = reinterpret_cast<const uint4*>(ws->hist + PER * tid);
+#pragma unroll
+        for (int q = 0; q < PER / 4; q++) {
+            const uint4 v = __ldcg(c4 + q);
+            t += v.x + v.y + v.z + v.w;
+        }
+    }
     uint32_t total = 0;
     const uint32_t excl = wsel_block_scan(t, &total);
     chunk[tid] = excl;
@@ -889,7 +886,7 @@ __global__ void __launch_bounds__(1024) k_wsel_plan(WselState* ws, int64_t n, in
         uint32_t before = chunk[lo];
         bool found = false;
         for (int q = 0; q < PER / 4 && !found; q++) {
-            const uint4 v = c4[q];
+            const uint4 v = __ldcg(c4 + q);
             const uint32_t w[4] = { v.x, v.y, v.z, v.w };
             for (int e = 0; e < 4; e++) {
                 if (before + w[e] > gp) { // rank gp lies in this bin
@@ -948,6 +945,21 @@ __global__ void __launch_bounds__(1024) k_wsel_plan(WselState* ws, int64_t n, in
         ws->list_off[nlist] = noff;
         ws->valid = 1;
     }
+}
+
+// Histogram of the 24-bit keys (those of k_wkey24, formed here and again in
+// k_wsel_collect from |w|), then the plan by the last block.
+__global__ void __launch_bounds__(1024) k_wsel_hist(const double* __restrict__ absw, int64_t n, const double* total,
+    WselState* ws, int P, const unsigned long long* ngood, unsigned int* err)
+{
+    const WKey kf(total, n);
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+        atomicAdd(&ws->hist[kf(absw[i]) >> (24 - WSEL_BINS_LOG)], 1u);
+    // no start bins yet (the plan marks them)
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < WSEL_BINS; b += gridDim.x * blockDim.x)
+        ws->binmap[b] = -1;
+    if (last_block(&ws->tickets[0]))
+        wsel_plan(ws, n, P, ngood, err);
 }
 
 __global__ void __launch_bounds__(256) k_wsel_collect(const double* __restrict__ absw, int64_t n, const double* total,
@@ -1023,7 +1035,7 @@ __device__ __forceinline__ void wsel_range(const WselState* ws, int p, int P, in
 }
 
 __global__ void __launch_bounds__(256) k_wsel_classify(const double* __restrict__ absw, int64_t n, int P,
-    const double* total, WselState* ws, uint16_t* plane16, unsigned int* err)
+    const double* total, WselState* ws, uint16_t* plane16, unsigned int* err, double* w_avg, int64_t* first)
 {
     __shared__ unsigned long long sbits[WSEL_MAXP];
     __shared__ uint32_t sidx[WSEL_MAXP];
@@ -1038,6 +1050,11 @@ __global__ void __launch_bounds__(256) k_wsel_classify(const double* __restrict_
         // (the host grids again on the sorting path)
         for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
             plane16[i] = 0;
+        if (blockIdx.x == 0)
+            for (int p = threadIdx.x; p < P; p += blockDim.x) {
+                w_avg[p] = 0.0;
+                first[p] = 0;
+            }
         return;
     }
     const double wmax = total[1];
@@ -1083,25 +1100,13 @@ __global__ void __launch_bounds__(256) k_wsel_classify(const double* __restrict_
         if (v)
             atomicAdd(&ws->sum[p], v);
     }
-}
-
-__global__ void __launch_bounds__(256) k_wsel_finish(const WselState* ws, int64_t n, int P, const double* total,
-    double* w_avg, int64_t* first)
-{
-    if (!ws->valid) {
+    // the last block: plane means and starts
+    if (last_block(&ws->tickets[1]))
         for (int p = threadIdx.x; p < P; p += blockDim.x) {
-            w_avg[p] = 0.0;
-            first[p] = 0;
+            const int64_t cnt = ws->G[p + 1] - ws->G[p];
+            w_avg[p] = cnt > 0 ? slo[p] + (double(__ldcg(&ws->sum[p])) / sscale[p]) / double(cnt) : 0.0;
+            first[p] = ws->G[p];
         }
-        return;
-    }
-    for (int p = threadIdx.x; p < P; p += blockDim.x) {
-        double lo, scale;
-        wsel_range(ws, p, P, n, total[1], lo, scale);
-        const int64_t cnt = ws->G[p + 1] - ws->G[p];
-        w_avg[p] = cnt > 0 ? lo + (double(ws->sum[p]) / scale) / double(cnt) : 0.0;
-        first[p] = ws->G[p];
-    }
 }
 
 // The |w| order from a stable sort on the 24-bit keys of k_wkey24 is exact
@@ -1527,35 +1532,6 @@ __global__ void k_cos_table(int arr, double* c)
         c[t] = cospi(2.0 * double(t) / double(arr));
 }
 
-// FP32 copies of the W-kernel tables for the single-precision gridders.
-// Per-snapshot scalars of a batch, gathered for one read-back.
-struct BatchScalars {
-    double total;
-    unsigned long long ngood;
-    uint32_t nitems;
-    uint32_t err;
-    int32_t max_support;
-    int32_t pad;
-};
-
-__global__ void k_collect_scalars(const double* total, const unsigned long long* ngood, const uint32_t* nitems,
-    const unsigned int* err, const int* psup, int nplanes, BatchScalars* out)
-{
-    if (threadIdx.x != 0 || blockIdx.x != 0)
-        return;
-    BatchScalars b;
-    b.total = total[0];
-    b.ngood = ngood[0];
-    b.nitems = nitems[0];
-    b.err = err[0];
-    int m = 0;
-    for (int p = 0; p < nplanes; p++)
-        m = max(m, psup[p]);
-    b.max_support = m;
-    b.pad = 0;
-    *out = b;
-}
-
 // Expanded W-kernel tables for the gridder: one block per (plane, oversampled
 // offset pair); entry j*K + i (column j, row i) holds the reference's cached
 // kernel value conv(|oy|, |ox|) * inv (aw_projection.cpp:415-448), formed in
@@ -1596,18 +1572,6 @@ __global__ void k_wk_expand(const double2* convd, const double* invd, const int*
     }
 }
 
-// The scalars a call reads back, gathered for one copy: sampling-grid
-// total, good visibilities, tile-list entries, error flags and the largest
-// plane support (one warp).
-struct ScalarPack {
-    double total;
-    unsigned long long ngood;
-    uint32_t nitems;
-    unsigned int err;
-    int max_support;
-    int pad;
-};
-
 // Copies of a call's results into page-locked host memory through its device
 // address: the na words of a, then the 16-byte units of b that hold the
 // first a[count_word] records of rec_bytes each (all nb units when
@@ -1625,22 +1589,6 @@ __global__ void k_copy_out(const uint32_t* a, uint32_t* ha, int na, const uint4*
         hb[i] = b[i];
 }
 
-__global__ void k_pack_scalars(const double* total, const unsigned long long* ngood, const uint32_t* nitems,
-    const unsigned int* err, const int* sup, int nsup, ScalarPack* out)
-{
-    int m = 0;
-    for (int i = threadIdx.x; i < nsup; i += 32)
-        m = max(m, sup[i]);
-    for (int o = 16; o > 0; o >>= 1)
-        m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (threadIdx.x == 0) {
-        out->total = *total;
-        out->ngood = *ngood;
-        out->nitems = *nitems;
-        out->err = *err;
-        out->max_support = m;
-        out->pad = 0;
-    }
-}
+__global__ void __launch_bounds__(32) k_pack_scalars(PackArgs k) { pack_scalars(k); }
 
 } // namespace stpgpu

@@ -175,27 +175,6 @@ struct SfStats {
     unsigned int stats_err; // the fused statistics kernel gave up at a grid barrier: the pass kernels must run
 };
 
-// True in exactly one block, the last to finish the pass; every other
-// block's writes before the call are visible to it (the barrier, then one
-// fenced ticket per block, as in a grid-wide barrier).  Resets the ticket
-// for the next pass.
-__device__ __forceinline__ bool last_block(unsigned int* ticket)
-{
-    __shared__ bool last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const unsigned int t = atomicAdd(ticket, 1u);
-        last = t == gridDim.x - 1;
-        if (last) {
-            *ticket = 0;
-            __threadfence();
-        }
-    }
-    __syncthreads();
-    return last;
-}
-
 // Sum NV-wide partials of nb blocks in a fixed order (one block of BT
 // threads: strided sums, warp trees, warps in order); the result is valid in
 // every thread.
