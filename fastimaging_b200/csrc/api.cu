@@ -398,6 +398,7 @@ std::string fkey(double v)
 }
 
 constexpr size_t pad256(size_t b) { return (b + 255) / 256 * 256; }
+constexpr size_t pad16(size_t b) { return (b + 15) / 16 * 16; }
 
 inline unsigned grid1d(int64_t n, int threads) { return unsigned(std::max<int64_t>(1, ceil_div(n, threads))); }
 
@@ -684,7 +685,7 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
 
     // ---- prepass (gridder.h:369-423, :504)
     Item<R>* items = c->buf<Item<R>>("items", nn);
-    const unsigned nb_pre = grid1d(n, GRID_THREADS);
+    const unsigned nb_pre = std::min<unsigned>(grid1d(n, GRID_THREADS), 148 * 8);
     double* wpart = c->buf<double>("wpart", nb_pre);
     unsigned long long* npart = c->buf<unsigned long long>("npart", nb_pre);
     g.d_total = c->buf<double>("total", 4);
@@ -827,7 +828,8 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
         int64_t* first = c->buf<int64_t>("pfirst", P);
         int64_t* last = c->buf<int64_t>("plast", P);
         double* w_avg = c->buf<double>("wavg", P);
-        k_wplanes<<<1, 1, 0, st>>>(cgood, absw_sorted, n, P, s.wmedian, first, last);
+        k_wplanes<<<std::min<unsigned>(grid1d(n, 256), 148 * 4), 256, 0, st>>>(cgood, n, P, c->buf<uint32_t>("goodpos", nn),
+            g.d_err + CF_TICKET, first, last);
         STPGPU_CHECK_LAUNCH();
         if (s.wmedian) {
             k_wplane_values<<<P, 256, 0, st>>>(cgood, absw_sorted, good_sorted, first, last, n, P, 1, w_avg);
@@ -983,9 +985,21 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
             hq.Cp = c->buf<double>("hkC", size_t(P) * 2 * hq.n);
             k_hankel_plane<<<P, 1024, 0, st>>>(wq, hq);
         } else {
-            const size_t ct_bytes = sizeof(double) * size_t(arr);
-            wq.ctab_in_smem = ct_bytes <= 24 * 1024;
-            k_wkernel_plane<<<P, 1024, wq.ctab_in_smem ? ct_bytes : 0, st>>>(wq);
+            // shared memory: the cosine table, Q and T in this order of
+            // preference (a kernel of 16 cells' support and oversampling 8
+            // takes 4 + 16 + 66 KB)
+            size_t smem = 0;
+            auto fits = [&](size_t bytes) {
+                if (smem + bytes > 160 * 1024)
+                    return 0;
+                smem += bytes;
+                return 1;
+            };
+            wq.smem_ctab = fits(pad16(sizeof(double) * size_t(arr)));
+            wq.smem_Q = fits(sizeof(double2) * size_t(half) * half);
+            wq.smem_T = fits(sizeof(double2) * size_t(Lh) * half);
+            STPGPU_CUDA_TRY(cudaFuncSetAttribute(k_wkernel_plane, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+            k_wkernel_plane<<<P, 1024, smem, st>>>(wq);
         }
         STPGPU_CHECK_LAUNCH();
         // per-offset K x K tables in the gridder's precision: worst-case
@@ -1009,8 +1023,8 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
             k_aproj_expand<KT><<<dim3(PT, cs * cs), 256, 0, st>>>(aconv, arr, plane_support, cs, os, wk, wk_off,
                 g.d_err + CF_MAX_SUPPORT);
         else
-            k_wk_expand<KT><<<dim3(P, cs * cs), 64, 0, st>>>(wq.convd, wq.invd, plane_support, P, cs, os, Lh, wk,
-                wk_off, g.d_err + CF_MAX_SUPPORT);
+            k_wk_expand<KT><<<dim3(P, cs * cs), 64, 0, st>>>(wq.convd, wq.invd, plane_support, P, cs, os, Lh,
+                large_support(s) ? 0u : uint32_t(cs * cs) * uint32_t(K * K), wk, wk_off, g.d_err + CF_MAX_SUPPORT);
         STPGPU_CHECK_LAUNCH();
         g.d_plane_support = plane_support;
         g.nplanes = PT;

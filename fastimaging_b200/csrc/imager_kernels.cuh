@@ -89,10 +89,10 @@ __global__ void __launch_bounds__(GRID_THREADS) k_prepass(PrepassParams p, Item<
     __shared__ double s_w[GRID_THREADS / 32];
     __shared__ unsigned long long s_n[GRID_THREADS / 32];
     __shared__ double s_m[GRID_THREADS / 32], s_a[GRID_THREADS / 32];
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     double wgood = 0.0, wmax = 0.0, wabs = 0.0;
     unsigned long long ngood = 0;
-    if (i < p.n) {
+    // a bounded number of blocks: the last one sums their partials
+    for (int64_t i = int64_t(blockIdx.x) * GRID_THREADS + threadIdx.x; i < p.n; i += int64_t(gridDim.x) * GRID_THREADS) {
         double u, v, w = 0.0;
         if (p.uv_is_pixels) {
             u = p.uv[i];
@@ -160,8 +160,8 @@ __global__ void __launch_bounds__(GRID_THREADS) k_prepass(PrepassParams p, Item<
         if (p.absw_key)
             p.absw_key[i] = fabs(w);
         if (fabs(w) <= 1.7976931348623157e308) { // finite
-            wmax = fabs(w);
-            wabs = fabs(w);
+            wmax = fmax(wmax, fabs(w));
+            wabs += fabs(w);
         }
         if (p.iota)
             p.iota[i] = uint32_t(i);
@@ -180,8 +180,8 @@ __global__ void __launch_bounds__(GRID_THREADS) k_prepass(PrepassParams p, Item<
         it.flags = uint8_t((w < 0.0 ? 1 : 0) | (-w < 0.0 ? 2 : 0));
         items[i] = it;
         if (good) {
-            wgood = wt;
-            ngood = 1;
+            wgood += wt;
+            ngood++;
             if (b.count)
                 count_entries(b, it, i, b.support);
         }
@@ -574,49 +574,39 @@ __global__ void k_reciprocal(const double* in, double* out, int n)
 
 // ---------------------------------------------------------------- W-projection
 
-// Plane boundaries and plane w (average_w_planes, gridder.cpp:68-146) from the
-// |w|-sorted order: cgood[k] = number of good visibilities among sorted[0..k).
-__global__ void k_wplanes(const uint32_t* cgood, const double* absw_sorted, int64_t n, int P, int median,
-    int64_t* first, int64_t* last)
+// Plane boundaries (average_w_planes, gridder.cpp:68-146) from the |w|-sorted
+// order: cgood[k] = number of good visibilities among sorted[0..k).  A plane
+// ends behind its last good visibility, so the boundaries are a chain with
+// one look-up per plane in goodpos (sorted position of every good
+// visibility), which all blocks fill and the last one then follows.  (A
+// binary search in cgood per plane: 199 us for 64 planes of 333k.)
+__global__ void __launch_bounds__(256) k_wplanes(const uint32_t* __restrict__ cgood, int64_t n, int P, uint32_t* goodpos,
+    unsigned int* ticket, int64_t* first, int64_t* last)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0)
+    for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += int64_t(gridDim.x) * blockDim.x) {
+        const uint32_t g = cgood[k];
+        if (cgood[k + 1] != g)
+            goodpos[g] = uint32_t(k);
+    }
+    if (!last_block(ticket) || threadIdx.x != 0)
         return;
     const uint64_t G = cgood[n];
-    uint64_t begin = 0;
-    if (G == uint64_t(n)) {
-        // every visibility is in bounds: sorted position == good count
-        for (int idx = 0; idx < P; idx++) {
-            const uint64_t plane_size = uint64_t(ceil(double(G - begin) / (P - idx)));
-            const uint64_t lo = min(uint64_t(n), begin + plane_size);
-            first[idx] = int64_t(begin);
-            last[idx] = int64_t(lo);
-            begin = lo;
-        }
-        return;
-    }
+    uint64_t begin = 0, before = 0; // good visibilities before `begin`
     for (int idx = 0; idx < P; idx++) {
-        uint64_t plane_size = uint64_t(ceil(double(G - begin) / (P - idx)));
-        // k: first index with cgood[k] == cgood[begin] + plane_size (or n)
-        const uint64_t remaining = uint64_t(cgood[n]) - uint64_t(cgood[begin]);
-        uint64_t lo = begin, hi = uint64_t(n);
+        const uint64_t plane_size = uint64_t(ceil(double(G - begin) / (P - idx)));
+        const uint64_t remaining = G - before;
+        uint64_t end = begin;
         if (plane_size > remaining) {
-            lo = uint64_t(n);
-        } else {
-            const uint64_t target = uint64_t(cgood[begin]) + plane_size;
-            while (lo < hi) {
-                uint64_t mid = (lo + hi) / 2;
-                if (uint64_t(cgood[mid]) >= target)
-                    hi = mid;
-                else
-                    lo = mid + 1;
-            }
+            end = uint64_t(n);
+            before = G;
+        } else if (plane_size > 0) {
+            before += plane_size;
+            end = uint64_t(__ldcg(goodpos + before - 1)) + 1;
         }
         first[idx] = int64_t(begin);
-        last[idx] = int64_t(lo);
-        begin = lo;
+        last[idx] = int64_t(end);
+        begin = end;
     }
-    (void)absw_sorted;
-    (void)median;
 }
 
 // One block per plane: plane w = mean |w| over good visibilities (or the
@@ -847,15 +837,24 @@ __device__ __forceinline__ void wsel_plan(WselState* ws, int64_t n, int P, const
     __shared__ uint32_t chunk[1025]; // prefix at each thread's first bin
     const int tid = threadIdx.x;
     const bool ok0 = ngood[0] == (unsigned long long)n && P >= 1 && P <= WSEL_MAXP;
-    uint32_t t = 0;
+    // totals of the 1024 chunks of 64 bins: half a warp a chunk, so that a
+    // load covers two whole chunks (a thread reading its own chunk touches 32
+    // lines per load)
     {
-        const uint4* c4 = reinterpret_cast<const uint4*>(ws->hist + PER * tid);
-#pragma unroll
-        for (int q = 0; q < PER / 4; q++) {
-            const uint4 v = __ldcg(c4 + q);
-            t += v.x + v.y + v.z + v.w;
+        const int lane = tid & 31, warp = tid >> 5;
+        const uint4* c4 = reinterpret_cast<const uint4*>(ws->hist) + warp * (32 * PER / 4);
+#pragma unroll 8
+        for (int c = 0; c < 32; c += 2) {
+            const uint4 v = __ldcg(c4 + c * (PER / 4) + lane);
+            uint32_t t = v.x + v.y + v.z + v.w;
+            for (int o = 8; o > 0; o >>= 1)
+                t += __shfl_xor_sync(0xffffffffu, t, o);
+            if ((lane & 15) == 0)
+                chunk[warp * 32 + c + (lane >> 4)] = t;
         }
+        __syncthreads();
     }
+    const uint32_t t = chunk[tid];
     uint32_t total = 0;
     const uint32_t excl = wsel_block_scan(t, &total);
     chunk[tid] = excl;
@@ -867,12 +866,15 @@ __device__ __forceinline__ void wsel_plan(WselState* ws, int64_t n, int P, const
         for (int p = tid; p <= P; p += blockDim.x)
             ws->G[p] = G(p);
     __syncthreads();
-    // plane p = tid: its start item's bin (the last b whose prefix is <= G_p)
-    // and rank within it, and the bin's size
-    const int p = tid;
-    const bool has = ok0 && p >= 1 && p < P && G(p) < n;
-    uint32_t bin = 0, m = 0;
-    if (has) {
+    // each plane's start item: its bin (the last b whose prefix is <= G_p), the
+    // rank within it and the bin's size.  One warp per plane, two bins of the
+    // start's chunk a lane: a thread walking the chunk alone waits for up to
+    // 16 loads in turn (19 us of a 5k-visibility call)
+    __shared__ uint32_t ssize[1024], srank[1024], sbin[1024];
+    const int lane = tid & 31;
+    for (int p = tid >> 5; p < 1024; p += 32) {
+        if (!(ok0 && p >= 1 && p < P && G(p) < n))
+            continue;
         const uint32_t gp = uint32_t(G(p));
         int lo = 0, hi = 1023;
         while (lo < hi) {
@@ -882,28 +884,34 @@ __device__ __forceinline__ void wsel_plan(WselState* ws, int64_t n, int P, const
             else
                 hi = mid - 1;
         }
-        const uint4* c4 = reinterpret_cast<const uint4*>(ws->hist + PER * lo);
-        uint32_t before = chunk[lo];
-        bool found = false;
-        for (int q = 0; q < PER / 4 && !found; q++) {
-            const uint4 v = __ldcg(c4 + q);
-            const uint32_t w[4] = { v.x, v.y, v.z, v.w };
-            for (int e = 0; e < 4; e++) {
-                if (before + w[e] > gp) { // rank gp lies in this bin
-                    bin = uint32_t(PER * lo + 4 * q + e);
-                    m = w[e];
-                    found = true;
-                    break;
-                }
-                before += w[e];
-            }
+        const uint2 v = __ldcg(reinterpret_cast<const uint2*>(ws->hist + PER * lo) + lane);
+        uint32_t x = v.x + v.y;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o)
+                x += y;
         }
-        ws->start_bin[p] = bin;
-        ws->start_rank[p] = gp - before;
+        const uint32_t end = chunk[lo] + x; // entries up to the lane's second bin
+        const int at = __ffs(int(__ballot_sync(0xffffffffu, end > gp))) - 1;
+        if (lane == at) {
+            const uint32_t first = end - v.x - v.y; // before the lane's first bin
+            const bool second = first + v.x <= gp;
+            sbin[p] = uint32_t(PER * lo + 2 * lane) + (second ? 1u : 0u);
+            srank[p] = gp - (second ? first + v.x : first);
+            ssize[p] = second ? v.y : v.x;
+        }
     }
-    __shared__ uint32_t sbin[1024];
+    __syncthreads();
+    const int p = tid;
+    const bool has = ok0 && p >= 1 && p < P && G(p) < n;
+    const uint32_t bin = has ? sbin[p] : 0u, m = has ? ssize[p] : 0u;
+    if (has) {
+        ws->start_bin[p] = bin;
+        ws->start_rank[p] = srank[p];
+    }
     __shared__ int bad;
-    sbin[tid] = bin;
+    if (!has)
+        sbin[tid] = 0;
     if (tid == 0)
         bad = !ok0;
     __syncthreads();
@@ -1188,7 +1196,7 @@ struct WkParams {
     const double* aa; // image-domain AA kernel over the workarea
     const double* ctab; // cos(2 pi t / arr), t < arr
     int half, arr, os, cs, max_support, lh_max;
-    int ctab_in_smem; // k_wkernel_plane: launched with arr doubles of dynamic shared memory
+    int smem_ctab, smem_Q, smem_T; // k_wkernel_plane: what the launch's dynamic shared memory holds
     double scaled_cell, trunc_perc;
     double2* Qs;   // scratch [P][half][half]
     double2* Ts;   // scratch [P][lh_max][half]
@@ -1213,48 +1221,82 @@ __device__ __forceinline__ double2 wk_value(const WkParams& q, double w, int px,
     return make_double2(re * q.aa[half + py], im * q.aa[half + py]);
 }
 
-// 1/sum(Re) of each oversampled sub-kernel of plane p (ty outer, tx inner as
-// in generate_kernel_cache, aw_projection.cpp:383-448); conv is the plane's
-// quadrant conv[|dy| * lh + |dx|].
+// 1/sum(Re) of each oversampled sub-kernel of plane p (generate_kernel_cache,
+// aw_projection.cpp:383-448); conv is the plane's quadrant
+// conv[|dy| * lh + |dx|].  One warp per sub-kernel: its K^2 loads are spread
+// over the lanes instead of being one thread's chain.
 __device__ void wk_inverse_sums(const WkParams& q, int p, const double2* conv, int S)
 {
     const int cs = q.cs, os = q.os, lh = q.lh_max;
     const int K = 2 * S + 1;
-    for (int t = threadIdx.x; t < cs * cs; t += blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    for (int t = threadIdx.x >> 5; t < cs * cs; t += blockDim.x >> 5) {
         const int x = t % cs, y = t / cs;
         double ks = 0.0;
-        for (int j = 0; j < K; j++) {
-            int ox = (j - S) * os + os / 2 - x;
+        for (int e = lane; e < K * K; e += 32) {
+            int ox = (e / K - S) * os + os / 2 - x;
+            int oy = (e % K - S) * os + os / 2 - y;
             ox = ox < 0 ? -ox : ox;
-            for (int i = 0; i < K; i++) {
-                int oy = (i - S) * os + os / 2 - y;
-                oy = oy < 0 ? -oy : oy;
-                ks += conv[size_t(oy) * lh + ox].x;
-            }
+            oy = oy < 0 ? -oy : oy;
+            ks += conv[size_t(oy) * lh + ox].x;
         }
-        q.invd[(size_t(p) * cs + y) * cs + x] = 1 / ks;
+        for (int o = 16; o > 0; o >>= 1)
+            ks += __shfl_xor_sync(0xffffffffu, ks, o);
+        if (lane == 0)
+            q.invd[(size_t(p) * cs + y) * cs + x] = 1 / ks;
     }
 }
 
+// sum_a m_a V[a * stride] cos(2 pi k a / arr), m_0 = 1, m_{>0} = 2
+__device__ __forceinline__ double2 cos_sum(const double2* V, int stride, int half, const double* ct, int k, int arr)
+{
+    double re = 0.0, im = 0.0;
+    int at = 0; // k a mod arr
+#pragma unroll 4
+    for (int a = 0; a < half; a++) {
+        const double c = (a == 0 ? 1.0 : 2.0) * ct[at];
+        const double2 v = V[size_t(a) * stride];
+        re += v.x * c;
+        im += v.y * c;
+        at += k;
+        at = at >= arr ? at - arr : at;
+    }
+    return make_double2(re, im);
+}
+
+// A plane's steps are a chain of short sums, so latency bounds them: the
+// cosine table, the image-domain quadrant Q and its row transforms T are kept
+// in shared memory where they fit (q.smem_*; the launch gives the room), the
+// position in the cosine table is carried instead of reduced modulo arr at
+// every term, and the truncation test runs in all threads.
 __global__ void __launch_bounds__(1024) k_wkernel_plane(WkParams q)
 {
     const int p = blockIdx.x;
     const int half = q.half, arr = q.arr, os = q.os, lh = q.lh_max;
     const double w = q.w_avg[p];
-    double2* Q = q.Qs + size_t(p) * half * half;
-    double2* T = q.Ts + size_t(p) * lh * half;
-    double2* conv = q.convd + size_t(p) * lh * lh;
     __shared__ double2 row0[1024];
     __shared__ int s_support;
-    // the cosine table in shared memory when the launch gave room for it
-    extern __shared__ double sct[];
-    const double* ct = q.ctab;
-    if (q.ctab_in_smem) {
-        for (int t = threadIdx.x; t < arr; t += blockDim.x)
-            sct[t] = q.ctab[t];
-        ct = sct;
+    extern __shared__ __align__(16) double sct[];
+    // 16-byte cells first, then the cosine table
+    double2* sm = reinterpret_cast<double2*>(sct);
+    double2* Q = q.Qs + size_t(p) * half * half;
+    double2* T = q.Ts + size_t(p) * lh * half;
+    if (q.smem_Q) {
+        Q = sm;
+        sm += size_t(half) * half;
     }
-    auto C = [&](int t) { return ct[t % arr]; };
+    if (q.smem_T) {
+        T = sm;
+        sm += size_t(lh) * half;
+    }
+    double2* conv = q.convd + size_t(p) * lh * lh;
+    const double* ct = q.ctab;
+    if (q.smem_ctab) {
+        double* sc = reinterpret_cast<double*>(sm);
+        for (int t = threadIdx.x; t < arr; t += blockDim.x)
+            sc[t] = q.ctab[t];
+        ct = sc;
+    }
     // 1. image-domain quadrant Q[a][b] (row a, column b)
     for (int t = threadIdx.x; t < half * half; t += blockDim.x) {
         const int a = t % half, b = t / half;
@@ -1269,76 +1311,43 @@ __global__ void __launch_bounds__(1024) k_wkernel_plane(WkParams q)
             v = wk_value(q, w, a, b);
         Q[size_t(b) * half + a] = v;
     }
+    if (threadIdx.x == 0)
+        s_support = 0;
     __syncthreads();
     // 2. T[0][a] = sum_b m_b Q[a][b]
-    for (int a = threadIdx.x; a < half; a += blockDim.x) {
-        double re = 0.0, im = 0.0;
-        for (int b = 0; b < half; b++) {
-            const double m = b == 0 ? 1.0 : 2.0;
-            const double2 v = Q[size_t(b) * half + a];
-            re += v.x * m;
-            im += v.y * m;
-        }
-        T[a] = make_double2(re, im);
-    }
+    for (int a = threadIdx.x; a < half; a += blockDim.x)
+        T[a] = cos_sum(Q + a, half, half, ct, 0, arr);
     __syncthreads();
     // 3. conv(k, 0) at k = i*os for the truncation (k <= arr/2)
     const int kmax0 = min(q.max_support * os, arr >> 1);
     const int nrow = kmax0 / os + 1;
-    for (int t = threadIdx.x; t < nrow && t < 1024; t += blockDim.x) {
-        const int k = t * os;
-        double re = 0.0, im = 0.0;
-        for (int a = 0; a < half; a++) {
-            const double c = (a == 0 ? 1.0 : 2.0) * C(k * a);
-            re += T[a].x * c;
-            im += T[a].y * c;
-        }
-        row0[t] = make_double2(re, im);
+    for (int t = threadIdx.x; t < nrow && t < 1024; t += blockDim.x)
+        row0[t] = cos_sum(T, 1, half, ct, t * os, arr);
+    __syncthreads();
+    if (q.trunc_perc > 0.0) {
+        // the last sample above the threshold (0 when none is)
+        const double minv = hypot(row0[0].x, row0[0].y) * (q.trunc_perc / 100.0);
+        for (int t = 1 + threadIdx.x; t < nrow && t < 1024; t += blockDim.x)
+            if (hypot(row0[t].x, row0[t].y) > minv)
+                atomicMax(&s_support, t);
+    } else if (threadIdx.x == 0) {
+        s_support = q.max_support;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int S = q.max_support;
-        if (q.trunc_perc > 0.0) {
-            const double minv = hypot(row0[0].x, row0[0].y) * (q.trunc_perc / 100.0);
-            unsigned i = unsigned(kmax0);
-            while (i > 0) {
-                const double2 v = row0[i / os];
-                if (hypot(v.x, v.y) > minv)
-                    break;
-                i -= os;
-            }
-            S = int(min(unsigned(i / os), unsigned(q.max_support)));
-        }
-        s_support = S;
+    const int S = min(s_support, q.max_support);
+    if (threadIdx.x == 0)
         q.support[p] = S;
-    }
-    __syncthreads();
-    const int S = s_support;
     const int L = min(S * os + os / 2 + 1, (arr >> 1) + 1);
-    // 4. T[l][a] for l < L
+    // 4. T[l][a] for l < L (l = 0 again: the same values)
     for (int t = threadIdx.x; t < L * half; t += blockDim.x) {
         const int a = t % half, l = t / half;
-        double re = 0.0, im = 0.0;
-        for (int b = 0; b < half; b++) {
-            const double c = (b == 0 ? 1.0 : 2.0) * C(l * b);
-            const double2 v = Q[size_t(b) * half + a];
-            re += v.x * c;
-            im += v.y * c;
-        }
-        T[size_t(l) * half + a] = make_double2(re, im);
+        T[size_t(l) * half + a] = cos_sum(Q + a, half, half, ct, l, arr);
     }
     __syncthreads();
     // 5. conv(k, l) for k, l < L
     for (int t = threadIdx.x; t < L * L; t += blockDim.x) {
         const int k = t % L, l = t / L;
-        double re = 0.0, im = 0.0;
-        const double2* Tl = T + size_t(l) * half;
-        for (int a = 0; a < half; a++) {
-            const double c = (a == 0 ? 1.0 : 2.0) * C(k * a);
-            re += Tl[a].x * c;
-            im += Tl[a].y * c;
-        }
-        conv[size_t(l) * lh + k] = make_double2(re, im);
+        conv[size_t(l) * lh + k] = cos_sum(T + size_t(l) * half, 1, half, ct, k, arr);
     }
     __syncthreads();
     wk_inverse_sums(q, p, conv, S);
@@ -1535,17 +1544,18 @@ __global__ void k_cos_table(int arr, double* c)
 // Expanded W-kernel tables for the gridder: one block per (plane, oversampled
 // offset pair); entry j*K + i (column j, row i) holds the reference's cached
 // kernel value conv(|oy|, |ox|) * inv (aw_projection.cpp:415-448), formed in
-// FP64 and rounded once to R.  Plane p's tables start at off[p] = sum over q <
-// p of cs^2 * K_q^2; *max_support (zeroed before) = the largest support.
+// FP64 and rounded once to R.  Plane p's tables start at off[p] = p * stride,
+// or (stride 0) right after those of the planes before; *max_support (zeroed
+// before) = the largest support.
 template <typename R>
 __global__ void k_wk_expand(const double2* convd, const double* invd, const int* support, int P, int cs, int os,
-    int lh, typename Cplx<R>::T* out, uint32_t* off, unsigned int* max_support)
+    int lh, uint32_t stride, typename Cplx<R>::T* out, uint32_t* off, unsigned int* max_support)
 {
     const int p = blockIdx.x;
     const int pair = blockIdx.y;
     const int cy = pair / cs, cx = pair % cs;
-    uint32_t base = 0;
-    for (int q = 0; q < p; q++) {
+    uint32_t base = uint32_t(p) * stride;
+    for (int q = 0; stride == 0 && q < p; q++) {
         const uint32_t Kq = uint32_t(2 * support[q] + 1);
         base += uint32_t(cs) * uint32_t(cs) * Kq * Kq;
     }
