@@ -2076,7 +2076,7 @@ void run_source_find(stpgpu_context* c, const T* d_img, int rows, int cols, cons
         listed = c->buf<uint32_t>("fg_listed", lcap);
     };
     auto moments_and_islands = [&](const FgSizes& z) {
-        k_label_sums<T><<<G, 128, 0, st>>>(z, d_img, rows, cols, v1, sb, se, sp, mom, ns);
+        k_label_sums<T><<<G, 32 * kSumWarps, 0, st>>>(z, d_img, rows, cols, v1, sb, se, sp, listed, &sfs->seg[1], mom, ns);
         STPGPU_CHECK_LAUNCH();
         k_islands<packed><<<G, 256, 0, st>>>(z, &sfs->st, ext, eidx, ns, mom, p.source_min_area, nvalid, nisl, raw);
         STPGPU_CHECK_LAUNCH();
