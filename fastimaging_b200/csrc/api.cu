@@ -520,6 +520,10 @@ BlockBins make_bins(stpgpu_context* c, const ImagerSetup& s, const GridOut& g, i
     return b;
 }
 
+// Visibilities per block of cells from which several warps share a block.
+constexpr int64_t kDensePerBlock = 24;
+constexpr int kDenseSplit = 8;
+
 // Where a call's items and kernel tables are, for grid_blocks.
 template <typename R>
 struct GridInputs {
@@ -595,10 +599,17 @@ void grid_blocks(stpgpu_context* c, const ImagerSetup& s, GridOut& g, int64_t n,
         p.grid = g.grid;
         p.beam = g.beam;
     };
-    const dim3 blocks(unsigned(ceil_div(ceil_div(b.rows, kBlk), kGridWarps)), unsigned(ceil_div(b.N, kBlk)));
-    auto launch = [&](auto kern, const auto& p) {
+    const int64_t nbr = ceil_div(b.rows, kBlk), nbc = ceil_div(b.N, kBlk);
+    // visibilities per block: above kDensePerBlock several warps share a block
+    const bool dense = n > kDensePerBlock * nbr * nbc;
+    auto run = [&](auto core, const auto& p) {
+        using C = decltype(core);
         c->mark(1);
-        kern<<<blocks, 32 * kGridWarps, 0, st>>>(p);
+        if (dense)
+            k_grid_dense<C, kDenseSplit><<<dim3(unsigned(ceil_div(nbr, kGridWarps / kDenseSplit)), unsigned(nbc)),
+                32 * kGridWarps, 0, st>>>(p);
+        else
+            k_grid_blocks<C><<<dim3(unsigned(ceil_div(nbr, kGridWarps)), unsigned(nbc)), 32 * kGridWarps, 0, st>>>(p);
         STPGPU_CHECK_LAUNCH();
         c->mark(2);
     };
@@ -615,8 +626,7 @@ void grid_blocks(stpgpu_context* c, const ImagerSetup& s, GridOut& g, int64_t n,
         p.max_support = in.max_support;
         by_cell([&](auto cell) {
             using G = decltype(cell);
-            s.beam ? launch(k_grid_blocks<WprojCore<R, G, T, ACC, true>>, p)
-                   : launch(k_grid_blocks<WprojCore<R, G, T, ACC, false>>, p);
+            s.beam ? run(WprojCore<R, G, T, ACC, true>(), p) : run(WprojCore<R, G, T, ACC, false>(), p);
         });
         return;
     }
@@ -644,11 +654,9 @@ void grid_blocks(stpgpu_context* c, const ImagerSetup& s, GridOut& g, int64_t n,
     by_cell([&](auto cell) {
         using G = decltype(cell);
         if (in.exact)
-            s.beam ? launch(k_grid_blocks<SepCore<R, G, true, true>>, p)
-                   : launch(k_grid_blocks<SepCore<R, G, true, false>>, p);
+            s.beam ? run(SepCore<R, G, true, true>(), p) : run(SepCore<R, G, true, false>(), p);
         else
-            s.beam ? launch(k_grid_blocks<SepCore<R, G, false, true>>, p)
-                   : launch(k_grid_blocks<SepCore<R, G, false, false>>, p);
+            s.beam ? run(SepCore<R, G, false, true>(), p) : run(SepCore<R, G, false, false>(), p);
     });
 }
 

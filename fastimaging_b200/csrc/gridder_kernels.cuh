@@ -50,14 +50,24 @@ __global__ void __launch_bounds__(256) k_exact_tables(int kf, double trunc, int 
 // One warp per 8 x 8 block of cells, eight warps (64 rows x 8 columns) per
 // CTA.  The cells stay in registers: nothing is read back, zeroed or
 // updated in memory, and every cell of the grid is written exactly once.
-// The warp walks its pad + 1 ranges of records as one stream, 32 at a time:
-// each lane fetches and decodes one record, those that reach the block are
-// packed into shared memory, and the core C accumulates them.  Blocks with
-// more than kHeavy entries (the centre of a concentrated uv coverage) are
-// taken by all eight warps of the CTA together, their partial cells summed
-// in a fixed order through shared memory.
+//
+// The CTA's entries are fetched and decoded once into shared memory (up to
+// kCtaEntries, footprints of up to 8 (kCtaBins - 1) + 1 cells): the bins of
+// neighbouring blocks overlap, and a block that stages its own entries spends
+// as much on its ranges and on decoding as on gridding when it holds a few
+// tens of them (138 M warp instructions on the 1M-visibility headline call,
+// 47 per entry and block, 26 of them the gridding).  Each warp then looks at
+// the entries of its own bins 32 at a time, lists those that reach its block
+// and hands the list to the core C.
+//
+// Denser CTAs take their entries block by block, 32 at a time through shared
+// memory, and blocks with more than kHeavy entries (the centre of a
+// concentrated uv coverage) are taken by all eight warps together, their
+// partial cells summed in a fixed order.
 constexpr int kGridWarps = 8;
 constexpr uint32_t kHeavy = 512;
+constexpr uint32_t kCtaEntries = 960;
+constexpr int kCtaBins = 5; // bins per axis that reach a block, at most, for staging by CTA
 
 struct BlockRanges {
     uint32_t pre, delta; // lane j: entries before range j, and range j's first record minus that
@@ -103,9 +113,39 @@ __device__ __forceinline__ uint32_t stream_record(const BlockRanges& r, uint32_t
     return t + d;
 }
 
+// Entries [first, first + n) of st, n <= 32, added to the block whose first
+// row is `row` (relative to the staged entries' origin): those that reach it
+// are listed by position and added by the core.
+template <class C>
+__device__ __forceinline__ void block_add(const typename C::Params& p, const typename C::Staged* st, uint32_t first, uint32_t n,
+    uint32_t dummy, int row, uint16_t* list, typename C::A (&acc)[C::NACC])
+{
+    const int lane = threadIdx.x & 31;
+    bool reach = false, odd = false;
+    if (uint32_t(lane) < n) {
+        const typename C::Staged& s = st[first + lane];
+        reach = C::reach(p, s, row);
+        odd = reach && C::odd(s);
+    }
+    const unsigned mask = __ballot_sync(0xffffffffu, reach && !odd);
+    const int m = __popc(mask);
+    if (reach && !odd)
+        list[__popc(mask & ((1u << lane) - 1u))] = uint16_t(first + lane);
+    if (lane < 3)
+        list[m + lane] = uint16_t(dummy); // up to a multiple of four
+    __syncwarp();
+    C::accumulate(p, st, list, m, row, acc);
+    if (C::kOdd) {
+        unsigned o = __ballot_sync(0xffffffffu, odd);
+        for (; o; o &= o - 1)
+            C::add_odd(p, st[first + __ffs(int(o)) - 1], row, acc);
+    }
+    __syncwarp();
+}
+
 template <class C>
 __device__ __forceinline__ void block_walk(const typename C::Params& p, const BlockRanges& r, int r0, int c0, int first,
-    int stride, typename C::Staged* st, typename C::A (&acc)[C::NACC])
+    int stride, typename C::Staged* st, uint16_t* list, typename C::A (&acc)[C::NACC])
 {
     const int lane = threadIdx.x & 31;
     uint32_t t = uint32_t(first) * 32u;
@@ -116,13 +156,9 @@ __device__ __forceinline__ void block_walk(const typename C::Params& p, const Bl
             raw = C::fetch(p, i);
     }
     while (t < r.total) {
-        typename C::Staged s;
-        const bool reach = C::decode(p, raw, r0, c0, s) && t + lane < r.total;
-        const unsigned mask = __ballot_sync(0xffffffffu, reach);
-        if (reach)
-            st[__popc(mask & ((1u << lane) - 1u))] = s;
-        const int m = __popc(mask);
-        C::fill_up(p, st, m);
+        const uint32_t n = min(32u, r.total - t);
+        if (uint32_t(lane) < n)
+            st[lane] = C::decode(p, raw, r0, c0);
         __syncwarp();
         // the next 32 records are in flight while these are gridded
         const uint32_t tn = t + uint32_t(stride) * 32u;
@@ -131,26 +167,76 @@ __device__ __forceinline__ void block_walk(const typename C::Params& p, const Bl
             if (tn + lane < r.total)
                 raw = C::fetch(p, i);
         }
-        C::accumulate(p, st, m, acc);
-        __syncwarp();
+        block_add<C>(p, st, 0, n, 32, 0, list, acc);
         t = tn;
     }
 }
 
 template <class C>
-__global__ void __launch_bounds__(32 * kGridWarps) k_grid_blocks(const __grid_constant__ typename C::Params p)
+__global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(const __grid_constant__ typename C::Params p)
 {
     using A = typename C::A;
-    constexpr size_t kStage = sizeof(typename C::Staged) * 36 * kGridWarps;
+    using Staged = typename C::Staged;
+    // entries of the CTA and a dummy per warp; or 32 and a dummy per warp; or
+    // the partial cells of a block taken by all warps
+    constexpr size_t kStage = sizeof(Staged) * (kCtaEntries + kGridWarps);
     constexpr size_t kRed = sizeof(A) * C::NACC * 32 * kGridWarps;
+    static_assert(kCtaEntries + kGridWarps >= 33 * kGridWarps, "staging by warp");
     __shared__ __align__(16) unsigned char smem[kStage > kRed ? kStage : kRed];
+    __shared__ uint16_t s_list[kGridWarps][36];
+    __shared__ uint32_t s_off[kCtaBins][kGridWarps + kCtaBins];
     __shared__ uint32_t s_heavy;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    typename C::Staged* st = reinterpret_cast<typename C::Staged*>(smem) + warp * 36;
+    Staged* all = reinterpret_cast<Staged*>(smem);
+    uint16_t* list = s_list[warp];
     const int nbr = (p.rows + kBlk - 1) / kBlk;
-    const int br = int(blockIdx.x) * kGridWarps + warp, bc = int(blockIdx.y);
-    const int nb = C::bins(p);      // bins that reach a block on either axis
+    const int br0 = int(blockIdx.x) * kGridWarps, br = br0 + warp, bc = int(blockIdx.y);
+    const int nb = C::bins(p);       // bins that reach a block on either axis
     const int skip = p.pad + 1 - nb; // (those further away cannot)
+    if (nb <= kCtaBins) {
+        // s_off[j]: the offsets of the CTA's bins in column j
+        const int no = kGridWarps + nb;
+        for (int t = threadIdx.x; t < nb * no; t += 32 * kGridWarps) {
+            const int j = t / no, i = t - j * no;
+            s_off[j][i] = p.off[size_t(bc + skip + j) * size_t(p.brn + 1) + size_t(min(br0 + skip + i, p.brn))];
+        }
+        __syncthreads();
+        uint32_t total = 0;
+        for (int j = 0; j < nb; j++)
+            total += s_off[j][no - 1] - s_off[j][0];
+        if (total <= kCtaEntries) {
+            for (uint32_t t = threadIdx.x; t < total; t += 32 * kGridWarps) {
+                uint32_t i = t, j = 0;
+                for (;; j++) {
+                    const uint32_t len = s_off[j][no - 1] - s_off[j][0];
+                    if (i < len)
+                        break;
+                    i -= len;
+                }
+                all[t] = C::decode(p, C::fetch(p, s_off[j][0] + i), br0 * kBlk, bc * kBlk);
+            }
+            if (threadIdx.x < kGridWarps)
+                all[kCtaEntries + threadIdx.x] = C::dummy(p, int(threadIdx.x) * kBlk);
+            __syncthreads();
+            if (br >= nbr)
+                return;
+            A acc[C::NACC] = {};
+            uint32_t before = 0;
+            for (int j = 0; j < nb; j++) {
+                const uint32_t o = s_off[j][0];
+                const uint32_t end = before + s_off[j][warp + nb] - o;
+                for (uint32_t e = before + s_off[j][warp] - o; e < end; e += 32)
+                    block_add<C>(p, all, e, min(32u, end - e), kCtaEntries + warp, warp * kBlk, list, acc);
+                before += s_off[j][no - 1] - o;
+            }
+            C::store(p, br * kBlk, bc * kBlk, acc);
+            return;
+        }
+        __syncthreads();
+    }
+    Staged* st = all + warp * 33;
+    if (lane == 0)
+        st[32] = C::dummy(p, 0);
     if (threadIdx.x == 0)
         s_heavy = 0;
     __syncthreads();
@@ -165,7 +251,7 @@ __global__ void __launch_bounds__(32 * kGridWarps) k_grid_blocks(const __grid_co
             heavy = total > kHeavy;
             if (heavy)
                 break;
-            block_walk<C>(p, r, br * kBlk, bc * kBlk, 0, 1, st, acc);
+            block_walk<C>(p, r, br * kBlk, bc * kBlk, 0, 1, st, list, acc);
         }
         if (heavy) {
             if (lane == 0)
@@ -177,11 +263,11 @@ __global__ void __launch_bounds__(32 * kGridWarps) k_grid_blocks(const __grid_co
     __syncthreads();
     for (uint32_t h = s_heavy; h; h &= h - 1) {
         const int hw = __ffs(int(h)) - 1;
-        const int hbr = int(blockIdx.x) * kGridWarps + hw;
+        const int hbr = br0 + hw;
         A acc[C::NACC] = {};
         for (int j = 0; j < nb; j += 32) {
             const BlockRanges r = block_ranges(p.off, p.brn, hbr + skip, bc + skip + j, nb, min(nb - j, 32));
-            block_walk<C>(p, r, hbr * kBlk, bc * kBlk, warp, kGridWarps, st, acc);
+            block_walk<C>(p, r, hbr * kBlk, bc * kBlk, warp, kGridWarps, st, list, acc);
         }
         __syncthreads(); // the staged records are read; the same memory takes the partial cells
         A* red = reinterpret_cast<A*>(smem);
@@ -198,7 +284,53 @@ __global__ void __launch_bounds__(32 * kGridWarps) k_grid_blocks(const __grid_co
             C::store(p, hbr * kBlk, bc * kBlk, acc);
         }
         __syncthreads();
+        if (lane == 0)
+            st[32] = C::dummy(p, 0); // overwritten by the partial cells
+        __syncwarp();
     }
+}
+
+// Dense grids: SPLIT warps share a block (every SPLIT-th 32 entries of its
+// stream each) and sum their cells in a fixed order; a CTA has 8 / SPLIT
+// blocks.  A small image with many visibilities has too few blocks to fill
+// the GPU with one warp each, and along uv tracks most of its entries fall
+// into a tenth of them.
+template <class C, int SPLIT>
+__global__ void __launch_bounds__(32 * kGridWarps) k_grid_dense(const __grid_constant__ typename C::Params p)
+{
+    using A = typename C::A;
+    using Staged = typename C::Staged;
+    constexpr size_t kStage = sizeof(Staged) * 33 * kGridWarps;
+    constexpr size_t kRed = sizeof(A) * C::NACC * 32 * kGridWarps;
+    __shared__ __align__(16) unsigned char smem[kStage > kRed ? kStage : kRed];
+    __shared__ uint16_t s_list[kGridWarps][36];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int sub = warp % SPLIT, first = warp - sub;
+    Staged* st = reinterpret_cast<Staged*>(smem) + warp * 33;
+    if (lane == 0)
+        st[32] = C::dummy(p, 0);
+    __syncwarp();
+    const int nbr = (p.rows + kBlk - 1) / kBlk;
+    const int br = int(blockIdx.x) * (kGridWarps / SPLIT) + warp / SPLIT, bc = int(blockIdx.y);
+    const int nb = C::bins(p), skip = p.pad + 1 - nb;
+    A acc[C::NACC] = {};
+    if (br < nbr)
+        for (int j = 0; j < nb; j += 32) {
+            const BlockRanges r = block_ranges(p.off, p.brn, br + skip, bc + skip + j, nb, min(nb - j, 32));
+            block_walk<C>(p, r, br * kBlk, bc * kBlk, sub, SPLIT, st, s_list[warp], acc);
+        }
+    __syncthreads(); // the staged records are read; the same memory takes the partial cells
+    A* red = reinterpret_cast<A*>(smem);
+    if (sub)
+        for (int q = 0; q < C::NACC; q++)
+            red[(q * kGridWarps + warp) * 32 + lane] = acc[q];
+    __syncthreads();
+    if (sub || br >= nbr)
+        return;
+    for (int w = first + 1; w < first + SPLIT; w++)
+        for (int q = 0; q < C::NACC; q++)
+            acc[q] += red[(q * kGridWarps + w) * 32 + lane];
+    C::store(p, br * kBlk, bc * kBlk, acc);
 }
 
 // ---------------------------------------------------------------- separable kernels
@@ -236,24 +368,27 @@ struct SepCore {
     using Params = SepParams<R>;
     using A = double;
     static constexpr int NACC = BEAM ? 6 : 4;
+    static constexpr int kMinBlocks = BEAM ? 3 : 5; // (4 blocks of 64 registers: 1460 us against 1421 on the 8192^2 call)
     struct Raw {
         GridRec<R> r;
         R w;
     };
+    // ty, tx: table position of the entry's tap at the origin's row / column;
+    // rc: row0 and col0 plus 512 (10 bits each), bit 20: exact, the mirrored
+    // copy; bit 21: not finite
     struct alignas(16) StagedB {
         double vr, vi;
-        int ty, tx;  // table position of the entry's tap at the block's first row / column
-        uint32_t vis; // exact: the visibility
-        int back;     // bit 0: exact, the mirrored copy; bit 1: not finite
+        int ty, tx;
+        uint32_t vis, rc; // vis: exact, the visibility
         double w, unused;
     };
     struct alignas(16) StagedP {
         double vr, vi;
         int ty, tx;
-        uint32_t vis;
-        int back;
+        uint32_t vis, rc;
     };
     using Staged = std::conditional_t<BEAM, StagedB, StagedP>;
+    static constexpr bool kOdd = true;
 
     static __device__ __forceinline__ int bins(const Params& p) { return p.pad + 1; }
     static __device__ __forceinline__ Raw fetch(const Params& p, uint32_t i)
@@ -264,8 +399,9 @@ struct SepCore {
             w.w = p.wts[i];
         return w;
     }
-    static __device__ __forceinline__ bool decode(const Params& p, const Raw& w, int r0, int c0, Staged& s)
+    static __device__ __forceinline__ Staged decode(const Params& p, const Raw& w, int r0, int c0)
     {
+        Staged s;
         const uint32_t g = w.r.geom;
         const int row0 = int((g - uint32_t(r0)) << 22) >> 22, col0 = int((g - (uint32_t(c0) << 10)) << 12) >> 22;
         s.vr = double(w.r.vr);
@@ -275,80 +411,70 @@ struct SepCore {
             s.w = double(w.w);
             chk += s.w;
         }
+        s.rc = uint32_t(row0 + 512) | (uint32_t(col0 + 512) << 10) | (((g >> 28) & 1u) << 20);
+        // a kernel whose samples sum to zero is not finite in all its taps
         if (EXACT) {
             s.ty = -row0;
             s.tx = -col0;
             s.vis = w.r.koff;
-            s.back = int((g >> 28) & 1u);
-        } else {
-            s.ty = int(w.r.koff & 0xffffu) * p.tw + 7 - row0;
-            s.tx = int(w.r.koff >> 16) * p.tw + 7 - col0;
-            s.vis = 0;
-            s.back = 0;
-        }
-        if (!(row0 + p.K > 0 && col0 + p.K > 0))
-            return false;
-        // a kernel whose samples sum to zero is not finite in all its taps
-        if (EXACT) {
             const double* t = p.tab + size_t(s.vis) * size_t(2 * p.K);
             chk += __ldg(t) + __ldg(t + p.K);
         } else {
-            chk += __ldg(p.tab + s.ty + row0) + __ldg(p.tab + s.tx + col0);
+            const int ky = int(w.r.koff & 0xffffu) * p.tw + 7, kx = int(w.r.koff >> 16) * p.tw + 7;
+            s.ty = ky - row0;
+            s.tx = kx - col0;
+            s.vis = 0;
+            chk += __ldg(p.tab + ky) + __ldg(p.tab + kx);
         }
         if (!(fabs(chk) <= 1.7976931348623157e308))
-            s.back |= 2;
-        return true;
+            s.rc |= 1u << 21;
+        return s;
     }
-    // entries of zero weight up to a multiple of four
-    static __device__ __forceinline__ void fill_up(const Params& p, Staged* st, int m)
-    {
-        const int lane = threadIdx.x & 31;
-        if (lane < ((4 - m) & 3))
-            st[m + lane] = none(p);
-    }
-    static __device__ __forceinline__ Staged none(const Params& p)
+    // an entry of zero weight for the block at `row`
+    static __device__ __forceinline__ Staged dummy(const Params& p, int row)
     {
         Staged z {};
-        z.ty = z.tx = EXACT ? -kBlk : p.zrow;
+        z.ty = EXACT ? -kBlk - row : p.zrow - row;
+        z.tx = EXACT ? -kBlk : p.zrow;
         return z;
     }
-    // the tap of either axis at the block's row / column q
+    static __device__ __forceinline__ int row0_of(const Staged& s) { return int(s.rc & 1023u) - 512; }
+    static __device__ __forceinline__ int col0_of(const Staged& s) { return int((s.rc >> 10) & 1023u) - 512; }
+    static __device__ __forceinline__ bool odd(const Staged& s) { return (s.rc >> 21) & 1u; }
+    static __device__ __forceinline__ bool reach(const Params& p, const Staged& s, int row)
+    {
+        const int row0 = row0_of(s) - row, col0 = col0_of(s);
+        return row0 + p.K > 0 && row0 < kBlk && col0 + p.K > 0 && col0 < kBlk;
+    }
+    // the taps of either axis at the origin's row / column
     static __device__ __forceinline__ void taps(const Params& p, const Staged& s, int row, int col, double& a, double& b)
     {
         if (EXACT) {
             const int K = p.K;
             const int dr = s.ty + row, dc = s.tx + col;
+            const bool back = (s.rc >> 20) & 1u;
             const double* t = p.tab + size_t(s.vis) * size_t(2 * K);
-            a = unsigned(dr) < unsigned(K) ? __ldg(t + (s.back & 1 ? K - 1 - dr : dr)) : 0.0;
-            b = unsigned(dc) < unsigned(K) ? __ldg(t + K + (s.back & 1 ? K - 1 - dc : dc)) : 0.0;
+            a = unsigned(dr) < unsigned(K) ? __ldg(t + (back ? K - 1 - dr : dr)) : 0.0;
+            b = unsigned(dc) < unsigned(K) ? __ldg(t + K + (back ? K - 1 - dc : dc)) : 0.0;
         } else {
             a = __ldg(p.tab + s.ty + row);
             b = __ldg(p.tab + s.tx + col);
         }
     }
-    static __device__ __noinline__ void odd_entries(const Params& p, Staged* st, int m, unsigned odd, A (&acc)[NACC])
+    // an entry that is not finite: its own footprint's cells only
+    static __device__ __forceinline__ void add_odd(const Params& p, const Staged& s, int row, A (&acc)[NACC])
     {
         const int lane = threadIdx.x & 31;
-        for (; odd; odd &= odd - 1) {
-            const int e = __ffs(int(odd)) - 1;
-            const Staged s = st[e];
-            const int tr = EXACT ? 0 : (s.ty / p.tw) * p.tw + 7, tc = EXACT ? 0 : (s.tx / p.tw) * p.tw + 7;
-            for (int k = 0; k < 2; k++) {
-                const int row = lane >> 2, col = 2 * (lane & 3) + k;
-                const int dr = s.ty + row - tr, dc = s.tx + col - tc;
-                if (unsigned(dr) < unsigned(p.K) && unsigned(dc) < unsigned(p.K)) {
-                    double a, b;
-                    taps(p, s, row, col, a, b);
-                    acc[k] += a * b * s.vr;
-                    acc[2 + k] += a * b * s.vi;
-                    if constexpr (BEAM)
-                        acc[4 + k] += a * b * s.w;
-                }
+        for (int k = 0; k < 2; k++) {
+            const int r = row + (lane >> 2), c = 2 * (lane & 3) + k;
+            if (unsigned(r - row0_of(s)) < unsigned(p.K) && unsigned(c - col0_of(s)) < unsigned(p.K)) {
+                double a, b;
+                taps(p, s, r, c, a, b);
+                acc[k] += a * b * s.vr;
+                acc[2 + k] += a * b * s.vi;
+                if constexpr (BEAM)
+                    acc[4 + k] += a * b * s.w;
             }
-            __syncwarp();
-            if (lane == 0)
-                st[e] = none(p);
-            __syncwarp();
         }
     }
     static __device__ __forceinline__ void mma(double& c0, double& c1, double a, double b)
@@ -357,17 +483,16 @@ struct SepCore {
             : "+d"(c0), "+d"(c1)
             : "d"(a), "d"(b));
     }
-    static __device__ __forceinline__ void accumulate(const Params& p, Staged* st, int m, A (&acc)[NACC])
+    static __device__ __forceinline__ void accumulate(const Params& p, const Staged* st, const uint16_t* list, int m, int row,
+        A (&acc)[NACC])
     {
         const int lane = threadIdx.x & 31;
-        const unsigned odd = __ballot_sync(0xffffffffu, lane < m && (st[lane].back & 2));
-        if (odd)
-            odd_entries(p, st, m, odd, acc);
+        const int q = lane >> 2;
 #pragma unroll 2
         for (int g = 0; g < m; g += 4) {
-            const Staged s = st[g + (lane & 3)];
+            const Staged& s = st[list[g + (lane & 3)]];
             double a, b;
-            taps(p, s, lane >> 2, lane >> 2, a, b);
+            taps(p, s, row + q, q, a, b);
             mma(acc[0], acc[1], a, b * s.vr);
             mma(acc[2], acc[3], a, b * s.vi);
             if constexpr (BEAM)
@@ -427,6 +552,7 @@ struct WprojCore {
     using Params = WprojParams<R, T>;
     using A = ACC;
     static constexpr int NACC = BEAM ? 8 : 4;
+    static constexpr int kMinBlocks = BEAM ? 2 : 4; // (5 blocks of 48 registers spill: 472 us against 490 on the headline call)
     struct Raw {
         GridRec<R> r;
         R w;
@@ -455,8 +581,12 @@ struct WprojCore {
             w.w = p.wts[i];
         return w;
     }
-    static __device__ __forceinline__ bool decode(const Params&, const Raw& w, int r0, int c0, Staged& s)
+    static constexpr bool kOdd = false; // (cells outside a footprint are not touched)
+    static __device__ __forceinline__ bool odd(const Staged&) { return false; }
+    static __device__ __forceinline__ void add_odd(const Params&, const Staged&, int, A (&)[NACC]) {}
+    static __device__ __forceinline__ Staged decode(const Params&, const Raw& w, int r0, int c0)
     {
+        Staged s;
         const uint32_t g = w.r.geom;
         s.row0 = int((g - uint32_t(r0)) << 22) >> 22;
         s.col0 = int((g - (uint32_t(c0) << 10)) << 12) >> 22;
@@ -467,9 +597,19 @@ struct WprojCore {
         s.kc = uint32_t(K) | ((g << 4) & 0x80000000u);
         if constexpr (BEAM)
             s.w = A(w.w);
-        return s.row0 + K > 0 && s.col0 + K > 0 && s.row0 < kBlk && s.col0 < kBlk;
+        return s;
     }
-    static __device__ __forceinline__ void fill_up(const Params&, Staged*, int) {}
+    // an entry without taps
+    static __device__ __forceinline__ Staged dummy(const Params&, int)
+    {
+        Staged z {};
+        return z;
+    }
+    static __device__ __forceinline__ bool reach(const Params&, const Staged& s, int row)
+    {
+        const int K = int(s.kc & 0xffffu), row0 = s.row0 - row;
+        return row0 + K > 0 && row0 < kBlk && s.col0 + K > 0 && s.col0 < kBlk;
+    }
     static __device__ __forceinline__ float flip(float x, uint32_t sign)
     {
         return __uint_as_float(__float_as_uint(x) ^ sign);
@@ -478,15 +618,16 @@ struct WprojCore {
     {
         return __hiloint2double(int(uint32_t(__double2hiint(x)) ^ sign), __double2loint(x));
     }
-    static __device__ __forceinline__ void accumulate(const Params& p, const Staged* st, int m, A (&acc)[NACC])
+    static __device__ __forceinline__ void accumulate(const Params& p, const Staged* st, const uint16_t* list, int m, int row,
+        A (&acc)[NACC])
     {
         using C2 = typename Cplx<T>::T;
         const int lane = threadIdx.x & 31;
-        const int r = lane & 7, c = lane >> 3;
+        const int r = row + (lane & 7), c = lane >> 3;
         const C2* __restrict__ wk = p.wk;
 #pragma unroll 4
         for (int e = 0; e < m; e++) {
-            const Staged s = st[e];
+            const Staged s = st[list[e]];
             const int K = int(s.kc & 0xffffu);
             const uint32_t sign = s.kc & 0x80000000u;
             const int dr = r - s.row0, dc = c - s.col0;
