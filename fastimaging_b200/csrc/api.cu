@@ -2340,7 +2340,7 @@ void run_source_find(stpgpu_context* c, const T* d_img, int rows, int cols, cons
             int* dit = c->buf<int>("fit_iter", nfit);
             STPGPU_CUDA_TRY(cudaMemcpyAsync(dkeys, keys.data(), sizeof(int) * nfit, cudaMemcpyHostToDevice, st));
             STPGPU_CUDA_TRY(cudaMemcpyAsync(dinit, init.data(), sizeof(double) * 6 * nfit, cudaMemcpyHostToDevice, st));
-            k_gauss_fit<T><<<nfit, 32, 0, st>>>(d_img, rows, cols, fit_pix, sb, se, sp, dkeys, dinit, nfit, dout, dit);
+            k_gauss_fit<T><<<nfit, FIT_THREADS, 0, st>>>(d_img, rows, cols, fit_pix, sb, se, sp, dkeys, dinit, nfit, dout, dit);
             STPGPU_CHECK_LAUNCH();
             std::vector<double> out(6 * size_t(nfit));
             std::vector<int> its(nfit);

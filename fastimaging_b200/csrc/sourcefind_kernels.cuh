@@ -1554,7 +1554,7 @@ __device__ __forceinline__ uint32_t seg_at(uint32_t b, uint32_t sp, uint32_t e, 
 // and multiply 32 pixels at once, then six lanes each add one of the sums in
 // pixel order.  Only the additions are a chain: with one thread per label the
 // loads were one too, and a bright source of 600 pixels kept the whole grid
-// waiting (60 us of the call on a 4096^2 image, now 6).
+// waiting (60 us of the call on a 4096^2 image, now 25).
 constexpr int kSumWarps = 4;
 template <typename T>
 __global__ void __launch_bounds__(32 * kSumWarps) k_label_sums(FgSizes z, const T* img, int rows, int cols,
@@ -1577,12 +1577,10 @@ __global__ void __launch_bounds__(32 * kSumWarps) k_label_sums(FgSizes z, const 
         const uint32_t l = listed[q];
         const uint32_t b = seg_begin[l], e = seg_end[l], sp = seg_split[l], len = e - b;
         double sum = 0.0;
-        uint32_t m = 0;
-        double val = 0.0;
-        if (uint32_t(lane) < len) {
-            m = vals[seg_at(b, sp, e, lane)];
-            val = ld(img, m);
-        }
+        // the pixel of the next 32 and the index of the 32 after are in flight
+        auto index = [&](uint32_t j) { return j < len ? vals[seg_at(b, sp, e, j)] : 0u; };
+        uint32_t m = index(lane), m1 = index(32 + lane);
+        double val = uint32_t(lane) < len ? ld(img, m) : 0.0;
         for (uint32_t j = 0; j < len; j += 32) {
             const int c = int(m / uint32_t(rows)), r = int(m - uint32_t(c) * uint32_t(rows));
             const double y = r < vs ? double(r + vs) : double(r - vs);
@@ -1595,10 +1593,10 @@ __global__ void __launch_bounds__(32 * kSumWarps) k_label_sums(FgSizes z, const 
             t[4][lane] = __dmul_rn(xb, y);
             t[5][lane] = val;
             __syncwarp();
-            if (j + 32 + lane < len) { // in flight during the additions
-                m = vals[seg_at(b, sp, e, j + 32 + lane)];
+            m = m1;
+            if (j + 32 + lane < len)
                 val = ld(img, m);
-            }
+            m1 = index(j + 64 + lane);
             if (lane < 6) {
                 const int n = int(min(32u, len - j));
 #pragma unroll 8
@@ -1675,10 +1673,15 @@ __global__ void k_islands(FgSizes z, const SfStats* st, const unsigned long long
 // src/stp/sourcefind/fitting.h:183-210; a, b, c from the standard deviations
 // and theta as there), starting from the moments fit
 // (sourcefind.cpp:719-760).  The reference minimises with Ceres; here a
-// Levenberg-Marquardt iteration with analytic derivatives: one warp per
-// island, lanes over the island's pixels, the 6x6 normal equations reduced
-// with shuffles and solved by every lane (Cholesky).
+// Levenberg-Marquardt iteration with analytic derivatives: one block per
+// island, threads over the island's pixels, the 6x6 normal equations reduced
+// with shuffles and through shared memory in a fixed order, and solved by
+// every thread (Cholesky).  The call waits for its largest island (a bright
+// source of 900 pixels): with one warp an island, and with the cost of a
+// step evaluated before its normal equations, the kernel took 205 us on 60
+// sources of a 1502 x 1998 image.
 constexpr int FIT_MAX_ITER = 100;
+constexpr int FIT_THREADS = 128;
 
 struct GaussTerms {
     double a, b, c, da_dsx, db_dsx, dc_dsx, da_dsy, db_dsy, dc_dsy, da_dt, db_dt, dc_dt;
@@ -1704,15 +1707,6 @@ __device__ __forceinline__ GaussTerms gauss_terms(const double* p)
     g.db_dt = c2t * (ix2 - iy2);
     g.dc_dt = 0.5 * s2t * (ix2 - iy2);
     return g;
-}
-
-// Sum over the warp, broadcast from lane 0 so that every lane holds the same
-// bits (the butterfly adds in a different order on each lane).
-__device__ __forceinline__ double warp_sum_bcast(double v)
-{
-    for (int o = 16; o > 0; o >>= 1)
-        v += __shfl_xor_sync(0xffffffffu, v, o);
-    return __shfl_sync(0xffffffffu, v, 0);
 }
 
 // Cholesky solve of the 6x6 SPD system m x = r (m: 21 packed lower entries).
@@ -1759,7 +1753,7 @@ __device__ __forceinline__ bool solve6(const double* m, const double* r, double*
 // x, y are display coordinates (the image is unshifted: display = memory
 // index shifted by half, sourcefind.cpp:230-245).
 template <typename T>
-__global__ void __launch_bounds__(32) k_gauss_fit(const T* __restrict__ img, int rows, int cols,
+__global__ void __launch_bounds__(FIT_THREADS) k_gauss_fit(const T* __restrict__ img, int rows, int cols,
     const uint32_t* __restrict__ pix, const uint32_t* __restrict__ sb, const uint32_t* __restrict__ se,
     const uint32_t* __restrict__ sp, const int* __restrict__ keys, const double* __restrict__ init, int nis,
     double* outp, int* iters)
@@ -1767,7 +1761,8 @@ __global__ void __launch_bounds__(32) k_gauss_fit(const T* __restrict__ img, int
     const int isl = blockIdx.x;
     if (isl >= nis)
         return;
-    const int lane = threadIdx.x;
+    __shared__ double part[FIT_THREADS / 32][28], tot[28];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int key = keys[isl];
     const uint32_t b = sb[key], e = se[key], split = sp[key];
     const int hs = cols / 2, vs = rows / 2;
@@ -1775,18 +1770,12 @@ __global__ void __launch_bounds__(32) k_gauss_fit(const T* __restrict__ img, int
     for (int k = 0; k < 6; k++)
         p[k] = init[6 * isl + k];
 
-    // cost (and optionally the normal equations) at parameters q
-    auto pass = [&](const double* q, bool normal, double* JtJ, double* Jtr) -> double {
+    // cost and normal equations at parameters q (the same bits in every thread)
+    auto pass = [&](const double* q, double* JtJ, double* Jtr) -> double {
         const GaussTerms g = gauss_terms(q);
         double cost = 0.0;
-        double jj[21], jr[6];
-        if (normal) {
-            for (int k = 0; k < 21; k++)
-                jj[k] = 0.0;
-            for (int k = 0; k < 6; k++)
-                jr[k] = 0.0;
-        }
-        for (uint32_t j = lane; j < e - b; j += 32) {
+        double jj[21] = {}, jr[6] = {};
+        for (uint32_t j = threadIdx.x; j < e - b; j += FIT_THREADS) {
             const uint32_t m = pix[seg_at(b, split, e, j)];
             const int rm = int(m % uint32_t(rows)), cm = int(m / uint32_t(rows));
             const double x = double(cm < hs ? cm + hs : cm - hs);
@@ -1796,34 +1785,53 @@ __global__ void __launch_bounds__(32) k_gauss_fit(const T* __restrict__ img, int
             const double ex = exp(-quad);
             const double r = q[0] * ex - double(img[m]);
             cost += r * r;
-            if (normal) {
-                const double ae = q[0] * ex;
-                double J[6];
-                J[0] = ex;
-                J[1] = ae * (2.0 * g.a * dx + g.b * dy);
-                J[2] = ae * (g.b * dx + 2.0 * g.c * dy);
-                J[3] = -ae * (g.da_dsx * dx * dx + g.db_dsx * dx * dy + g.dc_dsx * dy * dy);
-                J[4] = -ae * (g.da_dsy * dx * dx + g.db_dsy * dx * dy + g.dc_dsy * dy * dy);
-                J[5] = -ae * (g.da_dt * dx * dx + g.db_dt * dx * dy + g.dc_dt * dy * dy);
-                int u = 0;
-                for (int i = 0; i < 6; i++) {
-                    jr[i] += J[i] * r;
-                    for (int j = 0; j <= i; j++)
-                        jj[u++] += J[i] * J[j];
-                }
+            const double ae = q[0] * ex;
+            double J[6];
+            J[0] = ex;
+            J[1] = ae * (2.0 * g.a * dx + g.b * dy);
+            J[2] = ae * (g.b * dx + 2.0 * g.c * dy);
+            J[3] = -ae * (g.da_dsx * dx * dx + g.db_dsx * dx * dy + g.dc_dsx * dy * dy);
+            J[4] = -ae * (g.da_dsy * dx * dx + g.db_dsy * dx * dy + g.dc_dsy * dy * dy);
+            J[5] = -ae * (g.da_dt * dx * dx + g.db_dt * dx * dy + g.dc_dt * dy * dy);
+            int u = 0;
+#pragma unroll
+            for (int i = 0; i < 6; i++) {
+                jr[i] += J[i] * r;
+#pragma unroll
+                for (int k = 0; k <= i; k++)
+                    jj[u++] += J[i] * J[k];
             }
         }
-        if (normal) {
-            for (int k = 0; k < 21; k++)
-                JtJ[k] = warp_sum_bcast(jj[k]);
-            for (int k = 0; k < 6; k++)
-                Jtr[k] = warp_sum_bcast(jr[k]);
+        auto reduce = [&](double v, int k) {
+            for (int o = 16; o > 0; o >>= 1)
+                v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0)
+                part[warp][k] = v;
+        };
+#pragma unroll
+        for (int k = 0; k < 21; k++)
+            reduce(jj[k], k);
+#pragma unroll
+        for (int k = 0; k < 6; k++)
+            reduce(jr[k], 21 + k);
+        reduce(cost, 27);
+        __syncthreads();
+        if (threadIdx.x < 28) {
+            double v = 0.0;
+            for (int w = 0; w < FIT_THREADS / 32; w++)
+                v += part[w][threadIdx.x];
+            tot[threadIdx.x] = v;
         }
-        return warp_sum_bcast(cost);
+        __syncthreads();
+        for (int k = 0; k < 21; k++)
+            JtJ[k] = tot[k];
+        for (int k = 0; k < 6; k++)
+            Jtr[k] = tot[21 + k];
+        return tot[27];
     };
 
     double JtJ[21], Jtr[6];
-    double cost = pass(p, true, JtJ, Jtr);
+    double cost = pass(p, JtJ, Jtr);
     double lambda = 1e-3;
     int it = 0;
     while (it < FIT_MAX_ITER) {
@@ -1831,7 +1839,7 @@ __global__ void __launch_bounds__(32) k_gauss_fit(const T* __restrict__ img, int
         // (J^T J + lambda D) delta = -J^T r, D = diag(J^T J) floored at 1e-12 of its
         // largest entry (a parameter the residuals do not depend on, such as
         // theta of a circular Gaussian, then gets a zero step)
-        double m[21], rhs[6], d[6], q[6];
+        double m[21], rhs[6], d[6], q[6], JtJn[21], Jtrn[6];
         double dmax = 0.0;
         for (int i = 0; i < 6; i++)
             dmax = fmax(dmax, JtJ[i * (i + 1) / 2 + i]);
@@ -1849,8 +1857,7 @@ __global__ void __launch_bounds__(32) k_gauss_fit(const T* __restrict__ img, int
             ok = q[3] != 0.0 && q[4] != 0.0;
         }
         if (ok) {
-            double dummy1[21], dummy2[6];
-            cnew = pass(q, false, dummy1, dummy2);
+            cnew = pass(q, JtJn, Jtrn);
             ok = cnew == cnew && cnew < cost; // NaN-safe
         }
         if (ok) {
@@ -1860,7 +1867,11 @@ __global__ void __launch_bounds__(32) k_gauss_fit(const T* __restrict__ img, int
             const bool small = (cost - cnew) <= 1e-12 * cost || step <= 1e-10;
             for (int k = 0; k < 6; k++)
                 p[k] = q[k];
-            cost = pass(p, true, JtJ, Jtr);
+            cost = cnew;
+            for (int k = 0; k < 21; k++)
+                JtJ[k] = JtJn[k];
+            for (int k = 0; k < 6; k++)
+                Jtr[k] = Jtrn[k];
             lambda = fmax(lambda * 0.1, 1e-15);
             if (small)
                 break;
@@ -1870,7 +1881,7 @@ __global__ void __launch_bounds__(32) k_gauss_fit(const T* __restrict__ img, int
                 break;
         }
     }
-    if (lane == 0) {
+    if (threadIdx.x == 0) {
         for (int k = 0; k < 6; k++)
             outp[6 * isl + k] = p[k];
         iters[isl] = it;
