@@ -911,12 +911,15 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
         // WideFieldImaging gets real_t(arc_sec_to_rad(cell)), scaled by N/workarea
         wq.scaled_cell = arc_sec_to_rad(s.cell_size) * scaling;
         wq.trunc_perc = s.trunc_perc;
+        // CTAs that share a plane: by the kernel's rows at the largest support
+        // (a second costs little where the truncated kernel turns out small),
+        // as far as the planes leave SMs
+        const int wk_ctas = std::max(1, std::min({ 4, Lh / 16, 148 / std::max(P, 1) }));
         if (!s.hankel) {
-            wq.Qs = c->buf<double2>("wkQ", size_t(P) * half * half);
-            wq.Ts = c->buf<double2>("wkT", size_t(P) * Lh * half);
+            wq.Qs = c->buf<double2>("wkQ", size_t(P) * wk_ctas * half * half);
+            wq.Ts = c->buf<double2>("wkT", size_t(P) * (Lh + wk_ctas) * half);
         }
         wq.convd = c->buf<double2>("wkconv", size_t(P) * Lh * Lh);
-        wq.invd = c->buf<double>("wkinv", size_t(P) * cs * cs);
         const int T = std::max(s.ntimesteps, 1);
         const int PT = P * T;
         plane_support = c->buf<int>("psupport", PT);
@@ -1005,9 +1008,9 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
             };
             wq.smem_ctab = fits(pad16(sizeof(double) * size_t(arr)));
             wq.smem_Q = fits(sizeof(double2) * size_t(half) * half);
-            wq.smem_T = fits(sizeof(double2) * size_t(Lh) * half);
+            wq.smem_T = fits(sizeof(double2) * size_t(ceil_div(Lh, wk_ctas)) * half);
             STPGPU_CUDA_TRY(cudaFuncSetAttribute(k_wkernel_plane, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-            k_wkernel_plane<<<P, 1024, smem, st>>>(wq);
+            k_wkernel_plane<<<dim3(P, wk_ctas), 1024, smem, st>>>(wq);
         }
         STPGPU_CHECK_LAUNCH();
         // per-offset K x K tables in the gridder's precision: worst-case
@@ -1031,7 +1034,7 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
             k_aproj_expand<KT><<<dim3(PT, cs * cs), 256, 0, st>>>(aconv, arr, plane_support, cs, os, wk, wk_off,
                 g.d_err + CF_MAX_SUPPORT);
         else
-            k_wk_expand<KT><<<dim3(P, cs * cs), 64, 0, st>>>(wq.convd, wq.invd, plane_support, P, cs, os, Lh,
+            k_wk_expand<KT><<<dim3(P, cs * cs), kExpandThreads, 0, st>>>(wq.convd, plane_support, P, cs, os, Lh,
                 large_support(s) ? 0u : uint32_t(cs * cs) * uint32_t(K * K), wk, wk_off, g.d_err + CF_MAX_SUPPORT);
         STPGPU_CHECK_LAUNCH();
         g.d_plane_support = plane_support;

@@ -1188,9 +1188,8 @@ __global__ void k_fix_runs(const uint32_t* __restrict__ key32, uint32_t* perm, c
 // with m_0 = 1, m_{>0} = 2, and conv(+-k, +-l) = conv(|k|, |l|).  Only the
 // entries the cache samples are formed: first the l = 0 row for the
 // truncation, then the |offset| block of the truncated support.
-// Outputs per plane: support, conv quadrant conv[p][l][k] (stride lh_max)
-// and inv[p][y][x] = 1 / sum(Re) of each oversampled sub-kernel, so that the
-// reference's cached kernel value is conv * inv.
+// Outputs per plane: support and conv quadrant conv[p][l][k] (stride lh_max),
+// from which k_wk_expand forms the cached kernels.
 struct WkParams {
     const double* w_avg;
     const double* aa; // image-domain AA kernel over the workarea
@@ -1201,7 +1200,6 @@ struct WkParams {
     double2* Qs;   // scratch [P][half][half]
     double2* Ts;   // scratch [P][lh_max][half]
     double2* convd; // [P][lh_max][lh_max] FP64
-    double* invd;   // [P][cs][cs]
     int* support;
 };
 
@@ -1219,32 +1217,6 @@ __device__ __forceinline__ double2 wk_value(const WkParams& q, double w, int px,
     const double re = (cn / nn) * q.aa[half + px];
     const double im = (sn / nn) * q.aa[half + px];
     return make_double2(re * q.aa[half + py], im * q.aa[half + py]);
-}
-
-// 1/sum(Re) of each oversampled sub-kernel of plane p (generate_kernel_cache,
-// aw_projection.cpp:383-448); conv is the plane's quadrant
-// conv[|dy| * lh + |dx|].  One warp per sub-kernel: its K^2 loads are spread
-// over the lanes instead of being one thread's chain.
-__device__ void wk_inverse_sums(const WkParams& q, int p, const double2* conv, int S)
-{
-    const int cs = q.cs, os = q.os, lh = q.lh_max;
-    const int K = 2 * S + 1;
-    const int lane = threadIdx.x & 31;
-    for (int t = threadIdx.x >> 5; t < cs * cs; t += blockDim.x >> 5) {
-        const int x = t % cs, y = t / cs;
-        double ks = 0.0;
-        for (int e = lane; e < K * K; e += 32) {
-            int ox = (e / K - S) * os + os / 2 - x;
-            int oy = (e % K - S) * os + os / 2 - y;
-            ox = ox < 0 ? -ox : ox;
-            oy = oy < 0 ? -oy : oy;
-            ks += conv[size_t(oy) * lh + ox].x;
-        }
-        for (int o = 16; o > 0; o >>= 1)
-            ks += __shfl_xor_sync(0xffffffffu, ks, o);
-        if (lane == 0)
-            q.invd[(size_t(p) * cs + y) * cs + x] = 1 / ks;
-    }
 }
 
 // sum_a m_a V[a * stride] cos(2 pi k a / arr), m_0 = 1, m_{>0} = 2
@@ -1268,7 +1240,10 @@ __device__ __forceinline__ double2 cos_sum(const double2* V, int stride, int hal
 // cosine table, the image-domain quadrant Q and its row transforms T are kept
 // in shared memory where they fit (q.smem_*; the launch gives the room), the
 // position in the cosine table is carried instead of reduced modulo arr at
-// every term, and the truncation test runs in all threads.
+// every term, and the truncation test runs in all threads.  gridDim.y CTAs
+// share a plane: each forms Q and the truncation, then the rows l = blockIdx.y,
+// + gridDim.y, ... of T and of the kernel (at support 16 the kernel's 133^2
+// sums are most of the work: 193 us with one CTA a plane).
 __global__ void __launch_bounds__(1024) k_wkernel_plane(WkParams q)
 {
     const int p = blockIdx.x;
@@ -1278,16 +1253,18 @@ __global__ void __launch_bounds__(1024) k_wkernel_plane(WkParams q)
     __shared__ int s_support;
     extern __shared__ __align__(16) double sct[];
     // 16-byte cells first, then the cosine table
+    const int lrows = (lh + int(gridDim.y) - 1) / int(gridDim.y); // rows of T of this CTA, at most
+    const size_t cta = size_t(p) * gridDim.y + blockIdx.y;
     double2* sm = reinterpret_cast<double2*>(sct);
-    double2* Q = q.Qs + size_t(p) * half * half;
-    double2* T = q.Ts + size_t(p) * lh * half;
+    double2* Q = q.Qs + cta * half * half;
+    double2* T = q.Ts + cta * lrows * half;
     if (q.smem_Q) {
         Q = sm;
         sm += size_t(half) * half;
     }
     if (q.smem_T) {
         T = sm;
-        sm += size_t(lh) * half;
+        sm += size_t(lrows) * half;
     }
     double2* conv = q.convd + size_t(p) * lh * lh;
     const double* ct = q.ctab;
@@ -1335,22 +1312,22 @@ __global__ void __launch_bounds__(1024) k_wkernel_plane(WkParams q)
     }
     __syncthreads();
     const int S = min(s_support, q.max_support);
-    if (threadIdx.x == 0)
+    if (threadIdx.x == 0 && blockIdx.y == 0)
         q.support[p] = S;
     const int L = min(S * os + os / 2 + 1, (arr >> 1) + 1);
-    // 4. T[l][a] for l < L (l = 0 again: the same values)
-    for (int t = threadIdx.x; t < L * half; t += blockDim.x) {
-        const int a = t % half, l = t / half;
-        T[size_t(l) * half + a] = cos_sum(Q + a, half, half, ct, l, arr);
+    // 4. T[l][a] for this CTA's l < L
+    const int l0 = int(blockIdx.y), dl = int(gridDim.y);
+    const int nl = l0 < L ? (L - l0 + dl - 1) / dl : 0;
+    for (int t = threadIdx.x; t < nl * half; t += blockDim.x) {
+        const int a = t % half, i = t / half;
+        T[size_t(i) * half + a] = cos_sum(Q + a, half, half, ct, l0 + i * dl, arr);
     }
     __syncthreads();
-    // 5. conv(k, l) for k, l < L
-    for (int t = threadIdx.x; t < L * L; t += blockDim.x) {
-        const int k = t % L, l = t / L;
-        conv[size_t(l) * lh + k] = cos_sum(T + size_t(l) * half, 1, half, ct, k, arr);
+    // 5. conv(k, l) for k < L
+    for (int t = threadIdx.x; t < nl * L; t += blockDim.x) {
+        const int k = t % L, i = t / L;
+        conv[size_t(l0 + i * dl) * lh + k] = cos_sum(T + size_t(i) * half, 1, half, ct, k, arr);
     }
-    __syncthreads();
-    wk_inverse_sums(q, p, conv, S);
 }
 
 // Hankel-transform W-kernels (hankel_opt, aw_projection.cpp:211-287 and
@@ -1530,8 +1507,6 @@ __global__ void __launch_bounds__(1024) k_hankel_plane(WkParams q, HankelParams 
         const double r = dy == 0 ? double(dx) : (dx == 0 ? double(dy) : sqrt(double(dx * dx + dy * dy)));
         conv[size_t(dy) * lh + dx] = hankel_interp(h, Y, B, r);
     }
-    __syncthreads();
-    wk_inverse_sums(q, p, conv, S);
 }
 
 __global__ void k_cos_table(int arr, double* c)
@@ -1543,12 +1518,13 @@ __global__ void k_cos_table(int arr, double* c)
 
 // Expanded W-kernel tables for the gridder: one block per (plane, oversampled
 // offset pair); entry j*K + i (column j, row i) holds the reference's cached
-// kernel value conv(|oy|, |ox|) * inv (aw_projection.cpp:415-448), formed in
+// kernel value conv(|oy|, |ox|) / sum(Re) (aw_projection.cpp:415-448), formed in
 // FP64 and rounded once to R.  Plane p's tables start at off[p] = p * stride,
 // or (stride 0) right after those of the planes before; *max_support (zeroed
 // before) = the largest support.
+constexpr int kExpandThreads = 128;
 template <typename R>
-__global__ void k_wk_expand(const double2* convd, const double* invd, const int* support, int P, int cs, int os,
+__global__ void __launch_bounds__(kExpandThreads) k_wk_expand(const double2* convd, const int* support, int P, int cs, int os,
     int lh, uint32_t stride, typename Cplx<R>::T* out, uint32_t* off, unsigned int* max_support)
 {
     const int p = blockIdx.x;
@@ -1565,16 +1541,31 @@ __global__ void k_wk_expand(const double2* convd, const double* invd, const int*
         atomicMax(max_support, unsigned(S));
     }
     const int K = 2 * S + 1;
-    const double inv = invd[(size_t(p) * cs + cy) * cs + cx];
     const double2* conv = convd + size_t(p) * lh * lh;
-    typename Cplx<R>::T* dst = out + base + uint32_t(pair) * uint32_t(K * K);
-    for (int t = threadIdx.x; t < K * K; t += blockDim.x) {
+    auto at = [&](int t) { // |oy|, |ox| of entry t
         const int i = t % K, j = t / K;
         int oy = (i - S) * os + os / 2 - cy;
         int ox = (j - S) * os + os / 2 - cx;
         oy = oy < 0 ? -oy : oy;
         ox = ox < 0 ? -ox : ox;
-        const double2 v = conv[size_t(oy) * lh + ox];
+        return conv[size_t(oy) * lh + ox];
+    };
+    __shared__ double part[kExpandThreads / 32];
+    double ks = 0.0;
+    for (int t = threadIdx.x; t < K * K; t += kExpandThreads)
+        ks += at(t).x;
+    for (int o = 16; o > 0; o >>= 1)
+        ks += __shfl_xor_sync(0xffffffffu, ks, o);
+    if ((threadIdx.x & 31) == 0)
+        part[threadIdx.x >> 5] = ks;
+    __syncthreads();
+    ks = 0.0;
+    for (int w = 0; w < kExpandThreads / 32; w++)
+        ks += part[w];
+    const double inv = 1 / ks;
+    typename Cplx<R>::T* dst = out + base + uint32_t(pair) * uint32_t(K * K);
+    for (int t = threadIdx.x; t < K * K; t += kExpandThreads) {
+        const double2 v = at(t);
         typename Cplx<R>::T o;
         o.x = R(v.x * inv);
         o.y = R(v.y * inv);
