@@ -33,6 +33,7 @@
 #include "common.cuh"
 #include "imager_kernels.cuh"
 #include "gridder_kernels.cuh"
+#include "fft_kernels.cuh"
 #include "sourcefind_kernels.cuh"
 #include "visibility_kernels.cuh"
 #include "aproj_kernels.cuh"
@@ -140,6 +141,7 @@ struct GridOut {
     void* grid = nullptr;
     void* beam = nullptr;
     int image_rows = 0;
+    int ld = 0; // cells from one grid column to the next
     double* d_total = nullptr;             // [0] sample_grid_total
     unsigned long long* d_ngood = nullptr; // [0] good visibilities
     uint32_t* d_nitems = nullptr;          // binned entries
@@ -452,6 +454,7 @@ struct ImagerSetup {
     // compensated FP32 only: grid cells stored in double and the c2r done in
     // double precision (wide_fft_needed decides)
     int wide_fft = 0;
+    int own_c2r = 0; // the c2r on our own kernels (own_c2r_applies decides)
 };
 
 // W-projection with a maximum support above 32: the W-kernel tables and tile
@@ -584,7 +587,9 @@ void grid_blocks(stpgpu_context* c, const ImagerSetup& s, GridOut& g, int64_t n,
         k_bin_fill<R><<<grid1d(n, 256), 256, 0, st>>>(b, in.items, q);
         STPGPU_CHECK_LAUNCH();
     }
-    const size_t cells = size_t(b.rows) * b.N;
+    // columns that start on a 128-byte line where our own kernels read them
+    g.ld = s.own_c2r ? int(ceil_div(b.rows, 16)) * 16 : b.rows;
+    const size_t cells = size_t(g.ld) * b.N;
     const bool f64 = sizeof(R) == 8 || wide;
     g.grid = c->buf<unsigned char>("grid", cells * (f64 ? 16 : 8));
     g.beam = s.beam ? c->buf<unsigned char>("beamgrid", cells * (f64 ? 16 : 8)) : nullptr;
@@ -593,6 +598,7 @@ void grid_blocks(stpgpu_context* c, const ImagerSetup& s, GridOut& g, int64_t n,
         p.rows = b.rows;
         p.pad = b.pad;
         p.brn = b.brn;
+        p.ld = g.ld;
         p.off = b.off;
         p.recs = q.rec;
         p.wts = q.wts;
@@ -1118,6 +1124,123 @@ const double* device_gcf(stpgpu_context* c, const ImagerSetup& s)
     return gcf;
 }
 
+// Whether the c2r runs on our own kernels (k_fft_axis, k_c2r_normalise): grids
+// of a power of two from 256 to 16384 (others take cuFFT's 2-D transform and
+// k_normalise), an image that the kernel can store in pairs, and no
+// single-precision transform into a double image.
+bool own_c2r_applies(const ImagerSetup& s, bool fp64_fft, int out_f32, const void* image, const void* beam)
+{
+    const uintptr_t pair = out_f32 ? 8 : 16;
+    return s.halfplane && (s.N & (s.N - 1)) == 0 && s.N >= (2 << kC2rMinLog) && s.N <= (2 << kC2rMaxLog)
+        && (fp64_fft || out_f32) && reinterpret_cast<uintptr_t>(image) % pair == 0
+        && reinterpret_cast<uintptr_t>(beam) % pair == 0;
+}
+
+// One pass of the columns-axis transform over transforms of length L.
+template <typename T, bool FIRST>
+void launch_axis(stpgpu_context* c, const GridOut& g, void* grid, int N, int L, const void* tw)
+{
+    using C = typename Cplx<T>::T;
+    auto run = [&](auto len) {
+        constexpr int l = decltype(len)::value;
+        constexpr size_t smem = l > 16 ? size_t(axis_groups(l)) * l * 32 * sizeof(C) : 0;
+        auto kern = k_fft_axis<T, l, FIRST>;
+        if (smem > 48 * 1024)
+            STPGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        const dim3 blocks(grid1d(g.image_rows, 32), unsigned(N / l / axis_groups(l)));
+        kern<<<blocks, axis_threads(l), smem, c->stream>>>(static_cast<C*>(grid), g.ld, g.image_rows, N,
+            static_cast<const C*>(tw));
+        STPGPU_CHECK_LAUNCH();
+    };
+    switch (L) {
+    case 16:
+        return run(std::integral_constant<int, 16>());
+    case 32:
+        return run(std::integral_constant<int, 32>());
+    case 64:
+        return run(std::integral_constant<int, 64>());
+    case 128:
+        return run(std::integral_constant<int, 128>());
+    }
+    fail(STPGPU_ERR_UNSUPPORTED, "axis length");
+}
+
+template <typename T, typename RO, int LOGM>
+void launch_c2r(stpgpu_context* c, const ImagerSetup& s, int image_size, int correction, const GridOut& g, const void* F,
+    const void* tw, const double* ginv, void* out, ScalarPack* pack)
+{
+    using C = typename Cplx<T>::T;
+    constexpr size_t smem = c2r_smem(LOGM, sizeof(C));
+    auto kern = k_c2r_normalise<T, RO, LOGM>;
+    if (smem > 48 * 1024)
+        STPGPU_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    kern<<<grid1d(image_size, c2r_rows(LOGM)), c2r_threads(LOGM), smem, c->stream>>>(static_cast<const C*>(F), g.ld,
+        static_cast<const C*>(tw), image_size, g.d_total, ginv, correction, static_cast<RO*>(out), pack_args(g, pack));
+    STPGPU_CHECK_LAUNCH();
+}
+
+template <typename T, typename RO>
+void launch_c2r(stpgpu_context* c, const ImagerSetup& s, int image_size, int correction, const GridOut& g, const void* F,
+    const void* tw, const double* ginv, void* out, ScalarPack* pack)
+{
+    auto run = [&](auto lm) {
+        launch_c2r<T, RO, decltype(lm)::value>(c, s, image_size, correction, g, F, tw, ginv, out, pack);
+    };
+    switch (s.N) {
+    case 256:
+        return run(std::integral_constant<int, 7>());
+    case 512:
+        return run(std::integral_constant<int, 8>());
+    case 1024:
+        return run(std::integral_constant<int, 9>());
+    case 2048:
+        return run(std::integral_constant<int, 10>());
+    case 4096:
+        return run(std::integral_constant<int, 11>());
+    case 8192:
+        return run(std::integral_constant<int, 12>());
+    case 16384:
+        return run(std::integral_constant<int, 13>());
+    }
+    fail(STPGPU_ERR_UNSUPPORTED, "c2r size");
+}
+
+template <typename R>
+void finish_own(stpgpu_context* c, const ImagerSetup& s, int image_size, int correction, const GridOut& g, void* d_image,
+    void* d_beam, int out_f32, ScalarPack* pack)
+{
+    using C = typename Cplx<R>::T;
+    const int N = s.N;
+    C* tw = c->buf<C>("fft_tw", tw_size(N));
+    if (!c->memo("fft_tw", std::to_string(N) + "/" + std::to_string(sizeof(R)))) {
+        int logm = 0;
+        while ((2 << logm) < N)
+            logm++;
+        k_fft_tables<R><<<grid1d(tw_size(N), 256), 256, 0, c->stream>>>(N, logm, tw);
+        STPGPU_CHECK_LAUNCH();
+    }
+    if (correction)
+        device_gcf<R>(c, s);
+    const double* ginv = correction ? c->buf<double>("gcfinv", N) : nullptr;
+    auto one = [&](void* grid, void* out, ScalarPack* pk) {
+        launch_axis<R, true>(c, g, grid, N, axis_n1(N), tw);
+        launch_axis<R, false>(c, g, grid, N, N / axis_n1(N), tw);
+        if (pk)
+            c->mark(3);
+        if constexpr (sizeof(R) == 8) {
+            if (!out_f32) {
+                launch_c2r<R, double>(c, s, image_size, correction, g, grid, tw, ginv, out, pk);
+                return;
+            }
+        }
+        launch_c2r<R, float>(c, s, image_size, correction, g, grid, tw, ginv, out, pk);
+    };
+    one(g.grid, d_image, pack);
+    c->mark(4);
+    if (s.beam && d_beam)
+        one(g.beam, d_beam, nullptr);
+}
+
 // c2r FFT + crop/normalise of a gridded snapshot (fft.cpp:45-135,
 // imager.h:97-213) on the context's current stream; the call's scalars go
 // to `pack`.
@@ -1133,6 +1256,10 @@ void finish_imager(stpgpu_context* c, const ImagerSetup& s, int image_size, int 
     }
     cudaStream_t st = c->stream;
     const int N = s.N;
+    if (s.own_c2r) {
+        finish_own<R>(c, s, image_size, correction, g, d_image, d_beam, out_f32, pack);
+        return;
+    }
     R* img = c->buf<R>("fftimg", size_t(N) * N);
     const cufftType type = sizeof(R) == 8 ? CUFFT_Z2D : CUFFT_C2R;
     cufftHandle h = c->plan(N, type);
@@ -1257,6 +1384,7 @@ void run_imager(stpgpu_context* c, const ImagerSetup& s_in, int image_size, int 
         fail(STPGPU_ERR_INVALID_ARG, "image_size must be even, > 0 and <= padded_image_size");
     ImagerSetup s = s_in;
     s.wide_fft = (COMP == 1 && wide_fft_needed(s, image_size, correction)) ? 1 : 0;
+    s.own_c2r = own_c2r_applies(s, sizeof(R) == 8 || s.wide_fft, out_f32, d_image, d_beam);
     // W-planes without the |w| sort where they apply (mean |w| per plane, no
     // A-projection time steps); a size class whose data did not allow it on
     // its last call (visibilities outside the grid, non-finite w) sorts
@@ -1546,6 +1674,9 @@ void run_batch(stpgpu_context* c, const stpgpu_snapshot* sn, int nb, int precisi
         b.correction = x.pars.gridding_correction;
         if (precision == STPGPU_FP32C)
             b.s.wide_fft = wide_fft_needed(b.s, b.image_size, b.correction) ? 1 : 0;
+        // (host images go through an aligned device buffer)
+        b.s.own_c2r = own_c2r_applies(b.s, precision == STPGPU_FP64 || b.s.wide_fft, out_f32,
+            device_ptrs ? x.image : nullptr, nullptr);
         b.vis = x.vis;
         b.c64 = x.vis_dtype == STPGPU_C64;
         b.wts = x.weights;

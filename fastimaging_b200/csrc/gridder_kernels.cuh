@@ -338,6 +338,7 @@ __global__ void __launch_bounds__(32 * kGridWarps) k_grid_dense(const __grid_con
 template <typename R>
 struct SepParams {
     int N, rows, pad, brn;
+    int ld; // cells from one grid column to the next
     const uint32_t* off;
     const GridRec<R>* recs;
     const R* wts;      // per record (beam)
@@ -512,7 +513,7 @@ struct SepCore {
             const int c = c0 + 2 * (lane & 3) + k;
             if (c >= p.N)
                 continue;
-            const size_t i = size_t(c) * size_t(p.rows) + size_t(r);
+            const size_t i = size_t(c) * size_t(p.ld) + size_t(r);
             G2 v;
             v.x = G(acc[k]);
             v.y = G(acc[2 + k]);
@@ -532,6 +533,7 @@ struct SepCore {
 template <typename R, typename T>
 struct WprojParams {
     int N, rows, pad, brn;
+    int ld; // cells from one grid column to the next
     const uint32_t* off;
     const GridRec<R>* recs;
     const R* wts;                     // per record (beam)
@@ -668,7 +670,7 @@ struct WprojCore {
             const int c = c0 + (lane >> 3) + 4 * k;
             if (c >= p.N)
                 continue;
-            const size_t i = size_t(c) * size_t(p.rows) + size_t(r);
+            const size_t i = size_t(c) * size_t(p.ld) + size_t(r);
             G2 v;
             v.x = G(acc[2 * k]);
             v.y = G(acc[2 * k + 1]);
