@@ -660,9 +660,11 @@ void grid_blocks(stpgpu_context* c, const ImagerSetup& s, GridOut& g, int64_t n,
     by_cell([&](auto cell) {
         using G = decltype(cell);
         if (in.exact)
-            s.beam ? run(SepCore<R, G, true, true>(), p) : run(SepCore<R, G, true, false>(), p);
+            s.beam ? run(SepCore<R, G, true, true, false>(), p) : run(SepCore<R, G, true, false, false>(), p);
+        else if (p.zrow + p.tw <= SepCore<R, G, false, false, true>::kTab) // (oversampling 16 at support 4: 414 values)
+            s.beam ? run(SepCore<R, G, false, true, true>(), p) : run(SepCore<R, G, false, false, true>(), p);
         else
-            s.beam ? run(SepCore<R, G, false, true>(), p) : run(SepCore<R, G, false, false>(), p);
+            s.beam ? run(SepCore<R, G, false, true, false>(), p) : run(SepCore<R, G, false, false, false>(), p);
     });
 }
 

@@ -51,8 +51,8 @@ __global__ void __launch_bounds__(256) k_exact_tables(int kf, double trunc, int 
 // CTA.  The cells stay in registers: nothing is read back, zeroed or
 // updated in memory, and every cell of the grid is written exactly once.
 //
-// The CTA's entries are fetched and decoded once into shared memory (up to
-// kCtaEntries, footprints of up to 8 (kCtaBins - 1) + 1 cells): the bins of
+// The CTA's entries are fetched and decoded once into shared memory
+// (C::kCta at a time, footprints of up to 8 (kCtaBins - 1) + 1 cells): the bins of
 // neighbouring blocks overlap, and a block that stages its own entries spends
 // as much on its ranges and on decoding as on gridding when it holds a few
 // tens of them (138 M warp instructions on the 1M-visibility headline call,
@@ -60,13 +60,14 @@ __global__ void __launch_bounds__(256) k_exact_tables(int kf, double trunc, int 
 // the entries of its own bins 32 at a time, lists those that reach its block
 // and hands the list to the core C.
 //
-// Denser CTAs take their entries block by block, 32 at a time through shared
-// memory, and blocks with more than kHeavy entries (the centre of a
-// concentrated uv coverage) are taken by all eight warps together, their
-// partial cells summed in a fixed order.
+// CTAs with a block of more than 2 kHeavy entries (the centre of a
+// concentrated uv coverage) or, for W-kernels, with more than C::kCta in all,
+// and those of wider footprints, take their entries block by block, 32 at a
+// time through shared memory; blocks with more than kHeavy entries are then
+// taken by all eight warps together, their partial cells summed in a fixed
+// order.
 constexpr int kGridWarps = 8;
 constexpr uint32_t kHeavy = 512;
-constexpr uint32_t kCtaEntries = 960;
 constexpr int kCtaBins = 5; // bins per axis that reach a block, at most, for staging by CTA
 
 struct BlockRanges {
@@ -74,6 +75,25 @@ struct BlockRanges {
     uint32_t total;
     int nb;
 };
+
+// Ranges of `len` entries from `beg` on, lane j's for j < nb <= 32, as one
+// stream.
+__device__ __forceinline__ BlockRanges make_ranges(uint32_t beg, uint32_t len, int nb)
+{
+    const int lane = threadIdx.x & 31;
+    uint32_t incl = len;
+    for (int o = 1; o < nb; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o)
+            incl += y;
+    }
+    BlockRanges r;
+    r.pre = incl - len;
+    r.delta = beg - r.pre;
+    r.total = __shfl_sync(0xffffffffu, incl, nb - 1);
+    r.nb = nb;
+    return r;
+}
 
 // Ranges j0 .. j0 + nb - 1 (nb <= 32) of block (br, bc): the bins' columns.
 __device__ __forceinline__ BlockRanges block_ranges(const uint32_t* __restrict__ off, int brn, int br, int bc, int rows_nb,
@@ -86,19 +106,7 @@ __device__ __forceinline__ BlockRanges block_ranges(const uint32_t* __restrict__
         beg = o[0];
         len = o[rows_nb] - beg;
     }
-    uint32_t incl = len;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o)
-            incl += y;
-    }
-    BlockRanges r;
-    r.pre = incl - len;
-    r.delta = beg - r.pre;
-    r.total = __shfl_sync(0xffffffffu, incl, 31);
-    r.nb = nb;
-    return r;
+    return make_ranges(beg, len, nb);
 }
 
 // Record of stream position t.
@@ -113,39 +121,39 @@ __device__ __forceinline__ uint32_t stream_record(const BlockRanges& r, uint32_t
     return t + d;
 }
 
-// Entries [first, first + n) of st, n <= 32, added to the block whose first
-// row is `row` (relative to the staged entries' origin): those that reach it
-// are listed by position and added by the core.
+// Entries of st, one per lane (position `at`, if `valid`), added to the block
+// whose first row is `row` (relative to the staged entries' origin): those
+// that reach it are listed by position and added by the core.
 template <class C>
-__device__ __forceinline__ void block_add(const typename C::Params& p, const typename C::Staged* st, uint32_t first, uint32_t n,
-    uint32_t dummy, int row, uint16_t* list, typename C::A (&acc)[C::NACC])
+__device__ __forceinline__ void block_add(const typename C::Params& p, const double* stab, const typename C::Staged* st,
+    uint32_t at, bool valid, uint32_t dummy, int row, uint16_t* list, typename C::A (&acc)[C::NACC])
 {
     const int lane = threadIdx.x & 31;
     bool reach = false, odd = false;
-    if (uint32_t(lane) < n) {
-        const typename C::Staged& s = st[first + lane];
+    if (valid) {
+        const typename C::Staged& s = st[at];
         reach = C::reach(p, s, row);
         odd = reach && C::odd(s);
     }
     const unsigned mask = __ballot_sync(0xffffffffu, reach && !odd);
     const int m = __popc(mask);
     if (reach && !odd)
-        list[__popc(mask & ((1u << lane) - 1u))] = uint16_t(first + lane);
+        list[__popc(mask & ((1u << lane) - 1u))] = uint16_t(at);
     if (lane < 3)
         list[m + lane] = uint16_t(dummy); // up to a multiple of four
     __syncwarp();
-    C::accumulate(p, st, list, m, row, acc);
+    C::accumulate(p, stab, st, list, m, row, acc);
     if (C::kOdd) {
         unsigned o = __ballot_sync(0xffffffffu, odd);
         for (; o; o &= o - 1)
-            C::add_odd(p, st[first + __ffs(int(o)) - 1], row, acc);
+            C::add_odd(p, stab, st[__shfl_sync(0xffffffffu, at, __ffs(int(o)) - 1)], row, acc);
     }
     __syncwarp();
 }
 
 template <class C>
-__device__ __forceinline__ void block_walk(const typename C::Params& p, const BlockRanges& r, int r0, int c0, int first,
-    int stride, typename C::Staged* st, uint16_t* list, typename C::A (&acc)[C::NACC])
+__device__ __forceinline__ void block_walk(const typename C::Params& p, const double* stab, const BlockRanges& r, int r0,
+    int c0, int first, int stride, typename C::Staged* st, uint16_t* list, typename C::A (&acc)[C::NACC])
 {
     const int lane = threadIdx.x & 31;
     uint32_t t = uint32_t(first) * 32u;
@@ -167,7 +175,7 @@ __device__ __forceinline__ void block_walk(const typename C::Params& p, const Bl
             if (tn + lane < r.total)
                 raw = C::fetch(p, i);
         }
-        block_add<C>(p, st, 0, n, 32, 0, list, acc);
+        block_add<C>(p, stab, st, uint32_t(lane), uint32_t(lane) < n, 32, 0, list, acc);
         t = tn;
     }
 }
@@ -179,9 +187,9 @@ __global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(
     using Staged = typename C::Staged;
     // entries of the CTA and a dummy per warp; or 32 and a dummy per warp; or
     // the partial cells of a block taken by all warps
-    constexpr size_t kStage = sizeof(Staged) * (kCtaEntries + kGridWarps);
+    constexpr size_t kStage = sizeof(Staged) * (C::kCta + kGridWarps);
     constexpr size_t kRed = sizeof(A) * C::NACC * 32 * kGridWarps;
-    static_assert(kCtaEntries + kGridWarps >= 33 * kGridWarps, "staging by warp");
+    static_assert(C::kCta + kGridWarps >= 33 * kGridWarps, "staging by warp");
     __shared__ __align__(16) unsigned char smem[kStage > kRed ? kStage : kRed];
     __shared__ uint16_t s_list[kGridWarps][36];
     __shared__ uint32_t s_off[kCtaBins][kGridWarps + kCtaBins];
@@ -193,6 +201,8 @@ __global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(
     const int br0 = int(blockIdx.x) * kGridWarps, br = br0 + warp, bc = int(blockIdx.y);
     const int nb = C::bins(p);       // bins that reach a block on either axis
     const int skip = p.pad + 1 - nb; // (those further away cannot)
+    __shared__ double s_tab[C::kTab > 0 ? C::kTab : 1];
+    const double* stab = s_tab;
     if (nb <= kCtaBins) {
         // s_off[j]: the offsets of the CTA's bins in column j
         const int no = kGridWarps + nb;
@@ -201,38 +211,65 @@ __global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(
             s_off[j][i] = p.off[size_t(bc + skip + j) * size_t(p.brn + 1) + size_t(min(br0 + skip + i, p.brn))];
         }
         __syncthreads();
-        uint32_t total = 0;
-        for (int j = 0; j < nb; j++)
+        uint32_t total = 0, own = 0;
+        for (int j = 0; j < nb; j++) {
             total += s_off[j][no - 1] - s_off[j][0];
-        if (total <= kCtaEntries) {
-            for (uint32_t t = threadIdx.x; t < total; t += 32 * kGridWarps) {
-                uint32_t i = t, j = 0;
-                for (;; j++) {
-                    const uint32_t len = s_off[j][no - 1] - s_off[j][0];
-                    if (i < len)
-                        break;
-                    i -= len;
-                }
-                all[t] = C::decode(p, C::fetch(p, s_off[j][0] + i), br0 * kBlk, bc * kBlk);
-            }
-            if (threadIdx.x < kGridWarps)
-                all[kCtaEntries + threadIdx.x] = C::dummy(p, int(threadIdx.x) * kBlk);
-            __syncthreads();
-            if (br >= nbr)
-                return;
+            if (C::kWindows)
+                own += s_off[j][warp + nb] - s_off[j][warp];
+        }
+        if (total == 0) { // nothing reaches the CTA: most of a grid outside the uv coverage
             A acc[C::NACC] = {};
-            uint32_t before = 0;
-            for (int j = 0; j < nb; j++) {
-                const uint32_t o = s_off[j][0];
-                const uint32_t end = before + s_off[j][warp + nb] - o;
-                for (uint32_t e = before + s_off[j][warp] - o; e < end; e += 32)
-                    block_add<C>(p, all, e, min(32u, end - e), kCtaEntries + warp, warp * kBlk, list, acc);
-                before += s_off[j][no - 1] - o;
-            }
-            C::store(p, br * kBlk, bc * kBlk, acc);
+            if (br < nbr)
+                C::store(p, br * kBlk, bc * kBlk, acc);
             return;
         }
-        __syncthreads();
+        C::load_table(p, s_tab);
+        // (the barrier also orders the table before its first use)
+        const bool staged = C::kWindows ? !__syncthreads_or(own > 2 * kHeavy) : total <= C::kCta;
+        if (staged) {
+            if (threadIdx.x < kGridWarps)
+                all[C::kCta + threadIdx.x] = C::dummy(p, int(threadIdx.x) * kBlk);
+            // lane j < nb: column j's entries in the CTA's order, all and the warp's
+            uint32_t beg = 0, end = 0;
+            {
+                const uint32_t o = lane < nb ? s_off[lane][0] : 0u;
+                const BlockRanges c = make_ranges(0, lane < nb ? s_off[lane][no - 1] - o : 0u, nb);
+                if (lane < nb) {
+                    beg = c.pre + s_off[lane][warp] - o;
+                    end = c.pre + s_off[lane][warp + nb] - o;
+                }
+            }
+            A acc[C::NACC] = {};
+            uint32_t w0 = 0;
+            for (;;) {
+                const uint32_t w1 = C::kWindows ? min(total, w0 + C::kCta) : total;
+                for (uint32_t t = w0 + threadIdx.x; t < w1; t += 32 * kGridWarps) {
+                    uint32_t i = t, j = 0;
+                    for (;; j++) {
+                        const uint32_t len = s_off[j][no - 1] - s_off[j][0];
+                        if (i < len)
+                            break;
+                        i -= len;
+                    }
+                    all[t - w0] = C::decode(p, C::fetch(p, s_off[j][0] + i), br0 * kBlk, bc * kBlk);
+                }
+                __syncthreads();
+                const uint32_t lo = C::kWindows ? max(beg, w0) : beg, hi = C::kWindows ? min(end, w1) : end;
+                const BlockRanges r = make_ranges(lo - w0, hi > lo ? hi - lo : 0u, nb);
+                for (uint32_t t = 0; t < r.total; t += 32)
+                    block_add<C>(p, stab, all, stream_record(r, t + lane), t + lane < r.total, C::kCta + warp, warp * kBlk, list,
+                        acc);
+                if (!C::kWindows || w1 == total)
+                    break;
+                w0 = w1;
+                __syncthreads(); // the window's entries are gridded
+            }
+            if (br < nbr)
+                C::store(p, br * kBlk, bc * kBlk, acc);
+            return;
+        }
+    } else {
+        C::load_table(p, s_tab);
     }
     Staged* st = all + warp * 33;
     if (lane == 0)
@@ -251,7 +288,7 @@ __global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(
             heavy = total > kHeavy;
             if (heavy)
                 break;
-            block_walk<C>(p, r, br * kBlk, bc * kBlk, 0, 1, st, list, acc);
+            block_walk<C>(p, stab, r, br * kBlk, bc * kBlk, 0, 1, st, list, acc);
         }
         if (heavy) {
             if (lane == 0)
@@ -267,7 +304,7 @@ __global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(
         A acc[C::NACC] = {};
         for (int j = 0; j < nb; j += 32) {
             const BlockRanges r = block_ranges(p.off, p.brn, hbr + skip, bc + skip + j, nb, min(nb - j, 32));
-            block_walk<C>(p, r, hbr * kBlk, bc * kBlk, warp, kGridWarps, st, list, acc);
+            block_walk<C>(p, stab, r, hbr * kBlk, bc * kBlk, warp, kGridWarps, st, list, acc);
         }
         __syncthreads(); // the staged records are read; the same memory takes the partial cells
         A* red = reinterpret_cast<A*>(smem);
@@ -306,10 +343,13 @@ __global__ void __launch_bounds__(32 * kGridWarps) k_grid_dense(const __grid_con
     __shared__ uint16_t s_list[kGridWarps][36];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = warp % SPLIT, first = warp - sub;
+    __shared__ double s_tab[C::kTab > 0 ? C::kTab : 1];
+    const double* stab = s_tab;
     Staged* st = reinterpret_cast<Staged*>(smem) + warp * 33;
     if (lane == 0)
         st[32] = C::dummy(p, 0);
-    __syncwarp();
+    C::load_table(p, s_tab);
+    __syncthreads();
     const int nbr = (p.rows + kBlk - 1) / kBlk;
     const int br = int(blockIdx.x) * (kGridWarps / SPLIT) + warp / SPLIT, bc = int(blockIdx.y);
     const int nb = C::bins(p), skip = p.pad + 1 - nb;
@@ -317,7 +357,7 @@ __global__ void __launch_bounds__(32 * kGridWarps) k_grid_dense(const __grid_con
     if (br < nbr)
         for (int j = 0; j < nb; j += 32) {
             const BlockRanges r = block_ranges(p.off, p.brn, br + skip, bc + skip + j, nb, min(nb - j, 32));
-            block_walk<C>(p, r, br * kBlk, bc * kBlk, sub, SPLIT, st, s_list[warp], acc);
+            block_walk<C>(p, stab, r, br * kBlk, bc * kBlk, sub, SPLIT, st, s_list[warp], acc);
         }
     __syncthreads(); // the staged records are read; the same memory takes the partial cells
     A* red = reinterpret_cast<A*>(smem);
@@ -364,11 +404,12 @@ struct SepParams {
 // Products and sums are in double whatever the record's precision.  Entries
 // with a weight, visibility or kernel that is not finite are added tap by
 // tap instead, so that they reach their own footprint only.
-template <typename R, typename G, bool EXACT, bool BEAM>
+template <typename R, typename G, bool EXACT, bool BEAM, bool STAB>
 struct SepCore {
     using Params = SepParams<R>;
     using A = double;
     static constexpr int NACC = BEAM ? 6 : 4;
+    static constexpr uint32_t kCta = BEAM ? 384 : 512;
     static constexpr int kMinBlocks = BEAM ? 3 : 5; // (4 blocks of 64 registers: 1460 us against 1421 on the 8192^2 call)
     struct Raw {
         GridRec<R> r;
@@ -390,6 +431,19 @@ struct SepCore {
     };
     using Staged = std::conditional_t<BEAM, StagedB, StagedP>;
     static constexpr bool kOdd = true;
+    static constexpr bool kWindows = true; // CTAs of more than kCta entries in several rounds
+    // STAB: the padded table (at most kTab values) in shared memory.  The four
+    // entries of a product read four runs of eight taps, up to eight lines of
+    // L1 for a global load (which kept its data pipe 73 % busy on the 8192^2
+    // call), about half as many passes over the banks.
+    static constexpr int kTab = STAB ? 768 : 0;
+
+    static __device__ __forceinline__ void load_table(const Params& p, double* s_tab)
+    {
+        if (STAB)
+            for (int t = threadIdx.x; t < p.zrow + p.tw; t += blockDim.x)
+                s_tab[t] = p.tab[t];
+    }
 
     static __device__ __forceinline__ int bins(const Params& p) { return p.pad + 1; }
     static __device__ __forceinline__ Raw fetch(const Params& p, uint32_t i)
@@ -448,7 +502,8 @@ struct SepCore {
         return row0 + p.K > 0 && row0 < kBlk && col0 + p.K > 0 && col0 < kBlk;
     }
     // the taps of either axis at the origin's row / column
-    static __device__ __forceinline__ void taps(const Params& p, const Staged& s, int row, int col, double& a, double& b)
+    static __device__ __forceinline__ void taps(const Params& p, const double* stab, const Staged& s, int row, int col,
+        double& a, double& b)
     {
         if (EXACT) {
             const int K = p.K;
@@ -457,20 +512,24 @@ struct SepCore {
             const double* t = p.tab + size_t(s.vis) * size_t(2 * K);
             a = unsigned(dr) < unsigned(K) ? __ldg(t + (back ? K - 1 - dr : dr)) : 0.0;
             b = unsigned(dc) < unsigned(K) ? __ldg(t + K + (back ? K - 1 - dc : dc)) : 0.0;
+        } else if (STAB) {
+            a = stab[s.ty + row];
+            b = stab[s.tx + col];
         } else {
             a = __ldg(p.tab + s.ty + row);
             b = __ldg(p.tab + s.tx + col);
         }
     }
     // an entry that is not finite: its own footprint's cells only
-    static __device__ __forceinline__ void add_odd(const Params& p, const Staged& s, int row, A (&acc)[NACC])
+    static __device__ __forceinline__ void add_odd(const Params& p, const double* stab, const Staged& s, int row,
+        A (&acc)[NACC])
     {
         const int lane = threadIdx.x & 31;
         for (int k = 0; k < 2; k++) {
             const int r = row + (lane >> 2), c = 2 * (lane & 3) + k;
             if (unsigned(r - row0_of(s)) < unsigned(p.K) && unsigned(c - col0_of(s)) < unsigned(p.K)) {
                 double a, b;
-                taps(p, s, r, c, a, b);
+                taps(p, stab, s, r, c, a, b);
                 acc[k] += a * b * s.vr;
                 acc[2 + k] += a * b * s.vi;
                 if constexpr (BEAM)
@@ -484,8 +543,8 @@ struct SepCore {
             : "+d"(c0), "+d"(c1)
             : "d"(a), "d"(b));
     }
-    static __device__ __forceinline__ void accumulate(const Params& p, const Staged* st, const uint16_t* list, int m, int row,
-        A (&acc)[NACC])
+    static __device__ __forceinline__ void accumulate(const Params& p, const double* stab, const Staged* st,
+        const uint16_t* list, int m, int row, A (&acc)[NACC])
     {
         const int lane = threadIdx.x & 31;
         const int q = lane >> 2;
@@ -493,7 +552,7 @@ struct SepCore {
         for (int g = 0; g < m; g += 4) {
             const Staged& s = st[list[g + (lane & 3)]];
             double a, b;
-            taps(p, s, row + q, q, a, b);
+            taps(p, stab, s, row + q, q, a, b);
             mma(acc[0], acc[1], a, b * s.vr);
             mma(acc[2], acc[3], a, b * s.vi);
             if constexpr (BEAM)
@@ -554,6 +613,8 @@ struct WprojCore {
     using Params = WprojParams<R, T>;
     using A = ACC;
     static constexpr int NACC = BEAM ? 8 : 4;
+    // (960: most CTAs of the untruncated headline call in one go; 512: 2093 us against 1743)
+    static constexpr uint32_t kCta = BEAM ? 720 : 960;
     static constexpr int kMinBlocks = BEAM ? 2 : 4; // (5 blocks of 48 registers spill: 472 us against 490 on the headline call)
     struct Raw {
         GridRec<R> r;
@@ -583,9 +644,12 @@ struct WprojCore {
             w.w = p.wts[i];
         return w;
     }
+    static constexpr bool kWindows = false; // (the loop's registers: 206 -> 234 us on the double headline call)
     static constexpr bool kOdd = false; // (cells outside a footprint are not touched)
     static __device__ __forceinline__ bool odd(const Staged&) { return false; }
-    static __device__ __forceinline__ void add_odd(const Params&, const Staged&, int, A (&)[NACC]) {}
+    static __device__ __forceinline__ void add_odd(const Params&, const double*, const Staged&, int, A (&)[NACC]) {}
+    static constexpr int kTab = 0;
+    static __device__ __forceinline__ void load_table(const Params&, double*) {}
     static __device__ __forceinline__ Staged decode(const Params&, const Raw& w, int r0, int c0)
     {
         Staged s;
@@ -620,8 +684,8 @@ struct WprojCore {
     {
         return __hiloint2double(int(uint32_t(__double2hiint(x)) ^ sign), __double2loint(x));
     }
-    static __device__ __forceinline__ void accumulate(const Params& p, const Staged* st, const uint16_t* list, int m, int row,
-        A (&acc)[NACC])
+    static __device__ __forceinline__ void accumulate(const Params& p, const double* stab, const Staged* st,
+        const uint16_t* list, int m, int row, A (&acc)[NACC])
     {
         using C2 = typename Cplx<T>::T;
         const int lane = threadIdx.x & 31;
