@@ -709,9 +709,13 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
     g.d_err = c->buf<unsigned int>("err", CF_WORDS);
     BlockBins bins = make_bins(c, s, g, n, kernel_exact != 0);
     const bool use_wsel = wproj && n > 0 && s.wsel;
+    int wsel_log = WSEL_MIN_LOG;
+    while (wsel_log < WSEL_MAX_LOG && (int64_t(8) << wsel_log) < n)
+        wsel_log++;
     WselState* ws = use_wsel ? c->buf<WselState>("wsel", 1) : nullptr;
     zero_words(st, { { g.d_err, CF_WORDS }, { bins.count, int64_t(bins.brn) * bins.bcn },
-                       { ws, use_wsel ? int64_t(kWselZeroWords) : 0 } });
+                       { ws, use_wsel ? int64_t(1) << wsel_log : 0 },
+                       { ws ? ws->cursor : nullptr, use_wsel ? int64_t(kWselZeroWords) : 0 } });
     PrepassParams pp {};
     pp.n = n;
     pp.vis = d_vis;
@@ -773,14 +777,13 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
         // again on the sorting path
         const int P = s.nplanes;
         const unsigned g2 = std::min<unsigned>(grid1d(n, 256), 148 * 8);
-        static_assert(WSEL_BINS == 1024 * 64, "chunks of 64 bins, one per thread of the planning block");
-        k_wsel_hist<<<std::min<unsigned>(grid1d(n, 1024), 148), 1024, 0, st>>>(pp.absw_key, n, g.d_total, ws, P, g.d_ngood,
-            g.d_err);
+        k_wsel_hist<<<std::min<unsigned>(grid1d(n, 1024), 148), 1024, 0, st>>>(pp.absw_key, n, g.d_total, ws, wsel_log, P,
+            g.d_ngood, g.d_err);
         STPGPU_CHECK_LAUNCH();
         // members of the start bins: at most P - 1 bins of WSEL_CAP
         unsigned long long* mbits = c->buf<unsigned long long>("wsel_mb", size_t(std::max(P - 1, 1)) * WSEL_CAP);
         uint32_t* midx = c->buf<uint32_t>("wsel_mi", size_t(std::max(P - 1, 1)) * WSEL_CAP);
-        k_wsel_collect<<<g2, 256, 0, st>>>(pp.absw_key, n, g.d_total, ws, mbits, midx);
+        k_wsel_collect<<<g2, 256, 0, st>>>(pp.absw_key, n, g.d_total, ws, wsel_log, mbits, midx);
         STPGPU_CHECK_LAUNCH();
         if (P > 1) {
             k_wsel_resolve<<<P - 1, 256, 0, st>>>(ws, mbits, midx);
@@ -1006,7 +1009,7 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
         } else {
             // shared memory: the cosine table, Q and T in this order of
             // preference (a kernel of 16 cells' support and oversampling 8
-            // takes 4 + 16 + 66 KB)
+            // on four CTAs takes 4 + 16 + 17 KB)
             size_t smem = 0;
             auto fits = [&](size_t bytes) {
                 if (smem + bytes > 160 * 1024)

@@ -759,7 +759,7 @@ __global__ void k_gather_good(const uint32_t* perm, const Item<R>* items, const 
 // p)), so an item's plane follows from how many plane-start items precede
 // it in the sort order ((|w| bits, input index), the stable order).  Those
 // P - 1 items are found without sorting: a histogram of the 24-bit keys'
-// top 16 bits places each start rank in a bin and at a rank within it
+// top 12 to 16 bits places each start rank in a bin and at a rank within it
 // (k_wsel_hist and, in its last block, wsel_plan); the members of those bins are collected
 // (k_wsel_collect) and each start item is the member of its bin with the
 // wanted rank under the exact order (k_wsel_resolve: every member counts the
@@ -770,8 +770,10 @@ __global__ void k_gather_good(const uint32_t* perm, const Item<R>* items, const 
 // and plane starts.  Items not all good, non-finite |w|, more than WSEL_MAXP
 // planes or a start bin of more than WSEL_CAP members set bit 16 of the
 // error word: the host then runs the sorting path.
-constexpr int WSEL_BINS_LOG = 16;
-constexpr int WSEL_BINS = 1 << WSEL_BINS_LOG; // key24 >> 8
+// Bins: a power of two near n / 8 (about ten members in a start bin; small
+// calls plan over fewer bins), key24 >> (24 - blog).
+constexpr int WSEL_MIN_LOG = 12, WSEL_MAX_LOG = 16;
+constexpr int WSEL_BINS = 1 << WSEL_MAX_LOG;
 constexpr int WSEL_CAP = 2048;  // members of a start item's bin that k_wsel_resolve holds
 constexpr int WSEL_MAXP = 1024; // planes
 
@@ -793,7 +795,7 @@ struct WselState {
     int64_t G[WSEL_MAXP + 1];
     int valid;
 };
-constexpr size_t kWselZeroWords = (sizeof(uint32_t) * (WSEL_BINS + WSEL_MAXP + 2) + sizeof(unsigned long long) * WSEL_MAXP) / 4;
+constexpr size_t kWselZeroWords = (sizeof(uint32_t) * (WSEL_MAXP + 2) + sizeof(unsigned long long) * WSEL_MAXP) / 4; // beside hist
 
 // Exclusive scan over the 1024 threads of a block of the values v; *total =
 // their sum.
@@ -828,29 +830,29 @@ __device__ __forceinline__ uint32_t wsel_block_scan(uint32_t v, uint32_t* total)
 
 // One block of 1024 threads.  The plane starts have a closed form: with q =
 // n / P and r = n % P, ceil((n - G_p) / (P - p)) = q + [p < r], so G_p = p q +
-// min(p, r).  A block scan of the totals of 1024 chunks of 64 bins locates
+// min(p, r).  A block scan of the totals of 1024 chunks of bins locates
 // each start rank's chunk, and the plane's thread walks the chunk's bins to
 // the bin and the rank within it.  The start bins become lists in plane order.
-__device__ __forceinline__ void wsel_plan(WselState* ws, int64_t n, int P, const unsigned long long* ngood, unsigned int* err)
+__device__ __forceinline__ void wsel_plan(WselState* ws, int blog, int64_t n, int P, const unsigned long long* ngood,
+    unsigned int* err)
 {
-    constexpr int PER = WSEL_BINS / 1024;
+    const int per = 1 << (blog - 10); // bins per chunk, 4 to 64
     __shared__ uint32_t chunk[1025]; // prefix at each thread's first bin
     const int tid = threadIdx.x;
     const bool ok0 = ngood[0] == (unsigned long long)n && P >= 1 && P <= WSEL_MAXP;
-    // totals of the 1024 chunks of 64 bins: half a warp a chunk, so that a
-    // load covers two whole chunks (a thread reading its own chunk touches 32
-    // lines per load)
+    // totals of the 1024 chunks: four bins a lane, so that a load covers whole
+    // lines (a thread reading its own chunk touches 32 lines per load)
     {
-        const int lane = tid & 31, warp = tid >> 5;
-        const uint4* c4 = reinterpret_cast<const uint4*>(ws->hist) + warp * (32 * PER / 4);
+        const int lane = tid & 31, warp = tid >> 5, lanes = per / 4; // lanes per chunk
+        const uint4* c4 = reinterpret_cast<const uint4*>(ws->hist) + warp * (32 * lanes);
 #pragma unroll 8
-        for (int c = 0; c < 32; c += 2) {
-            const uint4 v = __ldcg(c4 + c * (PER / 4) + lane);
+        for (int c = 0; c < lanes; c++) {
+            const uint4 v = __ldcg(c4 + c * 32 + lane);
             uint32_t t = v.x + v.y + v.z + v.w;
-            for (int o = 8; o > 0; o >>= 1)
+            for (int o = lanes / 2; o > 0; o >>= 1)
                 t += __shfl_xor_sync(0xffffffffu, t, o);
-            if ((lane & 15) == 0)
-                chunk[warp * 32 + c + (lane >> 4)] = t;
+            if ((lane & (lanes - 1)) == 0)
+                chunk[warp * 32 + (c * 32 + lane) / lanes] = t;
         }
         __syncthreads();
     }
@@ -884,7 +886,7 @@ __device__ __forceinline__ void wsel_plan(WselState* ws, int64_t n, int P, const
             else
                 hi = mid - 1;
         }
-        const uint2 v = __ldcg(reinterpret_cast<const uint2*>(ws->hist + PER * lo) + lane);
+        const uint2 v = 2 * lane < per ? __ldcg(reinterpret_cast<const uint2*>(ws->hist + per * lo) + lane) : make_uint2(0u, 0u);
         uint32_t x = v.x + v.y;
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
@@ -896,7 +898,7 @@ __device__ __forceinline__ void wsel_plan(WselState* ws, int64_t n, int P, const
         if (lane == at) {
             const uint32_t first = end - v.x - v.y; // before the lane's first bin
             const bool second = first + v.x <= gp;
-            sbin[p] = uint32_t(PER * lo + 2 * lane) + (second ? 1u : 0u);
+            sbin[p] = uint32_t(per * lo + 2 * lane) + (second ? 1u : 0u);
             srank[p] = gp - (second ? first + v.x : first);
             ssize[p] = second ? v.y : v.x;
         }
@@ -958,27 +960,27 @@ __device__ __forceinline__ void wsel_plan(WselState* ws, int64_t n, int P, const
 // Histogram of the 24-bit keys (those of k_wkey24, formed here and again in
 // k_wsel_collect from |w|), then the plan by the last block.
 __global__ void __launch_bounds__(1024) k_wsel_hist(const double* __restrict__ absw, int64_t n, const double* total,
-    WselState* ws, int P, const unsigned long long* ngood, unsigned int* err)
+    WselState* ws, int blog, int P, const unsigned long long* ngood, unsigned int* err)
 {
     const WKey kf(total, n);
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-        atomicAdd(&ws->hist[kf(absw[i]) >> (24 - WSEL_BINS_LOG)], 1u);
+        atomicAdd(&ws->hist[kf(absw[i]) >> (24 - blog)], 1u);
     // no start bins yet (the plan marks them)
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < WSEL_BINS; b += gridDim.x * blockDim.x)
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < (1 << blog); b += gridDim.x * blockDim.x)
         ws->binmap[b] = -1;
     if (last_block(&ws->tickets[0]))
-        wsel_plan(ws, n, P, ngood, err);
+        wsel_plan(ws, blog, n, P, ngood, err);
 }
 
 __global__ void __launch_bounds__(256) k_wsel_collect(const double* __restrict__ absw, int64_t n, const double* total,
-    WselState* ws, unsigned long long* mbits, uint32_t* midx)
+    WselState* ws, int blog, unsigned long long* mbits, uint32_t* midx)
 {
     if (!ws->valid)
         return;
     const WKey kf(total, n);
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
         const double a = absw[i];
-        const int li = ws->binmap[kf(a) >> (24 - WSEL_BINS_LOG)];
+        const int li = ws->binmap[kf(a) >> (24 - blog)];
         if (li >= 0) {
             const uint32_t pos = ws->list_off[li] + atomicAdd(&ws->cursor[li], 1u);
             mbits[pos] = __double_as_longlong(a);
