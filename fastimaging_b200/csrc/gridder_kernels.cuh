@@ -121,39 +121,80 @@ __device__ __forceinline__ uint32_t stream_record(const BlockRanges& r, uint32_t
     return t + d;
 }
 
-// Entries of st, one per lane (position `at`, if `valid`), added to the block
-// whose first row is `row` (relative to the staged entries' origin): those
-// that reach it are listed by position and added by the core.
-template <class C>
-__device__ __forceinline__ void block_add(const typename C::Params& p, const double* stab, const typename C::Staged* st,
-    uint32_t at, bool valid, uint32_t dummy, int row, uint16_t* list, typename C::A (&acc)[C::NACC])
+// Positions of the entries that reach a warp's block, in PARTS lists: an entry
+// is on the list of every part of the block that it reaches, and the parts
+// take an entry each at a time.  The longest list counts, which over 32
+// entries (one bin's, often) is that of the part next to it, so two lists
+// gather entries over several rounds before they are added; one list is added
+// after each round.  Lists are filled up with a dummy to a multiple of four.
+template <int PARTS>
+struct BlockList {
+    static constexpr int kSize = PARTS > 1 ? 128 : 32;
+    uint16_t* list;
+    int m[PARTS];
+};
+
+// The entries listed added to the block whose first row is `row` (relative to
+// the staged entries' origin).
+template <class C, int PARTS>
+__device__ __forceinline__ void list_add(const typename C::Params& p, const double* stab, const typename C::Staged* st,
+    uint32_t dummy, int row, BlockList<PARTS>& b, typename C::A (&acc)[C::NACC])
 {
     const int lane = threadIdx.x & 31;
-    bool reach = false, odd = false;
+    int n = b.m[0];
+#pragma unroll
+    for (int h = 1; h < PARTS; h++)
+        n = max(n, b.m[h]);
+    n = (n + 3) & ~3;
+#pragma unroll
+    for (int h = 0; h < PARTS; h++)
+        for (int i = b.m[h] + lane; i < n; i += 32)
+            b.list[h * BlockList<PARTS>::kSize + i] = uint16_t(dummy);
+    __syncwarp();
+    C::template accumulate<PARTS>(p, stab, st, b.list, n, row, acc);
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < PARTS; h++)
+        b.m[h] = 0;
+}
+
+// Entries of st, one per lane (position `at`, if `valid`), listed if they
+// reach the block, and added if they are the only list's or a list may not
+// have room for 32 more.
+template <class C, int PARTS>
+__device__ __forceinline__ void block_add(const typename C::Params& p, const double* stab, const typename C::Staged* st,
+    uint32_t at, bool valid, uint32_t dummy, int row, BlockList<PARTS>& b, typename C::A (&acc)[C::NACC])
+{
+    const int lane = threadIdx.x & 31;
+    unsigned reach = 0; // bit h: part h
+    bool odd = false;
     if (valid) {
         const typename C::Staged& s = st[at];
-        reach = C::reach(p, s, row);
+        reach = C::template reach<PARTS>(p, s, row);
         odd = reach && C::odd(s);
     }
-    const unsigned mask = __ballot_sync(0xffffffffu, reach && !odd);
-    const int m = __popc(mask);
-    if (reach && !odd)
-        list[__popc(mask & ((1u << lane) - 1u))] = uint16_t(at);
-    if (lane < 3)
-        list[m + lane] = uint16_t(dummy); // up to a multiple of four
-    __syncwarp();
-    C::accumulate(p, stab, st, list, m, row, acc);
+    bool full = PARTS == 1;
+#pragma unroll
+    for (int h = 0; h < PARTS; h++) {
+        const bool in = ((reach >> h) & 1u) && !odd;
+        const unsigned mask = __ballot_sync(0xffffffffu, in);
+        if (in)
+            b.list[h * BlockList<PARTS>::kSize + b.m[h] + __popc(mask & ((1u << lane) - 1u))] = uint16_t(at);
+        b.m[h] += __popc(mask);
+        full |= b.m[h] > BlockList<PARTS>::kSize - 32;
+    }
     if (C::kOdd) {
         unsigned o = __ballot_sync(0xffffffffu, odd);
         for (; o; o &= o - 1)
             C::add_odd(p, stab, st[__shfl_sync(0xffffffffu, at, __ffs(int(o)) - 1)], row, acc);
     }
-    __syncwarp();
+    if (full)
+        list_add<C, PARTS>(p, stab, st, dummy, row, b, acc);
 }
 
 template <class C>
 __device__ __forceinline__ void block_walk(const typename C::Params& p, const double* stab, const BlockRanges& r, int r0,
-    int c0, int first, int stride, typename C::Staged* st, uint16_t* list, typename C::A (&acc)[C::NACC])
+    int c0, int first, int stride, typename C::Staged* st, BlockList<1>& list, typename C::A (&acc)[C::NACC])
 {
     const int lane = threadIdx.x & 31;
     uint32_t t = uint32_t(first) * 32u;
@@ -175,9 +216,64 @@ __device__ __forceinline__ void block_walk(const typename C::Params& p, const do
             if (tn + lane < r.total)
                 raw = C::fetch(p, i);
         }
-        block_add<C>(p, stab, st, uint32_t(lane), uint32_t(lane) < n, 32, 0, list, acc);
+        block_add<C, 1>(p, stab, st, uint32_t(lane), uint32_t(lane) < n, 32, 0, list, acc);
         t = tn;
     }
+}
+
+using CtaOffsets = uint32_t[kCtaBins][kGridWarps + kCtaBins];
+
+// A CTA's `total` entries (bins at off, nb to an axis), staged at `all`.
+template <class C, int PARTS>
+__device__ __forceinline__ void grid_staged(const typename C::Params& p, const double* stab, typename C::Staged* all,
+    const CtaOffsets& off, uint16_t* lists, int nb, uint32_t total)
+{
+    using A = typename C::A;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int br0 = int(blockIdx.x) * kGridWarps, br = br0 + warp, bc = int(blockIdx.y);
+    const int no = kGridWarps + nb;
+    const uint32_t dummy = C::kCta + uint32_t(warp);
+    BlockList<PARTS> list { lists, {} };
+    if (threadIdx.x < kGridWarps)
+        all[C::kCta + threadIdx.x] = C::dummy(p, int(threadIdx.x) * kBlk);
+    // lane j < nb: column j's entries in the CTA's order, all and the warp's
+    uint32_t beg = 0, end = 0;
+    {
+        const uint32_t o = lane < nb ? off[lane][0] : 0u;
+        const BlockRanges c = make_ranges(0, lane < nb ? off[lane][no - 1] - o : 0u, nb);
+        if (lane < nb) {
+            beg = c.pre + off[lane][warp] - o;
+            end = c.pre + off[lane][warp + nb] - o;
+        }
+    }
+    A acc[C::NACC] = {};
+    uint32_t w0 = 0;
+    for (;;) {
+        const uint32_t w1 = C::kWindows ? min(total, w0 + C::kCta) : total;
+        for (uint32_t t = w0 + threadIdx.x; t < w1; t += 32 * kGridWarps) {
+            uint32_t i = t, j = 0;
+            for (;; j++) {
+                const uint32_t len = off[j][no - 1] - off[j][0];
+                if (i < len)
+                    break;
+                i -= len;
+            }
+            all[t - w0] = C::decode(p, C::fetch(p, off[j][0] + i), br0 * kBlk, bc * kBlk);
+        }
+        __syncthreads();
+        const uint32_t lo = C::kWindows ? max(beg, w0) : beg, hi = C::kWindows ? min(end, w1) : end;
+        const BlockRanges r = make_ranges(lo - w0, hi > lo ? hi - lo : 0u, nb);
+        for (uint32_t t = 0; t < r.total; t += 32)
+            block_add<C, PARTS>(p, stab, all, stream_record(r, t + lane), t + lane < r.total, dummy, warp * kBlk, list, acc);
+        if (PARTS > 1)
+            list_add<C, PARTS>(p, stab, all, dummy, warp * kBlk, list, acc);
+        if (!C::kWindows || w1 == total)
+            break;
+        w0 = w1;
+        __syncthreads(); // the window's entries are gridded
+    }
+    if (br < (p.rows + kBlk - 1) / kBlk)
+        C::template store<PARTS>(p, br * kBlk, bc * kBlk, acc);
 }
 
 template <class C>
@@ -191,12 +287,12 @@ __global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(
     constexpr size_t kRed = sizeof(A) * C::NACC * 32 * kGridWarps;
     static_assert(C::kCta + kGridWarps >= 33 * kGridWarps, "staging by warp");
     __shared__ __align__(16) unsigned char smem[kStage > kRed ? kStage : kRed];
-    __shared__ uint16_t s_list[kGridWarps][36];
-    __shared__ uint32_t s_off[kCtaBins][kGridWarps + kCtaBins];
+    __shared__ uint16_t s_list[kGridWarps][C::kParts * BlockList<C::kParts>::kSize];
+    __shared__ CtaOffsets s_off;
     __shared__ uint32_t s_heavy;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Staged* all = reinterpret_cast<Staged*>(smem);
-    uint16_t* list = s_list[warp];
+    BlockList<1> list { s_list[warp], {} };
     const int nbr = (p.rows + kBlk - 1) / kBlk;
     const int br0 = int(blockIdx.x) * kGridWarps, br = br0 + warp, bc = int(blockIdx.y);
     const int nb = C::bins(p);       // bins that reach a block on either axis
@@ -220,52 +316,17 @@ __global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(
         if (total == 0) { // nothing reaches the CTA: most of a grid outside the uv coverage
             A acc[C::NACC] = {};
             if (br < nbr)
-                C::store(p, br * kBlk, bc * kBlk, acc);
+                C::template store<1>(p, br * kBlk, bc * kBlk, acc);
             return;
         }
         C::load_table(p, s_tab);
         // (the barrier also orders the table before its first use)
         const bool staged = C::kWindows ? !__syncthreads_or(own > 2 * kHeavy) : total <= C::kCta;
         if (staged) {
-            if (threadIdx.x < kGridWarps)
-                all[C::kCta + threadIdx.x] = C::dummy(p, int(threadIdx.x) * kBlk);
-            // lane j < nb: column j's entries in the CTA's order, all and the warp's
-            uint32_t beg = 0, end = 0;
-            {
-                const uint32_t o = lane < nb ? s_off[lane][0] : 0u;
-                const BlockRanges c = make_ranges(0, lane < nb ? s_off[lane][no - 1] - o : 0u, nb);
-                if (lane < nb) {
-                    beg = c.pre + s_off[lane][warp] - o;
-                    end = c.pre + s_off[lane][warp + nb] - o;
-                }
-            }
-            A acc[C::NACC] = {};
-            uint32_t w0 = 0;
-            for (;;) {
-                const uint32_t w1 = C::kWindows ? min(total, w0 + C::kCta) : total;
-                for (uint32_t t = w0 + threadIdx.x; t < w1; t += 32 * kGridWarps) {
-                    uint32_t i = t, j = 0;
-                    for (;; j++) {
-                        const uint32_t len = s_off[j][no - 1] - s_off[j][0];
-                        if (i < len)
-                            break;
-                        i -= len;
-                    }
-                    all[t - w0] = C::decode(p, C::fetch(p, s_off[j][0] + i), br0 * kBlk, bc * kBlk);
-                }
-                __syncthreads();
-                const uint32_t lo = C::kWindows ? max(beg, w0) : beg, hi = C::kWindows ? min(end, w1) : end;
-                const BlockRanges r = make_ranges(lo - w0, hi > lo ? hi - lo : 0u, nb);
-                for (uint32_t t = 0; t < r.total; t += 32)
-                    block_add<C>(p, stab, all, stream_record(r, t + lane), t + lane < r.total, C::kCta + warp, warp * kBlk, list,
-                        acc);
-                if (!C::kWindows || w1 == total)
-                    break;
-                w0 = w1;
-                __syncthreads(); // the window's entries are gridded
-            }
-            if (br < nbr)
-                C::store(p, br * kBlk, bc * kBlk, acc);
+            if (C::kParts > 1 && C::parts(p))
+                grid_staged<C, C::kParts>(p, s_tab, all, s_off, s_list[warp], nb, total);
+            else
+                grid_staged<C, 1>(p, s_tab, all, s_off, s_list[warp], nb, total);
             return;
         }
     } else {
@@ -294,7 +355,7 @@ __global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(
             if (lane == 0)
                 atomicOr(&s_heavy, 1u << warp);
         } else {
-            C::store(p, br * kBlk, bc * kBlk, acc);
+            C::template store<1>(p, br * kBlk, bc * kBlk, acc);
         }
     }
     __syncthreads();
@@ -318,7 +379,7 @@ __global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(
                     v += red[(q * kGridWarps + w) * 32 + lane];
                 acc[q] = v;
             }
-            C::store(p, hbr * kBlk, bc * kBlk, acc);
+            C::template store<1>(p, hbr * kBlk, bc * kBlk, acc);
         }
         __syncthreads();
         if (lane == 0)
@@ -340,12 +401,13 @@ __global__ void __launch_bounds__(32 * kGridWarps) k_grid_dense(const __grid_con
     constexpr size_t kStage = sizeof(Staged) * 33 * kGridWarps;
     constexpr size_t kRed = sizeof(A) * C::NACC * 32 * kGridWarps;
     __shared__ __align__(16) unsigned char smem[kStage > kRed ? kStage : kRed];
-    __shared__ uint16_t s_list[kGridWarps][36];
+    __shared__ uint16_t s_list[kGridWarps][C::kParts * BlockList<C::kParts>::kSize];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = warp % SPLIT, first = warp - sub;
     __shared__ double s_tab[C::kTab > 0 ? C::kTab : 1];
     const double* stab = s_tab;
     Staged* st = reinterpret_cast<Staged*>(smem) + warp * 33;
+    BlockList<1> list { s_list[warp], {} };
     if (lane == 0)
         st[32] = C::dummy(p, 0);
     C::load_table(p, s_tab);
@@ -357,7 +419,7 @@ __global__ void __launch_bounds__(32 * kGridWarps) k_grid_dense(const __grid_con
     if (br < nbr)
         for (int j = 0; j < nb; j += 32) {
             const BlockRanges r = block_ranges(p.off, p.brn, br + skip, bc + skip + j, nb, min(nb - j, 32));
-            block_walk<C>(p, stab, r, br * kBlk, bc * kBlk, sub, SPLIT, st, s_list[warp], acc);
+            block_walk<C>(p, stab, r, br * kBlk, bc * kBlk, sub, SPLIT, st, list, acc);
         }
     __syncthreads(); // the staged records are read; the same memory takes the partial cells
     A* red = reinterpret_cast<A*>(smem);
@@ -370,7 +432,7 @@ __global__ void __launch_bounds__(32 * kGridWarps) k_grid_dense(const __grid_con
     for (int w = first + 1; w < first + SPLIT; w++)
         for (int q = 0; q < C::NACC; q++)
             acc[q] += red[(q * kGridWarps + w) * 32 + lane];
-    C::store(p, br * kBlk, bc * kBlk, acc);
+    C::template store<1>(p, br * kBlk, bc * kBlk, acc);
 }
 
 // ---------------------------------------------------------------- separable kernels
@@ -496,7 +558,10 @@ struct SepCore {
     static __device__ __forceinline__ int row0_of(const Staged& s) { return int(s.rc & 1023u) - 512; }
     static __device__ __forceinline__ int col0_of(const Staged& s) { return int((s.rc >> 10) & 1023u) - 512; }
     static __device__ __forceinline__ bool odd(const Staged& s) { return (s.rc >> 21) & 1u; }
-    static __device__ __forceinline__ bool reach(const Params& p, const Staged& s, int row)
+    static constexpr int kParts = 1;
+    static __device__ __forceinline__ bool parts(const Params&) { return false; }
+    template <int>
+    static __device__ __forceinline__ unsigned reach(const Params& p, const Staged& s, int row)
     {
         const int row0 = row0_of(s) - row, col0 = col0_of(s);
         return row0 + p.K > 0 && row0 < kBlk && col0 + p.K > 0 && col0 < kBlk;
@@ -543,6 +608,7 @@ struct SepCore {
             : "+d"(c0), "+d"(c1)
             : "d"(a), "d"(b));
     }
+    template <int PARTS>
     static __device__ __forceinline__ void accumulate(const Params& p, const double* stab, const Staged* st,
         const uint16_t* list, int m, int row, A (&acc)[NACC])
     {
@@ -560,6 +626,7 @@ struct SepCore {
         }
     }
     // lane: row lane / 4, columns 2 (lane % 4) and the next
+    template <int PARTS>
     static __device__ __forceinline__ void store(const Params& p, int r0, int c0, const A (&acc)[NACC])
     {
         using G2 = typename Cplx<G>::T;
@@ -603,9 +670,10 @@ struct WprojParams {
 };
 
 // W-kernels: each lane keeps two cells of the block (row lane % 8, columns
-// lane / 8 and that + 4) in registers and adds the entries one after the
-// other: eight lanes read eight consecutive kernel values (rows of one
-// column), so a warp's load touches the footprint's columns once each.  The
+// lane / 8 and that + 4; in two parts, two columns of its part) in registers
+// and adds the entries one after the other: eight lanes read eight
+// consecutive kernel values (rows of one column), so a warp's load touches the
+// footprint's columns once each.  The
 // kernel values of the next entries are in flight while one is added.  Sums
 // (type A) are in double for FP64 and compensated FP32.
 template <typename R, typename G, typename T, typename ACC, bool BEAM>
@@ -613,8 +681,9 @@ struct WprojCore {
     using Params = WprojParams<R, T>;
     using A = ACC;
     static constexpr int NACC = BEAM ? 8 : 4;
-    // (960: most CTAs of the untruncated headline call in one go; 512: 2093 us against 1743)
-    static constexpr uint32_t kCta = BEAM ? 720 : 960;
+    // (most CTAs of the untruncated headline call in one go: 512 2093 us, 960 1743; and four CTAs an SM within
+    // 132 KB of shared memory, so that L1 keeps the rest)
+    static constexpr uint32_t kCta = BEAM ? 720 : 864;
     static constexpr int kMinBlocks = BEAM ? 2 : 4; // (5 blocks of 48 registers spill: 472 us against 490 on the headline call)
     struct Raw {
         GridRec<R> r;
@@ -671,10 +740,33 @@ struct WprojCore {
         Staged z {};
         return z;
     }
-    static __device__ __forceinline__ bool reach(const Params&, const Staged& s, int row)
+    // a lane's first column, and from that to its second
+    template <int PARTS>
+    static __device__ __forceinline__ int lane_col(int lane)
     {
-        const int K = int(s.kc & 0xffffu), row0 = s.row0 - row;
-        return row0 + K > 0 && row0 < kBlk && s.col0 + K > 0 && s.col0 < kBlk;
+        return PARTS == 2 ? (lane >> 4) * 4 + ((lane >> 3) & 1) : lane >> 3;
+    }
+    // Small footprints in two parts, columns 0 to 3 and 4 to 7, each half of the
+    // warp with an entry of its own: an entry of 5 x 5 cells reaches 11 of a
+    // block's 64 on average, and two of three entries only one part.  Kernel on
+    // the 1M-visibility 4096^2 call, one part and two: 196 and 178 us (largest
+    // support 16, truncated to 2 to 3 mostly), untruncated support 3 216 and 196
+    // (double 214 and 205), 6 401 and 371 (397 and 387), 8 538 and 512 (528 and
+    // 537); 12 909 and 879 to 968.
+    static constexpr int kParts = 2;
+    static __device__ __forceinline__ bool parts(const Params& p)
+    {
+        return p.max_support[0] <= (sizeof(T) == 4 ? 8u : 6u);
+    }
+    template <int PARTS>
+    static __device__ __forceinline__ unsigned reach(const Params&, const Staged& s, int row)
+    {
+        const int K = int(s.kc & 0xffffu), row0 = s.row0 - row, end = s.col0 + K;
+        if (row0 + K <= 0 || row0 >= kBlk)
+            return 0;
+        if (PARTS == 1)
+            return end > 0 && s.col0 < kBlk;
+        return unsigned(end > 0 && s.col0 < kBlk / 2) | unsigned(end > kBlk / 2 && s.col0 < kBlk) << 1;
     }
     static __device__ __forceinline__ float flip(float x, uint32_t sign)
     {
@@ -684,13 +776,17 @@ struct WprojCore {
     {
         return __hiloint2double(int(uint32_t(__double2hiint(x)) ^ sign), __double2loint(x));
     }
+    template <int PARTS>
     static __device__ __forceinline__ void accumulate(const Params& p, const double* stab, const Staged* st,
         const uint16_t* list, int m, int row, A (&acc)[NACC])
     {
         using C2 = typename Cplx<T>::T;
         const int lane = threadIdx.x & 31;
-        const int r = row + (lane & 7), c = lane >> 3;
+        const int r = row + (lane & 7), c = lane_col<PARTS>(lane);
+        constexpr int step = 4 / PARTS;
         const C2* __restrict__ wk = p.wk;
+        if (PARTS == 2)
+            list += (lane >> 4) * BlockList<PARTS>::kSize;
 #pragma unroll 4
         for (int e = 0; e < m; e++) {
             const Staged s = st[list[e]];
@@ -698,14 +794,14 @@ struct WprojCore {
             const uint32_t sign = s.kc & 0x80000000u;
             const int dr = r - s.row0, dc = c - s.col0;
             const bool in = unsigned(dr) < unsigned(K);
-            const bool in0 = in && unsigned(dc) < unsigned(K), in1 = in && unsigned(dc + 4) < unsigned(K);
+            const bool in0 = in && unsigned(dc) < unsigned(K), in1 = in && unsigned(dc + step) < unsigned(K);
             const uint32_t i = s.koff + uint32_t(dc * K + dr);
             C2 v[2];
             v[0].x = v[0].y = v[1].x = v[1].y = T(0);
             if (in0)
                 v[0] = __ldg(wk + i);
             if (in1)
-                v[1] = __ldg(wk + (i + uint32_t(4 * K)));
+                v[1] = __ldg(wk + (i + uint32_t(step * K)));
 #pragma unroll
             for (int k = 0; k < 2; k++) {
                 if (k ? in1 : in0) {
@@ -722,6 +818,7 @@ struct WprojCore {
             }
         }
     }
+    template <int PARTS>
     static __device__ __forceinline__ void store(const Params& p, int r0, int c0, const A (&acc)[NACC])
     {
         using G2 = typename Cplx<G>::T;
@@ -731,7 +828,7 @@ struct WprojCore {
             return;
 #pragma unroll
         for (int k = 0; k < 2; k++) {
-            const int c = c0 + (lane >> 3) + 4 * k;
+            const int c = c0 + lane_col<PARTS>(lane) + 4 / PARTS * k;
             if (c >= p.N)
                 continue;
             const size_t i = size_t(c) * size_t(p.ld) + size_t(r);

@@ -53,6 +53,35 @@ def test_dense_blocks_match_oracle(ctx, n):
     _compare(ctx, capi.GaussianSinc, 3, 64, uv, vis, wts, False, 8, True)
 
 
+def _uneven(seed, n, N):
+    """A grid with few entries a block on average: a quarter of them in the blocks around the origin (more than one
+    warp takes alone), a quarter at a few dozen entries a block (more than a CTA stages at once), the rest anywhere."""
+    uv, vis, wts = _points(seed, n, N, 1.02)
+    rng = np.random.default_rng(seed + 1)
+    uv[::4] = rng.normal(scale=4.0, size=uv[::4].shape)
+    uv[1::4] = rng.uniform(20.0, 100.0, size=uv[1::4].shape)
+    return uv, vis, wts
+
+
+@pytest.mark.parametrize("exact,S", [(False, 3), (True, 3), (False, 5), (True, 6)])
+def test_uneven_blocks_match_oracle(ctx, exact, S):
+    uv, vis, wts = _uneven(S, 16000, 512)
+    _compare(ctx, capi.PSWF, S, 512, uv, vis, wts, exact, 8, True)
+
+
+@pytest.mark.parametrize("smax", [3, 8, 12])
+def test_uneven_w_blocks_match_oracle(ctx, smax):
+    N, cell = 512, 20.0
+    uv, vis, wts = _uneven(smax, 16000, N)
+    w = np.random.default_rng(smax).uniform(-3000.0, 3000.0, len(vis))
+    kw = dict(num_wplanes=4, max_wpconv_support=smax, kernel_trunc_perc=1.0, w=w, cell_size=cell, analytic_gcf=False)
+    r = orc.convolve_to_grid(capi.GaussianSinc, 3, N, uv, vis, wts, False, 4, True, True, True,
+                             wproj=orc.WProj(4, smax, 1, 1.0), w=w, cell_size=cell, analytic_gcf=False)
+    g = ctx.convolve_to_grid(capi.GaussianSinc, 3.0, 3, N, uv, vis, wts, kernel_exact=False, oversampling=4, **kw)
+    assert np.abs(g[0] - r.vis_grid).max() <= 1e-11 * np.abs(r.vis_grid).max()
+    assert np.abs(g[1] - r.sampling_grid).max() <= 1e-11 * np.abs(r.sampling_grid).max()
+
+
 @pytest.mark.parametrize("exact", [True, False])
 def test_entries_that_are_not_finite_stay_in_their_footprint(ctx, exact):
     N, S = 64, 3
