@@ -276,7 +276,7 @@ def run_gpu(args):
     # algorithmic bytes per launch of each phase
     alg = {
         # grid loop: one 28-byte item record per gridded visibility read once, the half-plane grid written
-        # once (FP32 complex); the tile lists' replication is overhead, not algorithmic traffic
+        # once (FP32 complex); the binning's records are overhead, not algorithmic traffic
         "grid_loop": int(info32.n_good_vis) * 28 + rows * N * 8,
         # c2r FFT: read the half-plane grid, write the N x N image (FP32)
         "fft_c2r": rows * N * 8 + N * N * 4,
@@ -285,7 +285,7 @@ def run_gpu(args):
         # prepass + W-planes + binning: read vis/uvw/weights, write items, lists
         "grid_init": n * (16 + 24 + 8) + n * 28 + items * 4 * 2,
     }
-    # the dominant kernel: the tile gridder is the single most expensive launch of a step (the
+    # the dominant kernel: the block gridder is the single most expensive launch of a step (the
     # grid-init phase is ~20 short kernels, none above ~45 us)
     dom = names.index("grid_loop")
     dom_name = names[dom]
@@ -297,7 +297,7 @@ def run_gpu(args):
             traffic = json.load(open(tfile)).get(dom_name)
         except Exception:
             traffic = None
-    roofline = {"bound": "hbm", "kernel": "tile gridder, autotuned form (grid_loop phase)", "achieved": round(achieved, 1),
+    roofline = {"bound": "hbm", "kernel": "block gridder (grid_loop phase)", "achieved": round(achieved, 1),
                 "peak": hbm, "unit": "GB/s",
                 "frac": round(achieved / hbm, 4), "peak_source": peak_kind, "traffic": traffic,
                 "phase_ms": {k: round(float(v), 4) for k, v in zip(names, mean_ph)},
@@ -317,7 +317,7 @@ def run_gpu(args):
     line = {
         "metric": METRIC, "value": round(value, 2), "unit": "Mvis/s", "n_gpus": ws, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": round(tot32 / args.steps, 4), "higher_is_better": True,
-        "scaling": "weak", "vs_baseline": None, "dtype": "f32 (two-sum compensated), FP64 W-kernels/uvw/normalise",
+        "scaling": "weak", "vs_baseline": None, "dtype": "f32 with double cell sums, FP64 W-kernels/uvw/normalise",
         "data": "synthetic (seeded point sources + noise, config-2 shapes)",
         "config": {"workload": WORKLOAD, "n_vis": n, "image_size": N, "precision": "fp32c",
                    "l2": "flushed (256 MB write) before each timed step", "inputs": "resident in HBM",
@@ -395,7 +395,7 @@ def run_large_support(ctx, peaks, steps=3):
     res = {}
     for prec, name in ((capi.FP32C, "fp32c"), (capi.FP64, "fp64")):
         odt = capi.F64 if prec == capi.FP64 else capi.F32
-        # an untimed call first: the autotuner picks this size class's gridder layout
+        # an untimed call first: buffers and tables
         ctx.image_visibilities(dv, dw, duvw, N, s.cell_size, precision=prec, out_dtype=odt, device_ptrs=True,
                                image_out=outs[prec], **kw)
         ctx.set_timing(True)
@@ -417,7 +417,7 @@ def run_large_support(ctx, peaks, steps=3):
         res[name] = {"Mvis_per_s": round(n / (float(np.median(total)) * 1e-3) / 1e6, 2),
                      "ms": round(float(np.median(total)), 3), "grid_loop_ms": round(g, 3),
                      "max_plane_support": int(infos[-1].max_plane_support), "taps": taps,
-                     "roofline": {"bound": "fp", "kernel": "tile gridder (grid_loop phase)",
+                     "roofline": {"bound": "fp", "kernel": "block gridder (grid_loop phase)",
                                   "achieved": round(achieved, 2), "peak": peak, "unit": "TFLOP/s",
                                   "frac": round(achieved / peak, 4), "peak_source": "measured (FMA probe)"}}
     d = outs[capi.FP32C].double() - outs[capi.FP64]
@@ -515,7 +515,7 @@ def run_serving(rates=(10.0, 20.0, 50.0, 100.0, 200.0, 500.0), seconds=2.0, slot
     for rate in rates:
         srv = capi.Server(slots=slots, hbm_budget_bytes=64 << 30, precision=capi.FP32C)
         try:
-            # warm-up: every template once on every slot (buffers, cuFFT plans, gridder tuning), so that
+            # warm-up: every template once on every slot (buffers, cuFFT plans), so that
             # the timed arrivals allocate nothing
             for (v, w, uvw), kw, _ in pool:
                 srv.prepare(v, w, uvw, find_sources=True, want_image=False, **kw)

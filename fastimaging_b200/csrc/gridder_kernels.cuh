@@ -749,10 +749,10 @@ struct WprojCore {
     // Small footprints in two parts, columns 0 to 3 and 4 to 7, each half of the
     // warp with an entry of its own: an entry of 5 x 5 cells reaches 11 of a
     // block's 64 on average, and two of three entries only one part.  Kernel on
-    // the 1M-visibility 4096^2 call, one part and two: 196 and 178 us (largest
-    // support 16, truncated to 2 to 3 mostly), untruncated support 3 216 and 196
-    // (double 214 and 205), 6 401 and 371 (397 and 387), 8 538 and 512 (528 and
-    // 537); 12 909 and 879 to 968.
+    // the 1M-visibility 4096^2 call, one part and two: 196 and 179 us (truncated
+    // to support 3 at most); untruncated support 3 216 and 196 (double 214 and
+    // 205), 6 401 and 371 (397 and 387), 8 538 and 512 (528 and 537), 12 909 and
+    // 879 to 968.
     static constexpr int kParts = 2;
     static __device__ __forceinline__ bool parts(const Params& p)
     {

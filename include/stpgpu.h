@@ -50,8 +50,8 @@ typedef enum { STPGPU_ZEROMEDIAN = 0, STPGPU_BINMEDIAN, STPGPU_BINAPPROX, STPGPU
 
 /* Arithmetic of the imager.  FP64 is the plain form matched to the
  * reference's double build; FP32 uses single-precision visibilities, kernel
- * weights, grid and FFT; FP32C adds two-sum compensated accumulation of the
- * grid cells, and stores the grid in double with a double-precision c2r
+ * weights, grid and FFT; FP32C sums the grid cells in double, and stores the
+ * grid in double with a double-precision c2r
  * when the grid correction amplifies the FFT's rounding by more than 4096
  * (1/gcf_min^2 over the output field; e.g. PSWF kernels).  uvw -> pixel
  * scaling, W-kernel generation and the final normalisation stay FP64 in all
@@ -128,7 +128,8 @@ typedef struct {
     /* With stpgpu_set_timing(ctx, 1): device time of the phases the
      * reference reports (reduce/common_functions.cpp:164-228), ms:
      * [0] grid init (prepass, W-planes and W-kernels, binning),
-     * [1] grid loop (the tile gridder kernel), [2] FFT, [3] normalise. */
+     * [1] grid loop (the block gridder kernel), [2] FFT (power-of-two grids:
+     * its passes along the columns), [3] normalise (with the rest of it). */
     double phase_ms[4];
     int32_t n_launches; /* kernels of this library the call ran, graph replays included (cuFFT's excluded) */
     /* bit 0: the compensated-FP32 call kept its grid in double and ran the
@@ -281,19 +282,14 @@ typedef struct {
 typedef struct {
     double device_ms;        /* device time of the whole batch (CUDA events) */
     int32_t graph;           /* 1: ran as a replay of a captured CUDA graph */
-    int32_t gridder_launches; /* persistent gridder launches (one per kernel variant) */
-    int32_t tuned_classes;   /* size classes the tile autotuner measured in this call */
+    int32_t gridder_launches; /* gridder launches (one per snapshot) */
+    int32_t tuned_classes;   /* always 0: the gridder has no autotuner any more */
     int32_t n_launches;      /* kernels of this library the call ran, graph replays included (cuFFT's excluded) */
 } stpgpu_batch_info;
 
-/* Many snapshots of uneven sizes in one call: per-snapshot preparation on
- * parallel streams, ONE persistent gridder launch per kernel variant over a
- * (snapshot, tile) work queue, then the c2r transforms and normalisation of
- * every snapshot.  Results equal stpgpu_image_visibilities_ex on each
- * snapshot alone.  The tile width (32 or 16 grid columns) of each size class
- * (padded size, kernel mode, precision, support) is chosen by an autotuner
- * that times both shapes on the first batch containing that class.  With
- * device pointers, the second and later calls with the same snapshots
+/* Many snapshots of uneven sizes in one call: the snapshots are imaged on
+ * parallel streams, each its whole pipeline.  Results equal
+ * stpgpu_image_visibilities_ex on each snapshot alone.  With device pointers, the second and later calls with the same snapshots
  * (sizes, parameters and pointers) replay a CUDA graph captured from the
  * previous one.  infos: nullable, n_snapshots entries. No counterpart in the
  * reference (it images one snapshot per call, imager.h:233-376). */
@@ -366,9 +362,9 @@ STPGPU_API stpgpu_status stpgpu_server_destroy(stpgpu_server* server);
 STPGPU_API stpgpu_status stpgpu_server_submit(stpgpu_server* server, const stpgpu_request* request, int64_t* ticket);
 /* Run a request once on every slot, in the calling thread, while admission
  * is held (queued requests wait; the requests in flight finish first).  Each
- * slot then holds the buffers, cuFFT plans and tuned gridder layout of the
- * request's size class, so requests of that class admitted later pay no
- * allocation, plan creation or tuning (which can stall every slot on the
+ * slot then holds the buffers and cuFFT plans of the request's size class, so
+ * requests of that class admitted later pay no allocation or plan creation
+ * (which can stall every slot on the
  * device for up to a second).  Outputs go to the request's buffers; *result
  * (nullable) holds the last slot's outcome.  Not counted in the statistics. */
 STPGPU_API stpgpu_status stpgpu_server_prepare(stpgpu_server* server, const stpgpu_request* request,
