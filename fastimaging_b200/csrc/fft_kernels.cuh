@@ -197,10 +197,13 @@ __global__ void __launch_bounds__(axis_threads(L), sizeof(T) == 8 ? 512 / axis_t
     // column of point m: FIRST other * m + grp, else L * grp + m
     const size_t step = FIRST ? size_t(other) * size_t(ld) : size_t(ld);
     C* base = g + (FIRST ? size_t(grp) : size_t(L) * size_t(grp)) * size_t(ld) + size_t(live ? row : 0);
-    C v[16];
+    // (lanes beyond the last row read nothing: other blocks write the cells of every row there is)
+    C v[16] = {};
+    if (live) {
 #pragma unroll
-    for (int q = 0; q < 16; q++)
-        v[q] = base[size_t(t + q * TL) * step];
+        for (int q = 0; q < 16; q++)
+            v[q] = base[size_t(t + q * TL) * step];
+    }
     fft_points<16>(v);
     if constexpr (TL > 1) {
 #pragma unroll
