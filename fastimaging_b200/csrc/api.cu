@@ -2222,8 +2222,9 @@ void run_source_find(stpgpu_context* c, const T* d_img, int rows, int cols, cons
         bigl = c->buf<uint32_t>("fg_big", lcap);
         listed = c->buf<uint32_t>("fg_listed", lcap);
     };
-    auto moments_and_islands = [&](const FgSizes& z) {
-        k_label_sums<T><<<G, 32 * kSumWarps, 0, st>>>(z, d_img, rows, cols, v1, sb, se, sp, listed, &sfs->seg[1], mom, ns);
+    auto moments_and_islands = [&](const FgSizes& z, uint32_t longest) {
+        k_label_sums<T><<<G, 32 * kSumWarps, 0, st>>>(z, d_img, rows, cols, v1, sb, se, sp, listed, &sfs->seg[1], longest,
+            mom, ns);
         STPGPU_CHECK_LAUNCH();
         k_islands<packed><<<G, 256, 0, st>>>(z, &sfs->st, ext, eidx, ns, mom, p.source_min_area, nvalid, nisl, raw);
         STPGPU_CHECK_LAUNCH();
@@ -2254,7 +2255,7 @@ void run_source_find(stpgpu_context* c, const T* d_img, int rows, int cols, cons
         k_seg_sort_big<<<64, 1024, SEG_BIG * sizeof(uint32_t), st>>>(sb, se, slots, fm, split_m, v1, sp, bigl,
             &sfs->seg[2], sort_overflow);
         STPGPU_CHECK_LAUNCH();
-        moments_and_islands(z);
+        moments_and_islands(z, SEG_BIG);
     };
     // everything, then one read-back: state (statistics, counts, flags) and
     // the first island records
@@ -2400,7 +2401,7 @@ void run_source_find(stpgpu_context* c, const T* d_img, int rows, int cols, cons
         k_seg_mark<<<grid1d(nv, 256), 256, 0, st>>>(vk2, nv, fm, split_m, v1, sb, se, sp);
         STPGPU_CHECK_LAUNCH();
         STPGPU_CUDA_TRY(cudaMemsetAsync(cb.misc + 4, 0, 2 * sizeof(uint32_t), st));
-        moments_and_islands(FgSizes { cb.misc, lcap, fcap });
+        moments_and_islands(FgSizes { cb.misc, lcap, fcap }, ~0u);
         read_back_state();
     }
     const SfState h = *hstate;

@@ -1555,17 +1555,21 @@ __device__ __forceinline__ uint32_t seg_at(uint32_t b, uint32_t sp, uint32_t e, 
 // pixel order.  Only the additions are a chain: with one thread per label the
 // loads were one too, and a bright source of 600 pixels kept the whole grid
 // waiting (60 us of the call on a 4096^2 image, now 25).
+// Ranges of more than `longest` entries have no order yet (those that
+// k_seg_sort_big left to the host, which sums again behind its sort): nothing
+// is read through them, and their sums stay zero.
 constexpr int kSumWarps = 4;
 template <typename T>
 __global__ void __launch_bounds__(32 * kSumWarps) k_label_sums(FgSizes z, const T* img, int rows, int cols,
     const uint32_t* vals, const uint32_t* seg_begin, const uint32_t* seg_end, const uint32_t* seg_split,
-    const uint32_t* listed, const uint32_t* nlisted, double* mom, int* ns)
+    const uint32_t* listed, const uint32_t* nlisted, uint32_t longest, double* mom, int* ns)
 {
     __shared__ double terms[kSumWarps][6][33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     FG_LOOP(l, z.nl())
     {
-        if (seg_begin[l] == seg_end[l]) {
+        const uint32_t len = seg_end[l] - seg_begin[l];
+        if (len == 0 || len > longest) {
             for (int q = 0; q < 6; q++)
                 mom[6 * size_t(l) + q] = 0.0;
             ns[l] = 0;
@@ -1576,6 +1580,8 @@ __global__ void __launch_bounds__(32 * kSumWarps) k_label_sums(FgSizes z, const 
     for (uint32_t q = blockIdx.x * kSumWarps + warp, nq = *nlisted; q < nq; q += gridDim.x * kSumWarps) {
         const uint32_t l = listed[q];
         const uint32_t b = seg_begin[l], e = seg_end[l], sp = seg_split[l], len = e - b;
+        if (len > longest)
+            continue;
         double sum = 0.0;
         // the pixel of the next 32 and the index of the 32 after are in flight
         auto index = [&](uint32_t j) { return j < len ? vals[seg_at(b, sp, e, j)] : 0u; };

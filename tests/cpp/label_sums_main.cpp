@@ -1,0 +1,73 @@
+// k_label_sums on the CPU while a label has more pixels than the one-block
+// sort takes: their order is not formed yet (the host sorts all of them and
+// sums again), so nothing may be read through it.
+#include <algorithm>
+#include <atomic>
+
+static int g_pixels = 0;
+static std::atomic<int> g_outside { 0 };
+
+template <typename T>
+double ld(const T* p, int64_t i)
+{
+    if (i < 0 || i >= g_pixels) {
+        g_outside++;
+        return 0.0;
+    }
+    return double(p[i]);
+}
+
+#include "label_sums.cuh"
+
+int main()
+{
+    const int rows = 256, cols = 256;
+    g_pixels = rows * cols;
+    std::vector<float> img(g_pixels);
+    for (int i = 0; i < g_pixels; i++)
+        img[i] = float(i % 97) - 20.0f;
+    const uint32_t small = 100, large = SEG_BIG + 5;
+    const uint32_t misc[3] = { 2, 0, small + large };
+    const FgSizes z { misc, 2, small + large };
+    // ranges from k_seg_alloc (the split of a range that is not sorted is still zero), pixels from k_seg_sort
+    const std::vector<uint32_t> begin = { 0, small }, end = { small, small + large }, listed = { 1, 0 };
+    std::vector<uint32_t> split = { small, 0 }, pixels(small + large, 0xfffffff0u);
+    const uint32_t nlisted = 2;
+    for (uint32_t i = 0; i < small; i++)
+        pixels[i] = 3 * i; // all in the left half of the image
+    std::vector<double> mom(12);
+    std::vector<int> ns(2);
+    auto run = [&](uint32_t longest) {
+        std::fill(mom.begin(), mom.end(), -1.0);
+        launch(Dim3 { 2, 1, 1 }, 32 * kSumWarps, [&] {
+            k_label_sums<float>(z, img.data(), rows, cols, pixels.data(), begin.data(), end.data(), split.data(),
+                listed.data(), &nlisted, longest, mom.data(), ns.data());
+        });
+    };
+    int bad = 0;
+    auto check = [&](int l) {
+        double v = 0.0, x = 0.0;
+        for (uint32_t i = begin[l]; i < end[l]; i++) {
+            const uint32_t m = pixels[i], c = m / rows;
+            v += img[m];
+            x += double(c < 128 ? c + 128 : c - 128) * img[m];
+        }
+        if (std::abs(mom[6 * l] - x) > 1e-9 * std::abs(x) || std::abs(mom[6 * l + 5] - v) > 1e-9 * std::abs(v)
+            || ns[l] != int(end[l] - begin[l])) {
+            std::printf("label %d: sums %g %g, should be %g %g\n", l, mom[6 * l], mom[6 * l + 5], x, v);
+            bad++;
+        }
+    };
+    run(SEG_BIG);
+    check(0);
+    std::printf("pixels read outside the image: %d\n", int(g_outside));
+    bad += g_outside;
+    for (uint32_t i = 0; i < large; i++) // sorted by the host
+        pixels[small + i] = 400 + i;
+    split[1] = small + large;
+    run(~0u);
+    check(0);
+    check(1);
+    bad += g_outside;
+    return bad ? 1 : 0;
+}

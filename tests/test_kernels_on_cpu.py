@@ -34,3 +34,15 @@ inline void pack_scalars(const PackArgs&) {}
 }
 """
     _run(tmp_path, "fft_axis_main.cpp", {"imager_kernels.cuh": stub, "fft_kernels.cuh": _source("fft_kernels.cuh")})
+
+
+def test_label_sums_wait_for_the_order_of_a_large_label(tmp_path):
+    src = _source("sourcefind_kernels.cuh")
+
+    def cut(begin, end):
+        i = src.index(begin)
+        return src[i:src.index(end, i) + len(end)]
+
+    text = (cut("struct FgSizes {", "};\n") + cut("#define FG_LOOP", "blockDim.x)\n") + cut("constexpr int SEG_BIG", "\n")
+            + cut("__device__ __forceinline__ uint32_t seg_at", "\n}\n") + cut("constexpr int kSumWarps", "\n}\n"))
+    _run(tmp_path, "label_sums_main.cpp", {"label_sums.cuh": text})
