@@ -463,6 +463,58 @@ struct ImagerSetup {
 // captured into CUDA graphs.
 bool large_support(const ImagerSetup& s) { return s.nplanes > 0 && s.max_support > 32; }
 
+// Sizes of the W-kernel generation (WideFieldImaging, aw_projection.cpp:19-111).
+struct WkShape {
+    int64_t workarea = 2, arr = 0;
+    int half = 0, lh = 0;
+    int ctas = 1;                              // CTAs that share a plane in k_wkernel_plane
+    int smem_ctab = 0, smem_Q = 0, smem_T = 0; // what its shared memory holds
+    size_t smem = 0;
+    size_t q_cells = 0, t_cells = 0; // scratch for what it does not hold
+
+    bool too_large() const { return arr > 46340; } // arr^2 > 2^31: not generated
+};
+
+WkShape wk_shape(const ImagerSetup& s, int os)
+{
+    WkShape k;
+    const int K = 2 * s.max_support + 1;
+    const int u = s.undersampling > 0 ? int(std::pow(2, s.undersampling - 1)) : 0;
+    if (u > 0) {
+        while (k.workarea / u < K)
+            k.workarea *= 2;
+    } else {
+        while (k.workarea < s.N)
+            k.workarea *= 2;
+    }
+    k.arr = k.workarea * os;
+    if (k.too_large())
+        return k;
+    k.half = int(k.workarea / 2);
+    k.lh = int(std::min<int64_t>(int64_t(s.max_support) * os + os / 2 + 1, k.arr / 2 + 1));
+    // by the kernel's rows at the largest support (a second CTA costs little
+    // where the truncated kernel turns out small), as far as the planes leave SMs
+    k.ctas = std::max(1, std::min({ 4, k.lh / 16, 148 / std::max(s.nplanes, 1) }));
+    // shared memory: the cosine table, Q and T in this order of preference (a
+    // kernel of 16 cells' support and oversampling 8 on four CTAs takes 4 + 16
+    // + 17 KB)
+    auto fits = [&](size_t bytes) {
+        if (k.smem + bytes > 160 * 1024)
+            return 0;
+        k.smem += bytes;
+        return 1;
+    };
+    const size_t t_rows = size_t(ceil_div(k.lh, k.ctas));
+    k.smem_ctab = fits(pad16(sizeof(double) * size_t(k.arr)));
+    k.smem_Q = fits(sizeof(double2) * size_t(k.half) * k.half);
+    k.smem_T = fits(sizeof(double2) * t_rows * k.half);
+    if (!s.hankel && s.ntimesteps == 0) {
+        k.q_cells = k.smem_Q ? 0 : size_t(s.nplanes) * k.half * k.half;
+        k.t_cells = k.smem_T ? 0 : size_t(s.nplanes) * k.ctas * t_rows * k.half;
+    }
+    return k;
+}
+
 void check_pars(const ImagerSetup& s)
 {
     if (s.N <= 0 || (s.N % 2) != 0)
@@ -871,25 +923,15 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
         double* w_avg = c->buf<double>("wavg", P); // the plane means, from either path above
         // W-kernels in FP64 (WideFieldImaging, aw_projection.cpp:19-111,173-210,366-452)
         const int K = 2 * s.max_support + 1;
-        const int u = s.undersampling > 0 ? int(std::pow(2, s.undersampling - 1)) : 0;
-        int workarea = 2;
-        if (u > 0) {
-            while ((workarea / u) < K)
-                workarea *= 2;
-        } else {
-            while (workarea < N)
-                workarea *= 2;
-        }
-        if (workarea < K)
+        const WkShape ks = wk_shape(s, os);
+        if (ks.workarea < K)
             fail(STPGPU_ERR_INVALID_ARG, "W-kernel workarea smaller than the kernel size");
-        const double scaling = double(N) / double(workarea);
-        const int arr = workarea * os;
-        if (arr % 2)
+        if (ks.arr % 2)
             fail(STPGPU_ERR_INVALID_ARG, "array_size must be multiple of 2 for WideFieldImaging generation.");
-        if (int64_t(arr) * arr > (int64_t(1) << 31))
+        if (ks.too_large())
             fail(STPGPU_ERR_UNSUPPORTED, "W-kernel array too large");
-        const int half = workarea / 2;
-        const int Lh = std::min(s.max_support * os + os / 2 + 1, arr / 2 + 1);
+        const int workarea = int(ks.workarea), arr = int(ks.arr), half = ks.half, Lh = ks.lh;
+        const double scaling = double(N) / double(workarea);
         double* aa = c->buf<double>("aa", workarea);
         if (!c->memo("aa", std::to_string(s.kf) + "/" + fkey(s.trunc) + "/" + std::to_string(workarea) + "/"
                                + std::to_string(s.analytic))) {
@@ -922,14 +964,11 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
         // WideFieldImaging gets real_t(arc_sec_to_rad(cell)), scaled by N/workarea
         wq.scaled_cell = arc_sec_to_rad(s.cell_size) * scaling;
         wq.trunc_perc = s.trunc_perc;
-        // CTAs that share a plane: by the kernel's rows at the largest support
-        // (a second costs little where the truncated kernel turns out small),
-        // as far as the planes leave SMs
-        const int wk_ctas = std::max(1, std::min({ 4, Lh / 16, 148 / std::max(P, 1) }));
-        if (!s.hankel) {
-            wq.Qs = c->buf<double2>("wkQ", size_t(P) * wk_ctas * half * half);
-            wq.Ts = c->buf<double2>("wkT", size_t(P) * (Lh + wk_ctas) * half);
-        }
+        wq.smem_ctab = ks.smem_ctab;
+        wq.smem_Q = ks.smem_Q;
+        wq.smem_T = ks.smem_T;
+        wq.Qs = ks.q_cells ? c->buf<double2>("wkQ", ks.q_cells) : nullptr;
+        wq.Ts = ks.t_cells ? c->buf<double2>("wkT", ks.t_cells) : nullptr;
         wq.convd = c->buf<double2>("wkconv", size_t(P) * Lh * Lh);
         const int T = std::max(s.ntimesteps, 1);
         const int PT = P * T;
@@ -1007,21 +1046,12 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
             hq.Cp = c->buf<double>("hkC", size_t(P) * 2 * hq.n);
             k_hankel_plane<<<P, 1024, 0, st>>>(wq, hq);
         } else {
-            // shared memory: the cosine table, Q and T in this order of
-            // preference (a kernel of 16 cells' support and oversampling 8
-            // on four CTAs takes 4 + 16 + 17 KB)
-            size_t smem = 0;
-            auto fits = [&](size_t bytes) {
-                if (smem + bytes > 160 * 1024)
-                    return 0;
-                smem += bytes;
-                return 1;
-            };
-            wq.smem_ctab = fits(pad16(sizeof(double) * size_t(arr)));
-            wq.smem_Q = fits(sizeof(double2) * size_t(half) * half);
-            wq.smem_T = fits(sizeof(double2) * size_t(ceil_div(Lh, wk_ctas)) * half);
+            if (ks.q_cells) {
+                k_wk_quadrant<<<dim3(grid1d(int64_t(half) * half, 256), P), 256, 0, st>>>(wq);
+                STPGPU_CHECK_LAUNCH();
+            }
             STPGPU_CUDA_TRY(cudaFuncSetAttribute(k_wkernel_plane, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-            k_wkernel_plane<<<dim3(P, wk_ctas), 1024, smem, st>>>(wq);
+            k_wkernel_plane<<<dim3(P, ks.ctas), 1024, ks.smem, st>>>(wq);
         }
         STPGPU_CHECK_LAUNCH();
         // per-offset K x K tables in the gridder's precision: worst-case
@@ -2879,9 +2909,12 @@ int64_t request_bytes(const ImagerSetup& s, int image_size, int64_t n, int vis_c
     if (s.nplanes > 0) {
         b += n * (rb == 8 ? 48 : 32); // items in |w| order
         const int64_t os = std::max(1, (s.os >> 1) << 1), cs = (os / 2) * 2 + 1, K = 2 * conv + 1;
-        const int64_t lh = conv * os + os / 2 + 1;
-        b += n * 41;                                                  // |w| sort, planes
-        b += int64_t(s.nplanes) * (cs * cs * K * K * 2 * rb + lh * lh * 16 + 64 * 64 * 16);
+        const WkShape ks = wk_shape(s, int(os));
+        b += n * 55; // |w| sort (CUB's own buffers with it), planes
+        b += int64_t(s.nplanes) * (cs * cs * K * K * 2 * rb + int64_t(ks.lh) * ks.lh * 16);
+        b += int64_t(ks.q_cells + ks.t_cells) * 16 + (ks.workarea + ks.arr) * 8;
+        if (s.hankel && !ks.too_large())
+            b += int64_t(s.nplanes) * (ks.half * 16 + ks.arr * 48); // radial profiles, transforms, spline
     }
     b += rows * N * 2 * rb + N * N * rb + int64_t(image_size) * image_size * rb;
     if (precision == STPGPU_FP32C && wide_fft_needed(s, image_size, correction))

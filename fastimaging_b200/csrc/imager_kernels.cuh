@@ -1199,8 +1199,8 @@ struct WkParams {
     int half, arr, os, cs, max_support, lh_max;
     int smem_ctab, smem_Q, smem_T; // k_wkernel_plane: what the launch's dynamic shared memory holds
     double scaled_cell, trunc_perc;
-    double2* Qs;   // scratch [P][half][half]
-    double2* Ts;   // scratch [P][lh_max][half]
+    double2* Qs;   // [P][half][half] from k_wk_quadrant, without smem_Q
+    double2* Ts;   // scratch [P][CTAs of a plane][rows of T of a CTA][half], without smem_T
     double2* convd; // [P][lh_max][lh_max] FP64
     int* support;
 };
@@ -1238,14 +1238,37 @@ __device__ __forceinline__ double2 cos_sum(const double2* V, int stride, int hal
     return make_double2(re, im);
 }
 
+// Value (a, b) of the image-domain quadrant, t = a + b half.
+__device__ __forceinline__ double2 wk_quadrant(const WkParams& q, double w, int t)
+{
+    const int a = t % q.half, b = t / q.half;
+    if (a == 0 && b == 0)
+        return make_double2(q.aa[q.half] * q.aa[q.half], 0.0);
+    if (b == 0)
+        return wk_value(q, w, a, 0);
+    if (a == 0)
+        return wk_value(q, w, b, 0); // output(0, i) reuses value(i, 0)
+    return wk_value(q, w, a, b);
+}
+
+// The quadrants that shared memory does not hold, one for all the CTAs of a
+// plane (blockIdx.y): a copy for each would take four times the memory, 8.6 GB
+// instead of 2.1 for 32 planes on a workarea of 4096.
+__global__ void __launch_bounds__(256) k_wk_quadrant(WkParams q)
+{
+    const int t = int(blockIdx.x) * 256 + int(threadIdx.x);
+    if (t < q.half * q.half)
+        q.Qs[size_t(blockIdx.y) * q.half * q.half + t] = wk_quadrant(q, q.w_avg[blockIdx.y], t);
+}
+
 // A plane's steps are a chain of short sums, so latency bounds them: the
 // cosine table, the image-domain quadrant Q and its row transforms T are kept
 // in shared memory where they fit (q.smem_*; the launch gives the room), the
 // position in the cosine table is carried instead of reduced modulo arr at
 // every term, and the truncation test runs in all threads.  gridDim.y CTAs
-// share a plane: each forms Q and the truncation, then the rows l = blockIdx.y,
-// + gridDim.y, ... of T and of the kernel (at support 16 the kernel's 133^2
-// sums are most of the work: 193 us with one CTA a plane).
+// share a plane: each forms Q (in shared memory) and the truncation, then the
+// rows l = blockIdx.y, + gridDim.y, ... of T and of the kernel (at support 16
+// the kernel's 133^2 sums are most of the work: 193 us with one CTA a plane).
 __global__ void __launch_bounds__(1024) k_wkernel_plane(WkParams q)
 {
     const int p = blockIdx.x;
@@ -1258,7 +1281,7 @@ __global__ void __launch_bounds__(1024) k_wkernel_plane(WkParams q)
     const int lrows = (lh + int(gridDim.y) - 1) / int(gridDim.y); // rows of T of this CTA, at most
     const size_t cta = size_t(p) * gridDim.y + blockIdx.y;
     double2* sm = reinterpret_cast<double2*>(sct);
-    double2* Q = q.Qs + cta * half * half;
+    double2* Q = q.Qs + size_t(p) * half * half;
     double2* T = q.Ts + cta * lrows * half;
     if (q.smem_Q) {
         Q = sm;
@@ -1277,19 +1300,9 @@ __global__ void __launch_bounds__(1024) k_wkernel_plane(WkParams q)
         ct = sc;
     }
     // 1. image-domain quadrant Q[a][b] (row a, column b)
-    for (int t = threadIdx.x; t < half * half; t += blockDim.x) {
-        const int a = t % half, b = t / half;
-        double2 v;
-        if (a == 0 && b == 0)
-            v = make_double2(q.aa[half] * q.aa[half], 0.0);
-        else if (b == 0)
-            v = wk_value(q, w, a, 0);
-        else if (a == 0)
-            v = wk_value(q, w, b, 0); // output(0, i) reuses value(i, 0)
-        else
-            v = wk_value(q, w, a, b);
-        Q[size_t(b) * half + a] = v;
-    }
+    if (q.smem_Q)
+        for (int t = threadIdx.x; t < half * half; t += blockDim.x)
+            Q[t] = wk_quadrant(q, w, t);
     if (threadIdx.x == 0)
         s_support = 0;
     __syncthreads();

@@ -128,6 +128,25 @@ def test_w_kernels_match_oracle(ctx, N, P, smax, trunc, precision):
     assert np.abs(img - ref).max() <= 5e-6 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("smax,under,os,P", [(12, 0, 4, 3), (8, 0, 8, 40), (70, 1, 8, 2), (70, 1, 4, 2), (5, 3, 8, 2)])
+def test_w_kernel_generation_beyond_shared_memory(ctx, smax, under, os, P):
+    """Workareas whose quadrant (16 half^2 bytes), and with support 70 and oversampling 8 its row transforms too, do
+    not fit into shared memory, with one and with several CTAs a plane."""
+    N, cell = 256, 20.0
+    uv, vis, wts = _points(smax + os, 300, N, 0.7)
+    uv[:, :] *= 0.6 if smax > 40 else 1.0
+    w = np.random.default_rng(smax).uniform(-2000.0, 2000.0, len(vis))
+    r = orc.convolve_to_grid(capi.GaussianSinc, 3, N, uv, vis, wts, False, os, True, True, True,
+                             wproj=orc.WProj(P, smax, under, 0.0), w=w, cell_size=cell, analytic_gcf=False)
+    g = ctx.convolve_to_grid(capi.GaussianSinc, 3.0, 3, N, uv, vis, wts, kernel_exact=False, oversampling=os,
+                             num_wplanes=P, max_wpconv_support=smax, undersampling_opt=under, w=w, cell_size=cell,
+                             analytic_gcf=False)
+    assert np.abs(r.vis_grid).max() > 0
+    # double-precision cosine sums over up to 128^2 values in place of an FFT
+    assert np.abs(g[0] - r.vis_grid).max() <= 1e-11 * np.abs(r.vis_grid).max()
+    assert np.abs(g[1] - r.sampling_grid).max() <= 1e-11 * np.abs(r.sampling_grid).max()
+
+
 def test_w_kernel_entries_that_are_not_finite_stay_in_their_footprint(ctx):
     N, smax = 64, 4
     uv, vis, wts = _points(5, 200, N, 0.8)

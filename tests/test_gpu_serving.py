@@ -107,6 +107,36 @@ def test_fp32c_requests_same_alone_and_in_the_mix():
         assert peak_rel(img.astype(np.float64), rimg.astype(np.float64)) < 1e-6
 
 
+@pytest.mark.parametrize("kw", [dict(undersampling_opt=0, num_wplanes=16, max_wpconv_support=16, image_size=1000),
+                                dict(undersampling_opt=1, num_wplanes=8, max_wpconv_support=70, oversampling=8),
+                                dict(undersampling_opt=1, num_wplanes=32, max_wpconv_support=8, kernel_trunc_perc=1.0),
+                                dict(), dict(kernel_exact=True, kernel_support=8)])
+def test_admission_estimate_covers_the_request(kw):
+    """What a request takes on the device is within its admission estimate and the eighth that buffers are allocated
+    beyond their size (and 48 MB for the runtime's own: kernels, events, the page-locked stage)."""
+    import torch
+
+    rng = np.random.default_rng(5)
+    n, N, cell = 200000, 1024, 4.0
+    half = 0.4 / np.deg2rad(cell / 3600.0)
+    uvw = np.column_stack([rng.uniform(-half, half, (n, 2)), rng.uniform(-300.0, 300.0, n)])
+    vis, wts = rng.normal(size=n) + 0j, np.ones(n)
+    args = dict(image_size=N, cell_size=cell, kernel_func=capi.GaussianSinc, kernel_support=3, kernel_exact=False,
+                oversampling=8, analytic_gcf=False)
+    args.update(kw)
+    srv = capi.Server(slots=1, precision=capi.FP64)
+    try:
+        srv.prepare(vis[:10], wts[:10], uvw[:10], out_dtype=capi.F64, want_image=False, image_size=250, cell_size=cell)
+        free = torch.cuda.mem_get_info()[0]
+        res = srv.wait(srv.submit(vis, wts, uvw, out_dtype=capi.F64, want_image=False, **args))[3]
+        assert res.status == 0
+        est = res.est_bytes
+        used = free - torch.cuda.mem_get_info()[0]
+    finally:
+        srv.close()
+    assert used <= est * 1.125 + (48 << 20), (used, est)
+
+
 def test_admission_keeps_in_flight_within_budget():
     reqs = _requests()
     probe = capi.Server(slots=1, precision=capi.FP32C)
