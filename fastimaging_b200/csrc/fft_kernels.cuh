@@ -12,7 +12,8 @@ namespace stpgpu {
 //   [kTwRoots, + N)        exp(2 pi i k / N)
 //   [tw_c2r(N, p), ...)    pass p of the c2r: [q][k], k < 16^p
 //   [tw_axis(N, L), ...)   second half of an axis transform of L = 32, 64, 128: [q][k], k < 16
-constexpr int kC2rMinLog = 7, kC2rMaxLog = 13; // M: grids of 256 to 16384
+constexpr int kC2rMinLog = 7, kC2rMaxLog = 13; // M: grids of 256 to 16384,
+constexpr int kC2rMaxLogF = 12;                // in single precision to 8192
 __host__ __device__ constexpr int tw_c2r(int N, int pass) { return pass == 1 ? N : (pass == 2 ? N + 256 : N + 256 + 4096); }
 __host__ __device__ constexpr int tw_axis(int N, int L)
 {
@@ -299,7 +300,7 @@ __device__ __forceinline__ void c2r_store(const C* v, C* sm, int t)
 }
 
 template <typename T, typename RO, int LOGM>
-__global__ void __launch_bounds__(c2r_threads(LOGM), sizeof(T) == 8 ? (LOGM == 13 ? 1 : 2) : (LOGM == 13 ? 1 : 3))
+__global__ void __launch_bounds__(c2r_threads(LOGM), sizeof(T) == 8 ? (LOGM == 13 ? 1 : 2) : 3)
     k_c2r_normalise(const typename Cplx<T>::T* __restrict__ F, int ld, const typename Cplx<T>::T* __restrict__ tw,
         int image_size, const double* total, const double* __restrict__ ginv, int corr, RO* __restrict__ out, PackArgs pk)
 {
