@@ -578,6 +578,8 @@ BlockBins make_bins(stpgpu_context* c, const ImagerSetup& s, const GridOut& g, i
 // Visibilities per block of cells from which several warps share a block.
 constexpr int64_t kDensePerBlock = 24;
 constexpr int kDenseSplit = 8;
+// Columns of blocks that a CTA takes on sparse grids (k_grid_blocks).
+constexpr int kSparseCols = 8;
 
 // Where a call's items and kernel tables are, for grid_blocks.
 template <typename R>
@@ -660,6 +662,15 @@ void grid_blocks(stpgpu_context* c, const ImagerSetup& s, GridOut& g, int64_t n,
     const int64_t nbr = ceil_div(b.rows, kBlk), nbc = ceil_div(b.N, kBlk);
     // visibilities per block: above kDensePerBlock several warps share a block
     const bool dense = n > kDensePerBlock * nbr * nbc;
+    const unsigned nbr8 = unsigned(ceil_div(nbr, kGridWarps));
+    // Few visibilities: several columns of blocks a CTA, as long as the CTAs
+    // still fill the GPU.  One column and eight, us: 4096^2 (2112 CTAs of eight
+    // columns) at 0.2, 0.5 and 1 visibility a block 52 and 46, 54 and 50, 57 and
+    // 52 on disk coverage, 41 and 38, 44 and 44, 48 and 54 on a normal one;
+    // 6000^2 (4418 CTAs) at 0.5, 1 and 2 112 and 89, 118 and 94, 127 and 103,
+    // or 89 and 73, 98 and 87, 115 and 125.
+    const int64_t ctas = nbr8 * (nbc / kSparseCols);
+    const bool sparse = ctas >= 148 * 4 && (ctas >= 148 * 20 ? n : 2 * n) < nbr * nbc;
     auto run = [&](auto core, const auto& p) {
         using C = decltype(core);
         c->mark(1);
@@ -667,7 +678,8 @@ void grid_blocks(stpgpu_context* c, const ImagerSetup& s, GridOut& g, int64_t n,
             k_grid_dense<C, kDenseSplit><<<dim3(unsigned(ceil_div(nbr, kGridWarps / kDenseSplit)), unsigned(nbc)),
                 32 * kGridWarps, 0, st>>>(p);
         else
-            k_grid_blocks<C><<<dim3(unsigned(ceil_div(nbr, kGridWarps)), unsigned(nbc)), 32 * kGridWarps, 0, st>>>(p);
+            sparse ? k_grid_blocks<C, kSparseCols><<<dim3(nbr8, unsigned(ceil_div(nbc, kSparseCols))), 32 * kGridWarps, 0, st>>>(p)
+                   : k_grid_blocks<C, 1><<<dim3(nbr8, unsigned(nbc)), 32 * kGridWarps, 0, st>>>(p);
         STPGPU_CHECK_LAUNCH();
         c->mark(2);
     };

@@ -68,6 +68,7 @@ __global__ void __launch_bounds__(256) k_exact_tables(int kf, double trunc, int 
 // order.
 constexpr int kGridWarps = 8;
 constexpr uint32_t kHeavy = 512;
+constexpr uint32_t kFew = 256; // entries of a column of blocks that its warps take on their own (sparse grids)
 constexpr int kCtaBins = 5; // bins per axis that reach a block, at most, for staging by CTA
 
 struct BlockRanges {
@@ -221,16 +222,16 @@ __device__ __forceinline__ void block_walk(const typename C::Params& p, const do
     }
 }
 
-using CtaOffsets = uint32_t[kCtaBins][kGridWarps + kCtaBins];
+using CtaOffsets = uint32_t[kGridWarps + kCtaBins]; // of one column of bins
 
-// A CTA's `total` entries (bins at off, nb to an axis), staged at `all`.
+// The `total` entries of the blocks in column bc (bins at off, nb to an axis), staged at `all`.
 template <class C, int PARTS>
 __device__ __forceinline__ void grid_staged(const typename C::Params& p, const double* stab, typename C::Staged* all,
-    const CtaOffsets& off, uint16_t* lists, int nb, uint32_t total)
+    const CtaOffsets* off, uint16_t* lists, int bc, int nb, uint32_t total)
 {
     using A = typename C::A;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int br0 = int(blockIdx.x) * kGridWarps, br = br0 + warp, bc = int(blockIdx.y);
+    const int br0 = int(blockIdx.x) * kGridWarps, br = br0 + warp;
     const int no = kGridWarps + nb;
     const uint32_t dummy = C::kCta + uint32_t(warp);
     BlockList<PARTS> list { lists, {} };
@@ -276,63 +277,33 @@ __device__ __forceinline__ void grid_staged(const typename C::Params& p, const d
         C::template store<PARTS>(p, br * kBlk, bc * kBlk, acc);
 }
 
+// Zeros in 8 columns of 64 cells, a column per warp.
 template <class C>
-__global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(const __grid_constant__ typename C::Params p)
+__device__ __forceinline__ void store_zeros(const typename C::Params& p, int r0, int c0)
+{
+    const int c = c0 + int(threadIdx.x >> 5);
+    if (c >= p.N)
+        return;
+#pragma unroll
+    for (int k = 0; k < kGridWarps * kBlk / 32; k++) {
+        const int r = r0 + 32 * k + int(threadIdx.x & 31);
+        if (r < p.rows)
+            C::store_zero(p, size_t(c) * size_t(p.ld) + size_t(r));
+    }
+}
+
+// The blocks of column bc taken one by one, each warp's entries 32 at a time.
+template <class C>
+__device__ __forceinline__ void grid_unstaged(const typename C::Params& p, const double* stab, unsigned char* smem,
+    uint16_t (*s_list)[C::kParts * BlockList<C::kParts>::kSize], uint32_t& s_heavy, int bc, int nb, int skip)
 {
     using A = typename C::A;
     using Staged = typename C::Staged;
-    // entries of the CTA and a dummy per warp; or 32 and a dummy per warp; or
-    // the partial cells of a block taken by all warps
-    constexpr size_t kStage = sizeof(Staged) * (C::kCta + kGridWarps);
-    constexpr size_t kRed = sizeof(A) * C::NACC * 32 * kGridWarps;
-    static_assert(C::kCta + kGridWarps >= 33 * kGridWarps, "staging by warp");
-    __shared__ __align__(16) unsigned char smem[kStage > kRed ? kStage : kRed];
-    __shared__ uint16_t s_list[kGridWarps][C::kParts * BlockList<C::kParts>::kSize];
-    __shared__ CtaOffsets s_off;
-    __shared__ uint32_t s_heavy;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    Staged* all = reinterpret_cast<Staged*>(smem);
-    BlockList<1> list { s_list[warp], {} };
     const int nbr = (p.rows + kBlk - 1) / kBlk;
-    const int br0 = int(blockIdx.x) * kGridWarps, br = br0 + warp, bc = int(blockIdx.y);
-    const int nb = C::bins(p);       // bins that reach a block on either axis
-    const int skip = p.pad + 1 - nb; // (those further away cannot)
-    __shared__ double s_tab[C::kTab > 0 ? C::kTab : 1];
-    const double* stab = s_tab;
-    if (nb <= kCtaBins) {
-        // s_off[j]: the offsets of the CTA's bins in column j
-        const int no = kGridWarps + nb;
-        for (int t = threadIdx.x; t < nb * no; t += 32 * kGridWarps) {
-            const int j = t / no, i = t - j * no;
-            s_off[j][i] = p.off[size_t(bc + skip + j) * size_t(p.brn + 1) + size_t(min(br0 + skip + i, p.brn))];
-        }
-        __syncthreads();
-        uint32_t total = 0, own = 0;
-        for (int j = 0; j < nb; j++) {
-            total += s_off[j][no - 1] - s_off[j][0];
-            if (C::kWindows)
-                own += s_off[j][warp + nb] - s_off[j][warp];
-        }
-        if (total == 0) { // nothing reaches the CTA: most of a grid outside the uv coverage
-            A acc[C::NACC] = {};
-            if (br < nbr)
-                C::template store<1>(p, br * kBlk, bc * kBlk, acc);
-            return;
-        }
-        C::load_table(p, s_tab);
-        // (the barrier also orders the table before its first use)
-        const bool staged = C::kWindows ? !__syncthreads_or(own > 2 * kHeavy) : total <= C::kCta;
-        if (staged) {
-            if (C::kParts > 1 && C::parts(p))
-                grid_staged<C, C::kParts>(p, s_tab, all, s_off, s_list[warp], nb, total);
-            else
-                grid_staged<C, 1>(p, s_tab, all, s_off, s_list[warp], nb, total);
-            return;
-        }
-    } else {
-        C::load_table(p, s_tab);
-    }
-    Staged* st = all + warp * 33;
+    const int br0 = int(blockIdx.x) * kGridWarps, br = br0 + warp;
+    Staged* st = reinterpret_cast<Staged*>(smem) + warp * 33;
+    BlockList<1> list { s_list[warp], {} };
     if (lane == 0)
         st[32] = C::dummy(p, 0);
     if (threadIdx.x == 0)
@@ -385,6 +356,113 @@ __global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(
         if (lane == 0)
             st[32] = C::dummy(p, 0); // overwritten by the partial cells
         __syncwarp();
+    }
+}
+
+// The blocks of column bc on their own: each warp's few entries without a
+// barrier (the ranges from the CTA's offsets).
+template <class C>
+__device__ __forceinline__ void grid_few(const typename C::Params& p, const double* stab, typename C::Staged* st,
+    uint16_t* s_list, const CtaOffsets* off, int br, int bc, int nb)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (br >= (p.rows + kBlk - 1) / kBlk)
+        return;
+    if (lane == 0)
+        st[32] = C::dummy(p, 0);
+    uint32_t beg = 0, len = 0;
+    if (lane < nb) {
+        beg = off[lane][warp];
+        len = off[lane][warp + nb] - beg;
+    }
+    BlockList<1> list { s_list, {} };
+    typename C::A acc[C::NACC] = {};
+    block_walk<C>(p, stab, make_ranges(beg, len, nb), br * kBlk, bc * kBlk, 0, 1, st, list, acc);
+    C::template store<1>(p, br * kBlk, bc * kBlk, acc);
+}
+
+// COLS: columns of blocks that a CTA takes one after the other.  One, except
+// on sparse grids, where most blocks only get their zeros or a few entries: a
+// CTA for each column of eight blocks is then bound by its launch, the latency
+// of its offsets and its barriers.  Eight columns share the offsets, empty
+// ones are stored at once, and up to kFew entries are taken without a barrier
+// (64 instead of 256: 48 against 44 us for 65k normally distributed
+// visibilities on 4096^2).  Kernel with one column and eight, disk coverage,
+// single-precision cells: 5.2k visibilities on 8192^2 130 and 79 us, 105k 200
+// and 142, with W-kernels 260 and 154; 420k on 16384^2 785 and 521.
+template <class C, int COLS>
+__global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(const __grid_constant__ typename C::Params p)
+{
+    using A = typename C::A;
+    using Staged = typename C::Staged;
+    // entries of the CTA and a dummy per warp; or 32 and a dummy per warp; or
+    // the partial cells of a block taken by all warps
+    constexpr size_t kStage = sizeof(Staged) * (C::kCta + kGridWarps);
+    constexpr size_t kRed = sizeof(A) * C::NACC * 32 * kGridWarps;
+    static_assert(C::kCta + kGridWarps >= 33 * kGridWarps, "staging by warp");
+    __shared__ __align__(16) unsigned char smem[kStage > kRed ? kStage : kRed];
+    __shared__ uint16_t s_list[kGridWarps][C::kParts * BlockList<C::kParts>::kSize];
+    __shared__ CtaOffsets s_off[kCtaBins + COLS - 1];
+    __shared__ uint32_t s_heavy;
+    const int warp = threadIdx.x >> 5;
+    Staged* all = reinterpret_cast<Staged*>(smem);
+    const int br0 = int(blockIdx.x) * kGridWarps, bc0 = int(blockIdx.y) * COLS;
+    const int nb = C::bins(p);       // bins that reach a block on either axis
+    const int skip = p.pad + 1 - nb; // (those further away cannot)
+    const int cols = COLS == 1 ? 1 : min(COLS, (p.N + kBlk - 1) / kBlk - bc0);
+    __shared__ double s_tab[C::kTab > 0 ? C::kTab : 1];
+    const double* stab = s_tab;
+    const int no = kGridWarps + nb;
+    if (nb <= kCtaBins) {
+        // s_off[j]: the offsets of the CTA's bins in column j
+        for (int t = threadIdx.x; t < (nb + cols - 1) * no; t += 32 * kGridWarps) {
+            const int j = t / no, i = t - j * no;
+            s_off[j][i] = p.off[size_t(bc0 + skip + j) * size_t(p.brn + 1) + size_t(min(br0 + skip + i, p.brn))];
+        }
+        if (COLS > 1)
+            C::load_table(p, s_tab);
+        __syncthreads();
+    } else if (COLS > 1) {
+        C::load_table(p, s_tab);
+    }
+    bool shared = false; // the column before was one of the whole CTA
+    for (int k = 0; k < cols; k++) {
+        const int bc = bc0 + k;
+        const CtaOffsets* off = s_off + k;
+        uint32_t total = 1, own = 0;
+        if (nb <= kCtaBins) {
+            total = 0;
+            for (int j = 0; j < nb; j++) {
+                total += off[j][no - 1] - off[j][0];
+                if (C::kWindows)
+                    own += off[j][warp + nb] - off[j][warp];
+            }
+        }
+        if (total == 0) { // nothing reaches the blocks: most of a grid outside the uv coverage
+            store_zeros<C>(p, br0 * kBlk, bc * kBlk);
+            continue;
+        }
+        if (COLS > 1) {
+            if (shared)
+                __syncthreads(); // the entries of the column before are gridded
+            shared = total > kFew || nb > kCtaBins;
+            if (!shared) {
+                grid_few<C>(p, stab, all + warp * 33, s_list[warp], off, br0 + warp, bc, nb);
+                continue;
+            }
+            __syncthreads(); // no warp is still at a column of its own
+        } else {
+            C::load_table(p, s_tab);
+        }
+        bool staged = false;
+        if (nb <= kCtaBins) // (with one column, the barrier also orders the table before its first use)
+            staged = C::kWindows ? !__syncthreads_or(own > 2 * kHeavy) : total <= C::kCta;
+        if (!staged)
+            grid_unstaged<C>(p, s_tab, smem, s_list, s_heavy, bc, nb, skip);
+        else if (C::kParts > 1 && C::parts(p))
+            grid_staged<C, C::kParts>(p, stab, all, off, s_list[warp], bc, nb, total);
+        else
+            grid_staged<C, 1>(p, stab, all, off, s_list[warp], bc, nb, total);
     }
 }
 
@@ -625,6 +703,13 @@ struct SepCore {
                 mma(acc[4], acc[5], a, b * s.w);
         }
     }
+    static __device__ __forceinline__ void store_zero(const Params& p, size_t i)
+    {
+        using G2 = typename Cplx<G>::T;
+        static_cast<G2*>(p.grid)[i] = G2 {};
+        if constexpr (BEAM)
+            static_cast<G2*>(p.beam)[i] = G2 {};
+    }
     // lane: row lane / 4, columns 2 (lane % 4) and the next
     template <int PARTS>
     static __device__ __forceinline__ void store(const Params& p, int r0, int c0, const A (&acc)[NACC])
@@ -817,6 +902,13 @@ struct WprojCore {
                 }
             }
         }
+    }
+    static __device__ __forceinline__ void store_zero(const Params& p, size_t i)
+    {
+        using G2 = typename Cplx<G>::T;
+        static_cast<G2*>(p.grid)[i] = G2 {};
+        if constexpr (BEAM)
+            static_cast<G2*>(p.beam)[i] = G2 {};
     }
     template <int PARTS>
     static __device__ __forceinline__ void store(const Params& p, int r0, int c0, const A (&acc)[NACC])

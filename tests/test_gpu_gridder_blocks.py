@@ -69,6 +69,45 @@ def test_uneven_blocks_match_oracle(ctx, exact, S):
     _compare(ctx, capi.PSWF, S, 512, uv, vis, wts, exact, 8, True)
 
 
+def _sparse(seed, n, N):
+    """Few entries a block on average, so that a CTA takes eight columns of blocks: half of them anywhere (a warp's few
+    entries), the rest in a handful of blocks around the origin (more than one warp takes alone) and in a square of
+    some dozen entries a block (staged by the CTA)."""
+    uv, vis, wts = _points(seed, n, N, 1.02)
+    rng = np.random.default_rng(seed + 1)
+    uv[::4] = rng.normal(scale=5.0, size=uv[::4].shape)
+    uv[1::4] = rng.uniform(300.0, 340.0, size=uv[1::4].shape)
+    return uv, vis, wts
+
+
+@pytest.mark.parametrize("exact,S,os", [(False, 3, 8), (True, 3, 8), (False, 7, 64), (False, 20, 4), (True, 18, 4)])
+def test_sparse_grids_match_oracle(ctx, exact, S, os):
+    N = 2308  # 289 columns of blocks: the last CTA's group has one
+    uv, vis, wts = _sparse(S, 6000, N)
+    _compare(ctx, capi.PSWF, S, N, uv, vis, wts, exact, os, True)
+
+
+@pytest.mark.parametrize("smax,trunc", [(4, 0.0), (12, 1.0), (20, 0.0)])
+def test_sparse_w_grids_match_oracle(ctx, smax, trunc):
+    N, cell = 2308, 5.0
+    uv, vis, wts = _sparse(smax, 6000, N)
+    w = np.random.default_rng(smax).uniform(-3000.0, 3000.0, len(vis))
+    kw = dict(num_wplanes=4, max_wpconv_support=smax, kernel_trunc_perc=trunc, w=w, cell_size=cell, analytic_gcf=False)
+    r = orc.convolve_to_grid(capi.GaussianSinc, 3, N, uv, vis, wts, False, 4, True, True, True,
+                             wproj=orc.WProj(4, smax, 1, trunc), w=w, cell_size=cell, analytic_gcf=False)
+    g = ctx.convolve_to_grid(capi.GaussianSinc, 3.0, 3, N, uv, vis, wts, kernel_exact=False, oversampling=4, **kw)
+    assert np.abs(g[0] - r.vis_grid).max() <= 1e-11 * np.abs(r.vis_grid).max()
+    assert np.abs(g[1] - r.sampling_grid).max() <= 1e-11 * np.abs(r.sampling_grid).max()
+    # without the beam, in double and in single precision (tolerance as in test_w_kernels_match_oracle)
+    uvw = np.column_stack([uv / (N * np.deg2rad(cell / 3600.0)), w])
+    kwi = dict(kernel_func=capi.GaussianSinc, kernel_support=3, kernel_exact=False, oversampling=4, padded_image_size=N,
+               gridding_correction=False, num_wplanes=4, max_wpconv_support=smax, kernel_trunc_perc=trunc)
+    ref = ctx.image_visibilities(vis, wts, uvw, 300, cell, generate_beam=True, **kwi)[0]
+    for precision, tol in ((capi.FP64, 1e-12), (capi.FP32C, 5e-6), (capi.FP32, 5e-6)):
+        img = ctx.image_visibilities(vis, wts, uvw, 300, cell, precision=precision, **kwi)[0]
+        assert np.abs(img - ref).max() <= tol * np.abs(ref).max(), precision
+
+
 @pytest.mark.parametrize("smax", [3, 8, 12])
 def test_uneven_w_blocks_match_oracle(ctx, smax):
     N, cell = 512, 20.0
