@@ -1550,15 +1550,21 @@ __device__ __forceinline__ uint32_t seg_at(uint32_t b, uint32_t sp, uint32_t e, 
 // Ordered sums over each label's pixels, with explicitly rounded operations
 // (no FMA contraction), so the sums are bit-identical to the reference's.
 // mom: 6 doubles per label code: sum x v, y v, x^2 v, y^2 v, x y v, v (display
-// coordinates).  One warp per label with entries (`listed`): the lanes load
-// and multiply 32 pixels at once, then six lanes each add one of the sums in
-// pixel order.  Only the additions are a chain: with one thread per label the
-// loads were one too, and a bright source of 600 pixels kept the whole grid
-// waiting (60 us of the call on a 4096^2 image, now 25).
+// coordinates).  One warp per label with entries (`listed`) while there is a
+// warp for each: the lanes load and multiply 32 pixels at once, then six lanes
+// each add one of the sums in pixel order.  Only the additions are a chain:
+// with one thread per label the loads were one too, and a bright source of 600
+// pixels kept the whole grid waiting (60 us of the call on a 4096^2 image, now
+// 25).  With more labels than warps (low thresholds: half a million labels of
+// a few pixels) a warp takes up to 32 at a time, each lane one of at most
+// kSumThread pixels, and then together those that are larger: calls on 4096^2
+// single precision at 2.5 and at 2 sigma 510 and 844 us by threads, 573 and
+// 1250 by warps, 456 and 775 so.
 // Ranges of more than `longest` entries have no order yet (those that
 // k_seg_sort_big left to the host, which sums again behind its sort): nothing
 // is read through them, and their sums stay zero.
 constexpr int kSumWarps = 4;
+constexpr uint32_t kSumThread = 16;
 template <typename T>
 __global__ void __launch_bounds__(32 * kSumWarps) k_label_sums(FgSizes z, const T* img, int rows, int cols,
     const uint32_t* vals, const uint32_t* seg_begin, const uint32_t* seg_end, const uint32_t* seg_split,
@@ -1577,44 +1583,90 @@ __global__ void __launch_bounds__(32 * kSumWarps) k_label_sums(FgSizes z, const 
     }
     const int vs = rows / 2, hs = cols / 2;
     double(*t)[33] = terms[warp];
-    for (uint32_t q = blockIdx.x * kSumWarps + warp, nq = *nlisted; q < nq; q += gridDim.x * kSumWarps) {
-        const uint32_t l = listed[q];
-        const uint32_t b = seg_begin[l], e = seg_end[l], sp = seg_split[l], len = e - b;
-        if (len > longest)
-            continue;
-        double sum = 0.0;
-        // the pixel of the next 32 and the index of the 32 after are in flight
-        auto index = [&](uint32_t j) { return j < len ? vals[seg_at(b, sp, e, j)] : 0u; };
-        uint32_t m = index(lane), m1 = index(32 + lane);
-        double val = uint32_t(lane) < len ? ld(img, m) : 0.0;
-        for (uint32_t j = 0; j < len; j += 32) {
-            const int c = int(m / uint32_t(rows)), r = int(m - uint32_t(c) * uint32_t(rows));
-            const double y = r < vs ? double(r + vs) : double(r - vs);
-            const double x = c < hs ? double(c + hs) : double(c - hs);
-            const double xb = __dmul_rn(x, val), yb = __dmul_rn(y, val);
-            t[0][lane] = xb;
-            t[1][lane] = yb;
-            t[2][lane] = __dmul_rn(xb, x);
-            t[3][lane] = __dmul_rn(yb, y);
-            t[4][lane] = __dmul_rn(xb, y);
-            t[5][lane] = val;
-            __syncwarp();
-            m = m1;
-            if (j + 32 + lane < len)
-                val = ld(img, m);
-            m1 = index(j + 64 + lane);
-            if (lane < 6) {
-                const int n = int(min(32u, len - j));
-#pragma unroll 8
-                for (int i = 0; i < n; i++)
-                    sum = __dadd_rn(sum, t[lane][i]);
-            }
-            __syncwarp();
+    auto products = [&](uint32_t m, double val, double (&p)[6]) {
+        const int c = int(m / uint32_t(rows)), r = int(m - uint32_t(c) * uint32_t(rows));
+        const double y = r < vs ? double(r + vs) : double(r - vs);
+        const double x = c < hs ? double(c + hs) : double(c - hs);
+        p[0] = __dmul_rn(x, val);
+        p[1] = __dmul_rn(y, val);
+        p[2] = __dmul_rn(p[0], x);
+        p[3] = __dmul_rn(p[1], y);
+        p[4] = __dmul_rn(p[0], y);
+        p[5] = val;
+    };
+    const uint32_t nq = *nlisted, warps = gridDim.x * kSumWarps;
+    const uint32_t per = min(32u, (nq + warps - 1) / warps);
+    for (uint32_t q0 = (blockIdx.x * kSumWarps + warp) * per; q0 < nq; q0 += warps * per) {
+        // lane j < per: the warp's j-th label
+        uint32_t l = 0, b = 0, e = 0, sp = 0;
+        if (uint32_t(lane) < per && q0 + lane < nq) {
+            l = listed[q0 + lane];
+            b = seg_begin[l];
+            e = seg_end[l];
+            sp = seg_split[l];
         }
-        if (lane < 6)
-            mom[6 * size_t(l) + lane] = sum;
-        if (lane == 0)
-            ns[l] = int(len);
+        const uint32_t own = e - b > longest ? 0u : e - b;
+        const bool alone = per > 1 && own <= kSumThread;
+        if (alone && own > 0) {
+            double sum[6] = {};
+            // four pixels' loads in flight, then their sums in order
+            for (uint32_t j = 0; j < own; j += 4) {
+                uint32_t m[4];
+                double val[4];
+#pragma unroll
+                for (uint32_t i = 0; i < 4; i++)
+                    m[i] = j + i < own ? vals[seg_at(b, sp, e, j + i)] : 0u;
+#pragma unroll
+                for (uint32_t i = 0; i < 4; i++)
+                    val[i] = j + i < own ? ld(img, m[i]) : 0.0;
+#pragma unroll
+                for (uint32_t i = 0; i < 4; i++)
+                    if (j + i < own) {
+                        double p[6];
+                        products(m[i], val[i], p);
+#pragma unroll
+                        for (int k = 0; k < 6; k++)
+                            sum[k] = __dadd_rn(sum[k], p[k]);
+                    }
+            }
+            for (int k = 0; k < 6; k++)
+                mom[6 * size_t(l) + k] = sum[k];
+            ns[l] = int(own);
+        }
+        for (unsigned rest = __ballot_sync(0xffffffffu, own > 0 && !alone); rest; rest &= rest - 1) {
+            const int from = __ffs(int(rest)) - 1;
+            const uint32_t wl = __shfl_sync(0xffffffffu, l, from), wb = __shfl_sync(0xffffffffu, b, from);
+            const uint32_t we = __shfl_sync(0xffffffffu, e, from), wsp = __shfl_sync(0xffffffffu, sp, from);
+            const uint32_t len = we - wb;
+            double sum = 0.0;
+            // the pixel of the next 32 and the index of the 32 after are in flight
+            auto index = [&](uint32_t j) { return j < len ? vals[seg_at(wb, wsp, we, j)] : 0u; };
+            uint32_t m = index(lane), m1 = index(32 + lane);
+            double val = uint32_t(lane) < len ? ld(img, m) : 0.0;
+            for (uint32_t j = 0; j < len; j += 32) {
+                double p[6];
+                products(m, val, p);
+#pragma unroll
+                for (int k = 0; k < 6; k++)
+                    t[k][lane] = p[k];
+                __syncwarp();
+                m = m1;
+                if (j + 32 + lane < len)
+                    val = ld(img, m);
+                m1 = index(j + 64 + lane);
+                if (lane < 6) {
+                    const int n = int(min(32u, len - j));
+#pragma unroll 8
+                    for (int i = 0; i < n; i++)
+                        sum = __dadd_rn(sum, t[lane][i]);
+                }
+                __syncwarp();
+            }
+            if (lane < 6)
+                mom[6 * size_t(wl) + lane] = sum;
+            if (lane == 0)
+                ns[wl] = int(len);
+        }
     }
 }
 

@@ -38,6 +38,31 @@ inline std::vector<std::unique_ptr<std::barrier<>>> warp_barriers;
 
 inline void __syncthreads() { block_barrier->arrive_and_wait(); }
 inline void __syncwarp() { warp_barriers[threadIdx.x / 32]->arrive_and_wait(); }
+// every lane of a warp takes part
+inline std::vector<std::vector<uint64_t>> warp_slots;
+template <typename T>
+T __shfl_sync(unsigned, T v, int from)
+{
+    auto& slots = warp_slots[threadIdx.x / 32];
+    __builtin_memcpy(&slots[threadIdx.x % 32], &v, sizeof(T));
+    __syncwarp();
+    T r;
+    __builtin_memcpy(&r, &slots[from], sizeof(T));
+    __syncwarp();
+    return r;
+}
+inline unsigned __ballot_sync(unsigned, bool v)
+{
+    auto& slots = warp_slots[threadIdx.x / 32];
+    slots[threadIdx.x % 32] = v;
+    __syncwarp();
+    unsigned r = 0;
+    for (int i = 0; i < 32; i++)
+        r |= unsigned(slots[i] != 0) << i;
+    __syncwarp();
+    return r;
+}
+inline int __ffs(int v) { return __builtin_ffs(v); }
 template <typename T>
 inline T __ldg(const T* p)
 {
@@ -62,6 +87,7 @@ void launch(Dim3 grid, unsigned threads, F kernel)
             blockIdx = Dim3 { bx, by, 0 };
             block_barrier = std::make_unique<std::barrier<>>(threads);
             warp_barriers.clear();
+            warp_slots.assign((threads + 31) / 32, std::vector<uint64_t>(32));
             for (unsigned w = 0; w < threads; w += 32)
                 warp_barriers.push_back(std::make_unique<std::barrier<>>(std::min(32u, threads - w)));
             std::vector<std::thread> pool;

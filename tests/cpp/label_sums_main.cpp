@@ -69,5 +69,40 @@ int main()
     check(0);
     check(1);
     bad += g_outside;
+
+    // more labels than warps: a warp takes several, and small and large ones are summed in other ways; the sums of
+    // each are those of its pixels in memory order (the ones from the split on first), to the last bit
+    const int labels = 300;
+    std::vector<uint32_t> b2, e2, sp2, px, li;
+    for (int l = 0; l < labels; l++) {
+        const uint32_t len = l % 7 == 0 ? 17 + l % 60 : 1 + l % 16;
+        b2.push_back(uint32_t(px.size()));
+        sp2.push_back(b2[l] + len / 3);
+        for (uint32_t i = 0; i < len; i++)
+            px.push_back((uint32_t(l) * 211u + i * 97u) % uint32_t(g_pixels));
+        e2.push_back(uint32_t(px.size()));
+        li.push_back(uint32_t((l * 7) % labels));
+    }
+    const uint32_t misc2[3] = { uint32_t(labels), 0, uint32_t(px.size()) }, nl2 = labels;
+    std::vector<double> mom2(6 * labels, -1.0);
+    std::vector<int> ns2(labels, -1);
+    launch(Dim3 { 2, 1, 1 }, 32 * kSumWarps, [&] {
+        k_label_sums<float>(FgSizes { misc2, uint32_t(labels), misc2[2] }, img.data(), rows, cols, px.data(), b2.data(),
+            e2.data(), sp2.data(), li.data(), &nl2, SEG_BIG, mom2.data(), ns2.data());
+    });
+    for (int l = 0; l < labels; l++) {
+        double s[6] = {};
+        const uint32_t len = e2[l] - b2[l];
+        for (uint32_t j = 0; j < len; j++) {
+            const uint32_t m = px[seg_at(b2[l], sp2[l], e2[l], j)], c = m / rows, r = m % rows;
+            const double x = double(c < 128 ? c + 128 : c - 128), y = double(r < 128 ? r + 128 : r - 128), v = img[m];
+            const double xv = x * v, yv = y * v, terms[6] = { xv, yv, xv * x, yv * y, xv * y, v };
+            for (int k = 0; k < 6; k++)
+                s[k] += terms[k];
+        }
+        for (int k = 0; k < 6; k++)
+            bad += s[k] != mom2[6 * l + k];
+        bad += ns2[l] != int(len);
+    }
     return bad ? 1 : 0;
 }

@@ -36,7 +36,8 @@ inline void pack_scalars(const PackArgs&) {}
     _run(tmp_path, "fft_axis_main.cpp", {"imager_kernels.cuh": stub, "fft_kernels.cuh": _source("fft_kernels.cuh")})
 
 
-def test_label_sums_wait_for_the_order_of_a_large_label(tmp_path):
+def test_label_sums(tmp_path):
+    """No sums through a range that is not sorted yet; many labels, small and large."""
     src = _source("sourcefind_kernels.cuh")
 
     def cut(begin, end):
