@@ -151,8 +151,8 @@ def test_imager_wproj_untruncated(ctx):
 
 @pytest.mark.parametrize("trunc", [0.0, 1.0])
 def test_imager_wproj_large_support(ctx, trunc):
-    """W-kernel supports above 32 (the reference's W-projection configurations use up to 127): tables and tile
-    lists sized from the measured supports."""
+    """W-kernel supports above 32 (the reference's W-projection configurations use up to 127): tables sized from the
+    measured supports."""
     s = _imager_case(37, 256, 1500, w_range=(-4000.0, 4000.0))
     kw = dict(kernel_func=5, kernel_support=3, kernel_exact=False, oversampling=4, analytic_gcf=True,
               num_wplanes=3, max_wpconv_support=40, kernel_trunc_perc=trunc)
@@ -371,26 +371,103 @@ def test_repeated_device_calls_replay_graph_with_new_data(ctx):
         c2.close()
 
 
-@pytest.mark.parametrize("layout", ["32", "16", "32c", "16c", "32t", "16t", "8t", "32r", "16r", "8r"])
-@pytest.mark.parametrize("wproj", [False, True])
-def test_imager_every_gridder_layout_vs_oracle(layout, wproj, monkeypatch):
-    """Each tile width and gridder form the autotuner may pick gives the oracle's image (FP64 1e-10,
-    FP32C 1e-5); the image spans the grid edges (items near the uv origin wrap after the shift)."""
-    monkeypatch.setenv("STPGPU_GRIDDER_LAYOUT", layout)
-    s = _imager_case(61, 256, 8000, w_range=(-600.0, 600.0) if wproj else (0.0, 0.0))
-    kw = dict(kernel_func=4, kernel_support=3, kernel_exact=False, oversampling=8, analytic_gcf=False,
-              generate_beam=not wproj)
+# what selects the gridder's code: visibilities a block of 8 x 8 cells and their concentration, the length of the tap
+# table, the support, the kind of kernel and the cells' type (PSWF: double cells in compensated single precision)
+GRIDDER_BRANCHES = {
+    "staged": dict(n=8000),
+    "dense": dict(n=30000),
+    "concentrated": dict(n=8000, spread=0.03),
+    "double_cells": dict(n=8000, kernel_func=5),
+    "double_cells_dense": dict(n=30000, kernel_func=5),
+    "tap_table_in_memory": dict(n=4000, oversampling=64),
+    "tap_table_in_memory_dense": dict(n=30000, oversampling=64),
+    "wide_support": dict(n=2000, kernel_support=17),
+    "wide_support_dense": dict(n=26000, kernel_support=20),
+    "exact": dict(n=4000, kernel_exact=True),
+    "exact_dense": dict(n=26000, kernel_exact=True),
+    "exact_wide": dict(n=1000, kernel_exact=True, kernel_support=18),
+    "w_two_parts": dict(n=8000, max_wpconv_support=5),
+    "w_one_list": dict(n=8000, max_wpconv_support=12),
+    "w_unstaged": dict(n=2000, max_wpconv_support=20),
+    "w_concentrated": dict(n=8000, max_wpconv_support=5, spread=0.03),
+    "w_dense": dict(n=26000, max_wpconv_support=5),
+    "w_double_cells": dict(n=8000, max_wpconv_support=5, kernel_func=5),
+}
+
+
+@pytest.mark.parametrize("branch", list(GRIDDER_BRANCHES))
+def test_imager_every_gridder_branch_vs_oracle(ctx, branch):
+    """Each form of the gridder that sizes, kernels and types select gives the oracle's image and beam; the image
+    spans the grid edges (items near the uv origin wrap after the shift).  FP64 within 1e-10 and FP32C with double
+    cells within 1e-5 of the corrected image.  With single-precision cells and sums the uncorrected images are
+    compared (the correction multiplies their error by up to 890 at the field's edge): kernel values, weighted
+    visibilities and transform are rounded to 2^-24 each, 5e-6 of the peak in all."""
+    kw = dict(kernel_func=4, kernel_support=3, kernel_exact=False, oversampling=8, analytic_gcf=False)
+    kw.update(GRIDDER_BRANCHES[branch])
+    n, spread, wproj = kw.pop("n"), kw.pop("spread", 1.0), "max_wpconv_support" in kw
+    s = _imager_case(61, 256, n, w_range=(-600.0, 600.0) if wproj else (0.0, 0.0))
+    uvw = np.asfortranarray(s.uvw * np.array([spread, spread, 1.0]))
     if wproj:
-        kw.update(num_wplanes=5, max_wpconv_support=8, kernel_trunc_perc=1.0)
-    ref, rbeam = orc.image_visibilities(s.vis, s.weights, s.uvw, 256, s.cell_size, **kw)
-    c = capi.Context(0)
-    try:
-        img, beam, _ = c.image_visibilities(s.vis, s.weights, s.uvw, 256, s.cell_size, **kw)
+        kw.update(num_wplanes=5, kernel_trunc_perc=0.0)
+    args = (s.vis, s.weights, uvw, 256, s.cell_size)
+    wide = kw["kernel_func"] == 5
+    ref, rbeam = orc.image_visibilities(*args, generate_beam=True, **kw)
+    for beam in (True, False):
+        img, bm, _ = ctx.image_visibilities(*args, generate_beam=beam, **kw)
         assert peak_rel(img, ref) < TOL64
-        if not wproj:
-            assert peak_rel(beam, rbeam) < TOL64
-        img32, _, _ = c.image_visibilities(s.vis, s.weights, s.uvw, 256, s.cell_size, precision=capi.FP32C,
-                                           out_dtype=capi.F32, **kw)
-        assert peak_rel(img32.astype(np.float64), ref) < TOL32
-    finally:
-        c.close()
+        assert not beam or peak_rel(bm, rbeam) < TOL64
+    if not wide:
+        kw["gridding_correction"] = False
+        ref, rbeam = orc.image_visibilities(*args, generate_beam=True, **kw)
+    for precision in (capi.FP32C,) if wide else (capi.FP32C, capi.FP32):
+        for beam in (True, False):
+            img, bm, info = ctx.image_visibilities(*args, generate_beam=beam, precision=precision, out_dtype=capi.F32,
+                                                   **kw)
+            assert (info.flags & 1) == int(wide)
+            assert peak_rel(img.astype(np.float64), ref) < (TOL32 if wide else 5e-6)
+            assert not beam or peak_rel(bm.astype(np.float64), rbeam) < (TOL32 if wide else 5e-6)
+
+
+@pytest.mark.parametrize("precision", [capi.FP64, capi.FP32C])
+def test_device_image_aligned_to_one_element(ctx, precision):
+    """An output that the transform's kernel cannot store in pairs takes the other transform: the same image."""
+    import torch
+
+    s = _imager_case(62, 256, 4000)
+    kw = dict(kernel_func=4, kernel_support=3, kernel_exact=False, oversampling=8, analytic_gcf=False)
+    dv, dw = torch.from_numpy(s.vis).cuda(), torch.from_numpy(s.weights).cuda()
+    duvw = torch.from_numpy(np.ascontiguousarray(s.uvw.T)).cuda()
+    # (two single-precision transforms, each within TOL32 of the exact image)
+    dtype, odt, tol = ((torch.float64, capi.F64, 1e-12) if precision == capi.FP64
+                       else (torch.float32, capi.F32, 2 * TOL32))
+    got = []
+    for offset in (0, 1):
+        out = torch.full((256 * 256 + 8,), -1.0, dtype=dtype, device="cuda")
+        view = out[offset:offset + 256 * 256]
+        for _ in range(3):  # the third call replays the captured graph
+            ctx.image_visibilities(dv, dw, duvw, 256, s.cell_size, precision=precision, out_dtype=odt, device_ptrs=True,
+                                   image_out=view, **kw)
+        got.append(view.double().cpu().numpy())
+        assert (out[:offset] == -1.0).all() and (out[offset + 256 * 256:] == -1.0).all()
+    assert peak_rel(got[1], got[0]) < tol
+
+
+def test_imager_wproj_crowded_w():
+    """Three of four |w| in 2^-9 of each other: more of them share a bin with a plane's start than are looked at there,
+    whatever the number of bins, and the planes are found by sorting."""
+    for n in (4000, 20000):  # histograms of 2^12 bins
+        s = _imager_case(63, 256, n, w_range=(-300.0, 300.0))
+        uvw = np.array(s.uvw, order="F")
+        rng = np.random.default_rng(n)
+        uvw[:, 2] = np.where(np.arange(n) % 4 != 0, 150.0 * (1.0 + 2.0 ** -9 * rng.random(n)), uvw[:, 2])
+        kw = dict(kernel_func=4, kernel_support=3, kernel_exact=False, oversampling=8, analytic_gcf=False, num_wplanes=8,
+                  max_wpconv_support=8, undersampling_opt=1, kernel_trunc_perc=1.0)
+        fresh = capi.Context(0)
+        try:
+            for _ in range(2):
+                img, _, info = fresh.image_visibilities(s.vis, s.weights, uvw, 256, s.cell_size, **kw)
+                ri, _, g = orc.image_visibilities(s.vis, s.weights, uvw, 256, s.cell_size, return_grid=True, **kw)
+                assert info.max_plane_support == max(g.plane_supports)
+                assert peak_rel(img, ri) < TOL64
+        finally:
+            fresh.close()
