@@ -1737,7 +1737,11 @@ __global__ void k_islands(FgSizes z, const SfStats* st, const unsigned long long
 // every thread (Cholesky).  The call waits for its largest island (a bright
 // source of 900 pixels): with one warp an island, and with the cost of a
 // step evaluated before its normal equations, the kernel took 205 us on 60
-// sources of a 1502 x 1998 image.
+// sources of a 1502 x 1998 image.  A step's cost and this thread's part of its
+// normal equations come from one pass over the pixels; the 27 sums of the
+// latter are formed for steps that are taken only (faint islands of a few
+// pixels reject most of theirs: 1688 islands in a call of 1466 us, 1525 when
+// every step formed them, 1497 with one warp an island).
 constexpr int FIT_MAX_ITER = 100;
 constexpr int FIT_THREADS = 128;
 
@@ -1819,7 +1823,8 @@ __global__ void __launch_bounds__(FIT_THREADS) k_gauss_fit(const T* __restrict__
     const int isl = blockIdx.x;
     if (isl >= nis)
         return;
-    __shared__ double part[FIT_THREADS / 32][28], tot[28];
+    constexpr int W = FIT_THREADS / 32;
+    __shared__ double part[W][27], tot[27], costs[2][W];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int key = keys[isl];
     const uint32_t b = sb[key], e = se[key], split = sp[key];
@@ -1828,11 +1833,22 @@ __global__ void __launch_bounds__(FIT_THREADS) k_gauss_fit(const T* __restrict__
     for (int k = 0; k < 6; k++)
         p[k] = init[6 * isl + k];
 
-    // cost and normal equations at parameters q (the same bits in every thread)
-    auto pass = [&](const double* q, double* JtJ, double* Jtr) -> double {
+    auto warp_sum = [](double v) {
+        for (int o = 16; o > 0; o >>= 1)
+            v += __shfl_xor_sync(0xffffffffu, v, o);
+        return v;
+    };
+    // cost at parameters q (the same bits in every thread), and this thread's
+    // part of the normal equations
+    double jj[21], jr[6];
+    int turn = 0;
+    auto pass = [&](const double* q) -> double {
         const GaussTerms g = gauss_terms(q);
         double cost = 0.0;
-        double jj[21] = {}, jr[6] = {};
+        for (double& v : jj)
+            v = 0.0;
+        for (double& v : jr)
+            v = 0.0;
         for (uint32_t j = threadIdx.x; j < e - b; j += FIT_THREADS) {
             const uint32_t m = pix[seg_at(b, split, e, j)];
             const int rm = int(m % uint32_t(rows)), cm = int(m / uint32_t(rows));
@@ -1860,23 +1876,28 @@ __global__ void __launch_bounds__(FIT_THREADS) k_gauss_fit(const T* __restrict__
                     jj[u++] += J[i] * J[k];
             }
         }
-        auto reduce = [&](double v, int k) {
-            for (int o = 16; o > 0; o >>= 1)
-                v += __shfl_xor_sync(0xffffffffu, v, o);
+        cost = warp_sum(cost);
+        turn ^= 1; // (a slow thread may still read the costs of the pass before)
+        if (lane == 0)
+            costs[turn][warp] = cost;
+        __syncthreads();
+        cost = 0.0;
+        for (int w = 0; w < W; w++)
+            cost += costs[turn][w];
+        return cost;
+    };
+    // the normal equations at the parameters of the last pass
+    auto normal = [&](double* JtJ, double* Jtr) {
+#pragma unroll
+        for (int k = 0; k < 27; k++) {
+            const double v = warp_sum(k < 21 ? jj[k < 21 ? k : 0] : jr[k < 21 ? 0 : k - 21]);
             if (lane == 0)
                 part[warp][k] = v;
-        };
-#pragma unroll
-        for (int k = 0; k < 21; k++)
-            reduce(jj[k], k);
-#pragma unroll
-        for (int k = 0; k < 6; k++)
-            reduce(jr[k], 21 + k);
-        reduce(cost, 27);
+        }
         __syncthreads();
-        if (threadIdx.x < 28) {
+        if (threadIdx.x < 27) {
             double v = 0.0;
-            for (int w = 0; w < FIT_THREADS / 32; w++)
+            for (int w = 0; w < W; w++)
                 v += part[w][threadIdx.x];
             tot[threadIdx.x] = v;
         }
@@ -1885,11 +1906,11 @@ __global__ void __launch_bounds__(FIT_THREADS) k_gauss_fit(const T* __restrict__
             JtJ[k] = tot[k];
         for (int k = 0; k < 6; k++)
             Jtr[k] = tot[21 + k];
-        return tot[27];
     };
 
     double JtJ[21], Jtr[6];
-    double cost = pass(p, JtJ, Jtr);
+    double cost = pass(p);
+    normal(JtJ, Jtr);
     double lambda = 1e-3;
     int it = 0;
     while (it < FIT_MAX_ITER) {
@@ -1897,7 +1918,7 @@ __global__ void __launch_bounds__(FIT_THREADS) k_gauss_fit(const T* __restrict__
         // (J^T J + lambda D) delta = -J^T r, D = diag(J^T J) floored at 1e-12 of its
         // largest entry (a parameter the residuals do not depend on, such as
         // theta of a circular Gaussian, then gets a zero step)
-        double m[21], rhs[6], d[6], q[6], JtJn[21], Jtrn[6];
+        double m[21], rhs[6], d[6], q[6];
         double dmax = 0.0;
         for (int i = 0; i < 6; i++)
             dmax = fmax(dmax, JtJ[i * (i + 1) / 2 + i]);
@@ -1915,7 +1936,7 @@ __global__ void __launch_bounds__(FIT_THREADS) k_gauss_fit(const T* __restrict__
             ok = q[3] != 0.0 && q[4] != 0.0;
         }
         if (ok) {
-            cnew = pass(q, JtJn, Jtrn);
+            cnew = pass(q);
             ok = cnew == cnew && cnew < cost; // NaN-safe
         }
         if (ok) {
@@ -1926,10 +1947,7 @@ __global__ void __launch_bounds__(FIT_THREADS) k_gauss_fit(const T* __restrict__
             for (int k = 0; k < 6; k++)
                 p[k] = q[k];
             cost = cnew;
-            for (int k = 0; k < 21; k++)
-                JtJ[k] = JtJn[k];
-            for (int k = 0; k < 6; k++)
-                Jtr[k] = Jtrn[k];
+            normal(JtJ, Jtr);
             lambda = fmax(lambda * 0.1, 1e-15);
             if (small)
                 break;
