@@ -575,9 +575,27 @@ BlockBins make_bins(stpgpu_context* c, const ImagerSetup& s, const GridOut& g, i
     return b;
 }
 
-// Visibilities per block of cells from which several warps share a block.
-constexpr int64_t kDensePerBlock = 24;
+// Visibilities per block of cells above which several warps share a block.  On
+// a small grid a warp a block leaves most of the GPU idle, and a block of a
+// concentrated coverage keeps the rest waiting; on a large one there are warps
+// enough, and a CTA that stages its entries once spends less on them.  The
+// host knows neither the coverage nor the fullest block, so the line lies
+// between the two: kernel, a warp a block and eight, us, disk / normal / tracks
+// coverage at 24.5, 40 and 80 visibilities a block, W-kernels (support 2 to 3)
+// in compensated single precision:
+//   512^2   25 31, 41 34, 111 47 / 116 46, 174 60, 324 106 / 129 40, 140 53, 256 86
+//   1500^2  64 178, 120 201, 286 292 / 182 156, 272 206, 527 335 / 186 151, 250 198, 455 325
+//   2048^2  105 320, 198 358, 480 533 / 225 266, 355 353, 688 578 / 221 258, 336 339, 609 560
+//   3000^2  205 673, 395 760, 947 1123 / 365 541, 560 718, 1062 1162 / 373 520, 573 684, 1095 1110
+//   4096^2  368 1256, 716 1409 at 24.5 and 40 / 592 992, 910 1313 / 627 947, 938 1251
+// and separable kernels on 2048^2 72 118, 111 149, 216 232 / 142 127, 168 162,
+// 330 254 / 123 120, 155 154, 309 245.  With a beam in single precision (two
+// CTAs an SM) 299 370 and 770 562 at 40 and 80 on 2048^2 / 435 372, 851 601.
 constexpr int kDenseSplit = 8;
+int64_t dense_per_block(int64_t blocks, bool beam, bool single)
+{
+    return blocks <= 20000 ? 24 : blocks / (beam && single ? 980 : 490);
+}
 // Columns of blocks that a CTA takes on sparse grids (k_grid_blocks).
 constexpr int kSparseCols = 8;
 
@@ -660,8 +678,7 @@ void grid_blocks(stpgpu_context* c, const ImagerSetup& s, GridOut& g, int64_t n,
         p.beam = g.beam;
     };
     const int64_t nbr = ceil_div(b.rows, kBlk), nbc = ceil_div(b.N, kBlk);
-    // visibilities per block: above kDensePerBlock several warps share a block
-    const bool dense = n > kDensePerBlock * nbr * nbc;
+    const bool dense = n > dense_per_block(nbr * nbc, s.beam, sizeof(T) == 4) * nbr * nbc;
     const unsigned nbr8 = unsigned(ceil_div(nbr, kGridWarps));
     // Few visibilities: several columns of blocks a CTA, as long as the CTAs
     // still fill the GPU.  One column and eight, us: 4096^2 (2112 CTAs of eight
