@@ -681,13 +681,15 @@ void grid_blocks(stpgpu_context* c, const ImagerSetup& s, GridOut& g, int64_t n,
     const bool dense = n > dense_per_block(nbr * nbc, s.beam, sizeof(T) == 4) * nbr * nbc;
     const unsigned nbr8 = unsigned(ceil_div(nbr, kGridWarps));
     // Few visibilities: several columns of blocks a CTA, as long as the CTAs
-    // still fill the GPU.  One column and eight, us: 4096^2 (2112 CTAs of eight
-    // columns) at 0.2, 0.5 and 1 visibility a block 52 and 46, 54 and 50, 57 and
-    // 52 on disk coverage, 41 and 38, 44 and 44, 48 and 54 on a normal one;
-    // 6000^2 (4418 CTAs) at 0.5, 1 and 2 112 and 89, 118 and 94, 127 and 103,
-    // or 89 and 73, 98 and 87, 115 and 125.
+    // still fill the GPU.  One column and eight, us, W-kernels in double at
+    // disk / normal coverage: 4096^2 (2112 CTAs of eight columns) at 0.3, 1 and
+    // 2 visibilities a block 74 51, 84 68, 96 88 / 59 53, 72 92, 88 121; 5000^2
+    // (3120) at 1 and 2 125 92, 143 123 / 107 117, 131 154; 6000^2 (4418) at 1,
+    // 2 and 4 180 129, 207 174, 264 258 / 154 155, 189 195, 270 385; 8192^2 336
+    // 234, 391 319, 506 487 / 284 250, 351 327, 499 605.
     const int64_t ctas = nbr8 * (nbc / kSparseCols);
-    const bool sparse = ctas >= 148 * 4 && (ctas >= 148 * 20 ? n : 2 * n) < nbr * nbc;
+    const double line = ctas < 148 * 4 ? 0.0 : (ctas < 148 * 20 ? 0.5 : (ctas < 4000 ? 1.5 : 2.0));
+    const bool sparse = double(n) < line * double(nbr * nbc);
     auto run = [&](auto core, const auto& p) {
         using C = decltype(core);
         c->mark(1);

@@ -368,16 +368,18 @@ __device__ __forceinline__ void grid_few(const typename C::Params& p, const doub
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (br >= (p.rows + kBlk - 1) / kBlk)
         return;
-    if (lane == 0)
-        st[32] = C::dummy(p, 0);
     uint32_t beg = 0, len = 0;
     if (lane < nb) {
         beg = off[lane][warp];
         len = off[lane][warp + nb] - beg;
     }
-    BlockList<1> list { s_list, {} };
     typename C::A acc[C::NACC] = {};
-    block_walk<C>(p, stab, make_ranges(beg, len, nb), br * kBlk, bc * kBlk, 0, 1, st, list, acc);
+    if (__any_sync(0xffffffffu, len != 0)) {
+        if (lane == 0)
+            st[32] = C::dummy(p, 0);
+        BlockList<1> list { s_list, {} };
+        block_walk<C>(p, stab, make_ranges(beg, len, nb), br * kBlk, bc * kBlk, 0, 1, st, list, acc);
+    }
     C::template store<1>(p, br * kBlk, bc * kBlk, acc);
 }
 
@@ -387,9 +389,11 @@ __device__ __forceinline__ void grid_few(const typename C::Params& p, const doub
 // of its offsets and its barriers.  Eight columns share the offsets, empty
 // ones are stored at once, and up to kFew entries are taken without a barrier
 // (64 instead of 256: 48 against 44 us for 65k normally distributed
-// visibilities on 4096^2).  Kernel with one column and eight, disk coverage,
-// single-precision cells: 5.2k visibilities on 8192^2 130 and 79 us, 105k 200
-// and 142, with W-kernels 260 and 154; 420k on 16384^2 785 and 521.
+// visibilities on 4096^2); what is left is bound by the instructions of a block
+// (fetching the next column's records ahead gave nothing, 94 against 98 us).
+// Kernel with one column and eight, disk coverage, single-precision cells: 26k
+// visibilities on 8192^2 169 and 98 us, 157k 203 and 135, with W-kernels 260 and
+// 135; 56k on 12000^2 357 and 193.
 template <class C, int COLS>
 __global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(const __grid_constant__ typename C::Params p)
 {
@@ -426,18 +430,17 @@ __global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(
         C::load_table(p, s_tab);
     }
     bool shared = false; // the column before was one of the whole CTA
+    uint32_t totals = 1; // lane k: entries of column k
+    if (nb <= kCtaBins) {
+        const int lane = threadIdx.x & 31, k = COLS == 1 ? 0 : min(lane, cols - 1);
+        totals = 0;
+        for (int j = 0; j < nb; j++)
+            totals += s_off[k + j][no - 1] - s_off[k + j][0];
+    }
     for (int k = 0; k < cols; k++) {
         const int bc = bc0 + k;
         const CtaOffsets* off = s_off + k;
-        uint32_t total = 1, own = 0;
-        if (nb <= kCtaBins) {
-            total = 0;
-            for (int j = 0; j < nb; j++) {
-                total += off[j][no - 1] - off[j][0];
-                if (C::kWindows)
-                    own += off[j][warp + nb] - off[j][warp];
-            }
-        }
+        const uint32_t total = COLS == 1 ? totals : __shfl_sync(0xffffffffu, totals, k);
         if (total == 0) { // nothing reaches the blocks: most of a grid outside the uv coverage
             store_zeros<C>(p, br0 * kBlk, bc * kBlk);
             continue;
@@ -455,8 +458,14 @@ __global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(
             C::load_table(p, s_tab);
         }
         bool staged = false;
-        if (nb <= kCtaBins) // (with one column, the barrier also orders the table before its first use)
+        if (nb <= kCtaBins) {
+            uint32_t own = 0;
+            if (C::kWindows)
+                for (int j = 0; j < nb; j++)
+                    own += off[j][warp + nb] - off[j][warp];
+            // (with one column, the barrier also orders the table before its first use)
             staged = C::kWindows ? !__syncthreads_or(own > 2 * kHeavy) : total <= C::kCta;
+        }
         if (!staged)
             grid_unstaged<C>(p, s_tab, smem, s_list, s_heavy, bc, nb, skip);
         else if (C::kParts > 1 && C::parts(p))
