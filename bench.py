@@ -8,7 +8,7 @@ with uvw uniform in a uv disk and w ~ U[-2000, 2000] lambda, 20 point sources
 Synthetic, seeded data (no dataset exists for it).
 
 A step = one full imaging pass of one snapshot through the library (prepass,
-W-planes and FP64 W-kernels, binning, gridding, cuFFT c2r, gcf/normalise).
+W-planes and FP64 W-kernels, binning, gridding, c2r with gcf/normalise).
 value = visibilities imaged per second (Mvis/s), compensated FP32 (FP32C),
 inputs resident in HBM, L2 flushed (256 MB write) before every timed step.
 The FP64 plain form is timed the same way and reported beside it together
@@ -267,26 +267,26 @@ def run_gpu(args):
         assert abs(float(o.double().max()) - float(out32.double().max())) <= 1e-6 * peak
 
     # ---- roofline of the dominant phase (phase timers over the timed FP32C steps)
-    ph = np.array(ph)  # steps x [grid init, grid loop, FFT, normalise]
+    ph = np.array(ph)  # steps x [grid init, grid loop, columns-axis transform, c2r with crop and normalisation]
     mean_ph = ph.mean(axis=0)
-    names = ["grid_init", "grid_loop", "fft_c2r", "normalise"]
+    names = ["grid_init", "grid_loop", "fft_columns", "c2r_normalise"]
     hbm, peak_kind = _peaks()
     rows = N // 2 + 1
     items = info32.n_grid_items
     # algorithmic bytes per launch of each phase
     alg = {
-        # grid loop: one 28-byte item record per gridded visibility read once, the half-plane grid written
-        # once (FP32 complex); the binning's records are overhead, not algorithmic traffic
-        "grid_loop": int(info32.n_good_vis) * 28 + rows * N * 8,
-        # c2r FFT: read the half-plane grid, write the N x N image (FP32)
-        "fft_c2r": rows * N * 8 + N * N * 4,
-        # normalise: read image, write image (FP32)
-        "normalise": N * N * 4 * 2,
-        # prepass + W-planes + binning: read vis/uvw/weights, write items, lists
-        "grid_init": n * (16 + 24 + 8) + n * 28 + items * 4 * 2,
+        # grid loop: one 16-byte record per entry read once, the half-plane grid written once (FP32 complex)
+        "grid_loop": items * 16 + rows * N * 8,
+        # the columns-axis transform in place: the half-plane grid read once and written once (it takes two
+        # passes, so twice that is moved)
+        "fft_columns": rows * N * 8 * 2,
+        # c2r along the rows, crop, correction: the grid read, the FP32 image written
+        "c2r_normalise": rows * N * 8 + N * N * 4,
+        # prepass + W-planes + binning: read vis/uvw/weights, write the items (32 bytes) and the records
+        "grid_init": n * (16 + 24 + 8) + n * 32 + items * 16,
     }
     # the dominant kernel: the block gridder is the single most expensive launch of a step (the
-    # grid-init phase is ~20 short kernels, none above ~45 us)
+    # grid-init phase is 11 short kernels, none above ~30 us)
     dom = names.index("grid_loop")
     dom_name = names[dom]
     achieved = alg[dom_name] / (mean_ph[dom] / 1e3) / 1e9
