@@ -453,7 +453,7 @@ class Server:
                 island_capacity=4096, want_image=True, **imager_kw):
         """Run a request (the arguments of submit) once on every slot while
         admission is held, so that requests of its size class admitted later
-        allocate, plan and tune nothing.  -> Result of the last slot."""
+        allocate and plan nothing.  -> Result of the last slot."""
         req, _keep = self._request(vis, weights, uvw, find_sources, out_dtype, sf, want_labels, island_capacity,
                                     want_image, imager_kw)
         res = Result()

@@ -457,10 +457,9 @@ struct ImagerSetup {
     int own_c2r = 0; // the c2r on our own kernels (own_c2r_applies decides)
 };
 
-// W-projection with a maximum support above 32: the W-kernel tables and tile
-// lists are sized from the measured plane supports and list length (two
-// host round trips) instead of from the worst case, so such calls are not
-// captured into CUDA graphs.
+// W-projection with a maximum support above 32: the W-kernel tables are sized
+// from the measured plane supports (a host round trip) instead of from the
+// worst case, so such calls are not captured into CUDA graphs.
 bool large_support(const ImagerSetup& s) { return s.nplanes > 0 && s.max_support > 32; }
 
 // Sizes of the W-kernel generation (WideFieldImaging, aw_projection.cpp:19-111).
@@ -820,7 +819,6 @@ GridOut run_gridder(stpgpu_context* c, const ImagerSetup& s, const void* d_vis, 
     pp.absw_key = wproj ? c->buf<double>("absw", nn) : nullptr;
     pp.wmax_part = (wproj && !s.full_wsort) ? c->buf<double>("wmaxpart", 2 * size_t(nb_pre)) : nullptr;
     pp.iota = (wproj && !s.wsel) ? c->buf<uint32_t>("perm_in", nn) : nullptr;
-    pp.w_out = nullptr;
     pp.ticket = g.d_err + CF_TICKET;
     pp.total = g.d_total;
     pp.ngood = g.d_ngood;
@@ -2929,7 +2927,7 @@ struct ServerJob {
     bool done = false;
 };
 
-// Device working set of one request (inputs, items, tile lists, W-planes and
+// Device working set of one request (inputs, items, binned entries, W-planes and
 // W-kernel tables, grid, FFT output, image, source-finder arrays), bytes.
 int64_t request_bytes(const ImagerSetup& s, int image_size, int64_t n, int vis_c64, int precision, int find_sources,
     int correction)

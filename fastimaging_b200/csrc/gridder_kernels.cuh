@@ -775,8 +775,9 @@ struct WprojCore {
     using Params = WprojParams<R, T>;
     using A = ACC;
     static constexpr int NACC = BEAM ? 8 : 4;
-    // (most CTAs of the untruncated headline call in one go: 512 2093 us, 960 1743; and four CTAs an SM within
-    // 132 KB of shared memory, so that L1 keeps the rest)
+    // Most CTAs of the untruncated call of 1M visibilities on 4096^2 (support 16) in one go: 512 entries 2093 us, 960
+    // 1743; 864 leave L1 a little more beside four CTAs an SM (132 KB of shared memory): 1726 with lists gathered for
+    // one part, 960 1737.
     static constexpr uint32_t kCta = BEAM ? 720 : 864;
     static constexpr int kMinBlocks = BEAM ? 2 : 4; // (5 blocks of 48 registers spill: 472 us against 490 on the headline call)
     struct Raw {

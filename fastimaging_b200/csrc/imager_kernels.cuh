@@ -3,10 +3,13 @@
 // Pipeline (one snapshot):
 //   k_prepass      uvw -> pixel scaling, half-plane conversion, rint split,
 //                  bounds check, uv shift, oversampled index  (gridder.h:369-504)
-//   [W-proj]       |w| sort (CUB), plane boundaries/averages, FP64 W-kernels
-//   k_bin_*, k_grid_blocks  binning and gridding (gridder_kernels.cuh)
-//   cuFFT Z2D/C2R  (fft.cpp:45-135)
-//   k_normalise    crop + 1/sum + gcf division                    (imager.h:97-150)
+//   [W-proj]       plane boundaries/averages (k_wsel_*; a |w| sort, CUB, for
+//                  what these do not take), FP64 W-kernels
+//   k_bin_*, k_grid_blocks, k_grid_dense  binning and gridding
+//                  (binning_kernels.cuh, gridder_kernels.cuh)
+//   k_fft_axis, k_c2r_normalise  c2r, crop, 1/sum and gcf division of
+//                  power-of-two grids (fft_kernels.cuh; fft.cpp:45-135,
+//                  imager.h:97-150); other sizes cuFFT Z2D/C2R and k_normalise
 #pragma once
 
 #include "common.cuh"
@@ -30,7 +33,6 @@ struct PrepassParams {
     double* wsum_part; // per-block partial sums of good weights
     unsigned long long* ngood_part;
     double* absw_key; // n |w| (W-proj only), may be null
-    double* w_out;    // n half-plane-converted w (W-proj), may be null
     double* wmax_part; // per block: the maximum and the sum of the finite |w| (W-proj), may be null
     uint32_t* iota;    // n identity permutation (W-proj), may be null
     unsigned int* ticket; // blocks done (zeroed before)
@@ -165,8 +167,6 @@ __global__ void __launch_bounds__(GRID_THREADS) k_prepass(PrepassParams p, Item<
         }
         if (p.iota)
             p.iota[i] = uint32_t(i);
-        if (p.w_out)
-            p.w_out[i] = w;
         Item<R> it;
         it.vr = R(vr);
         it.vi = R(vi);
@@ -381,13 +381,6 @@ __global__ void k_kernel_table(int kf, double trunc, int support, int os, double
     const double s = a1 + a2;
     for (int i = 0; i < K; i++)
         out[c * K + i] = out[c * K + i] / s;
-}
-
-__global__ void k_d2f(const double* in, float* out, int64_t n)
-{
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n)
-        out[i] = float(in[i]);
 }
 
 // ImgDomKernel (conv_func.h:351-412).  Analytic: gcf((i - c)/c).  Otherwise
@@ -1394,9 +1387,9 @@ __device__ __forceinline__ double2 hankel_interp(const HankelParams& h, const do
     return make_double2(((a.x * t + b.x) * t + c.x) * t + y.x, ((a.y * t + b.y) * t + c.y) * t + y.y);
 }
 
-// One block per W-plane.  Writes the plane's support, its quadrant
-// conv[|dy| * lh + |dx|] = f(sqrt(dx^2 + dy^2)) and the sub-kernel
-// normalisations, the same outputs as k_wkernel_plane.
+// One block per W-plane.  Writes the plane's support and its quadrant
+// conv[|dy| * lh + |dx|] = f(sqrt(dx^2 + dy^2)), the same outputs as
+// k_wkernel_plane.
 __global__ void __launch_bounds__(1024) k_hankel_plane(WkParams q, HankelParams h)
 {
     const int p = blockIdx.x;
