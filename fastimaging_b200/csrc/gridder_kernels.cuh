@@ -135,11 +135,11 @@ struct BlockList {
     int m[PARTS];
 };
 
-// The entries listed added to the block whose first row is `row` (relative to
-// the staged entries' origin).
+// The entries listed added to the block whose first cell is (row, col)
+// (relative to the staged entries' origin).
 template <class C, int PARTS>
 __device__ __forceinline__ void list_add(const typename C::Params& p, const double* stab, const typename C::Staged* st,
-    uint32_t dummy, int row, BlockList<PARTS>& b, typename C::A (&acc)[C::NACC])
+    uint32_t dummy, int row, int col, BlockList<PARTS>& b, typename C::A (&acc)[C::NACC])
 {
     const int lane = threadIdx.x & 31;
     int n = b.m[0];
@@ -152,7 +152,7 @@ __device__ __forceinline__ void list_add(const typename C::Params& p, const doub
         for (int i = b.m[h] + lane; i < n; i += 32)
             b.list[h * BlockList<PARTS>::kSize + i] = uint16_t(dummy);
     __syncwarp();
-    C::template accumulate<PARTS>(p, stab, st, b.list, n, row, acc);
+    C::template accumulate<PARTS>(p, stab, st, b.list, n, row, col, acc);
     __syncwarp();
 #pragma unroll
     for (int h = 0; h < PARTS; h++)
@@ -164,14 +164,14 @@ __device__ __forceinline__ void list_add(const typename C::Params& p, const doub
 // have room for 32 more.
 template <class C, int PARTS>
 __device__ __forceinline__ void block_add(const typename C::Params& p, const double* stab, const typename C::Staged* st,
-    uint32_t at, bool valid, uint32_t dummy, int row, BlockList<PARTS>& b, typename C::A (&acc)[C::NACC])
+    uint32_t at, bool valid, uint32_t dummy, int row, int col, BlockList<PARTS>& b, typename C::A (&acc)[C::NACC])
 {
     const int lane = threadIdx.x & 31;
     unsigned reach = 0; // bit h: part h
     bool odd = false;
     if (valid) {
         const typename C::Staged& s = st[at];
-        reach = C::template reach<PARTS>(p, s, row);
+        reach = C::template reach<PARTS>(p, s, row, col);
         odd = reach && C::odd(s);
     }
     bool full = PARTS == 1;
@@ -187,10 +187,10 @@ __device__ __forceinline__ void block_add(const typename C::Params& p, const dou
     if (C::kOdd) {
         unsigned o = __ballot_sync(0xffffffffu, odd);
         for (; o; o &= o - 1)
-            C::add_odd(p, stab, st[__shfl_sync(0xffffffffu, at, __ffs(int(o)) - 1)], row, acc);
+            C::add_odd(p, stab, st[__shfl_sync(0xffffffffu, at, __ffs(int(o)) - 1)], row, col, acc);
     }
     if (full)
-        list_add<C, PARTS>(p, stab, st, dummy, row, b, acc);
+        list_add<C, PARTS>(p, stab, st, dummy, row, col, b, acc);
 }
 
 template <class C>
@@ -217,7 +217,7 @@ __device__ __forceinline__ void block_walk(const typename C::Params& p, const do
             if (tn + lane < r.total)
                 raw = C::fetch(p, i);
         }
-        block_add<C, 1>(p, stab, st, uint32_t(lane), uint32_t(lane) < n, 32, 0, list, acc);
+        block_add<C, 1>(p, stab, st, uint32_t(lane), uint32_t(lane) < n, 32, 0, 0, list, acc);
         t = tn;
     }
 }
@@ -236,7 +236,7 @@ __device__ __forceinline__ void grid_staged(const typename C::Params& p, const d
     const uint32_t dummy = C::kCta + uint32_t(warp);
     BlockList<PARTS> list { lists, {} };
     if (threadIdx.x < kGridWarps)
-        all[C::kCta + threadIdx.x] = C::dummy(p, int(threadIdx.x) * kBlk);
+        all[C::kCta + threadIdx.x] = C::dummy(p, int(threadIdx.x) * kBlk, 0);
     // lane j < nb: column j's entries in the CTA's order, all and the warp's
     uint32_t beg = 0, end = 0;
     {
@@ -265,9 +265,10 @@ __device__ __forceinline__ void grid_staged(const typename C::Params& p, const d
         const uint32_t lo = C::kWindows ? max(beg, w0) : beg, hi = C::kWindows ? min(end, w1) : end;
         const BlockRanges r = make_ranges(lo - w0, hi > lo ? hi - lo : 0u, nb);
         for (uint32_t t = 0; t < r.total; t += 32)
-            block_add<C, PARTS>(p, stab, all, stream_record(r, t + lane), t + lane < r.total, dummy, warp * kBlk, list, acc);
+            block_add<C, PARTS>(p, stab, all, stream_record(r, t + lane), t + lane < r.total, dummy, warp * kBlk, 0, list,
+                acc);
         if (PARTS > 1)
-            list_add<C, PARTS>(p, stab, all, dummy, warp * kBlk, list, acc);
+            list_add<C, PARTS>(p, stab, all, dummy, warp * kBlk, 0, list, acc);
         if (!C::kWindows || w1 == total)
             break;
         w0 = w1;
@@ -305,7 +306,7 @@ __device__ __forceinline__ void grid_unstaged(const typename C::Params& p, const
     Staged* st = reinterpret_cast<Staged*>(smem) + warp * 33;
     BlockList<1> list { s_list[warp], {} };
     if (lane == 0)
-        st[32] = C::dummy(p, 0);
+        st[32] = C::dummy(p, 0, 0);
     if (threadIdx.x == 0)
         s_heavy = 0;
     __syncthreads();
@@ -354,7 +355,7 @@ __device__ __forceinline__ void grid_unstaged(const typename C::Params& p, const
         }
         __syncthreads();
         if (lane == 0)
-            st[32] = C::dummy(p, 0); // overwritten by the partial cells
+            st[32] = C::dummy(p, 0, 0); // overwritten by the partial cells
         __syncwarp();
     }
 }
@@ -376,11 +377,54 @@ __device__ __forceinline__ void grid_few(const typename C::Params& p, const doub
     typename C::A acc[C::NACC] = {};
     if (__any_sync(0xffffffffu, len != 0)) {
         if (lane == 0)
-            st[32] = C::dummy(p, 0);
+            st[32] = C::dummy(p, 0, 0);
         BlockList<1> list { s_list, {} };
         block_walk<C>(p, stab, make_ranges(beg, len, nb), br * kBlk, bc * kBlk, 0, 1, st, list, acc);
     }
     C::template store<1>(p, br * kBlk, bc * kBlk, acc);
+}
+
+// kFewCols blocks beside each other: where the warp has at most 32 entries for
+// all of them, these are fetched and decoded once.
+constexpr int kFewCols = 4;
+template <class C>
+__device__ __forceinline__ void grid_few_columns(const typename C::Params& p, const double* stab, typename C::Staged* st,
+    uint16_t* s_list, const CtaOffsets* off, int br, int bc, int nb)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (br >= (p.rows + kBlk - 1) / kBlk)
+        return;
+    uint32_t beg = 0, len = 0;
+    if (lane < nb + kFewCols - 1) {
+        beg = off[lane][warp];
+        len = off[lane][warp + nb] - beg;
+    }
+    const BlockRanges r = make_ranges(beg, len, nb + kFewCols - 1);
+    if (r.total > 32) {
+#pragma unroll 1
+        for (int k = 0; k < kFewCols; k++)
+            grid_few<C>(p, stab, st, s_list, off + k, br, bc + k, nb);
+        return;
+    }
+    const bool valid = uint32_t(lane) < r.total;
+    if (r.total > 0) {
+        const uint32_t i = stream_record(r, lane);
+        if (valid)
+            st[lane] = C::decode(p, C::fetch(p, i), br * kBlk, bc * kBlk);
+    }
+    BlockList<1> list { s_list, {} };
+#pragma unroll 1
+    for (int k = 0; k < kFewCols; k++) {
+        typename C::A acc[C::NACC] = {};
+        if (r.total > 0) {
+            if (lane == 0)
+                st[32] = C::dummy(p, 0, k * kBlk);
+            __syncwarp();
+            block_add<C, 1>(p, stab, st, uint32_t(lane), valid, 32, 0, k * kBlk, list, acc);
+        }
+        C::template store<1>(p, br * kBlk, (bc + k) * kBlk, acc);
+    }
+    __syncwarp();
 }
 
 // COLS: columns of blocks that a CTA takes one after the other.  One, except
@@ -437,9 +481,24 @@ __global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(
         for (int j = 0; j < nb; j++)
             totals += s_off[k + j][no - 1] - s_off[k + j][0];
     }
+    const unsigned few = COLS == 1 || nb > kCtaBins ? 0u : __ballot_sync(0xffffffffu, totals <= kFew);
+    const unsigned some = COLS == 1 ? 1u : __ballot_sync(0xffffffffu, totals != 0);
     for (int k = 0; k < cols; k++) {
         const int bc = bc0 + k;
         const CtaOffsets* off = s_off + k;
+        if (COLS > 1 && k % kFewCols == 0 && k + kFewCols <= cols && ((~few >> k) & ((1u << kFewCols) - 1u)) == 0) {
+            if (((some >> k) & ((1u << kFewCols) - 1u)) == 0) {
+                for (int c = 0; c < kFewCols; c++)
+                    store_zeros<C>(p, br0 * kBlk, (bc + c) * kBlk);
+            } else {
+                if (shared)
+                    __syncthreads(); // the entries of the column before are gridded
+                shared = false;
+                grid_few_columns<C>(p, stab, all + warp * 33, s_list[warp], off, br0 + warp, bc, nb);
+            }
+            k += kFewCols - 1;
+            continue;
+        }
         const uint32_t total = COLS == 1 ? totals : __shfl_sync(0xffffffffu, totals, k);
         if (total == 0) { // nothing reaches the blocks: most of a grid outside the uv coverage
             store_zeros<C>(p, br0 * kBlk, bc * kBlk);
@@ -496,7 +555,7 @@ __global__ void __launch_bounds__(32 * kGridWarps) k_grid_dense(const __grid_con
     Staged* st = reinterpret_cast<Staged*>(smem) + warp * 33;
     BlockList<1> list { s_list[warp], {} };
     if (lane == 0)
-        st[32] = C::dummy(p, 0);
+        st[32] = C::dummy(p, 0, 0);
     C::load_table(p, s_tab);
     __syncthreads();
     const int nbr = (p.rows + kBlk - 1) / kBlk;
@@ -634,12 +693,12 @@ struct SepCore {
             s.rc |= 1u << 21;
         return s;
     }
-    // an entry of zero weight for the block at `row`
-    static __device__ __forceinline__ Staged dummy(const Params& p, int row)
+    // an entry of zero weight for the block at (row, col)
+    static __device__ __forceinline__ Staged dummy(const Params& p, int row, int col)
     {
         Staged z {};
         z.ty = EXACT ? -kBlk - row : p.zrow - row;
-        z.tx = EXACT ? -kBlk : p.zrow;
+        z.tx = EXACT ? -kBlk - col : p.zrow - col;
         return z;
     }
     static __device__ __forceinline__ int row0_of(const Staged& s) { return int(s.rc & 1023u) - 512; }
@@ -648,9 +707,9 @@ struct SepCore {
     static constexpr int kParts = 1;
     static __device__ __forceinline__ bool parts(const Params&) { return false; }
     template <int>
-    static __device__ __forceinline__ unsigned reach(const Params& p, const Staged& s, int row)
+    static __device__ __forceinline__ unsigned reach(const Params& p, const Staged& s, int row, int col)
     {
-        const int row0 = row0_of(s) - row, col0 = col0_of(s);
+        const int row0 = row0_of(s) - row, col0 = col0_of(s) - col;
         return row0 + p.K > 0 && row0 < kBlk && col0 + p.K > 0 && col0 < kBlk;
     }
     // the taps of either axis at the origin's row / column
@@ -673,12 +732,12 @@ struct SepCore {
         }
     }
     // an entry that is not finite: its own footprint's cells only
-    static __device__ __forceinline__ void add_odd(const Params& p, const double* stab, const Staged& s, int row,
+    static __device__ __forceinline__ void add_odd(const Params& p, const double* stab, const Staged& s, int row, int col,
         A (&acc)[NACC])
     {
         const int lane = threadIdx.x & 31;
         for (int k = 0; k < 2; k++) {
-            const int r = row + (lane >> 2), c = 2 * (lane & 3) + k;
+            const int r = row + (lane >> 2), c = col + 2 * (lane & 3) + k;
             if (unsigned(r - row0_of(s)) < unsigned(p.K) && unsigned(c - col0_of(s)) < unsigned(p.K)) {
                 double a, b;
                 taps(p, stab, s, r, c, a, b);
@@ -697,7 +756,7 @@ struct SepCore {
     }
     template <int PARTS>
     static __device__ __forceinline__ void accumulate(const Params& p, const double* stab, const Staged* st,
-        const uint16_t* list, int m, int row, A (&acc)[NACC])
+        const uint16_t* list, int m, int row, int col, A (&acc)[NACC])
     {
         const int lane = threadIdx.x & 31;
         const int q = lane >> 2;
@@ -705,7 +764,7 @@ struct SepCore {
         for (int g = 0; g < m; g += 4) {
             const Staged& s = st[list[g + (lane & 3)]];
             double a, b;
-            taps(p, stab, s, row + q, q, a, b);
+            taps(p, stab, s, row + q, col + q, a, b);
             mma(acc[0], acc[1], a, b * s.vr);
             mma(acc[2], acc[3], a, b * s.vi);
             if constexpr (BEAM)
@@ -811,7 +870,7 @@ struct WprojCore {
     static constexpr bool kWindows = false; // (the loop's registers: 206 -> 234 us on the double headline call)
     static constexpr bool kOdd = false; // (cells outside a footprint are not touched)
     static __device__ __forceinline__ bool odd(const Staged&) { return false; }
-    static __device__ __forceinline__ void add_odd(const Params&, const double*, const Staged&, int, A (&)[NACC]) {}
+    static __device__ __forceinline__ void add_odd(const Params&, const double*, const Staged&, int, int, A (&)[NACC]) {}
     static constexpr int kTab = 0;
     static __device__ __forceinline__ void load_table(const Params&, double*) {}
     static __device__ __forceinline__ Staged decode(const Params&, const Raw& w, int r0, int c0)
@@ -830,7 +889,7 @@ struct WprojCore {
         return s;
     }
     // an entry without taps
-    static __device__ __forceinline__ Staged dummy(const Params&, int)
+    static __device__ __forceinline__ Staged dummy(const Params&, int, int)
     {
         Staged z {};
         return z;
@@ -854,14 +913,14 @@ struct WprojCore {
         return p.max_support[0] <= (sizeof(T) == 4 ? 8u : 6u);
     }
     template <int PARTS>
-    static __device__ __forceinline__ unsigned reach(const Params&, const Staged& s, int row)
+    static __device__ __forceinline__ unsigned reach(const Params&, const Staged& s, int row, int col)
     {
-        const int K = int(s.kc & 0xffffu), row0 = s.row0 - row, end = s.col0 + K;
+        const int K = int(s.kc & 0xffffu), row0 = s.row0 - row, col0 = s.col0 - col, end = col0 + K;
         if (row0 + K <= 0 || row0 >= kBlk)
             return 0;
         if (PARTS == 1)
-            return end > 0 && s.col0 < kBlk;
-        return unsigned(end > 0 && s.col0 < kBlk / 2) | unsigned(end > kBlk / 2 && s.col0 < kBlk) << 1;
+            return end > 0 && col0 < kBlk;
+        return unsigned(end > 0 && col0 < kBlk / 2) | unsigned(end > kBlk / 2 && col0 < kBlk) << 1;
     }
     static __device__ __forceinline__ float flip(float x, uint32_t sign)
     {
@@ -873,11 +932,11 @@ struct WprojCore {
     }
     template <int PARTS>
     static __device__ __forceinline__ void accumulate(const Params& p, const double* stab, const Staged* st,
-        const uint16_t* list, int m, int row, A (&acc)[NACC])
+        const uint16_t* list, int m, int row, int col, A (&acc)[NACC])
     {
         using C2 = typename Cplx<T>::T;
         const int lane = threadIdx.x & 31;
-        const int r = row + (lane & 7), c = lane_col<PARTS>(lane);
+        const int r = row + (lane & 7), c = col + lane_col<PARTS>(lane);
         constexpr int step = 4 / PARTS;
         const C2* __restrict__ wk = p.wk;
         if (PARTS == 2)
