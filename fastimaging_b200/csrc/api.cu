@@ -680,12 +680,15 @@ void grid_blocks(stpgpu_context* c, const ImagerSetup& s, GridOut& g, int64_t n,
     const bool dense = n > dense_per_block(nbr * nbc, s.beam, sizeof(T) == 4) * nbr * nbc;
     const unsigned nbr8 = unsigned(ceil_div(nbr, kGridWarps));
     // Few visibilities: several columns of blocks a CTA, as long as the CTAs
-    // still fill the GPU.  One column and eight, us, W-kernels in double at
-    // disk / normal coverage: 4096^2 (2112 CTAs of eight columns) at 0.3, 1 and
-    // 2 visibilities a block 74 51, 84 68, 96 88 / 59 53, 72 92, 88 121; 5000^2
-    // (3120) at 1 and 2 125 92, 143 123 / 107 117, 131 154; 6000^2 (4418) at 1,
-    // 2 and 4 180 129, 207 174, 264 258 / 154 155, 189 195, 270 385; 8192^2 336
-    // 234, 391 319, 506 487 / 284 250, 351 327, 499 605.
+    // still fill the GPU.  One column and eight, us, at disk / normal coverage,
+    // separable kernels in single precision, then W-kernels in double: 4096^2
+    // (2112 CTAs of eight columns) at 0.3, 0.5 and 1 visibility a block 56 32,
+    // 56 34, 60 36 / 44 33, 46 37, 50 48, then 74 53, 77 57, 84 65 / 59 62, 63
+    // 72, 72 98; 5000^2 (3120) at 1 and 2 85 47, 93 68 / 71 60, 84 88, then 126
+    // 87, 143 131 / 108 129, 132 158; 6000^2 (4418) at 1, 2 and 3 124 63, 133
+    // 88, 142 109 / 103 74, 120 107, 139 157, then 180 122, 207 183, 235 227 /
+    // 154 166, 189 209, 224 263; 8192^2 at 2 and 3 248 160, 266 199 / 219 174,
+    // 251 236, then 390 333, 446 422 / 350 332, 418 423.
     const int64_t ctas = nbr8 * (nbc / kSparseCols);
     const double line = ctas < 148 * 4 ? 0.0 : (ctas < 148 * 20 ? 0.5 : (ctas < 4000 ? 1.5 : 2.0));
     const bool sparse = double(n) < line * double(nbr * nbc);

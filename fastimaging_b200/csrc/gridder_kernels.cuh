@@ -433,11 +433,12 @@ __device__ __forceinline__ void grid_few_columns(const typename C::Params& p, co
 // of its offsets and its barriers.  Eight columns share the offsets, empty
 // ones are stored at once, and up to kFew entries are taken without a barrier
 // (64 instead of 256: 48 against 44 us for 65k normally distributed
-// visibilities on 4096^2); what is left is bound by the instructions of a block
-// (fetching the next column's records ahead gave nothing, 94 against 98 us).
-// Kernel with one column and eight, disk coverage, single-precision cells: 26k
-// visibilities on 8192^2 169 and 98 us, 157k 203 and 135, with W-kernels 260 and
-// 135; 56k on 12000^2 357 and 193.
+// visibilities on 4096^2).  What is left is bound by the instructions that a
+// block costs whatever it holds (74 % of the issue slots), hence four columns
+// at once (135 -> 99 us below); fetching the next column's records ahead gave
+// nothing.  Kernel with one column and eight, disk coverage, single-precision
+// cells: 26k visibilities on 8192^2 169 and 83 us, 157k 203 and 99, with
+// W-kernels 260 and 127; 56k on 12000^2 357 and 166.
 template <class C, int COLS>
 __global__ void __launch_bounds__(32 * kGridWarps, C::kMinBlocks) k_grid_blocks(const __grid_constant__ typename C::Params p)
 {
