@@ -121,9 +121,10 @@ def test_uneven_w_blocks_match_oracle(ctx, smax):
     assert np.abs(g[1] - r.sampling_grid).max() <= 1e-11 * np.abs(r.sampling_grid).max()
 
 
+@pytest.mark.parametrize("N", [64, 2308])  # (the second takes the form of sparse grids)
 @pytest.mark.parametrize("exact", [True, False])
-def test_entries_that_are_not_finite_stay_in_their_footprint(ctx, exact):
-    N, S = 64, 3
+def test_entries_that_are_not_finite_stay_in_their_footprint(ctx, exact, N):
+    S = 3
     uv, vis, wts = _points(3, 200, N, 0.8)
     vis[17] = np.nan
     wts[40] = np.inf
